@@ -263,3 +263,77 @@ def tolerance(case):
     if case["train"]:
         return {"rel": 8e-6, "max": 4e-4}
     return {"rel": 2e-6, "max": 2e-5, "differ": 1e-4}
+
+
+def _messages(h, e, ctx, soft):
+    """New messages [N,L] of N pixels from their predecessors' terms h [N,L] and edge weights e [N]."""
+    v = e.view(-1, 1, 1) * ctx + h.unsqueeze(1)
+    m = (torch.softmax(-v, dim=2) * v).sum(2) if soft else v.amin(2)
+    return m - m.amin(1, keepdim=True)
+
+
+def _sweep(direction, uu, rho, e, ctx, soft):
+    """Messages [B,H,W,L] of one direction, from uu [B,H,W,L] and edge weights e [B,H,W]."""
+    hs, ws = ((0, 1), (0, -1), (1, 0), (-1, 0), (1, 1), (-1, -1), (1, -1), (-1, 1))[direction]
+    if hs == 0:   # walk over columns: a vertical sweep of the transposed image
+        new = _lines(uu.transpose(1, 2), e.transpose(1, 2), ws, 0, rho, ctx, soft)
+        return new.transpose(1, 2)
+    return _lines(uu, e, hs, ws, rho, ctx, soft)
+
+
+def _lines(uu, e, step, shift, rho, ctx, soft):
+    b, h, w, n = uu.shape
+    new = torch.zeros(uu.shape, device=uu.device, dtype=uu.dtype)
+    to, frm = slice(max(shift, 0), w + min(shift, 0)), slice(max(-shift, 0), w + min(-shift, 0))
+    order = range(1, h) if step > 0 else range(h - 2, -1, -1)
+    for y in order:
+        term = rho * new[:, y - step, frm] + uu[:, y - step, frm]
+        new[:, y, to] = _messages(term.reshape(-1, n), e[:, y, to].reshape(-1), ctx, soft).view(b, -1, n)
+    return new
+
+
+def exact(case, seed):
+    """Final costs in 64 bits.  Gradients have no such value: near-equal candidates resolve to another
+    label in another precision, and the gradient follows the label; nor have labellings.  The case
+    with images starts from whole-number matching costs of its own and is left out."""
+    if case["images"]:
+        return None
+    state = prepare(case, seed)
+    with torch.no_grad():
+        u = state["unary"].detach().double()
+        if case["scores"]:
+            u = u.amax(1, keepdim=True) - u
+        else:
+            u = u[:, 0]
+        u = u.permute(0, 2, 3, 1).contiguous()
+        n, dirs = case["labels"], case["dirs"]
+        ctx = state["context"].detach().double()
+        if ctx.dim() == 1:
+            k = torch.arange(n, device="cuda")
+            ctx = ctx[(k.view(n, 1) - k).abs()]
+        if state["weights"] is None:
+            e = torch.ones(u.shape[0], dirs, *u.shape[1:3], device="cuda", dtype=torch.float64)
+        else:
+            e = state["weights"].detach().double()
+        soft, trwp = case["mode"] == "SOFT", case["mode"] in ("SOFT", "TRWP")
+        rho = 0.5 if trwp else 1.0
+        msg = [torch.zeros_like(u) for _ in range(dirs)]
+        for _ in range(case["iters"]):
+            read = msg if trwp else list(msg)
+            for d in range(dirs):
+                rest = u + sum(read[k] for k in range(dirs) if k != d)
+                msg[d] = _sweep(d, rho * rest - read[d ^ 1], rho, e[:, d], ctx, soft)
+        cost = (dirs if case["mode"] == "SGM" else 1) * u + sum(msg)
+        cost = cost.permute(0, 3, 1, 2)
+        cost = -cost if case["scores"] else cost.unsqueeze(1)
+    return [cost] + [None] * (len(_output_names(case)) - 1)
+
+
+def _output_names(case):
+    """Names of what run returns."""
+    names = ["scores" if case["scores"] else "costs"]
+    if case["train"]:
+        names += ["unary gradient", "context gradient"] + (["weight gradient"] if case["weights"] else [])
+    elif case["keep_labels"] and not case["scores"]:
+        names += ["labels"]
+    return names
