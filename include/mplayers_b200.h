@@ -81,6 +81,24 @@ typedef struct mpl_problem {
                                separate layout pass.  Every other tensor keeps the labels last. */
 } mpl_problem;
 
+/* Row layout and start of a call through the *_rows entry points (the entry points without the suffix
+ * are the same calls with both members 0). */
+typedef struct mpl_rows {
+  int32_t label_stride;     /* elements from one pixel's labels to the next one's in every labels-last tensor
+                               (unary, msg, msg_update, msg_min_index, cost_final and their gradients).
+                               0 or n_disp: packed, the reference's layout; else n_disp rounded up to a
+                               multiple of 4, the elements between n_disp and label_stride being padding
+                               whose values do not matter on input and are unspecified on output.
+                               Rows of 16-byte multiples let label counts that are no multiple of 4 take
+                               the bulk-copy and several-labels-per-lane kernels (mpl_label_stride
+                               proposes a value).  A padded forward call needs a larger workspace
+                               (mpl_forward_workspace_bytes_rows), where the per-iteration sums are kept:
+                               a labels-first cost_final has no padding. */
+  int32_t messages_zero;    /* forward calls: 1 = the iterations start from zero messages whatever `msg` (and
+                               `msg_update`) hold, which then need not be initialised; on return `msg` is
+                               complete.  Ignored by backward calls. */
+} mpl_rows;
+
 /* Analyses a rank-1 context (and the edge weights, may be NULL) for mpl_problem::context_window:
  * *window receives R > 0 if min over the 2R-1 nearest labels plus one global term is exact (see
  * above), else -1.  Synchronous (waits for `stream`); call it once per context, not per step.
@@ -88,8 +106,13 @@ typedef struct mpl_problem {
 int mpl_analyze_context(const mpl_problem* p, const float* context, const float* edge_weights,
                         int32_t* window, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The mpl_rows::label_stride with which mpl_trwp_* (isgmr = 0) or mpl_isgmr_* (isgmr = 1) calls of `p` run
+ * fastest; n_disp where packed rows are as good.  0 if `p` is invalid. */
+int32_t mpl_label_stride(const mpl_problem* p, int32_t isgmr);
+
 /* Bytes of device scratch the forward / backward entry points need for `p` (never 0). */
 size_t mpl_forward_workspace_bytes(const mpl_problem* p);
+size_t mpl_forward_workspace_bytes_rows(const mpl_problem* p, const mpl_rows* rows);
 size_t mpl_backward_workspace_bytes(const mpl_problem* p);
 
 /* TRWP forward.  Replaces TRWP.forward of the reference extension
@@ -228,6 +251,25 @@ int mpl_isgmr_backward_combine(const mpl_problem* p, int32_t dir_first, int32_t 
 int mpl_backward_context_finish(const mpl_problem* p, void* workspace, size_t workspace_bytes,
                                 float* dcontext, void* stream);
 
+/* The four calls on padded label rows and / or from zero messages. */
+int mpl_trwp_forward_rows(const mpl_problem* p, const mpl_rows* rows, const float* unary, const float* context,
+                          const float* edge_weights, float* msg, float* cost_final, uint8_t* msg_min_index,
+                          uint8_t* msg_norm_index, uint8_t* label_all, void* workspace, size_t workspace_bytes,
+                          void* stream);
+int mpl_isgmr_forward_rows(const mpl_problem* p, const mpl_rows* rows, const float* unary,
+                           const float* context, const float* edge_weights, float* msg, float* msg_update,
+                           float* cost_final, uint8_t* msg_min_index, uint8_t* msg_norm_index,
+                           uint8_t* label_all, void* workspace, size_t workspace_bytes, void* stream);
+int mpl_trwp_backward_rows(const mpl_problem* p, const mpl_rows* rows, const float* context,
+                           const float* edge_weights, const float* dcost_final, const uint8_t* msg_min_index,
+                           const uint8_t* msg_norm_index, float* dunary, float* dcontext, float* dedge_weights,
+                           float* dmsg, void* workspace, size_t workspace_bytes, void* stream);
+int mpl_isgmr_backward_rows(const mpl_problem* p, const mpl_rows* rows, const float* context,
+                            const float* edge_weights, const float* dcost_final, const uint8_t* msg_min_index,
+                            const uint8_t* msg_norm_index, float* dunary, float* dcontext,
+                            float* dedge_weights, float* dmsg, float* dmsg_update, void* workspace,
+                            size_t workspace_bytes, void* stream);
+
 /* Layout glue around the layer.  Network code holds class scores as [B,L,H,W] planes; the layer
  * takes costs [B,(cv=1),H,W,L].  The reference converts with six elementwise passes: costs = -scores,
  * minus the per-pixel minimum, permute, layer, permute back, negate (mpnet.py:161-169,
@@ -252,6 +294,17 @@ int mpl_permute_lhw_to_hwl(const float* in, float* out, int32_t batch, int32_t n
                            int32_t width, void* stream);
 int mpl_permute_hwl_to_lhw(const float* in, float* out, int32_t batch, int32_t n_disp, int32_t height,
                            int32_t width, void* stream);
+/* The same changes of layout with label rows of label_stride >= n_disp elements on the labels-last side
+ * (mpl_rows::label_stride; the padding is written as 0 and not read). */
+int mpl_scores_to_cost_rows(const float* scores, float* costs, uint8_t* argmax, int32_t batch, int32_t n_disp,
+                            int32_t height, int32_t width, int32_t label_stride, void* stream);
+int mpl_scores_to_cost_rows_backward(const float* dcosts, const uint8_t* argmax, float* dscores, int32_t batch,
+                                     int32_t n_disp, int32_t height, int32_t width, int32_t label_stride,
+                                     void* stream);
+int mpl_permute_lhw_to_rows(const float* in, float* out, int32_t batch, int32_t n_disp, int32_t height,
+                            int32_t width, int32_t label_stride, void* stream);
+int mpl_permute_rows_to_lhw(const float* in, float* out, int32_t batch, int32_t n_disp, int32_t height,
+                            int32_t width, int32_t label_stride, void* stream);
 
 /* Energy of labellings on the MRF the layers minimise, for energy-versus-iteration curves from the
  * per-iteration labels `label_all` of a forward call.  energy [n_labelings, 2] (f64, device):

@@ -17,6 +17,7 @@ import torch.nn as nn
 from . import glue as _glue
 
 from . import ISGMR as _ISGMR
+from . import _lib
 from . import TRWP as _TRWP
 from .label_context import create_label_context
 
@@ -69,11 +70,12 @@ class TRWPFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, unary, label_context, edge_weights, args):
-        batch, cv, h, w, n_disp = unary.size()
+        batch, cv, h, w, row = unary.size()   # row >= n_disp elements per pixel (padded label rows)
+        n_disp = _labels_in_row(args, row)
         rho, n_iter, n_dir, is_training = args.rho, args.mpnet_max_iter, args.mpnet_n_dirs, args.training
         unary = unary.contiguous()
         label_context = label_context.contiguous()
-        message = unary.new_zeros(n_dir, batch, cv, h, w, n_disp)
+        message = unary.new_empty(n_dir, batch, cv, h, w, row)   # starts as zeros: messages_zero below
         lf = bool(getattr(args, "cost_labels_first", False))  # cost_final as [B,cv,L,H,W]
         cost_final = unary.new_empty(batch, cv, n_disp, h, w) if lf else torch.empty_like(unary)
         message_index, cost_index, label_all = _alloc_indices(unary, n_iter, n_dir, is_training,
@@ -82,8 +84,10 @@ class TRWPFunction(torch.autograd.Function):
         ew = edge_weights.contiguous() if enable_edge_weights else _empty_f32(unary.device)
         _TRWP.forward(rho, int(n_iter), int(args.enable_min_a_dir), unary, label_context, ew, message,
                       cost_final, message_index, cost_index, _empty_f32(unary.device), label_all,
-                      context_window=int(getattr(args, "context_window", 0) or 0), cost_labels_first=lf)
+                      context_window=int(getattr(args, "context_window", 0) or 0), cost_labels_first=lf,
+                      n_disp=n_disp, messages_zero=True)
         ctx.cost_labels_first = lf
+        ctx.n_disp = n_disp
         ctx.intermediate_results = rho, message_index, cost_index, label_context, ew, enable_edge_weights
         ctx.context_window = int(getattr(args, "context_window", 0) or 0)
         ctx.norm_index_override = _norm_index_override(args, cost_index, n_disp)
@@ -100,15 +104,15 @@ class TRWPFunction(torch.autograd.Function):
         if ctx.norm_index_override is not None:
             cost_index = ctx.norm_index_override
         dcost_final = dcost_final.contiguous()
-        n_iter, n_dir, batch, cv, h, w, n_disp = message_index.size()
-        dunary = dcost_final.new_empty(batch, cv, h, w, n_disp)
-        dmessage = dcost_final.new_empty(n_dir, batch, cv, h, w, n_disp)
+        n_iter, n_dir, batch, cv, h, w, row = message_index.size()
+        dunary = dcost_final.new_empty(batch, cv, h, w, row)
+        dmessage = dcost_final.new_empty(n_dir, batch, cv, h, w, row)
         dlabel_context = torch.zeros_like(label_context)
         dedge_weights = torch.zeros_like(ew) if enable_edge_weights else _empty_f32(dcost_final.device)
         _TRWP.backward(rho, label_context, ew, dcost_final, message_index, cost_index, dunary,
                        dlabel_context, dedge_weights, dmessage, _empty_f32(dcost_final.device),
                        keep_diag=ctx._forward_cls.keep_diag, context_window=ctx.context_window,
-                       cost_labels_first=ctx.cost_labels_first)
+                       cost_labels_first=ctx.cost_labels_first, n_disp=ctx.n_disp)
         return dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None
 
 
@@ -117,12 +121,13 @@ class ISGMRFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, unary, label_context, edge_weights, args):
-        batch, cv, h, w, n_disp = unary.size()
+        batch, cv, h, w, row = unary.size()   # row >= n_disp elements per pixel (padded label rows)
+        n_disp = _labels_in_row(args, row)
         rho, n_iter, n_dir, is_training = args.rho, args.mpnet_max_iter, args.mpnet_n_dirs, args.training
         unary = unary.contiguous()
         label_context = label_context.contiguous()
-        message = unary.new_zeros(n_dir, batch, cv, h, w, n_disp)
-        message_tmp = unary.new_zeros(n_dir, batch, cv, h, w, n_disp)
+        message = unary.new_empty(n_dir, batch, cv, h, w, row)   # starts as zeros: messages_zero below
+        message_tmp = torch.empty_like(message)
         lf = bool(getattr(args, "cost_labels_first", False))  # cost_final as [B,cv,L,H,W]
         cost_final = unary.new_empty(batch, cv, n_disp, h, w) if lf else torch.empty_like(unary)
         message_index, cost_index, label_all = _alloc_indices(unary, n_iter, n_dir, is_training,
@@ -132,8 +137,10 @@ class ISGMRFunction(torch.autograd.Function):
         _ISGMR.forward(int(args.enable_sgm), rho, int(n_iter), int(args.enable_min_a_dir), unary,
                        label_context, ew, message, cost_final, message_index, cost_index,
                        _empty_f32(unary.device), message_tmp, label_all,
-                       context_window=int(getattr(args, "context_window", 0) or 0), cost_labels_first=lf)
+                       context_window=int(getattr(args, "context_window", 0) or 0), cost_labels_first=lf,
+                      n_disp=n_disp, messages_zero=True)
         ctx.cost_labels_first = lf
+        ctx.n_disp = n_disp
         ctx.intermediate_results = args.enable_sgm, rho, message_index, cost_index, label_context, ew, \
             enable_edge_weights
         ctx.context_window = int(getattr(args, "context_window", 0) or 0)
@@ -149,17 +156,34 @@ class ISGMRFunction(torch.autograd.Function):
             raise RuntimeError("backward needs the indices saved by a training-mode forward "
                                "(args.training was False)")
         dcost_final = dcost_final.contiguous()
-        n_iter, n_dir, batch, cv, h, w, n_disp = message_index.size()
-        dunary = dcost_final.new_empty(batch, cv, h, w, n_disp)
-        dmessage = dcost_final.new_empty(n_dir, batch, cv, h, w, n_disp)
-        dmessage_tmp = dcost_final.new_empty(n_dir, batch, cv, h, w, n_disp)
+        n_iter, n_dir, batch, cv, h, w, row = message_index.size()
+        dunary = dcost_final.new_empty(batch, cv, h, w, row)
+        dmessage = dcost_final.new_empty(n_dir, batch, cv, h, w, row)
+        dmessage_tmp = torch.empty_like(dmessage)
         dlabel_context = torch.zeros_like(label_context)
         dedge_weights = torch.zeros_like(ew) if enable_edge_weights else _empty_f32(dcost_final.device)
         _ISGMR.backward(int(enable_sgm), rho, label_context, ew, dcost_final, message_index, cost_index,
                         dunary, dlabel_context, dedge_weights, dmessage,
                         _empty_f32(dcost_final.device), dmessage_tmp, context_window=ctx.context_window,
-                        cost_labels_first=ctx.cost_labels_first)
+                        cost_labels_first=ctx.cost_labels_first, n_disp=ctx.n_disp)
         return dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None
+
+
+def _labels_in_row(args, row):
+    """Label count of a call whose label rows have `row` elements; what the module said about padding
+    counts for one call."""
+    n_disp, args.labels_in_row = int(getattr(args, 'labels_in_row', 0) or row), 0
+    return n_disp
+
+
+def _row_elements(args, unary, direction_comm=None):
+    """Elements per label row of the layer's labels-last tensors for a module call on unary
+    [B,cv,L,H,W]: padded to a multiple of four where the kernels profit (mpl_label_stride)."""
+    n_disp = unary.size(2)
+    if direction_comm is not None or not unary.is_cuda or unary.dim() != 5:
+        return n_disp   # direction-sharded calls take packed rows
+    return _lib.label_stride(args.mpnet_max_iter, args.mpnet_n_dirs, unary.size(0), unary.size(1), unary.size(3),
+                             unary.size(4), n_disp, 2, args.mpnet_mrf_mode in {'ISGMR', 'SGM'})
 
 
 def _empty_f32(device):
@@ -246,7 +270,6 @@ class MPModule(torch.nn.Module):
         key = (id(src), src._version, src.data_ptr(), getattr(self.args, 'mpnet_smoothness_train', None),
                getattr(self.args, 'mpnet_term_weight', None), getattr(self.args, 'mpnet_diag_value', None))
         if getattr(self, "_window_key", None) != key:
-            from . import _lib
             self._window_value = _lib.analyze_context(label_context)
             self._window_key = key
         return self._window_value
@@ -258,6 +281,7 @@ class MPModule(torch.nn.Module):
         label_context = self._transformed_label_context()
         self.args.training = self.training
         self.args.cost_labels_first = False
+        self.args.labels_in_row = 0   # packed
         self.args.context_window = self._context_window(label_context, edge_weights)
         if self.args.mpnet_mrf_mode in {'ISGMR', 'SGM'}:
             cost_final, _ = ISGMRFunction.apply(unary, label_context, edge_weights, self.args)
@@ -265,9 +289,27 @@ class MPModule(torch.nn.Module):
             cost_final, _ = TRWPFunction.apply(unary, label_context, edge_weights, self.args)
         return cost_final, label_context.unsqueeze(0)
 
+    def row_elements(self, unary):
+        """Elements per label row with which forward_rows / forward run fastest on unary [B,cv,L,H,W]."""
+        return _row_elements(self.args, unary, self.direction_comm)
+
+    def forward_rows(self, unary, n_disp, edge_weights=None):
+        """forward_native on padded label rows: unary [B,cv,H,W,row] of which the first n_disp elements of a
+        row count -> (cost_final [B,cv,n_disp,H,W], label_context)."""
+        label_context = self._transformed_label_context()
+        self.args.training = self.training
+        self.args.cost_labels_first = True
+        self.args.labels_in_row = n_disp
+        self.args.context_window = self._context_window(label_context, edge_weights)
+        fn = ISGMRFunction if self.args.mpnet_mrf_mode in {'ISGMR', 'SGM'} else TRWPFunction
+        cost_final, _ = fn.apply(unary, label_context, edge_weights, self.args)
+        self.args.cost_labels_first = False
+        return cost_final, label_context.unsqueeze(0)
+
     def forward(self, unary, edge_weights=None):
         # unary [B,cv,L,H,W]; edge_weights [B,D,H,W]
-        unary = _glue.labels_last(unary)
+        self.args.labels_in_row = unary.size(2)
+        unary = _glue.label_rows(unary, _row_elements(self.args, unary, self.direction_comm))
         edge_weights = edge_weights.unsqueeze(1).permute(2, 0, 1, 3, 4).contiguous() \
             if (edge_weights is not None) else edge_weights
         if self.args.mpnet_mrf_mode == 'SGM':

@@ -15,7 +15,7 @@ from . import glue as _glue
 
 from . import TRWP as _TRWP
 from .MP_module import TRWPFunction as _TRWPFunctionBase
-from .MP_module import _norm_index_override
+from .MP_module import _norm_index_override, _row_elements
 from .label_context import create_label_context
 
 
@@ -106,7 +106,10 @@ class MPModule(torch.nn.Module):
         # normalisation indices in the backward pass
         self.args.msg_norm_index = msg_norm_index
         assert self.args.mpnet_mrf_mode == 'TRWP'
-        unary = _glue.labels_last(unary)
+        soft = getattr(self.args, 'mpnet_enable_soft', False)   # the soft kernels take packed rows
+        self.args.labels_in_row = 0 if soft else unary.size(2)
+        unary = _glue.labels_last(unary) if soft else \
+            _glue.label_rows(unary, _row_elements(self.args, unary))
         edge_weights = edge_weights.unsqueeze(1).permute(2, 0, 1, 3, 4).contiguous() \
             if (edge_weights is not None) else edge_weights
         label_context = self.label_context * self.args.mpnet_term_weight
@@ -124,7 +127,7 @@ class MPModule(torch.nn.Module):
             assert unary.size()[-3:-1] == edge_weights.size()[-2:]
         self.args.training = self.training
         self.args.cost_labels_first = False
-        if getattr(self.args, 'mpnet_enable_soft', False):
+        if soft:
             cost_final, cost_all, message_vector, message_index = \
                 TRWPSoftFunction.apply(unary, label_context, edge_weights, self.args)
             cost_final = _glue.labels_first(cost_final)

@@ -17,19 +17,23 @@ keep_diag = False  # TRWP_hard_soft accumulates dcontext on the diagonal, the TR
 
 
 def _problem(n_iter, msg_shape, context, rho, enable_min_a_dir=0, enable_sgm=0, keep_diag_=0,
-             context_window=0, cost_labels_first=False):
-    n_dir, batch, n_cv, h, w, n_disp = msg_shape
+             context_window=0, cost_labels_first=False, n_disp=0):
+    n_dir, batch, n_cv, h, w, stride = msg_shape
+    n_disp = n_disp or stride
     return _lib.Problem(int(n_iter), n_dir, batch, n_cv, h, w, n_disp,
                         _lib.context_rank(context, n_disp), int(enable_min_a_dir), int(enable_sgm),
                         int(keep_diag_), float(rho), int(context_window), 0, 0, int(bool(cost_labels_first)))
 
 
 def forward(rho, n_iter, enable_min_a_dir, unary, context, edge_weights, msg, cost_final,
-            msg_min_index, msg_norm_index, unary_update, label_all, context_window=0, cost_labels_first=False):
+            msg_min_index, msg_norm_index, unary_update, label_all, context_window=0, cost_labels_first=False, n_disp=0,
+            messages_zero=False):
     """`context_window` (keyword, not in the reference's signature): see mpl_problem::context_window;
     0 lets the library find out by itself, which makes an inference call with a rank-1 context and
     more than 32 labels wait for the stream once.  `cost_labels_first` (keyword): cost_final is
-    [B,cv,L,H,W] instead of [B,cv,H,W,L] (mpl_problem::cost_labels_first)."""
+    [B,cv,L,H,W] instead of [B,cv,H,W,L] (mpl_problem::cost_labels_first).  `n_disp` (keyword): the label
+    count where the label rows of the labels-last tensors are padded (mpl_rows::label_stride);
+    `messages_zero` (keyword): start from zero messages, `msg` need not be initialised."""
     dev = unary.device
     for t, n in ((unary, "unary"), (context, "context"), (edge_weights, "edge_weights"), (msg, "msg"),
                  (cost_final, "cost_final")):
@@ -40,12 +44,13 @@ def forward(rho, n_iter, enable_min_a_dir, unary, context, edge_weights, msg, co
     if msg.dim() != 6 or tuple(unary.shape) != tuple(msg.shape[1:]):
         raise RuntimeError("msg must be [D,B,cv,H,W,L] matching unary [B,cv,H,W,L]")
     prob = _problem(n_iter, tuple(msg.shape), context, rho, enable_min_a_dir, context_window=context_window,
-                    cost_labels_first=cost_labels_first)
+                    cost_labels_first=cost_labels_first, n_disp=n_disp)
+    rows = _lib.Rows(unary.size(-1), int(bool(messages_zero)))
     with torch.cuda.device(dev):
-        nbytes = _lib.lib().mpl_forward_workspace_bytes(ctypes.byref(prob))
+        nbytes = _lib.lib().mpl_forward_workspace_bytes_rows(ctypes.byref(prob), ctypes.byref(rows))
         ws = _lib.workspace(nbytes, dev)
-        _lib.check(_lib.lib().mpl_trwp_forward(
-            ctypes.byref(prob), _lib.ptr(unary), _lib.ptr(context), _lib.ptr(edge_weights),
+        _lib.check(_lib.lib().mpl_trwp_forward_rows(
+            ctypes.byref(prob), ctypes.byref(rows), _lib.ptr(unary), _lib.ptr(context), _lib.ptr(edge_weights),
             _lib.ptr(msg), _lib.ptr(cost_final), _lib.ptr(msg_min_index), _lib.ptr(msg_norm_index),
             _lib.ptr(label_all), _lib.ptr(ws), nbytes, _lib.stream_ptr(dev)))
         _lib.check_status(ws, "TRWP.forward")
@@ -53,7 +58,7 @@ def forward(rho, n_iter, enable_min_a_dir, unary, context, edge_weights, msg, co
 
 def backward(rho, context, edge_weights, dcost_final, msg_min_index, msg_norm_index, dunary,
              dcontext, dedge_weights, dmsg, dunary_update, keep_diag=None, context_window=0,
-             cost_labels_first=False):
+             cost_labels_first=False, n_disp=0):
     """`context_window` (keyword, not in the reference's signature): in the backward pass only a hint
     for how the scatter of a rank-1 context with more than 32 labels is split; any value gives the
     same sums."""
@@ -69,12 +74,12 @@ def backward(rho, context, edge_weights, dcost_final, msg_min_index, msg_norm_in
     kd = globals()["keep_diag"] if keep_diag is None else keep_diag
     prob = _problem(msg_min_index.size(0), tuple(msg_min_index.shape[1:]), context, rho,
                     keep_diag_=kd, context_window=max(int(context_window), 0),
-                    cost_labels_first=cost_labels_first)
+                    cost_labels_first=cost_labels_first, n_disp=n_disp)
     with torch.cuda.device(dev):
         nbytes = _lib.lib().mpl_backward_workspace_bytes(ctypes.byref(prob))
         ws = _lib.workspace(nbytes, dev)
-        _lib.check(_lib.lib().mpl_trwp_backward(
-            ctypes.byref(prob), _lib.ptr(context), _lib.ptr(edge_weights), _lib.ptr(dcost_final),
+        _lib.check(_lib.lib().mpl_trwp_backward_rows(
+            ctypes.byref(prob), ctypes.byref(_lib.Rows(msg_min_index.size(-1), 0)), _lib.ptr(context), _lib.ptr(edge_weights), _lib.ptr(dcost_final),
             _lib.ptr(msg_min_index), _lib.ptr(msg_norm_index), _lib.ptr(dunary), _lib.ptr(dcontext),
             _lib.ptr(dedge_weights), _lib.ptr(dmsg), _lib.ptr(ws), nbytes, _lib.stream_ptr(dev)))
         _lib.check_status(ws, "TRWP.backward")

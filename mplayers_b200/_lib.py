@@ -27,6 +27,11 @@ class Problem(ctypes.Structure):
                                                                    ("cost_labels_first", ctypes.c_int32)]
 
 
+class Rows(ctypes.Structure):
+    """struct mpl_rows of include/mplayers_b200.h"""
+    _fields_ = [("label_stride", ctypes.c_int32), ("messages_zero", ctypes.c_int32)]
+
+
 _lib = None
 
 
@@ -55,6 +60,13 @@ def lib():
         L.mpl_isgmr_backward.restype = ctypes.c_int
         L.mpl_isgmr_backward.argtypes = [pp] + [vp] * 11 + [sz, vp]
         i32 = ctypes.c_int32
+        rp = ctypes.POINTER(Rows)
+        L.mpl_forward_workspace_bytes_rows.restype = sz
+        L.mpl_forward_workspace_bytes_rows.argtypes = [pp, rp]
+        for name, n_ptr in (("trwp_forward", 9), ("trwp_backward", 10), ("isgmr_forward", 10), ("isgmr_backward", 11)):
+            fn = getattr(L, "mpl_%s_rows" % name)
+            fn.restype = ctypes.c_int
+            fn.argtypes = [pp, rp] + [vp] * n_ptr + [sz, vp]
         L.mpl_isgmr_forward_directions.restype = ctypes.c_int
         L.mpl_isgmr_forward_directions.argtypes = [pp, i32, i32] + [vp] * 8 + [sz, vp]
         L.mpl_sum_directions.restype = ctypes.c_int
@@ -83,6 +95,14 @@ def lib():
         for name in ("mpl_permute_lhw_to_hwl", "mpl_permute_hwl_to_lhw"):
             getattr(L, name).restype = ctypes.c_int
             getattr(L, name).argtypes = [vp, vp, i32, i32, i32, i32, vp]
+        L.mpl_label_stride.restype = i32
+        L.mpl_label_stride.argtypes = [pp, i32]
+        for name in ("mpl_permute_lhw_to_rows", "mpl_permute_rows_to_lhw"):
+            getattr(L, name).restype = ctypes.c_int
+            getattr(L, name).argtypes = [vp, vp, i32, i32, i32, i32, i32, vp]
+        for name in ("mpl_scores_to_cost_rows", "mpl_scores_to_cost_rows_backward"):
+            getattr(L, name).restype = ctypes.c_int
+            getattr(L, name).argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, vp]
         L.mpl_energy_workspace_bytes.restype = sz
         L.mpl_energy_workspace_bytes.argtypes = [pp]
         L.mpl_labeling_energy.restype = ctypes.c_int
@@ -121,6 +141,13 @@ def lib():
         L.mpl_version.restype = ctypes.c_int32
         _lib = L
     return _lib
+
+
+def label_stride(n_iter, n_dir, batch, n_cv, h, w, n_disp, rank, isgmr):
+    """Elements per label row with which a call of this shape runs fastest (mpl_label_stride); n_disp
+    where the library has no opinion."""
+    prob = Problem(int(n_iter), int(n_dir), int(batch), int(n_cv), int(h), int(w), int(n_disp), int(rank))
+    return int(lib().mpl_label_stride(ctypes.byref(prob), int(isgmr))) or int(n_disp)
 
 
 def kernel_launches():

@@ -125,13 +125,31 @@ int cuda_fail(cudaError_t e, const char* what) {
     if (e__ != cudaSuccess) return cuda_fail(e__, #expr); \
   } while (0)
 
+// Layout of every workspace (forward, backward, the built-in scratch): bytes [0, 64) context
+// analysis, [64, 68) the device status word, [256, ...) the backward's partial label-context
+// tables, or the per-iteration sums of a forward call with padded label rows.
+constexpr size_t kStatusOffset = 64, kTablesOffset = 256;
+inline float* ws_tables(void* workspace) { return reinterpret_cast<float*>(static_cast<char*>(workspace) + kTablesOffset); }
+inline int* ws_status(void* workspace) { return reinterpret_cast<int*>(static_cast<char*>(workspace) + kStatusOffset); }
+
 struct Dims {
   long long nimg, npix, slice;
+  int ls;  // elements from one pixel's labels to the next
   int ctx_elems;
 };
 
-int validate(const mpl_problem* p, Dims* d) {
-  if (!p) return fail(MPL_ERR_INVALID, "problem is NULL");
+// A call's problem with its row layout and start (packed rows, messages as given unless rows say otherwise).
+struct Problem : mpl_problem {
+  int32_t label_stride, messages_zero;
+};
+Problem with_rows(const mpl_problem* p, const mpl_rows* rows) {
+  Problem q{};
+  static_cast<mpl_problem&>(q) = *p;
+  if (rows) q.label_stride = rows->label_stride, q.messages_zero = rows->messages_zero;
+  return q;
+}
+
+int validate(const Problem* p, Dims* d) {
   if (p->n_iter < 0 || p->batch < 1 || p->n_cv < 1 || p->height < 1 || p->width < 1)
     return fail(MPL_ERR_INVALID, "bad shape: n_iter=%d batch=%d n_cv=%d height=%d width=%d", p->n_iter,
                 p->batch, p->n_cv, p->height, p->width);
@@ -141,18 +159,28 @@ int validate(const mpl_problem* p, Dims* d) {
     return fail(MPL_ERR_UNSUPPORTED, "n_dir=%d: must be even and in 2..16", p->n_dir);
   if (p->context_rank != 1 && p->context_rank != 2)
     return fail(MPL_ERR_INVALID, "context_rank=%d: must be 1 or 2", p->context_rank);
-  const long long per_img = (long long)p->height * p->width * p->n_disp;
+  d->ls = p->label_stride == 0 ? p->n_disp : p->label_stride;
+  if (d->ls != p->n_disp && d->ls != ((p->n_disp + 3) & ~3))
+    return fail(MPL_ERR_INVALID, "label_stride=%d: must be 0, n_disp=%d or the next multiple of 4", p->label_stride,
+                p->n_disp);
+  const long long per_img = (long long)p->height * p->width * d->ls;
   if (per_img >= (1ll << 31))
-    return fail(MPL_ERR_UNSUPPORTED, "height*width*n_disp=%lld must be below 2^31", per_img);
+    return fail(MPL_ERR_UNSUPPORTED, "height*width*(label stride)=%lld must be below 2^31", per_img);
   d->nimg = (long long)p->batch * p->n_cv;
   d->npix = d->nimg * p->height * p->width;
-  d->slice = d->npix * p->n_disp;
+  d->slice = d->npix * d->ls;
   if (d->nimg * 4096ll >= (1ll << 31) || d->npix >= (1ll << 40))
     return fail(MPL_ERR_UNSUPPORTED, "batch*n_cv=%lld too large", d->nimg);
   d->ctx_elems = p->context_rank == 2 ? p->n_disp * p->n_disp : p->n_disp;
   if (p->chain_parts > 1 && (p->chain_part < 0 || p->chain_part >= p->chain_parts))
     return fail(MPL_ERR_INVALID, "chain_part=%d outside 0..%d", p->chain_part, p->chain_parts - 1);
   return MPL_OK;
+}
+
+int validate(const mpl_problem* p, Dims* d) {
+  if (!p) return fail(MPL_ERR_INVALID, "problem is NULL");
+  const Problem q = with_rows(p, nullptr);
+  return validate(&q, d);
 }
 
 int check_chain_count(const mpl_problem* p, const Dims& d) {
@@ -173,6 +201,7 @@ void fill_forward(mpl::FwdParams& fp, const mpl_problem* p, const Dims& d, const
   fp.H = p->height;
   fp.W = p->width;
   fp.L = p->n_disp;
+  fp.ls = d.ls;
   fp.D = p->n_dir;
   fp.nimg = (int)d.nimg;
   fp.slice = d.slice;
@@ -238,10 +267,13 @@ int prepare_forward(mpl::FwdParams& fp, const mpl_problem* p, const Dims& d, con
   return MPL_OK;
 }
 
-int forward_common(bool isgmr, const mpl_problem* p, const float* unary, const float* context,
+int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows, const float* unary, const float* context,
                    const float* edge_weights, float* msg, float* msg_update, float* cost_final,
                    uint8_t* msg_min_index, uint8_t* msg_norm_index, uint8_t* label_all,
                    void* workspace, size_t workspace_bytes, void* stream) {
+  if (!problem) return fail(MPL_ERR_INVALID, "problem is NULL");
+  const Problem q = with_rows(problem, rows);
+  const Problem* p = &q;
   Dims d;
   if (int rc = validate(p, &d)) return rc;
   if (int rc = check_chain_count(p, d)) return rc;
@@ -249,12 +281,15 @@ int forward_common(bool isgmr, const mpl_problem* p, const float* unary, const f
     return fail(MPL_ERR_INVALID, "NULL tensor pointer");
   if ((msg_min_index == nullptr) != (msg_norm_index == nullptr))
     return fail(MPL_ERR_INVALID, "msg_min_index and msg_norm_index must both be given or both be NULL");
-  if (!workspace || workspace_bytes < mpl_forward_workspace_bytes(p))
+  if (!workspace || workspace_bytes < mpl_forward_workspace_bytes_rows(p, rows))
     return fail(MPL_ERR_INVALID, "workspace too small: %zu < %zu", workspace_bytes,
-                mpl_forward_workspace_bytes(p));
+                mpl_forward_workspace_bytes_rows(p, rows));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool train = msg_min_index != nullptr;
   const int D = p->n_dir, L = p->n_disp;
+  // Where the per-iteration sums go: `cost_final` is free until the end, but without padding it may be
+  // too small for rows of the padded stride; then they live in the workspace.
+  float* sums = d.ls == L ? cost_final : reinterpret_cast<float*>(static_cast<char*>(workspace) + kTablesOffset);
 
   mpl::FwdParams fp{};
   if (int rc = prepare_forward(fp, p, d, unary, context, edge_weights, workspace, train, st)) return rc;
@@ -269,28 +304,48 @@ int forward_common(bool isgmr, const mpl_problem* p, const float* unary, const f
     rd = wr == msg ? msg_update : msg;
     // The iterations start from the messages in `msg`, as in the reference.  With an odd iteration
     // count the first sweep writes `msg`, so its input moves to `msg_update` first.
-    if (rd != msg && p->n_iter > 0)
+    if (rd != msg && p->n_iter > 0 && !p->messages_zero)
       MPL_CUDA(cudaMemcpyAsync(msg_update, msg, (size_t)D * d.slice * sizeof(float), cudaMemcpyDeviceToDevice, st));
   }
+  // With few labels and directions an ISGMR sweep sums U + sum_k M_k itself faster than a separate
+  // pass over all messages does (measured 5.13 -> 4.99 ms on 2x512x512, L = 21, D = 4); with
+  // 256 labels the extra staged rows cost more than the pass (28.4 -> 29.2 ms).
+  const bool use_agg = isgmr && !(L <= 32 && D <= 4);
+  // Zero start: messages known to be zero are neither written nor read where the sweeps can leave them
+  // out (375 x 1242 x 128, eight directions, one iteration: 3.40 ms with them).  Either way the
+  // pixels that no sweep visits -- the chains' first ones -- have to hold zeros in every buffer.
+  bool skip_zero = false;
+  if (p->messages_zero) {
+    fp.agg = use_agg ? 1 : 0;
+    fp.msg_read = rd;
+    skip_zero = p->n_iter > 0 && mpl::forward_skips_zero_slices(fp, train);
+    if (!skip_zero) MPL_CUDA(cudaMemsetAsync(rd, 0, (size_t)D * d.slice * sizeof(float), st));
+    // (directions beyond 3 of a TRWP iteration read all slices)
+    if (skip_zero && !isgmr && D > 4)
+      MPL_CUDA(cudaMemsetAsync(rd + 4 * d.slice, 0, (size_t)(D - 4) * d.slice * sizeof(float), st));
+    if (p->n_iter > 0 && (skip_zero || isgmr)) {
+      set_dirs(fp, 0, D);
+      MPL_CUDA(mpl::launch_zero_chain_starts(fp, wr, skip_zero && isgmr ? rd : nullptr, st));
+    }
+    if (p->n_iter == 0 && rd != msg) MPL_CUDA(cudaMemsetAsync(msg, 0, (size_t)D * d.slice * sizeof(float), st));
+  }
+  bool have_sums = false;
   for (int it = 0; it < p->n_iter; ++it) {
     fp.min_idx = train ? msg_min_index + (long long)it * D * d.slice : nullptr;
     fp.norm_idx = train ? msg_norm_index + (long long)it * D * d.npix : nullptr;
     fp.msg_read = rd;
     fp.msg_write = wr;
+    fp.first = it == 0 && skip_zero;
     if (isgmr) {
       // Every direction reads the previous iteration's messages.  Their sum with the unaries is
-      // formed once (in `cost_final`, which is otherwise unused until the end) so that a sweep
-      // stages three arrays instead of D+1.  The first iteration forms it too: the messages the
-      // caller passes in count, as they do in the reference and in the other path.
-      // With few labels and directions the sweep sums U + sum_k M_k itself faster than a separate
-      // pass over all messages does (measured 5.13 -> 4.99 ms on 2x512x512, L = 21, D = 4); with
-      // 256 labels the extra staged rows cost more than the pass (28.4 -> 29.2 ms).
-      const bool use_agg = !(L <= 32 && D <= 4);
+      // formed once per iteration so that a sweep stages three arrays instead of D+1.  The first
+      // iteration forms it too unless the messages are known to be zero: those the caller passes
+      // in count, as they do in the reference and in the other path.
       fp.agg = use_agg ? 1 : 0;
       fp.unary = unary;
-      if (use_agg) {
-        MPL_CUDA(mpl::launch_aggregate(unary, rd, cost_final, nullptr, d.npix, L, D, d.slice, 1.f, 0, st));
-        fp.unary = cost_final;
+      if (use_agg && !(it == 0 && p->messages_zero)) {
+        if (!have_sums) MPL_CUDA(mpl::launch_aggregate(unary, rd, sums, nullptr, d.npix, L, d.ls, D, d.slice, 1.f, 0, st));
+        fp.unary = sums;
       }
       set_dirs(fp, 0, D);
       MPL_CUDA(mpl::launch_forward_sweep(fp, train, st));
@@ -305,28 +360,24 @@ int forward_common(bool isgmr, const mpl_problem* p, const float* unary, const f
     }
     if (label_all) {
       const float* cur = isgmr ? rd : msg;  // after the swap `rd` holds this iteration's messages
-      MPL_CUDA(mpl::launch_aggregate(unary, cur, cost_final, label_all + (long long)it * d.npix, d.npix,
-                                     L, D, d.slice, factor, p->enable_min_a_dir, st));
+      // the sums behind an iteration's labels are those the next iteration's sweeps start from
+      have_sums = isgmr && !(L <= 32 && D <= 4) && factor == 1.f && !p->enable_min_a_dir && it + 1 < p->n_iter;
+      MPL_CUDA(mpl::launch_aggregate(unary, cur, have_sums ? sums : nullptr, label_all + (long long)it * d.npix,
+                                     d.npix, L, d.ls, D, d.slice, factor, p->enable_min_a_dir, st));
     }
   }
   const float* fin = isgmr ? rd : msg;
   if (isgmr && p->n_iter > 0 && fin != msg)
     return fail(MPL_ERR_CUDA, "internal: ISGMR buffer parity");
   if (p->cost_labels_first) {
-    MPL_CUDA(mpl::launch_aggregate_lhw(unary, msg, cost_final, (int)d.nimg, L, (long long)p->height * p->width, D,
+    MPL_CUDA(mpl::launch_aggregate_lhw(unary, msg, cost_final, (int)d.nimg, L, d.ls, (long long)p->height * p->width, D,
                                        d.slice, factor, p->enable_min_a_dir, st));
   } else {
-    MPL_CUDA(mpl::launch_aggregate(unary, msg, cost_final, nullptr, d.npix, L, D, d.slice, factor,
+    MPL_CUDA(mpl::launch_aggregate(unary, msg, cost_final, nullptr, d.npix, L, d.ls, D, d.slice, factor,
                                    p->enable_min_a_dir, st));
   }
   return MPL_OK;
 }
-
-// Layout of every workspace (forward, backward, the built-in scratch): bytes [0, 64) context
-// analysis, [64, 68) the device status word, [256, ...) the backward's partial label-context tables.
-constexpr size_t kStatusOffset = 64, kTablesOffset = 256;
-inline float* ws_tables(void* workspace) { return reinterpret_cast<float*>(static_cast<char*>(workspace) + kTablesOffset); }
-inline int* ws_status(void* workspace) { return reinterpret_cast<int*>(static_cast<char*>(workspace) + kStatusOffset); }
 
 void fill_backward(mpl::BwdParams& bp, const mpl_problem* p, const Dims& d, const float* context,
                    const float* edge_weights, float* dunary, float* part, int n_slots, int cp, int* status) {
@@ -338,6 +389,7 @@ void fill_backward(mpl::BwdParams& bp, const mpl_problem* p, const Dims& d, cons
   bp.H = p->height;
   bp.W = p->width;
   bp.L = p->n_disp;
+  bp.ls = d.ls;
   bp.D = p->n_dir;
   bp.nimg = (int)d.nimg;
   bp.slice = d.slice;
@@ -350,11 +402,14 @@ void fill_backward(mpl::BwdParams& bp, const mpl_problem* p, const Dims& d, cons
   bp.status = status;
 }
 
-int backward_common(bool isgmr, const mpl_problem* p, const float* context, const float* edge_weights,
+int backward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows, const float* context, const float* edge_weights,
                     const float* dcost_final, const uint8_t* msg_min_index,
                     const uint8_t* msg_norm_index, float* dunary, float* dcontext,
                     float* dedge_weights, float* dmsg, float* dmsg_update, void* workspace,
                     size_t workspace_bytes, void* stream) {
+  if (!problem) return fail(MPL_ERR_INVALID, "problem is NULL");
+  const Problem q = with_rows(problem, rows);
+  const Problem* p = &q;
   Dims d;
   if (int rc = validate(p, &d)) return rc;
   if (int rc = check_chain_count(p, d)) return rc;
@@ -377,15 +432,15 @@ int backward_common(bool isgmr, const mpl_problem* p, const float* context, cons
   // see BwdParams::cp_scheme; everything else updates dunary and the D slices directly.
   // (L <= 64 in multiples of four at 16-byte aligned buffers runs the two-labels-per-lane kernel,
   // which knows the C + P scheme as well.)
-  const bool pair_cp = L <= 64 && (L & 3) == 0 && ((((uintptr_t)dunary | (uintptr_t)dmsg) & 15) == 0) &&
+  const bool pair_cp = L <= 64 && (d.ls & 3) == 0 && ((((uintptr_t)dunary | (uintptr_t)dmsg) & 15) == 0) &&
                        !mpl::pair_kernels_disabled();
   // (a rank-1 context with 32 < L <= 256 runs the several-labels-per-lane kernel, C + P too)
-  const bool wide_cp = mpl::bwd_wide_eligible(L, p->context_rank, 1, dunary, dmsg, dmsg);
+  const bool wide_cp = mpl::bwd_wide_eligible(L, d.ls, p->context_rank, 1, dunary, dmsg, dmsg);
   const int cp = isgmr ? 2 : ((L <= 32 || pair_cp || wide_cp) ? 1 : 0);
   float* X = isgmr ? dmsg_update : dmsg;  // gradients of the messages the sweeps produced
   float* Y = isgmr ? dmsg : dmsg;         // gradients of the messages the sweeps read
   if (p->cost_labels_first) {
-    MPL_CUDA(mpl::launch_backward_init_lhw(dcost_final, dunary, X, (int)d.nimg, L, (long long)p->height * p->width,
+    MPL_CUDA(mpl::launch_backward_init_lhw(dcost_final, dunary, X, (int)d.nimg, L, d.ls, (long long)p->height * p->width,
                                            D, factor, cp == 1, st));
   } else {
     MPL_CUDA(mpl::launch_backward_init(dcost_final, dunary, X, d.slice, D, factor, cp == 1, st));
@@ -446,10 +501,28 @@ int mpl_analyze_context(const mpl_problem* p, const float* context, const float*
   return MPL_OK;
 }
 
-size_t mpl_forward_workspace_bytes(const mpl_problem* p) {
-  (void)p;
-  return 256;
+int32_t mpl_label_stride(const mpl_problem* p, int32_t isgmr) {
+  Dims d;
+  if (validate(p, &d) != MPL_OK) return 0;
+  const int L = p->n_disp, padded = (L + 3) & ~3;
+  if (L > 32) return padded;
+  // up to 32 labels: the axis directions of an image whose width is a multiple of 4 have aligned row
+  // segments whatever L is; everything else goes through kernels that stage one label row per
+  // pixel, in 16-byte pieces where rows are aligned and one float per lane elsewhere
+  const bool row_staged =
+      (p->width & 3) || p->n_dir > 4 || (isgmr && d.nimg * (p->height < p->width ? p->height : p->width) < 256);
+  return row_staged ? padded : L;
 }
+
+size_t mpl_forward_workspace_bytes_rows(const mpl_problem* p, const mpl_rows* rows) {
+  Dims d;
+  if (!p) return kTablesOffset;
+  const Problem q = with_rows(p, rows);
+  if (validate(&q, &d) != MPL_OK || d.ls == p->n_disp) return kTablesOffset;
+  return kTablesOffset + (size_t)d.slice * sizeof(float);  // header + per-iteration sums
+}
+
+size_t mpl_forward_workspace_bytes(const mpl_problem* p) { return mpl_forward_workspace_bytes_rows(p, nullptr); }
 
 size_t mpl_backward_workspace_bytes(const mpl_problem* p) {
   Dims d;
@@ -458,40 +531,70 @@ size_t mpl_backward_workspace_bytes(const mpl_problem* p) {
   return kTablesOffset + (size_t)n_slots * d.ctx_elems * sizeof(float);  // header + tables
 }
 
+int mpl_trwp_forward_rows(const mpl_problem* p, const mpl_rows* rows, const float* unary, const float* context,
+                     const float* edge_weights, float* msg, float* cost_final, uint8_t* msg_min_index,
+                     uint8_t* msg_norm_index, uint8_t* label_all, void* workspace,
+                     size_t workspace_bytes, void* stream) {
+  return forward_common(false, p, rows, unary, context, edge_weights, msg, nullptr, cost_final, msg_min_index,
+                        msg_norm_index, label_all, workspace, workspace_bytes, stream);
+}
 int mpl_trwp_forward(const mpl_problem* p, const float* unary, const float* context,
                      const float* edge_weights, float* msg, float* cost_final, uint8_t* msg_min_index,
                      uint8_t* msg_norm_index, uint8_t* label_all, void* workspace,
                      size_t workspace_bytes, void* stream) {
-  return forward_common(false, p, unary, context, edge_weights, msg, nullptr, cost_final, msg_min_index,
-                        msg_norm_index, label_all, workspace, workspace_bytes, stream);
+  return mpl_trwp_forward_rows(p, nullptr, unary, context, edge_weights, msg, cost_final, msg_min_index,
+                               msg_norm_index, label_all, workspace, workspace_bytes, stream);
 }
 
+int mpl_isgmr_forward_rows(const mpl_problem* p, const mpl_rows* rows, const float* unary, const float* context,
+                      const float* edge_weights, float* msg, float* msg_update, float* cost_final,
+                      uint8_t* msg_min_index, uint8_t* msg_norm_index, uint8_t* label_all,
+                      void* workspace, size_t workspace_bytes, void* stream) {
+  return forward_common(true, p, rows, unary, context, edge_weights, msg, msg_update, cost_final,
+                        msg_min_index, msg_norm_index, label_all, workspace, workspace_bytes, stream);
+}
 int mpl_isgmr_forward(const mpl_problem* p, const float* unary, const float* context,
                       const float* edge_weights, float* msg, float* msg_update, float* cost_final,
                       uint8_t* msg_min_index, uint8_t* msg_norm_index, uint8_t* label_all,
                       void* workspace, size_t workspace_bytes, void* stream) {
-  return forward_common(true, p, unary, context, edge_weights, msg, msg_update, cost_final,
-                        msg_min_index, msg_norm_index, label_all, workspace, workspace_bytes, stream);
+  return mpl_isgmr_forward_rows(p, nullptr, unary, context, edge_weights, msg, msg_update, cost_final,
+                                msg_min_index, msg_norm_index, label_all, workspace, workspace_bytes, stream);
 }
 
+int mpl_trwp_backward_rows(const mpl_problem* p, const mpl_rows* rows, const float* context, const float* edge_weights,
+                      const float* dcost_final, const uint8_t* msg_min_index,
+                      const uint8_t* msg_norm_index, float* dunary, float* dcontext,
+                      float* dedge_weights, float* dmsg, void* workspace, size_t workspace_bytes,
+                      void* stream) {
+  return backward_common(false, p, rows, context, edge_weights, dcost_final, msg_min_index, msg_norm_index,
+                         dunary, dcontext, dedge_weights, dmsg, nullptr, workspace, workspace_bytes,
+                         stream);
+}
 int mpl_trwp_backward(const mpl_problem* p, const float* context, const float* edge_weights,
                       const float* dcost_final, const uint8_t* msg_min_index,
                       const uint8_t* msg_norm_index, float* dunary, float* dcontext,
                       float* dedge_weights, float* dmsg, void* workspace, size_t workspace_bytes,
                       void* stream) {
-  return backward_common(false, p, context, edge_weights, dcost_final, msg_min_index, msg_norm_index,
-                         dunary, dcontext, dedge_weights, dmsg, nullptr, workspace, workspace_bytes,
-                         stream);
+  return mpl_trwp_backward_rows(p, nullptr, context, edge_weights, dcost_final, msg_min_index, msg_norm_index,
+                                dunary, dcontext, dedge_weights, dmsg, workspace, workspace_bytes, stream);
 }
 
+int mpl_isgmr_backward_rows(const mpl_problem* p, const mpl_rows* rows, const float* context, const float* edge_weights,
+                       const float* dcost_final, const uint8_t* msg_min_index,
+                       const uint8_t* msg_norm_index, float* dunary, float* dcontext,
+                       float* dedge_weights, float* dmsg, float* dmsg_update, void* workspace,
+                       size_t workspace_bytes, void* stream) {
+  return backward_common(true, p, rows, context, edge_weights, dcost_final, msg_min_index, msg_norm_index,
+                         dunary, dcontext, dedge_weights, dmsg, dmsg_update, workspace,
+                         workspace_bytes, stream);
+}
 int mpl_isgmr_backward(const mpl_problem* p, const float* context, const float* edge_weights,
                        const float* dcost_final, const uint8_t* msg_min_index,
                        const uint8_t* msg_norm_index, float* dunary, float* dcontext,
                        float* dedge_weights, float* dmsg, float* dmsg_update, void* workspace,
                        size_t workspace_bytes, void* stream) {
-  return backward_common(true, p, context, edge_weights, dcost_final, msg_min_index, msg_norm_index,
-                         dunary, dcontext, dedge_weights, dmsg, dmsg_update, workspace,
-                         workspace_bytes, stream);
+  return mpl_isgmr_backward_rows(p, nullptr, context, edge_weights, dcost_final, msg_min_index, msg_norm_index,
+                                 dunary, dcontext, dedge_weights, dmsg, dmsg_update, workspace, workspace_bytes, stream);
 }
 
 // ---- ISGMR one iteration at a time over a subset of directions (direction sharding) -------------
@@ -669,10 +772,10 @@ int mpl_trwp_soft_forward(const mpl_problem* p, const float* unary, const float*
       MPL_CUDA(mpl::launch_forward_soft_sweep(fp, train, st));
     }
     if (label_all)
-      MPL_CUDA(mpl::launch_aggregate(unary, msg, cost_final, label_all + (long long)it * d.npix, d.npix, L, D,
+      MPL_CUDA(mpl::launch_aggregate(unary, msg, cost_final, label_all + (long long)it * d.npix, d.npix, L, d.ls, D,
                                      d.slice, 1.f, 0, st));
   }
-  MPL_CUDA(mpl::launch_aggregate(unary, msg, cost_final, nullptr, d.npix, L, D, d.slice, 1.f, 0, st));
+  MPL_CUDA(mpl::launch_aggregate(unary, msg, cost_final, nullptr, d.npix, L, d.ls, D, d.slice, 1.f, 0, st));
   return MPL_OK;
 }
 
@@ -722,11 +825,13 @@ int mpl_trwp_soft_backward(const mpl_problem* p, const float* context, const flo
 // ---- layout glue: class scores [B,L,H,W] <-> costs [B,H,W,L] -------------------------------------
 namespace {
 int layout_call(int kind, const float* in, float* out, uint8_t* amax, int32_t batch, int32_t n_disp,
-                int32_t height, int32_t width, void* stream) {
+                int32_t height, int32_t width, void* stream, int32_t label_stride = 0) {
   if (!in || !out || ((kind == 1 || kind == 3) && !amax)) return fail(MPL_ERR_INVALID, "NULL tensor pointer");
   if (batch < 1 || height < 1 || width < 1 || n_disp < 1 || n_disp > 256 || batch > 65535)
     return fail(MPL_ERR_INVALID, "bad shape: batch=%d n_disp=%d height=%d width=%d", batch, n_disp, height, width);
-  MPL_CUDA(mpl::launch_layout(kind, in, out, amax, batch, n_disp, (long long)height * width,
+  if (label_stride == 0) label_stride = n_disp;
+  if (label_stride < n_disp) return fail(MPL_ERR_INVALID, "label_stride=%d below n_disp=%d", label_stride, n_disp);
+  MPL_CUDA(mpl::launch_layout(kind, in, out, amax, batch, n_disp, label_stride, (long long)height * width,
                               static_cast<cudaStream_t>(stream)));
   return MPL_OK;
 }
@@ -749,6 +854,24 @@ int mpl_negate_hwl_to_lhw(const float* in, float* out, int32_t batch, int32_t n_
   return layout_call(2, in, out, nullptr, batch, n_disp, height, width, stream);
 }
 
+int mpl_permute_lhw_to_rows(const float* in, float* out, int32_t batch, int32_t n_disp, int32_t height, int32_t width,
+                            int32_t label_stride, void* stream) {
+  return layout_call(4, in, out, nullptr, batch, n_disp, height, width, stream, label_stride);
+}
+int mpl_permute_rows_to_lhw(const float* in, float* out, int32_t batch, int32_t n_disp, int32_t height, int32_t width,
+                            int32_t label_stride, void* stream) {
+  return layout_call(5, in, out, nullptr, batch, n_disp, height, width, stream, label_stride);
+}
+int mpl_scores_to_cost_rows(const float* scores, float* costs, uint8_t* argmax, int32_t batch, int32_t n_disp,
+                            int32_t height, int32_t width, int32_t label_stride, void* stream) {
+  return layout_call(1, scores, costs, argmax, batch, n_disp, height, width, stream, label_stride);
+}
+int mpl_scores_to_cost_rows_backward(const float* dcosts, const uint8_t* argmax, float* dscores, int32_t batch,
+                                     int32_t n_disp, int32_t height, int32_t width, int32_t label_stride,
+                                     void* stream) {
+  return layout_call(3, dcosts, dscores, const_cast<uint8_t*>(argmax), batch, n_disp, height, width, stream,
+                     label_stride);
+}
 int mpl_permute_lhw_to_hwl(const float* in, float* out, int32_t batch, int32_t n_disp, int32_t height,
                            int32_t width, void* stream) {
   return layout_call(4, in, out, nullptr, batch, n_disp, height, width, stream);
@@ -969,7 +1092,7 @@ int mpl_trwp_backward_static(const mpl_problem* p, const float* context, const f
     scratch = addr[dev];
   }
   // backward_common clears the part of the scratch it uses (partial tables and status word)
-  return backward_common(false, p, context, edge_weights, dcost_final, msg_min_index, msg_norm_index, dunary,
+  return backward_common(false, p, nullptr, context, edge_weights, dcost_final, msg_min_index, msg_norm_index, dunary,
                          dcontext, dedge_weights, dmsg, nullptr, scratch, MPL_STATIC_SCRATCH_BYTES, stream);
 }
 

@@ -18,6 +18,7 @@
 //     alone: the part carried from the successor pixel sums to zero (it is itself the output of
 //     a normalisation backward), so only rounding noise is dropped.
 #include <cstdlib>
+#include <type_traits>
 
 #include "mp_common.cuh"
 #include "mp_minplus.cuh"
@@ -36,26 +37,30 @@ __device__ __forceinline__ void warp_sum2(float& a, float& b) {
 
 // ------------------------------------------------------------------------------------------------
 // L <= 32, generic: one warp per chain, lane = label, any direction / alignment.
-// DT = compile-time direction count (0: from params); CP = gradient bookkeeping scheme.
+// SCH = gradient bookkeeping scheme: 1 (C + P, TRWP) or 2 (scatter field, ISGMR).
 //
 // The chain is walked in blocks of 32 steps; the stored message gradients of a whole block are
-// staged in shared memory one block ahead with cp.async.
+// staged in shared memory one block ahead with cp.async: in 16-byte pieces spread over the lanes where
+// pixel rows are multiples of 16 bytes (V4), in 4-byte pieces, one label per lane, elsewhere.
+// LMAX = padded label count of the scatter's gather.
 // ------------------------------------------------------------------------------------------------
 constexpr int kRB = 64;  // ring rows: two blocks of 32 steps
 constexpr int kRS = 33;  // padded row stride (conflict-free both along and across rows)
+constexpr int kRS4 = 36;  // V4: rows start 16-byte aligned
 
 __host__ __device__ inline int bwd_warp_floats(int L, int rank, int cp) {
-  const int tab = rank == 2 ? L * (L | 1) : 32;
-  return (cp ? 2 : 1) * kRB * kRS + 32 * kRS + 128 + ((tab + 3) & ~3);
+  (void)rank;  // the per-chain table is kept per (c, f) pair for both context conventions
+  return (cp ? 2 : 1) * kRB * kRS4 + 32 * kRS + 128 + ((L * (L | 1) + 3) & ~3);
 }
 
-template <int DT, int SCH>
+template <int LMAX, int SCH, bool V4>
 __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant__ BwdParams p) {
   constexpr bool CP = SCH == 1;   // C + P bookkeeping
   constexpr bool QM = SCH == 2;   // store the scatter field only
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = p.L, D = DT ? DT : p.D;
+  constexpr int RS = V4 ? kRS4 : kRS;
+  const int L = p.L, LR = p.ls;
   const int LS = L | 1;  // odd row stride: private rows without bank conflicts
   // full (symmetric / Toeplitz) context table shared by the CTA
   float* ctab = smem;
@@ -67,10 +72,10 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
   BChain ch;
   if (!decode_bchain(p, g, ch)) return;
   const int dir = ch.dir, inv = dir ^ 1;
-  const int tab = p.ctx_rank == 2 ? L * LS : 32;
+  const int tab = L * LS;
   float* ring = smem + ctab_floats + warp * bwd_warp_floats(L, p.ctx_rank, CP);  // [kRB][kRS] (x2 if CP)
-  float* ring2 = ring + kRB * kRS;                                              // CP: P_dir rows
-  float* dtile = ring + (CP ? 2 : 1) * kRB * kRS;                               // [32][kRS]
+  float* ring2 = ring + kRB * RS;                                              // CP: P_dir rows
+  float* dtile = ring + (CP ? 2 : 1) * kRB * kRS4;                               // [32][kRS]
   float* ts = dtile + 32 * kRS;                                                 // [2][32]
   float* is = ts + 64;                                                          // [2][32] argmin as float
   float* acc = ts + 128;                                                        // context-gradient table
@@ -78,34 +83,50 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
   for (int i = lane; i < tab; i += 32) acc[i] = 0.f;
   is[lane] = -1.f;
   is[32 + lane] = -1.f;
+  ts[lane] = 0.f;
+  ts[32 + lane] = 0.f;
 
   const long long ibase = (long long)ch.img * p.H * p.W;
-  float* DMrl = p.dm_read + (long long)dir * p.slice + ibase * L + lane;  // dM_dir, or P_dir
-  float* DMal = p.dm_acc + ibase * L + lane;
-  float* DUl = p.dunary + ibase * L + lane;                              // dU, or C
+  float* DMrl = p.dm_read + (long long)dir * p.slice + ibase * LR + lane;  // dM_dir, or P_dir
+  float* DMal = p.dm_acc + ibase * LR + lane;
+  float* DUl = p.dunary + ibase * LR + lane;                              // dU, or C
   const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
   float* DE = p.dew ? p.dew + (long long)dir * p.pslice + ibase : nullptr;
-  const uint8_t* MIl = p.min_idx + (long long)dir * p.slice + ibase * L + lane;
+  const uint8_t* MIl = p.min_idx + (long long)dir * p.slice + ibase * LR + lane;
   const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
   const int len = ch.len;
-  const int pstep = ch.pstep, ostep = ch.pstep * L;
+  const int pstep = ch.pstep, ostep = ch.pstep * LR;
   const int pixl = ch.h0 * p.W + ch.w0 + (len - 1) * pstep;  // last pixel of the chain
   const float rho = p.rho;
-  const float rinv = rho - 1.f;  // dM_inv += rho*q - q
   const int nsteps = len - 1;    // steps with a predecessor pixel (s = 0 .. len-2)
 
   // step s visits chain pixel len-1-s at image pixel pixl - s*pstep
+  const int nch = LR >> 2;  // V4: 16-byte pieces per row
   auto stage_block = [&](int b) {  // stored gradients of the 32 steps of block b -> ring rows
-    if (act) {
+    if constexpr (V4) {
+      // lane -> (row u, piece j) with nch lanes per row, 32 / nch rows per round
+      const int rpr = 32 / nch, u0 = lane / nch, j = lane - u0 * nch, s = 32 * b;
+      if (u0 < rpr) {
+        const int last = (CP ? len : nsteps) - s;
+        const float* c4 = (CP ? DUl : DMrl) - lane + 4 * j;
+        const float* p4 = DMrl - lane + 4 * j;
+        float* dst = ring + (s & (kRB - 1)) * RS + 4 * j;
+        for (int u = u0; u < 32 && u < last; u += rpr) {
+          const int o = (pixl - (s + u) * pstep) * LR;
+          cp_async16(dst + u * RS, c4 + o);
+          if (CP) cp_async16(dst + kRB * RS + u * RS, p4 + o);
+        }
+      }
+    } else if (act) {
       const int s = 32 * b;
-      int o = (pixl - s * pstep) * L;
-      float* dst = ring + (s & (kRB - 1)) * kRS + lane;
+      int o = (pixl - s * pstep) * LR;
+      float* dst = ring + (s & (kRB - 1)) * RS + lane;
 #pragma unroll 8
       for (int u = 0; u < 32; ++u) {
         // CP also needs the values of the chain-start pixel (its C is rewritten there)
         if (s + u < (CP ? len : nsteps)) {
-          cp_async4(dst + u * kRS, CP ? DUl + o : DMrl + o);
-          if (CP) cp_async4(dst + kRB * kRS + u * kRS, DMrl + o);
+          cp_async4(dst + u * RS, CP ? DUl + o : DMrl + o);
+          if (CP) cp_async4(dst + kRB * RS + u * RS, DMrl + o);
         }
         o -= ostep;
       }
@@ -129,10 +150,10 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
   load_blk(0, e_cur, n_cur);
   int fa[8], fb[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) fa[u] = (u < nsteps && act) ? (int)MIl[(pixl - u * pstep) * L] : -1;
+  for (int u = 0; u < 8; ++u) fa[u] = (u < nsteps && act) ? (int)MIl[(pixl - u * pstep) * LR] : -1;
 
   float q = 0.f;  // lane f: sum of t[c] of the successor pixel over labels c whose argmin was f
-  int of = pixl * L;
+  int of = pixl * LR;
   const int nblocks = (len + 31) >> 5;
   for (int b = 0; b < nblocks; ++b) {
     stage_block(b + 1);
@@ -142,8 +163,9 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
     // normalisation sums of this block: lane j sums row j of the staged gradients
     float s_cur = 0.f;
     {
-      const float* row = ring + ((32 * b + lane) & (kRB - 1)) * kRS;
-      for (int c = 0; c < L; ++c) s_cur += CP ? row[c] + row[kRB * kRS + c] : row[c];
+      const float* row = ring + ((32 * b + lane) & (kRB - 1)) * RS;
+#pragma unroll 4
+      for (int c = 0; c < L; ++c) s_cur += CP ? row[c] + row[kRB * RS + c] : row[c];
     }
     for (int g8 = 0; g8 < 4; ++g8) {
       const int s0 = 32 * b + 8 * g8;
@@ -151,7 +173,7 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
 #pragma unroll
       for (int u = 0; u < 8; ++u) {  // argmin indices of the next group of 8 steps
         const int s = s0 + 8 + u;
-        fb[u] = (s < nsteps && act) ? (int)MIl[(pixl - s * pstep) * L] : -1;
+        fb[u] = (s < nsteps && act) ? (int)MIl[(pixl - s * pstep) * LR] : -1;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
@@ -159,26 +181,21 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
         if (s < len) {
           const float rq = rho * q;
           float qn = 0.f;
-          const float x0 = ring[(s & (kRB - 1)) * kRS + lane];  // dM_dir, or C
+          const float x0 = ring[(s & (kRB - 1)) * RS + lane];  // dM_dir, or C
           if (s < nsteps) {
             const int sl = s & 31;
             const float e = __shfl_sync(0xffffffffu, e_cur, sl);
             const int n = __shfl_sync(0xffffffffu, n_cur, sl);
             const float S = __shfl_sync(0xffffffffu, s_cur, sl);
             const int f = fa[u];
-            const float x = CP ? x0 + ring2[(s & (kRB - 1)) * kRS + lane] : x0;
+            const float x = CP ? x0 + ring2[(s & (kRB - 1)) * RS + lane] : x0;
             const float t0 = act ? x + rq : 0.f;
             const float t = (lane == n) ? t0 - S : t0;  // MPLayers/commonCUDA.cuh:131-145
             float cv = 0.f;
             if (act) {
               cv = ctab[lane * LS + f];
-              if (lane != f || p.keep_diag) {
-                if (p.ctx_rank == 2) {
-                  acc[lane * LS + f] += e * t;
-                } else {
-                  atomicAdd(acc + (lane > f ? lane - f : f - lane), e * t);
-                }
-              }
+              // the diagonal is accumulated like every other cell and dropped at the flush unless wanted
+              acc[lane * LS + f] = fmaf(e, t, acc[lane * LS + f]);
             }
             dtile[sl * kRS + lane] = cv * t;
             float* tb = ts + (s & 1) * 32;
@@ -186,24 +203,16 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
             tb[lane] = t;
             if (act) ib[lane] = (float)f;
             __syncwarp();
-            qn = gather_q<0>(tb, ib, L, (float)lane);
+            qn = gather_q<LMAX>(tb, ib, L, (float)lane);
           }
           if (act) {
             if (QM) {
               DMal[(long long)dir * p.slice + of] = q;  // scatter field of this direction at this pixel
-            } else if (CP) {
+            } else {
               const float cnew = x0 + rq;  // dU and every dM_k (k != dir, inv) receive rho*q
               DUl[of] = cnew;
               DMrl[of] = -cnew;            // dM_dir = C + P_dir = 0 after its sweep
               atomicAdd(DMal + inv * p.slice + of, -q);
-            } else {
-              // UpdateUnaryKernelBack (MPLayers/TRWP/TRWP_backward.cu:26-47) applied to this pixel
-#pragma unroll
-              for (int k = 0; k < (DT ? DT : 16); ++k) {
-                if (k < D && k != dir) atomicAdd(DMal + k * p.slice + of, k == inv ? rinv * q : rq);
-              }
-              atomicAdd(DUl + of, rq);
-              DMrl[of] = 0.f;
             }
           }
           q = qn;
@@ -235,11 +244,16 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
   float* part = p.dctx_part + (long long)(g % p.n_slots) * (p.ctx_rank == 2 ? L * L : L);
   if (p.ctx_rank == 2) {
     for (int i = lane; i < L * L; i += 32) {
-      const float v = acc[(i / L) * LS + (i % L)];
-      if (v != 0.f) atomicAdd(part + i, v);
+      const int c = i / L, f = i - c * L;
+      const float v = acc[c * LS + f];
+      if (v != 0.f && (c != f || p.keep_diag)) atomicAdd(part + i, v);
     }
-  } else if (act) {
-    const float v = acc[lane];
+  } else if (act && (lane > 0 || p.keep_diag)) {  // lane k folds every (c, f) with |c - f| == k, in a fixed order
+    float v = 0.f;
+    for (int c = 0; c < L; ++c) {
+      if (c - lane >= 0) v += acc[c * LS + c - lane];
+      if (lane > 0 && c + lane < L) v += acc[c * LS + c + lane];
+    }
     if (v != 0.f) atomicAdd(part + lane, v);
   }
 }
@@ -262,7 +276,7 @@ __host__ __device__ inline int bwd_tma_warp_floats(int L, int rank) {
 
 // QM: scatter-field scheme (ISGMR): only the gradient slice of the direction is staged and only the
 // scatter field is stored.
-template <int LT, bool VERT, bool REV, bool QM = false>
+template <int LT, bool PAD, bool VERT, bool REV, bool QM = false>
 __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__ BwdParams p,
                                                          const __grid_constant__ TmaMaps maps) {
   // No static shared memory in this kernel: the dynamic region starts at the CTA's shared window
@@ -270,13 +284,13 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
   // pointer up by hand would hide its address space from the compiler and turn every shared
   // access into a slower generic one.)
   extern __shared__ __align__(128) float smem[];
-  const int L = LT ? LT : p.L, H = p.H, W = p.W, NS = p.tma_stages;
+  const int L = LT ? LT : p.L, LR = LT ? (PAD ? (LT + 3) / 4 * 4 : LT) : p.ls, H = p.H, W = p.W, NS = p.tma_stages;
   const int LS = L | 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int dir = p.dir, inv = dir ^ 1;
   const int len = VERT ? H : W;
   const int nstages = (len + kBK - 1) / kBK;
-  const int tile_floats = 2 * kBK * 4 * L;  // C and P_dir, kBK steps, four chains
+  const int tile_floats = 2 * kBK * 4 * LR;  // C and P_dir, kBK steps, four chains
 
   float* tiles = smem;                                         // [NS][tile_floats]
   float* ctab = tiles + NS * tile_floats;                      // [L][LS]
@@ -310,7 +324,7 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
   // step st of the walk visits coordinate (REV ? len-1-st : st) along the chain direction
   if (warp == 4) {
     // ---------------------------------- producer ----------------------------------
-    const unsigned row_bytes = 16u * L;
+    const unsigned row_bytes = 16u * LR;
     for (int s = 0; s < nstages; ++s) {
       const int slot = s % NS;
       if (s >= NS && !mbar_wait(&empty[slot], ((s / NS) - 1) & 1)) {
@@ -324,11 +338,11 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
         if (lane == 0) {
           mbar_arrive_expect_tx(&full[slot], (QM ? 1u : 2u) * kBK * row_bytes);
           const int y0 = img0 * H + (REV ? H - (s + 1) * kBK : s * kBK);
-          if (!QM) tma_load_2d(T, &maps.a, w0 * L, y0, &full[slot]);
-          tma_load_2d(T + kBK * 4 * L, &maps.b, w0 * L, dir * p.nimg * H + y0, &full[slot]);
+          if (!QM) tma_load_2d(T, &maps.a, w0 * LR, y0, &full[slot]);
+          tma_load_2d(T + kBK * 4 * LR, &maps.b, w0 * LR, dir * p.nimg * H + y0, &full[slot]);
         }
       } else {
-        if (lane == 0) mbar_arrive_expect_tx(&full[slot], (unsigned)nact * (unsigned)npix * (QM ? 4u : 8u) * L);
+        if (lane == 0) mbar_arrive_expect_tx(&full[slot], (unsigned)nact * (unsigned)npix * (QM ? 4u : 8u) * LR);
         __syncwarp();
         const int ncopy = nact * 2;
         for (int c = lane; c < ncopy; c += 32) {
@@ -336,8 +350,8 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
           if (QM && a == 0) continue;
           const int wlo = REV ? W - s * kBK - npix : s * kBK;
           const long long pix = (long long)(chain0 + qd) * W + wlo;
-          const float* src = (a == 0 ? p.dunary : p.dm_read + (long long)dir * p.slice) + pix * L;
-          bulk_g2s(T + (qd * 2 + a) * kBK * L, src, (unsigned)npix * 4u * L, &full[slot]);
+          const float* src = (a == 0 ? p.dunary : p.dm_read + (long long)dir * p.slice) + pix * LR;
+          bulk_g2s(T + (qd * 2 + a) * kBK * LR, src, (unsigned)npix * 4u * LR, &full[slot]);
         }
       }
     }
@@ -365,17 +379,17 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
     fix = (chain0 + wc) - img * H;
   }
   const long long ibase = (long long)img * H * W;
-  float* Cl = QM ? nullptr : p.dunary + ibase * L + lc;
-  float* Pdl = p.dm_read + (long long)dir * p.slice + ibase * L + lc;
-  float* Pil = p.dm_read + (long long)inv * p.slice + ibase * L + lc;
-  float* Ql = p.dm_acc + (long long)dir * p.slice + ibase * L + lc;   // QM: scatter field of this direction
+  float* Cl = QM ? nullptr : p.dunary + ibase * LR + lc;
+  float* Pdl = p.dm_read + (long long)dir * p.slice + ibase * LR + lc;
+  float* Pil = p.dm_read + (long long)inv * p.slice + ibase * LR + lc;
+  float* Ql = p.dm_acc + (long long)dir * p.slice + ibase * LR + lc;   // QM: scatter field of this direction
   const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
   float* DE = p.dew ? p.dew + (long long)dir * p.pslice + ibase : nullptr;
-  const uint8_t* MIl = p.min_idx + (long long)dir * p.slice + ibase * L + lc;
+  const uint8_t* MIl = p.min_idx + (long long)dir * p.slice + ibase * LR + lc;
   const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
   const float rho = p.rho;
-  const int sa = VERT ? kBK * 4 * L : kBK * L;        // C -> P_dir inside a tile
-  const int sk = (VERT ? 4 * L : L) * (REV ? -1 : 1);  // consecutive steps inside a tile
+  const int sa = VERT ? kBK * 4 * LR : kBK * LR;        // C -> P_dir inside a tile
+  const int sk = (VERT ? 4 * LR : LR) * (REV ? -1 : 1);  // consecutive steps inside a tile
   const int pstep = VERT ? (REV ? -W : W) : (REV ? -1 : 1);
   const int px0 = VERT ? (REV ? H - 1 : 0) * W + fix : fix * W + (REV ? W - 1 : 0);  // first step
   const int nsteps = len - 1;  // steps that have a predecessor pixel
@@ -397,14 +411,14 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
   };
   auto load_idx = [&](int s, int (&fi)[kBK]) {
     if ((s + 1) * kBK <= nsteps) {  // every step of the stage has a predecessor: no per-load checks
-      const uint8_t* b = MIl + (px0 + s * kBK * pstep) * L;
+      const uint8_t* b = MIl + (px0 + s * kBK * pstep) * LR;
 #pragma unroll
-      for (int u = 0; u < kBK; ++u) fi[u] = (int)b[u * pstep * L];
+      for (int u = 0; u < kBK; ++u) fi[u] = (int)b[u * pstep * LR];
     } else {
 #pragma unroll
       for (int u = 0; u < kBK; ++u) {
         const int st = s * kBK + u;
-        fi[u] = st < nsteps ? (int)MIl[(px0 + st * pstep) * L] : 0;
+        fi[u] = st < nsteps ? (int)MIl[(px0 + st * pstep) * LR] : 0;
       }
     }
   };
@@ -415,11 +429,11 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
   load_idx(0, fa);
 
   // output rows of the current pixel, moved by one pixel per step
-  const long long ostep = (long long)pstep * L;
-  float* pC = QM ? nullptr : Cl + (long long)px0 * L;
-  float* pPd = Pdl + (long long)px0 * L;
-  float* pPi = Pil + (long long)px0 * L;
-  float* pQ = Ql + (long long)px0 * L;
+  const long long ostep = (long long)pstep * LR;
+  float* pC = QM ? nullptr : Cl + (long long)px0 * LR;
+  float* pPd = Pdl + (long long)px0 * LR;
+  float* pPi = Pil + (long long)px0 * LR;
+  float* pQ = Ql + (long long)px0 * LR;
   // one step: t = tile pointer of this pixel (C at t[0], P_dir at t[sa]), k = step inside the stage
   auto step = [&](const float* t, int k, int f, float S_st, bool has_front) {
     const float cval = QM ? 0.f : t[0];
@@ -470,9 +484,9 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
     const float* T = tiles + slot * tile_floats;
     const float* t0p;
     if (VERT) {  // box rows ascend in memory; a downward walk starts at the last row of the box
-      t0p = T + wc * L + (REV ? (kBK - 1) * 4 * L : 0);
+      t0p = T + wc * LR + (REV ? (kBK - 1) * 4 * LR : 0);
     } else {
-      t0p = T + wc * 2 * kBK * L + (REV ? (npix - 1) * L : 0);
+      t0p = T + wc * 2 * kBK * LR + (REV ? (npix - 1) * LR : 0);
     }
     // normalisation sums of the stage: lane j sums (C + P_dir) over the labels of step j
     float S_st = 0.f;
@@ -528,7 +542,7 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
 }
 
 // ------------------------------------------------------------------------------------------------
-// 32 < L <= 64, L % 4 == 0: one WARP per chain, TWO labels per lane (2*lane, 2*lane + 1), schemes
+// 32 < L <= 64, rows of 16-byte multiples: one WARP per chain, TWO labels per lane (2*lane, 2*lane + 1), schemes
 // 1 (C + P) and 2 (scatter field).  No block barrier: the CTA-per-chain kernel pays two per step
 // plus a cross-warp reduction.  The stored gradients are staged kPB steps per stage by the warp
 // itself (lane-parallel cp.async.bulk copies: one per array and stage for horizontal chains, one
@@ -538,9 +552,9 @@ constexpr int kPB = 16;   // steps per stage (and per block of per-pixel scalars
 constexpr int kPNS = 2;   // stages in flight
 
 // floats of shared memory per warp (the CTA adds one [L][L|1] context table)
-__host__ __device__ inline int bwd_pair_floats(int L, int rank, int sch) {
+__host__ __device__ inline int bwd_pair_floats(int L, int ls, int rank, int sch) {
   const int tab = rank == 2 ? L * (L | 1) : 64;
-  return kPNS * (sch == 1 ? 2 : 1) * kPB * L + kPNS * kPB * L / 4 + kPB * 33 + 256 + ((tab + 3) & ~3) + 2 * kPNS + 2;
+  return kPNS * (sch == 1 ? 2 : 1) * kPB * ls + kPNS * kPB * ls / 4 + kPB * 33 + 256 + ((tab + 3) & ~3) + 2 * kPNS + 2;
 }
 
 // q0 / q1: scatter sums of labels me0, me0 + 1 over the 64 (padded) labels of one pixel.
@@ -562,7 +576,7 @@ __device__ __forceinline__ void gather_q2(const float* tb, const float* ib, int 
 #pragma unroll
     for (int v = 0; v < 16; ++v) body(v);
   } else {
-    const int nv = L >> 2;
+    const int nv = (L + 3) >> 2;  // entries beyond L hold t = 0 and an index that matches nothing
 #pragma unroll 3
     for (int v = 0; v < nv; ++v) body(v);
   }
@@ -580,16 +594,16 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
   constexpr int NA = CP ? 2 : 1;  // staged arrays: (C, P_dir) or the gradient slice of the direction
   extern __shared__ __align__(128) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = FULL ? 64 : p.L, LS = L | 1;
+  const int L = FULL ? 64 : p.L, LR = FULL ? 64 : p.ls, LS = L | 1;
   const int ctab_floats = (L * LS + 3) & ~3;
   float* ctab = smem;                              // [L][LS] full context table of the CTA
   for (int i = threadIdx.x; i < L * L; i += blockDim.x)
     ctab[(i / L) * LS + (i % L)] = ctx_value(p.ctx, p.ctx_rank, L, i / L, i % L);
-  const int per_warp = (bwd_pair_floats(L, p.ctx_rank, SCH) + 3) & ~3;
+  const int per_warp = (bwd_pair_floats(L, LR, p.ctx_rank, SCH) + 3) & ~3;
   float* ring = smem + ctab_floats + warp * per_warp;  // [kPNS][NA][kPB][L]
-  const int stage_floats = NA * kPB * L;
+  const int stage_floats = NA * kPB * LR;
   uint8_t* itile = reinterpret_cast<uint8_t*>(ring + kPNS * stage_floats);  // [kPNS][kPB][L] argmin indices
-  float* dtile = ring + kPNS * stage_floats + kPNS * kPB * L / 4;           // [kPB][33]
+  float* dtile = ring + kPNS * stage_floats + kPNS * kPB * LR / 4;           // [kPB][33]
   float* ts = dtile + kPB * 33;                    // [2][64]  (kPB * 33 is a multiple of 4)
   float* is = ts + 128;                            // [2][64] argmin as float
   float* acc = is + 128;                           // context-gradient table of this chain
@@ -607,17 +621,17 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
   if (!decode_bchain(p, g, ch)) return;
   const int dir = ch.dir, inv = dir ^ 1;
   const int c0 = 2 * lane;
-  const bool act = c0 < L;  // L is even: a lane owns two labels or none
+  const bool act = c0 < L, act1 = FULL || c0 + 1 < L;  // a lane owns two labels, one (the last of an odd L) or none
 
   const long long ibase = (long long)ch.img * p.H * p.W;
-  float* DMr = p.dm_read + (long long)dir * p.slice + ibase * L;  // dM_dir, or P_dir
-  float* DMa = p.dm_acc + ibase * L;
-  float* DU = p.dunary + ibase * L;                               // dU, or C
+  float* DMr = p.dm_read + (long long)dir * p.slice + ibase * LR;  // dM_dir, or P_dir
+  float* DMa = p.dm_acc + ibase * LR;
+  float* DU = p.dunary + ibase * LR;                               // dU, or C
   const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
   float* DE = p.dew ? p.dew + (long long)dir * p.pslice + ibase : nullptr;
-  const uint8_t* MI = p.min_idx + (long long)dir * p.slice + ibase * L;
+  const uint8_t* MI = p.min_idx + (long long)dir * p.slice + ibase * LR;
   const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
-  const int len = ch.len, pstep = ch.pstep, ostep = pstep * L;
+  const int len = ch.len, pstep = ch.pstep, ostep = pstep * LR;
   const int pixl = ch.h0 * p.W + ch.w0 + (len - 1) * pstep;  // last pixel of the chain
   const float rho = p.rho;
   const int nsteps = len - 1;               // steps with a predecessor pixel
@@ -639,31 +653,31 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
       float* T = ring + slot * stage_floats;
       if (lane == 0) {
         fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&full[slot], (unsigned)(rows * NA * L) * 4u);
+        mbar_arrive_expect_tx(&full[slot], (unsigned)(rows * NA * LR) * 4u);
       }
       __syncwarp();
       if (contiguous) {
         const int first = pstep == 1 ? pixl - (s0 + rows - 1) : pixl + s0;
         if (lane < NA)
-          bulk_g2s(T + lane * kPB * L, (CP && lane == 0 ? DU : DMr) + (long long)first * L,
-                   (unsigned)(rows * L) * 4u, &full[slot]);
+          bulk_g2s(T + lane * kPB * LR, (CP && lane == 0 ? DU : DMr) + (long long)first * LR,
+                   (unsigned)(rows * LR) * 4u, &full[slot]);
       } else {
         for (int q = lane; q < rows * NA; q += 32) {
           const int u = q / NA, a = q - u * NA;
           const int px = pixl - (s0 + u) * pstep;
-          bulk_g2s(T + (a * kPB + u) * L, (CP && a == 0 ? DU : DMr) + (long long)px * L, (unsigned)L * 4u,
+          bulk_g2s(T + (a * kPB + u) * LR, (CP && a == 0 ? DU : DMr) + (long long)px * LR, (unsigned)LR * 4u,
                    &full[slot]);
         }
       }
     }
     // argmin indices of the steps with a predecessor: four labels per lane and step
-    if (4 * lane < L) {
-      uint8_t* dst = itile + (slot * kPB) * L + 4 * lane;
-      const uint8_t* src = MI + (long long)(pixl - s0 * pstep) * L + 4 * lane;
+    if (4 * lane < LR) {
+      uint8_t* dst = itile + (slot * kPB) * LR + 4 * lane;
+      const uint8_t* src = MI + (long long)(pixl - s0 * pstep) * LR + 4 * lane;
 #pragma unroll 4
       for (int u = 0; u < kPB; ++u) {
         if (s0 + u < nsteps)
-          cp_async4(reinterpret_cast<float*>(dst + u * L), reinterpret_cast<const float*>(src - (long long)u * ostep));
+          cp_async4(reinterpret_cast<float*>(dst + u * LR), reinterpret_cast<const float*>(src - (long long)u * ostep));
       }
     }
     cp_async_commit();
@@ -686,15 +700,15 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
 
   float q0 = 0.f, q1 = 0.f;  // scatter sums carried from the successor pixel (labels c0, c0 + 1)
   // output rows of the current pixel (labels c0, c0 + 1), moved by one pixel per step
-  float* pA = (CP ? DU : DMa + (long long)dir * p.slice) + (long long)pixl * L + c0;  // C, or the scatter field
-  float* pB = DMr + (long long)pixl * L + c0;                                         // P_dir
-  float* pI = DMa + (long long)inv * p.slice + (long long)pixl * L + c0;              // P_inv
+  float* pA = (CP ? DU : DMa + (long long)dir * p.slice) + (long long)pixl * LR + c0;  // C, or the scatter field
+  float* pB = DMr + (long long)pixl * LR + c0;                                         // P_dir
+  float* pI = DMa + (long long)inv * p.slice + (long long)pixl * LR + c0;              // P_inv
   for (int b = 0; b < nblocks; ++b) {
     load_blk(b + 1, e_nxt, n_nxt);
     const int rows = stage_rows(b);
     const int slot = b % kPNS;
     const float* T = ring + slot * stage_floats;
-    const uint8_t* IT = itile + (slot * kPB) * L + c0;
+    const uint8_t* IT = itile + (slot * kPB) * LR + c0;
     cp_async_wait<kPNS - 1>();
     if (rows > 0 && !mbar_wait(&full[slot], (b / kPNS) & 1)) {
       if (lane == 0) atomicExch(p.status, 141);
@@ -707,34 +721,36 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
     {
       const int u = lane & (kPB - 1), half = lane >> 4;
       if (u < rows) {
-        const int hl = L >> 1;  // even halves (L % 4 == 0)
-        const float* row = T + (flip ? rows - 1 - u : u) * L + half * hl;
+        const int hl = ((L + 3) >> 2) << 1;  // even first half; the second one ends at the last label
+        const int hn = FULL ? 32 : (half ? L - hl : hl);
+        const float* row = T + (flip ? rows - 1 - u : u) * LR + half * hl;
         float sa = 0.f, sb = 0.f;
-        int c = lane >= hl ? lane - hl : lane;  // rotated start: lanes hit distinct banks
+        int c = lane >= hn ? lane - hn : lane;  // rotated start: lanes hit distinct banks
 #pragma unroll 4
-        for (int i = 0; i < hl; i += 2) {
-          sa += CP ? row[c] + row[c + kPB * L] : row[c];
-          c = c + 1 >= hl ? 0 : c + 1;
-          sb += CP ? row[c] + row[c + kPB * L] : row[c];
-          c = c + 1 >= hl ? 0 : c + 1;
+        for (int i = 0; i + 1 < hn; i += 2) {
+          sa += CP ? row[c] + row[c + kPB * LR] : row[c];
+          c = c + 1 >= hn ? 0 : c + 1;
+          sb += CP ? row[c] + row[c + kPB * LR] : row[c];
+          c = c + 1 >= hn ? 0 : c + 1;
         }
+        if (!FULL && (hn & 1)) sa += CP ? row[c] + row[c + kPB * LR] : row[c];
         s_cur = sa + sb;
       }
       s_cur += __shfl_xor_sync(0xffffffffu, s_cur, 16);
     }
     const int send = len - kPB * b < kPB ? len - kPB * b : kPB;
-    const float* row = T + (flip ? rows - 1 : 0) * L + c0;
-    const int rstep = flip ? -L : L;
+    const float* row = T + (flip ? rows - 1 : 0) * LR + c0;
+    const int rstep = flip ? -LR : LR;
     const uint8_t* irow = IT;
     float* drow = dtile + lane;
-    for (int sl = 0; sl < send; ++sl, row += rstep, irow += L, drow += 33, pA -= ostep, pB -= ostep, pI -= ostep) {
+    for (int sl = 0; sl < send; ++sl, row += rstep, irow += LR, drow += 33, pA -= ostep, pB -= ostep, pI -= ostep) {
       const int s = kPB * b + sl;
       const float rq0 = rho * q0, rq1 = rho * q1;
       float qn0 = 0.f, qn1 = 0.f;
       float2 x0 = make_float2(0.f, 0.f), x1 = make_float2(0.f, 0.f);
       if (act && sl < rows) {
         x0 = *reinterpret_cast<const float2*>(row);
-        if (CP) x1 = *reinterpret_cast<const float2*>(row + kPB * L);
+        if (CP) x1 = *reinterpret_cast<const float2*>(row + kPB * LR);
       }
       if (s < nsteps) {
         const float e = __shfl_sync(0xffffffffu, e_cur, sl);
@@ -743,25 +759,26 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
         float t0 = 0.f, t1 = 0.f, cv0 = 0.f, cv1 = 0.f;
         if (act) {
           const uchar2 fi = *reinterpret_cast<const uchar2*>(irow);
-          const int f0 = fi.x, f1 = fi.y;
+          const int f0 = fi.x, f1 = act1 ? fi.y : 0;
           t0 = x0.x + x1.x + rq0;
           t1 = x0.y + x1.y + rq1;
           t0 = (c0 == n) ? t0 - S : t0;  // MPLayers/commonCUDA.cuh:131-145
           t1 = (c0 + 1 == n) ? t1 - S : t1;
+          if (!act1) t1 = 0.f;
           cv0 = ctab[c0 * LS + f0];
-          cv1 = ctab[(c0 + 1) * LS + f1];
+          if (act1) cv1 = ctab[(c0 + 1) * LS + f1];
           if (p.ctx_rank == 2) {
             // the diagonal is accumulated like every other cell and dropped at the flush unless wanted
             acc[c0 * LS + f0] = fmaf(e, t0, acc[c0 * LS + f0]);
-            acc[(c0 + 1) * LS + f1] = fmaf(e, t1, acc[(c0 + 1) * LS + f1]);
+            if (act1) acc[(c0 + 1) * LS + f1] = fmaf(e, t1, acc[(c0 + 1) * LS + f1]);
           } else {
             if (c0 != f0 || p.keep_diag) atomicAdd(acc + (c0 > f0 ? c0 - f0 : f0 - c0), e * t0);
-            if (c0 + 1 != f1 || p.keep_diag) atomicAdd(acc + (c0 + 1 > f1 ? c0 + 1 - f1 : f1 - c0 - 1), e * t1);
+            if (act1 && (c0 + 1 != f1 || p.keep_diag)) atomicAdd(acc + (c0 + 1 > f1 ? c0 + 1 - f1 : f1 - c0 - 1), e * t1);
           }
           float* tb = ts + (s & 1) * 64;
           float* ib = is + (s & 1) * 64;
           *reinterpret_cast<float2*>(tb + c0) = make_float2(t0, t1);
-          *reinterpret_cast<float2*>(ib + c0) = make_float2((float)f0, (float)f1);
+          *reinterpret_cast<float2*>(ib + c0) = make_float2((float)f0, act1 ? (float)f1 : -1.f);
         }
         *drow = fmaf(cv0, t0, cv1 * t1);
         __syncwarp();
@@ -1048,7 +1065,7 @@ __global__ void __launch_bounds__(256) bwd_cta_kernel(const __grid_constant__ Bw
   extern __shared__ __align__(16) float smem[];
   BChain ch;
   if (!decode_bchain(p, blockIdx.x, ch)) return;  // uniform
-  const int L = p.L, D = p.D, dir = ch.dir, inv = dir ^ 1, NT = blockDim.x, c = threadIdx.x;
+  const int L = p.L, LR = p.ls, D = p.D, dir = ch.dir, inv = dir ^ 1, NT = blockDim.x, c = threadIdx.x;
   const int nw = NT >> 5, lane = c & 31, warp = c >> 5;
   const bool qmode = p.cp_scheme == 2;
   const int LS = L | 1;
@@ -1065,12 +1082,12 @@ __global__ void __launch_bounds__(256) bwd_cta_kernel(const __grid_constant__ Bw
   __syncthreads();
 
   const long long ibase = (long long)ch.img * p.H * p.W;
-  float* DMr = p.dm_read + (long long)dir * p.slice + ibase * L;
-  float* DMa = p.dm_acc + ibase * L;
-  float* DU = p.dunary + ibase * L;
+  float* DMr = p.dm_read + (long long)dir * p.slice + ibase * LR;
+  float* DMa = p.dm_acc + ibase * LR;
+  float* DU = p.dunary + ibase * LR;
   const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
   float* DE = p.dew ? p.dew + (long long)dir * p.pslice + ibase : nullptr;
-  const uint8_t* MI = p.min_idx + (long long)dir * p.slice + ibase * L;
+  const uint8_t* MI = p.min_idx + (long long)dir * p.slice + ibase * LR;
   const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
   const int len = ch.len;
   const int pixl = ch.h0 * p.W + ch.w0 + (len - 1) * ch.pstep;
@@ -1079,11 +1096,11 @@ __global__ void __launch_bounds__(256) bwd_cta_kernel(const __grid_constant__ Bw
 
   auto issue = [&](int s) {
     if (s < len - 1 && act)
-      cp_async4(ring + (s & (kPFB - 1)) * NT + c, DMr + (long long)(pixl - s * ch.pstep) * L + c);
+      cp_async4(ring + (s & (kPFB - 1)) * NT + c, DMr + (long long)(pixl - s * ch.pstep) * LR + c);
     cp_async_commit();
   };
   auto load_idx = [&](int s) -> int {
-    return (s < len - 1 && act) ? (int)MI[(long long)(pixl - s * ch.pstep) * L + c] : -1;
+    return (s < len - 1 && act) ? (int)MI[(long long)(pixl - s * ch.pstep) * LR + c] : -1;
   };
   auto load_blk = [&](int b, float& eb, int& nb) {
     const int s = 32 * b + lane;
@@ -1113,7 +1130,7 @@ __global__ void __launch_bounds__(256) bwd_cta_kernel(const __grid_constant__ Bw
     }
     cp_async_wait<kPFB - 1>();
     const int px = pixl - s * ch.pstep;
-    const long long o = (long long)px * L + c;
+    const long long o = (long long)px * LR + c;
     const bool has_front = s < len - 1;
     const float rq = rho * q;
     float qn = 0.f;
@@ -1209,7 +1226,7 @@ __global__ void backward_init_kernel(const float* __restrict__ g, float* __restr
 // The same prologue reading g with the labels first ([nimg, L, H*W] planes): one block per 32 pixels
 // of an image, through a shared-memory tile.
 __global__ void __launch_bounds__(256)
-backward_init_lhw_kernel(const float* __restrict__ g, float* __restrict__ dunary, float* __restrict__ dm, int L,
+backward_init_lhw_kernel(const float* __restrict__ g, float* __restrict__ dunary, float* __restrict__ dm, int L, int ls,
                          long long HW, long long n, int D, float factor, int cp) {
   extern __shared__ float tile[];  // [L][33]
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -1218,10 +1235,10 @@ backward_init_lhw_kernel(const float* __restrict__ g, float* __restrict__ dunary
   const float* src = g + b * L * HW + p0;
   for (int l = ty; l < L; l += 8) tile[l * 33 + tx] = tx < np ? src[(long long)l * HW + tx] : 0.f;
   __syncthreads();
-  const long long base = (b * HW + p0) * L;
-  for (int i = threadIdx.x; i < np * L; i += 256) {
-    const int px = i / L, l = i - px * L;
-    const float v = tile[l * 33 + px];
+  const long long base = (b * HW + p0) * ls;
+  for (int i = threadIdx.x; i < np * ls; i += 256) {
+    const int px = i / ls, l = i - px * ls;
+    const float v = l < L ? tile[l * 33 + px] : 0.f;
     dunary[base + i] = cp ? v : factor * v;
     for (int k = 0; k < D; ++k) dm[k * n + base + i] = cp ? 0.f : v;
   }
@@ -1313,38 +1330,38 @@ __global__ void dctx_reduce2_kernel(const float* __restrict__ part, int n_slots,
 
 constexpr int kSmemTableMaxL = 128;  // rank-2 table L*(L|1) floats fits next to the staging ring
 
-size_t bwd_tma_smem_bytes(int L, int rank, int stages) {
-  return ((size_t)stages * 2 * kBK * 4 * L + ((L * (L | 1) + 3) & ~3) + 4 * (size_t)bwd_tma_warp_floats(L, rank)) *
+size_t bwd_tma_smem_bytes(int L, int ls, int rank, int stages) {
+  return ((size_t)stages * 2 * kBK * 4 * ls + ((L * (L | 1) + 3) & ~3) + 4 * (size_t)bwd_tma_warp_floats(L, rank)) *
              sizeof(float) +
          2 * stages * 8 + 16 + 128;
 }
 
 bool bwd_tma_eligible(const BwdParams& p) {
   if (p.cp_scheme == 0 || p.dir > 3 || p.L > 32 || p.ndirs > 1) return false;
-  if ((p.W & 3) || (((long long)p.W * p.L) & 3)) return false;
+  if (p.W & 3) return false;
   if (((uintptr_t)(p.cp_scheme == 1 ? p.dunary : nullptr) | (uintptr_t)p.dm_read) & 15) return false;
   return true;
 }
 
 bool bwd_pair_eligible(const BwdParams& p) {
-  if (p.L <= 32 || p.L > 64 || (p.L & 3) || p.cp_scheme == 0) return false;
+  if (p.L <= 32 || p.L > 64 || (p.ls & 3) || p.cp_scheme == 0) return false;
   if (((uintptr_t)p.dunary | (uintptr_t)p.dm_read | (uintptr_t)p.dm_acc) & 15) return false;
   const char* e = getenv("MPL_NO_PAIR");  // tuning / comparison knob
   return !(e && e[0] == '1');
 }
 
-template <int LT>
+template <int LT, bool PAD>
 cudaError_t launch_bwd_tma(const BwdParams& p, cudaStream_t st) {
   const bool vert = p.dir >= 2;
   const bool rev = (p.dir & 1) == 0;  // forward walk upwards -> backward walk downwards
   const int groups = vert ? p.nimg * (p.W >> 2) : (p.nimg * p.H + 3) >> 2;
-  const size_t smem = bwd_tma_smem_bytes(p.L, p.ctx_rank, p.tma_stages);
+  const size_t smem = bwd_tma_smem_bytes(p.L, p.ls, p.ctx_rank, p.tma_stages);
   TmaMaps maps{};
   const bool qm = p.cp_scheme == 2;
   if (vert) {
-    const unsigned long long inner = (unsigned long long)p.W * p.L, rows = (unsigned long long)p.nimg * p.H;
-    if ((!qm && !encode_tmap_2d(&maps.a, p.dunary, inner, rows, 4 * p.L, kBK)) ||
-        !encode_tmap_2d(&maps.b, p.dm_read, inner, rows * p.D, 4 * p.L, kBK))
+    const unsigned long long inner = (unsigned long long)p.W * p.ls, rows = (unsigned long long)p.nimg * p.H;
+    if ((!qm && !encode_tmap_2d(&maps.a, p.dunary, inner, rows, 4 * p.ls, kBK)) ||
+        !encode_tmap_2d(&maps.b, p.dm_read, inner, rows * p.D, 4 * p.ls, kBK))
       return cudaErrorNotSupported;
   }
   auto go = [&](auto kernel) -> cudaError_t {
@@ -1356,11 +1373,11 @@ cudaError_t launch_bwd_tma(const BwdParams& p, cudaStream_t st) {
     return cudaSuccess;
   };
   if (qm) {
-    if (vert) return rev ? go(bwd_tma_kernel<LT, true, true, true>) : go(bwd_tma_kernel<LT, true, false, true>);
-    return rev ? go(bwd_tma_kernel<LT, false, true, true>) : go(bwd_tma_kernel<LT, false, false, true>);
+    if (vert) return rev ? go(bwd_tma_kernel<LT, PAD, true, true, true>) : go(bwd_tma_kernel<LT, PAD, true, false, true>);
+    return rev ? go(bwd_tma_kernel<LT, PAD, false, true, true>) : go(bwd_tma_kernel<LT, PAD, false, false, true>);
   }
-  if (vert) return rev ? go(bwd_tma_kernel<LT, true, true>) : go(bwd_tma_kernel<LT, true, false>);
-  return rev ? go(bwd_tma_kernel<LT, false, true>) : go(bwd_tma_kernel<LT, false, false>);
+  if (vert) return rev ? go(bwd_tma_kernel<LT, PAD, true, true>) : go(bwd_tma_kernel<LT, PAD, true, false>);
+  return rev ? go(bwd_tma_kernel<LT, PAD, false, true>) : go(bwd_tma_kernel<LT, PAD, false, false>);
 }
 
 }  // namespace
@@ -1424,12 +1441,12 @@ cudaError_t launch_backward_init(const float* dcost, float* dunary, float* dm, l
   return cudaGetLastError();
 }
 
-cudaError_t launch_backward_init_lhw(const float* dcost, float* dunary, float* dm, int nimg, int L, long long HW,
+cudaError_t launch_backward_init_lhw(const float* dcost, float* dunary, float* dm, int nimg, int L, int ls, long long HW,
                                      int D, float factor, int cp_scheme, cudaStream_t st) {
   const dim3 grid((unsigned)((HW + 31) / 32), (unsigned)nimg);
   const size_t smem = (size_t)L * 33 * sizeof(float);
   ProfScope prof(kProfElementwise, st);
-  backward_init_lhw_kernel<<<grid, 256, smem, st>>>(dcost, dunary, dm, L, HW, (long long)nimg * HW * L, D, factor,
+  backward_init_lhw_kernel<<<grid, 256, smem, st>>>(dcost, dunary, dm, L, ls, HW, (long long)nimg * HW * ls, D, factor,
                                                     cp_scheme);
   count_launch();
   return cudaGetLastError();
@@ -1470,7 +1487,9 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
   ProfScope prof(kProfBwdSweep, st);
   if (L <= 32 && p.parts <= 1 && bwd_tma_eligible(p)) {
     p.tma_stages = tma_stage_override() ? tma_stage_override() : 4;
-    cudaError_t e = L == 21 ? launch_bwd_tma<21>(p, st) : launch_bwd_tma<0>(p, st);
+    cudaError_t e = L == 21 && p.ls == 21   ? launch_bwd_tma<21, false>(p, st)
+                    : L == 21 && p.ls == 24 ? launch_bwd_tma<21, true>(p, st)
+                                            : launch_bwd_tma<0, false>(p, st);
     if (e != cudaSuccess) return e;
   } else if (L <= 32) {
     const int wpb = total >= 148 * 32 ? 4 : 1;
@@ -1484,21 +1503,23 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
       kernel<<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
       return cudaSuccess;
     };
-    cudaError_t e;
-    if (p.cp_scheme == 1) {
-      e = go(bwd_warp_kernel<0, 1>);
-    } else if (p.cp_scheme == 2) {
-      e = go(bwd_warp_kernel<0, 2>);
-    } else {
-      e = p.D == 4 ? go(bwd_warp_kernel<4, 0>) : p.D == 8 ? go(bwd_warp_kernel<8, 0>) : go(bwd_warp_kernel<0, 0>);
-    }
+    // rows of 16-byte multiples at 16-byte aligned bases: staged in 16-byte pieces
+    const bool v4 = (p.ls & 3) == 0 && (((uintptr_t)(p.cp_scheme == 1 ? p.dunary : nullptr) | (uintptr_t)p.dm_read) & 15) == 0;
+    auto pick = [&](auto lmax) -> cudaError_t {
+      constexpr int LM = decltype(lmax)::value;
+      if (p.cp_scheme == 1) return v4 ? go(bwd_warp_kernel<LM, 1, true>) : go(bwd_warp_kernel<LM, 1, false>);
+      return v4 ? go(bwd_warp_kernel<LM, 2, true>) : go(bwd_warp_kernel<LM, 2, false>);
+    };
+    const cudaError_t e = L <= 16   ? pick(std::integral_constant<int, 16>{})
+                          : L <= 21 ? pick(std::integral_constant<int, 21>{})
+                                    : pick(std::integral_constant<int, 32>{});
     if (e != cudaSuccess) return e;
-  } else if (bwd_wide_eligible(L, p.ctx_rank, p.cp_scheme, p.dunary, p.dm_read, p.dm_acc)) {
+  } else if (bwd_wide_eligible(L, p.ls, p.ctx_rank, p.cp_scheme, p.dunary, p.dm_read, p.dm_acc)) {
     // rank-1 context, 32 < L <= 256: several labels per lane, scatter split into near and far indices
     cudaError_t e = launch_backward_wide(p, total, st);
     if (e != cudaSuccess) return e;
   } else if (bwd_pair_eligible(p)) {
-    const size_t per_warp = (size_t)((bwd_pair_floats(L, p.ctx_rank, p.cp_scheme) + 3) & ~3) * sizeof(float);
+    const size_t per_warp = (size_t)((bwd_pair_floats(L, p.ls, p.ctx_rank, p.cp_scheme) + 3) & ~3) * sizeof(float);
     const size_t table = (size_t)((L * LS + 3) & ~3) * sizeof(float);
     int wpb = (int)((227 * 1024 - table) / per_warp);
     wpb = wpb > 8 ? 8 : wpb;

@@ -87,6 +87,7 @@ struct CtxInfo {
   int R;          // first offset at which ctx has reached its final value
   float cmax;     // ctx[L-1]
   int ew_min_bits;  // order-preserving int image of min(edge weight)
+  int zero_min;     // 1: no value of ctx is below ctx[0]
 };
 
 struct FwdParams {
@@ -101,7 +102,8 @@ struct FwdParams {
   const CtxInfo* info;
   int* status;            // device word: 0 = ok, else the code of a wait that gave up
   int H, W, L, D, nimg;
-  long long slice;        // nimg*H*W*L
+  int ls;                 // floats from one pixel's labels to the next (>= L; argmin indices: bytes)
+  long long slice;        // nimg*H*W*ls
   long long pslice;       // nimg*H*W
   float rho;
   int ctx_rank;
@@ -113,6 +115,10 @@ struct FwdParams {
   // stages A, M_dir and M_inv only: UU = (A - M_dir) * rho - M_inv, bit-identical to the
   // reference's ((U + M_0 + ... + M_{D-1}) - M_dir) * rho - M_inv.
   int agg;
+  // first != 0: the messages this launch reads are zero, except -- in a TRWP iteration -- the slices
+  // below `dir0`, which earlier sweeps of the iteration have written.  Only where
+  // forward_skips_zero_slices() says so; other launches read slices that hold zeros.
+  int first;
   int host_windowed;      // host copy of the context analysis (rank-1, L > 32): windowed path is exact
   int host_R;             //   ... and its window half-width
   int dir0, ndirs;        // this launch covers directions dir0 .. dir0+ndirs-1
@@ -135,6 +141,7 @@ struct BwdParams {
   float* dctx_part;       // [n_slots, ctx_table] partial tables
   int n_slots;
   int H, W, L, D, nimg;
+  int ls;                 // floats from one pixel's labels to the next (>= L; argmin indices: bytes)
   long long slice, pslice;
   float rho;
   int ctx_rank, keep_diag;
@@ -199,6 +206,11 @@ __device__ __forceinline__ float warp_sum(float v) {
 __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem_src) : "memory");
+}
+// dst, src 16-byte aligned
+__device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_src) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -301,21 +313,31 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
 cudaError_t launch_analyze(const float* ctx, int L, int rank, const float* ew, long long n_ew,
                            CtxInfo* info, cudaStream_t st);
 cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st);
+// mp_fwd_tma.cu
+bool forward_tma_eligible(const FwdParams& p, int dir, int* stages);
+cudaError_t launch_forward_tma(const FwdParams& p, int dir, int stages, bool train, cudaStream_t st);
+// Does a sweep described by p run without reading message slices that are known to be zero
+// (FwdParams::first)?  Those it would read otherwise have to hold zeros.
+bool forward_skips_zero_slices(const FwdParams& p, bool train);
+// Zeroes the rows of the chains' first pixels in the D slices of `a` and (if not null) `b`: they have no
+// predecessor, so no sweep writes them.  p describes all directions.
+cudaError_t launch_zero_chain_starts(const FwdParams& p, float* a, float* b, cudaStream_t st);
 cudaError_t launch_forward_wide(const FwdParams& p, bool train, cudaStream_t st);  // mp_wide.cu
+// ls: floats per pixel row of unary / msg / cost (>= L)
 cudaError_t launch_aggregate(const float* unary, const float* msg, float* cost, uint8_t* label,
-                             long long npix, int L, int D, long long slice, float factor,
+                             long long npix, int L, int ls, int D, long long slice, float factor,
                              int min_a_dir, cudaStream_t st);
 cudaError_t launch_backward_init(const float* dcost, float* dunary, float* dm, long long n, int D,
                                  float factor, int cp_scheme, cudaStream_t st);
 // labels-first variants (mpl_problem::cost_labels_first): cost / dcost as [nimg, L, H*W] planes
-cudaError_t launch_aggregate_lhw(const float* unary, const float* msg, float* cost, int nimg, int L,
+cudaError_t launch_aggregate_lhw(const float* unary, const float* msg, float* cost, int nimg, int L, int ls,
                                  long long HW, int D, long long slice, float factor, int min_a_dir,
                                  cudaStream_t st);
-cudaError_t launch_backward_init_lhw(const float* dcost, float* dunary, float* dm, int nimg, int L, long long HW,
+cudaError_t launch_backward_init_lhw(const float* dcost, float* dunary, float* dm, int nimg, int L, int ls, long long HW,
                                      int D, float factor, int cp_scheme, cudaStream_t st);
 cudaError_t launch_backward_sweep(const BwdParams& p, cudaStream_t st);
 // mp_wide_bwd.cu: rank-1 context, 32 < L <= 256, L % 4 == 0, schemes 1 and 2
-bool bwd_wide_eligible(int L, int ctx_rank, int cp_scheme, const void* dunary, const void* dm_read,
+bool bwd_wide_eligible(int L, int ls, int ctx_rank, int cp_scheme, const void* dunary, const void* dm_read,
                        const void* dm_acc);
 cudaError_t launch_backward_wide(const BwdParams& p, int total, cudaStream_t st);
 cudaError_t launch_isgmr_combine_total(const float* q_total, const float* q, float* dm, float* dunary, long long n,
@@ -339,7 +361,8 @@ cudaError_t launch_smoothness_context(int L, int method, float smax, float* out,
 bool edge_weights_reduces(int mode);
 cudaError_t launch_edge_weights(const float* img, int B, int C, int H, int W, int D, int mode, float sigma,
                                 float threshold, float penalty, float* out, double* sums, cudaStream_t st);
-cudaError_t launch_layout(int kind, const float* in, float* out, uint8_t* amax, int B, int L, long long HW,
+// ls: floats per pixel row on the labels-last side (>= L)
+cudaError_t launch_layout(int kind, const float* in, float* out, uint8_t* amax, int B, int L, int ls, long long HW,
                           cudaStream_t st);
 cudaError_t launch_energy(const float* unary, const float* ctx, const float* ew, const uint8_t* label,
                           long long npix, int H, int W, int L, int D, int rank, double* part, double* out,

@@ -88,18 +88,25 @@ __device__ __forceinline__ float soft_regrow(const float* hb, const float (&cr)[
 // Generic kernel: any direction, any alignment.  Inputs are staged through a ring of 4-byte
 // cp.async copies kPF pixels ahead (a register ring of plain loads was measured slower: waiting on
 // a register load drains every younger load too, whereas cp.async groups retire in order).
-// DT = compile-time direction count (0: read it from the params).
+// DT = compile-time number of staged message slices (0: read it from the params; 2: aggregate mode,
+// FwdParams::agg, slices M_dir and M_inv).
+// V4: pixel rows are multiples of 16 bytes at 16-byte aligned bases.  The rows of a pixel's unary
+// and messages are then copied in 16-byte pieces, lane q piece q of their concatenation: one
+// copy instruction for 21 labels and four directions (30 pieces) where the 4-byte form, which also
+// serves unaligned rows, needs one per row and keeps every lane's address arithmetic in the step.
 // SOFT: the soft (expected-value) message instead of the minimum; in training it saves the L x L
 // edge values of every pixel (entry [f][c] for even directions, [c][f] for odd ones, as the
 // reference does, MPLayers/TRWP_hard_soft/TRWP_forward_soft.cu:50-59) and no argmin indices.
 // EXACT: the label count equals LMAX (lets the compiler drop every "f < L" test; used by the soft path).
-template <int LMAX, int DT, bool TRAIN, bool SOFT = false, bool EXACT = false>
+template <int LMAX, int DT, bool TRAIN, bool V4 = false, bool SOFT = false, bool EXACT = false>
 __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
   if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
-  const int L = EXACT ? LMAX : p.L, D = p.agg ? 2 : (DT ? DT : p.D), rows = D + 2;  // D = staged message slices
+  constexpr bool AGG = DT == 2;
+  const int L = EXACT ? LMAX : p.L, LR = SOFT ? L : p.ls;
+  const int D = DT ? DT : p.D, rows = D + 2;  // D = staged message slices
   const int slot_floats = rows * 32;
   float* ring = smem + warp * (kPF * slot_floats + 64 + (SOFT ? 32 * 33 : 0));
   float* hbuf = ring + kPF * slot_floats;
@@ -112,14 +119,20 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
 #pragma unroll
   for (int f = 0; f < LMAX; ++f) cr[f] = (act && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, lane, f) : 0.f;
 
+  float colmin = kInf, colmax = -kInf;  // smallest and largest entry of the lane's column (= its row) of the context
+#pragma unroll
+  for (int f = 0; f < LMAX; ++f) {
+    if (f < L) colmin = fminf(colmin, cr[f]), colmax = fmaxf(colmax, cr[f]);
+  }
+
   const long long ibase = (long long)ch.img * p.H * p.W;
   // per-lane base pointers; everything below addresses them with 32-bit element offsets
-  const float* Ul = p.unary + ibase * L + lc;
-  const float* Ml = p.msg_read + ibase * L + lc;
-  float* Mwl = p.msg_write + (long long)ch.dir * p.slice + ibase * L + lc;
+  const float* Ul = p.unary + ibase * LR + lc;
+  const float* Ml = p.msg_read + ibase * LR + lc;
+  float* Mwl = p.msg_write + (long long)ch.dir * p.slice + ibase * LR + lc;
   const bool has_e = p.ew != nullptr;
   const float* E = has_e ? p.ew + (long long)ch.dir * p.pslice + ibase : p.unary;
-  uint8_t* MIl = (TRAIN && !SOFT) ? p.min_idx + (long long)ch.dir * p.slice + ibase * L + lc : nullptr;
+  uint8_t* MIl = (TRAIN && !SOFT) ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR + lc : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
   float* EL = (TRAIN && SOFT) ? p.edge_label + ((long long)ch.dir * p.pslice + ibase) * L * L : nullptr;
   const bool l2r = (ch.dir & 1) == 0;  // layout of the saved edge values
@@ -132,28 +145,54 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
     toff[k] = c * 33 + (i - c * L);
   }
   const int len = ch.len;
-  const int ostep = ch.pstep * L;
-  const int dir_row = (1 + ch.dir) * 32, inv_row = (1 + ch.inv) * 32;
+  const int ostep = ch.pstep * LR;
+  const int dir_row = AGG ? 32 : (1 + ch.dir) * 32, inv_row = AGG ? 64 : (1 + ch.inv) * 32;
 
   // Staging of chain pixel j (its unary and D messages, used when it is the predecessor, and its
   // edge weight, used when it is the current pixel).  Pixels past the chain end are replaced by
   // the last pixel (the copies land in slots nobody reads), which keeps the loop branch-free.
   const int px_last = ch.h0 * p.W + ch.w0 + (len - 1) * ch.pstep;
   int px_pf = ch.h0 * p.W + ch.w0;
+  // V4: pieces q = lane, lane + 32, ... of the (D + 1) rows of LR / 4 pieces each
+  constexpr int kRounds = V4 ? ((DT ? DT : 16) * 8 + 8 + 31) / 32 : 1;
+  const int nch = LR >> 2, npiece = (D + 1) * nch;
+  const float* src4[kRounds];
+  int dst4[kRounds];
+  if constexpr (V4) {
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k) {
+      const int q = lane + 32 * k, a = q / nch, j = q - a * nch;
+      const int sid = AGG ? (a == 1 ? ch.dir : ch.inv) : a - 1;
+      src4[k] = (a == 0 || q >= npiece ? p.unary : p.msg_read + sid * p.slice) + ibase * LR + 4 * j;
+      dst4[k] = a * 32 + 4 * j;
+    }
+  }
   auto issue = [&](int j) {
+    if constexpr (V4) {
+      float* dst = ring + (j & (kPF - 1)) * slot_floats;
+      const int pxc = j < len ? px_pf : px_last;
+      const int o = pxc * LR;
+#pragma unroll
+      for (int k = 0; k < kRounds; ++k)
+        if (lane + 32 * k < npiece) cp_async16(dst + dst4[k], src4[k] + o);
+      if (has_e && lane == 31) cp_async4(dst + (D + 1) * 32, E + pxc);
+      cp_async_commit();
+      px_pf += ch.pstep;
+      return;
+    }
     float* dst = ring_lane + (j & (kPF - 1)) * slot_floats;
     const int pxc = j < len ? px_pf : px_last;
-    const int o = pxc * L;
+    const int o = pxc * LR;
     cp_async4(dst, Ul + o);
 #pragma unroll
     for (int k = 0; k < (DT ? DT : 16); ++k)
-      if (k < D) cp_async4(dst + (1 + k) * 32, Ml + (p.agg ? (k == 0 ? ch.dir : ch.inv) : k) * p.slice + o);
+      if (k < D) cp_async4(dst + (1 + k) * 32, Ml + (AGG ? (k == 0 ? ch.dir : ch.inv) : k) * p.slice + o);
     cp_async4(dst + (D + 1) * 32, E + pxc);
     cp_async_commit();
     px_pf += ch.pstep;
   };
   auto uu_of = [&](const float* sl) {  // sl: this lane's column of a ring slot
-    if (p.agg) return fmaf(sl[0] - sl[32], rho, -sl[64]);  // rows: A, M_dir, M_inv
+    if (AGG) return fmaf(sl[0] - sl[32], rho, -sl[64]);  // rows: A, M_dir, M_inv
     float s = sl[0];
 #pragma unroll
     for (int k = 0; k < (DT ? DT : 16); ++k)
@@ -165,22 +204,26 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
 #pragma unroll
   for (int j = 0; j < kPF; ++j) issue(j);
   cp_async_wait<kPF - 1>();
-  float uu = uu_of(ring_lane);
+  __syncwarp();
+  float uu = uu_of(ring + lc);
+  __syncwarp();
   issue(kPF);
   float r = 0.f;
   int px = ch.h0 * p.W + ch.w0 + ch.pstep;  // pixel i = 1
-  int of = px * L;
+  int of = px * LR;
 
   for (int i = 1; i < len; ++i) {
-    cp_async_wait<kPF - 1>();  // everything staged for chain pixel i has landed
-    const float* sl = ring_lane + (i & (kPF - 1)) * slot_floats;
-    const float e = has_e ? sl[(D + 1) * 32] : 1.f;
-    // Old values at pixel i are consumed BEFORE the new message of pixel i is stored (TRWP updates
-    // the message slice in place).
-    const float uu_next = uu_of(sl);
     float* hb = hbuf + (i & 1) * 32;
     hb[lane] = act ? fmaf(rho, r, uu) : kInf;
+    cp_async_wait<kPF - 1>();  // everything staged for chain pixel i has landed
     __syncwarp();
+    const float* sl = ring + (i & (kPF - 1)) * slot_floats;
+    const float e = has_e ? sl[(D + 1) * 32 + (V4 ? 0 : lane)] : 1.f;
+    // Old values at pixel i are consumed BEFORE the new message of pixel i is stored (TRWP updates
+    // the message slice in place).
+    const float uu_next = uu_of(sl + lc);
+    float m_col = 0.f;
+    if constexpr (!SOFT && !TRAIN) m_col = warp_min(act ? fmaf(e, e >= 0.f ? colmin : colmax, hb[lane]) : kInf);
     float best;
     int bi = 0;
     if constexpr (SOFT) {
@@ -212,7 +255,8 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
     } else {
       minplus_regrow<LMAX, TRAIN>(hb, cr, e, best, bi);
     }
-    const float m = warp_min(act ? best : kInf);
+    // the minimum over the labels, known before the candidates (see fwd_tma_kernel)
+    const float m = SOFT || TRAIN ? warp_min(act ? best : kInf) : m_col;
     r = best - m;
     if (act) Mwl[of] = r;
     if (TRAIN) {
@@ -220,253 +264,13 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
       if (!SOFT && act) MIl[of] = (uint8_t)bi;
       if (lane == 0) NI[px] = (uint8_t)(31 - __clz(bal));
     }
+    __syncwarp();  // every lane has read the slot that is refilled next
     issue(i + kPF);
     uu = uu_next;
     px += ch.pstep;
     of += ostep;
   }
   cp_async_wait<0>();
-}
-
-// ------------------------------------------------------------------------------------------------
-// L <= 32, directions 0..3, 16-byte-aligned rows: bulk-copy (TMA) staged kernel.
-//
-// A CTA walks four neighbouring chains (four image rows for the horizontal directions, four
-// adjacent columns for the vertical ones) with one consumer warp each; a fifth warp is the
-// producer.  Per stage of kTK chain pixels the producer issues plain (non-multicast)
-// cp.async.bulk copies of whole row segments -- kTK*L floats per array and chain horizontally,
-// 4*L floats per array and image row vertically -- into a ring of shared-memory tiles; completion
-// is counted in bytes on one mbarrier per stage, and consumers hand a tile back through a second
-// mbarrier.  The consumers therefore spend no instruction on global loads or their addresses.
-// Every wait is bounded: after about a second it records a code in *status and the warp leaves.
-// ------------------------------------------------------------------------------------------------
-constexpr int kTK = 16;
-
-// LT = compile-time label count (0: runtime, up to LMAX = 32); FWD = the chain walks towards
-// increasing coordinates (directions 0 and 2).
-template <int LMAX, int LT, int DT, bool TRAIN, bool VERT, bool FWD>
-__global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__ FwdParams p,
-                                                         const __grid_constant__ TmaMaps maps) {
-  // No static shared memory in this kernel: the dynamic region starts at the CTA's shared window
-  // base, which satisfies the 128-byte alignment the tiled TMA destination needs.  (Rounding the
-  // pointer up by hand would hide its address space from the compiler and turn every shared
-  // access into a slower generic one.)
-  extern __shared__ __align__(128) float smem[];
-  constexpr bool AGG = DT == 2;  // aggregate mode (see FwdParams::agg): arrays A, M_dir, M_inv
-  constexpr int A = DT + 1;      // staged arrays: unary (or aggregate) + DT message slices
-  constexpr int AE = A + 1;   // ... + edge weights
-  const int L = LT ? LT : p.L, H = p.H, W = p.W, NS = p.tma_stages;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int dir = p.dir0, inv = dir ^ 1;
-  const bool has_e = p.ew != nullptr;
-  const int len = VERT ? H : W;
-  const int nstages = (len + kTK - 1) / kTK;
-  const int tile_floats = A * kTK * 4 * L;
-
-  float* tiles = smem;                                   // [NS][tile_floats]
-  float* etiles = tiles + NS * tile_floats;              // [NS][64]
-  float* hbufs = etiles + NS * 64;                       // [4][64]
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(hbufs + 4 * 64);  // [NS]
-  unsigned long long* empty = full + NS;                 // [NS]
-
-  // the four chains of this CTA
-  int nact, img0 = 0, w0 = 0, chain0 = 0;
-  if (VERT) {
-    const int gpi = W >> 2;
-    img0 = blockIdx.x / gpi;
-    w0 = (blockIdx.x - img0 * gpi) << 2;
-    nact = 4;
-  } else {
-    chain0 = blockIdx.x << 2;  // flattened (image, row)
-    const int total = p.nimg * H;
-    nact = total - chain0 < 4 ? total - chain0 : 4;
-  }
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NS; ++i) {
-      mbar_init(&full[i], 1);
-      mbar_init(&empty[i], nact);
-    }
-    mbar_fence_init();
-  }
-  __syncthreads();
-
-  if (warp == 4) {
-    // ---------------------------------- producer ----------------------------------
-    const unsigned row_bytes = VERT ? 16u * L : 0u;
-    for (int s = 0; s < nstages; ++s) {
-      const int slot = s % NS;
-      if (s >= NS && !mbar_wait(&empty[slot], ((s / NS) - 1) & 1)) {
-        if (lane == 0) atomicExch(p.status, 101);
-        break;
-      }
-      const int npix = len - s * kTK < kTK ? len - s * kTK : kTK;
-      float* T = tiles + slot * tile_floats;
-      float* ET = etiles + slot * 64;
-      if (VERT) {
-        // 2-D tiled TMA: one copy per staged array brings kTK image rows of the 4-pixel column
-        // group (box 4L x kTK).  Rows outside the tensor read as zero, rows of a neighbouring image
-        // are never used; the full box is always transferred.
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&full[slot], (unsigned)(A * kTK * row_bytes + (has_e ? kTK * 16u : 0u)));
-          const int y0 = img0 * H + (FWD ? s * kTK : H - (s + 1) * kTK);
-          tma_load_2d(T, &maps.a, w0 * L, y0, &full[slot]);
-#pragma unroll
-          for (int a = 1; a < A; ++a)
-            tma_load_2d(T + a * kTK * 4 * L, &maps.b, w0 * L,
-                        (AGG ? (a == 1 ? dir : inv) : a - 1) * p.nimg * H + y0, &full[slot]);
-          if (has_e) tma_load_2d(ET, &maps.c, w0, dir * p.nimg * H + y0, &full[slot]);
-        }
-      } else {
-        if (lane == 0)
-          mbar_arrive_expect_tx(&full[slot], (unsigned)nact * (unsigned)npix * (A * 4u * L + (has_e ? 4u : 0u)));
-        __syncwarp();
-        const int ncopy = nact * AE;
-        for (int c = lane; c < ncopy; c += 32) {
-          const int q = c / AE, a = c - q * AE;
-          const int wlo = FWD ? s * kTK : W - s * kTK - npix;
-          const long long pix = (long long)(chain0 + q) * W + wlo;  // first pixel, over all images
-          if (a < A) {
-            const int sid = AGG ? (a == 1 ? dir : inv) : a - 1;
-            const float* src = (a == 0 ? p.unary : p.msg_read + (long long)sid * p.slice) + pix * L;
-            bulk_g2s(T + (q * A + a) * kTK * L, src, (unsigned)npix * 4u * L, &full[slot]);
-          } else if (has_e) {
-            bulk_g2s(ET + q * kTK, p.ew + (long long)dir * p.pslice + pix, (unsigned)npix * 4u, &full[slot]);
-          }
-        }
-      }
-    }
-    return;
-  }
-
-  // ---------------------------------- consumers ----------------------------------
-  const int wc = warp;
-  if (wc >= nact) return;
-  const bool act = lane < L;
-  // Idle lanes (lane >= L) mirror the last label: same loads, same arithmetic, same `best`, so the
-  // warp-wide minimum needs no select; only their stores are masked.
-  const int lc = act ? lane : L - 1;
-  const unsigned lmask = L >= 32 ? 0xffffffffu : (1u << L) - 1u;
-  const float rho = p.rho;
-  float cr[LMAX];
-#pragma unroll
-  for (int f = 0; f < LMAX; ++f) cr[f] = f < L ? ctx_value(p.ctx, p.ctx_rank, L, lc, f) : 0.f;
-
-  int img, fix;  // fix = the coordinate that stays constant along the chain
-  if (VERT) {
-    img = img0;
-    fix = w0 + wc;
-  } else {
-    img = (chain0 + wc) / H;
-    fix = (chain0 + wc) - img * H;
-  }
-  const long long ibase = (long long)img * H * W;
-  float* Mwl = p.msg_write + (long long)dir * p.slice + ibase * L + lc;
-  uint8_t* MIl = TRAIN ? p.min_idx + (long long)dir * p.slice + ibase * L + lc : nullptr;
-  uint8_t* NI = TRAIN ? p.norm_idx + (long long)dir * p.pslice + ibase : nullptr;
-  float* hbuf = hbufs + wc * 64;
-  for (int i = lane; i < 64; i += 32) hbuf[i] = kInf;  // labels >= L (LMAX > L) never win
-  if (!has_e)  // no edge weights: the producer copies none, every staged weight reads as 1
-    for (int i = lane; i < NS * 64; i += 32) etiles[i] = 1.f;
-  __syncwarp();
-  const int sa = VERT ? kTK * 4 * L : kTK * L;        // stride between staged arrays
-  const int sk = (VERT ? 4 * L : L) * (FWD ? 1 : -1);  // stride between consecutive chain pixels
-  const int ek = (VERT ? 4 : 1) * (FWD ? 1 : -1);
-  const int pstep = VERT ? (FWD ? W : -W) : (FWD ? 1 : -1);
-  const int px0 = VERT ? (FWD ? 0 : H - 1) * W + fix : fix * W + (FWD ? 0 : W - 1);  // chain pixel 0
-  const int dir_off = (AGG ? 1 : 1 + dir) * sa, inv_off = (AGG ? 2 : 1 + inv) * sa;
-
-  float uu = 0.f, r = 0.f;
-  // inputs of one chain pixel -> UU of that pixel (reference order of the additions)
-  auto uu_at = [&](const float* t) {
-    float sum = t[0];
-    if (!AGG) {
-#pragma unroll
-      for (int a = 1; a <= DT; ++a) sum += t[a * sa];
-    }
-    sum -= t[dir_off];
-    return fmaf(sum, rho, -t[inv_off]);
-  };
-  // Output rows of the current chain pixel, moved by one pixel per step (running pointers: one
-  // 64-bit add each instead of an index multiplication and a widening add per store).
-  const long long ostep = (long long)pstep * L;
-  float* mw = Mwl + (long long)px0 * L;
-  uint8_t* mip = TRAIN ? MIl + (long long)px0 * L : nullptr;
-  uint8_t* nip = TRAIN ? NI + px0 : nullptr;
-  // message of the current chain pixel from its predecessor's UU (in `uu`) and running message `r`
-  auto step = [&](const float* t, float e, int par) {
-    const float uu_next = uu_at(t);
-    float* hb = hbuf + par * 32;
-    if (LT == 0 || LMAX != LT) {
-      if (act) hb[lane] = fmaf(rho, r, uu);
-    } else {
-      hb[lane] = fmaf(rho, r, uu);  // entries >= L are written but never read
-    }
-    __syncwarp();
-    // The warp-wide minimum is issued as soon as the lane's own minimum is known: its latency
-    // runs behind the argmin flags, which need only the lane's candidates.
-    float val[LMAX];
-    minplus_vals<LMAX>(hb, cr, e, val);
-    const float best = min_tree<LMAX>(val);
-    const float m = warp_min(best);
-    int bi = 0;
-    if (TRAIN) bi = highest_equal<LMAX>(val, best);
-    r = best - m;
-    // Unpredicated stores: idle lanes hold the same values as lane L-1 and write the same
-    // address, and the normalisation index is warp-uniform.
-    *mw = r;
-    if (TRAIN) {
-      const unsigned bal = __ballot_sync(0xffffffffu, best == m) & lmask;
-      *mip = (uint8_t)bi;
-      *nip = (uint8_t)(31 - __clz(bal));
-    }
-    uu = uu_next;
-  };
-  auto advance = [&]() {
-    mw += ostep;
-    if (TRAIN) {
-      mip += ostep;
-      nip += pstep;
-    }
-  };
-
-  for (int s = 0; s < nstages; ++s) {
-    const int slot = s % NS;
-    if (!mbar_wait(&full[slot], (s / NS) & 1)) {
-      if (lane == 0) atomicExch(p.status, 102);
-      return;
-    }
-    const int npix = len - s * kTK < kTK ? len - s * kTK : kTK;
-    const float* T = tiles + slot * tile_floats + lc;
-    const float* ET = etiles + slot * 64;
-    const float* t0;
-    const float* e0;
-    if (VERT) {  // box rows ascend in memory; a downward walk starts at the last row of the box
-      t0 = T + wc * L + (FWD ? 0 : (kTK - 1) * 4 * L);
-      e0 = ET + wc + (FWD ? 0 : (kTK - 1) * 4);
-    } else {
-      t0 = T + wc * A * kTK * L + (FWD ? 0 : (npix - 1) * L);
-      e0 = ET + wc * kTK + (FWD ? 0 : npix - 1);
-    }
-    if (s > 0 && npix == kTK) {
-      // full stage: fully unrolled, every tile offset is an immediate
-#pragma unroll
-      for (int k = 0; k < kTK; ++k) {
-        step(t0 + k * sk, e0[k * ek], k & 1);
-        advance();
-      }
-    } else {
-      for (int k = 0; k < npix; ++k) {
-        if (s + k == 0) {
-          uu = uu_at(t0);  // chain pixel 0 only provides the inputs of pixel 1
-        } else {
-          step(t0 + k * sk, e0[k * ek], k & 1);
-        }
-        advance();
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[slot]);
-  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -598,7 +402,7 @@ __global__ void __launch_bounds__(256) fwd_cta_kernel(const __grid_constant__ Fw
   extern __shared__ __align__(16) float smem[];
   ChainCtx ch;
   if (!decode_chain(p, blockIdx.x, ch)) return;  // uniform for the CTA
-  const int L = p.L, D = p.agg ? 2 : p.D, rows = D + 2, NT = blockDim.x, c = threadIdx.x, nw = NT >> 5;
+  const int L = p.L, LR = p.ls, D = p.agg ? 2 : p.D, rows = D + 2, NT = blockDim.x, c = threadIdx.x, nw = NT >> 5;
   float* ring = smem;                  // [kPF][rows][NT]
   float* hbuf = ring + kPF * rows * NT;  // [NT]
   float* ctx1 = hbuf + NT;             // [NT]   (MODE 1)
@@ -613,11 +417,11 @@ __global__ void __launch_bounds__(256) fwd_cta_kernel(const __grid_constant__ Fw
   __syncthreads();
 
   const long long ibase = (long long)ch.img * p.H * p.W;
-  const float* U = p.unary + ibase * L;
-  const float* Mr = p.msg_read + ibase * L;
-  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * L;
+  const float* U = p.unary + ibase * LR;
+  const float* Mr = p.msg_read + ibase * LR;
+  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * LR;
   const float* E = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
-  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * L : nullptr;
+  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
   const int pix0 = ch.h0 * p.W + ch.w0;
   const int len = ch.len;
@@ -627,10 +431,10 @@ __global__ void __launch_bounds__(256) fwd_cta_kernel(const __grid_constant__ Fw
       float* dst = ring + (j & (kPF - 1)) * rows * NT + c;
       const int px = pix0 + j * ch.pstep;
       if (act && j < len - 1) {
-        cp_async4(dst, U + (long long)px * L + c);
+        cp_async4(dst, U + (long long)px * LR + c);
         for (int k = 0; k < D; ++k)
           cp_async4(dst + (1 + k) * NT,
-                    Mr + (p.agg ? (k == 0 ? ch.dir : ch.inv) : k) * p.slice + (long long)px * L + c);
+                    Mr + (p.agg ? (k == 0 ? ch.dir : ch.inv) : k) * p.slice + (long long)px * LR + c);
       }
       if (E && j >= 1) cp_async4(dst + (D + 1) * NT, E + px);
     }
@@ -655,9 +459,9 @@ __global__ void __launch_bounds__(256) fwd_cta_kernel(const __grid_constant__ Fw
     cta_minplus<MODE, TRAIN>(p, cc, h, e, act, c, L, nw, hbuf, ctx1, redA_v, redA_i, redB_v, redB_i, best, bi, m, n);
     r = best - m;
     const int px = pix0 + i * ch.pstep;
-    if (act) Mw[(long long)px * L + c] = r;
+    if (act) Mw[(long long)px * LR + c] = r;
     if (TRAIN) {
-      if (act) MI[(long long)px * L + c] = (uint8_t)bi;
+      if (act) MI[(long long)px * LR + c] = (uint8_t)bi;
       if (c == 0) NI[px] = (uint8_t)n;
     }
     issue(i + kPF);
@@ -677,11 +481,11 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   extern __shared__ __align__(128) float smem[];
   ChainCtx ch;
   if (!decode_chain(p, blockIdx.x, ch)) return;  // uniform for the CTA
-  const int L = p.L, D = p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
+  const int L = p.L, LR = p.ls, D = p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   const int NT = blockDim.x - 32, c = threadIdx.x, nw = NT >> 5;
   const bool producer = c >= NT;
-  const int tile_floats = A * K * L;
-  float* tiles = smem;                        // [NS][A][K][L]
+  const int tile_floats = A * K * LR;
+  float* tiles = smem;                        // [NS][A][K][LR]
   float* etile = tiles + NS * tile_floats;    // [2][K]
   float* hbuf = etile + 2 * K;                // [NT]
   float* ctx1 = hbuf + NT;                    // [NT]
@@ -715,8 +519,8 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
 
   if (producer) {
     const int lane = c - NT;
-    const float* U = p.unary + ibase * L;
-    const float* Mr = p.msg_read + ibase * L;
+    const float* U = p.unary + ibase * LR;
+    const float* Mr = p.msg_read + ibase * LR;
     for (int s = 0; s < nstages; ++s) {
       const int slot = s % NS;
       if (s >= NS && !mbar_wait(&empty[slot], ((s / NS) - 1) & 1)) {
@@ -725,23 +529,23 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
       }
       const int np = len - s * K < K ? len - s * K : K;
       float* T = tiles + slot * tile_floats;
-      if (lane == 0) mbar_arrive_expect_tx(&full[slot], (unsigned)(np * A * L) * 4u);
+      if (lane == 0) mbar_arrive_expect_tx(&full[slot], (unsigned)(np * A * LR) * 4u);
       __syncwarp();
       if (contiguous) {
         // pixels s*K .. s*K+np-1 are adjacent in memory (ascending for pstep=1, descending for -1)
         const int first = ch.pstep == 1 ? pix0 + s * K : pix0 - (s * K + np - 1);
         if (lane < A) {
           const int sid = p.agg ? (lane == 1 ? ch.dir : ch.inv) : lane - 1;
-          const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * L;
-          bulk_g2s(T + lane * K * L, src, (unsigned)(np * L) * 4u, &full[slot]);
+          const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * LR;
+          bulk_g2s(T + lane * K * LR, src, (unsigned)(np * LR) * 4u, &full[slot]);
         }
       } else {
         for (int q = lane; q < np * A; q += 32) {
           const int k = q / A, a = q - k * A;
           const int px = pix0 + (s * K + k) * ch.pstep;
           const int sid = p.agg ? (a == 1 ? ch.dir : ch.inv) : a - 1;
-          const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * L;
-          bulk_g2s(T + (a * K + k) * L, src, (unsigned)L * 4u, &full[slot]);
+          const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * LR;
+          bulk_g2s(T + (a * K + k) * LR, src, (unsigned)LR * 4u, &full[slot]);
         }
       }
     }
@@ -749,11 +553,11 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   }
 
   // ---------------------------------- consumers ----------------------------------
-  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * L;
+  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * LR;
   const float* E = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
-  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * L : nullptr;
+  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
-  const int dir_off = (p.agg ? 1 : 1 + ch.dir) * K * L, inv_off = (p.agg ? 2 : 1 + ch.inv) * K * L;
+  const int dir_off = (p.agg ? 1 : 1 + ch.dir) * K * LR, inv_off = (p.agg ? 2 : 1 + ch.inv) * K * LR;
   auto load_e = [&](int s) -> float {  // thread k < K: weight of chain pixel s*K + k
     const int j = s * K + c;
     return (E && c < K && j < len && j >= 1) ? E[pix0 + j * ch.pstep] : 1.f;
@@ -775,12 +579,12 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
     const int kstep = (contiguous && ch.pstep == -1) ? -1 : 1;
     cta_sync(NT);  // the weights of this stage (written at the end of the previous one) are visible
     for (int k = 0; k < np; ++k) {
-      const float* t = T + (kbase + k * kstep) * L + c;
+      const float* t = T + (kbase + k * kstep) * LR + c;
       float uu_next = 0.f;
       if (act) {
         float sum = t[0];
         if (!p.agg)
-          for (int a = 1; a <= D; ++a) sum += t[a * K * L];
+          for (int a = 1; a <= D; ++a) sum += t[a * K * LR];
         sum -= t[dir_off];
         uu_next = fmaf(sum, p.rho, -t[inv_off]);
       }
@@ -793,9 +597,9 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
                                  m, n, NT);
         r = best - m;
         const int px = pix0 + (s * K + k) * ch.pstep;
-        if (act) Mw[(long long)px * L + c] = r;
+        if (act) Mw[(long long)px * LR + c] = r;
         if (TRAIN) {
-          if (act) MI[(long long)px * L + c] = (uint8_t)bi;
+          if (act) MI[(long long)px * LR + c] = (uint8_t)bi;
           if (c == 0) NI[px] = (uint8_t)n;
         }
       }
@@ -809,183 +613,30 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------
-// 32 < L <= 64, rank-2 (dense) context, L % 4 == 0: one WARP per chain, TWO labels per lane, both
-// context rows of the lane in registers.  No block barrier (the CTA-per-chain kernel needs two per
-// step and two warps per chain).  Every warp stages its own inputs: lane-parallel cp.async.bulk
-// copies (one per array and stage for horizontal chains, one label row per pixel otherwise) into a
-// private ring, completion on the warp's own mbarriers, refilled by the warp itself as soon as it
-// has consumed a stage (no producer warp: it would hold as many registers as a consumer).
-// ------------------------------------------------------------------------------------------------
-constexpr int kPairWarps = 4;  // chains per CTA
-
-template <bool TRAIN>
-__global__ void __launch_bounds__(kPairWarps * 32, 1) fwd_pair_kernel(const __grid_constant__ FwdParams p) {
-  extern __shared__ __align__(128) float smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = p.L, D = p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
-  const int tile_floats = A * K * L;
-  const int per_warp = NS * tile_floats + 2 * 64 + 2 * K + 2 * NS + 2;  // floats (barriers are 2 each)
-  float* wbase = smem + warp * ((per_warp + 3) & ~3);
-  float* tiles = wbase;                               // [NS][A][K][L]
-  float* hbuf = tiles + NS * tile_floats;             // [2][64]
-  float* etile = hbuf + 128;                          // [2][K]
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(etile + 2 * K + ((2 * K) & 1));
-  if (lane == 0)
-    for (int i = 0; i < NS; ++i) mbar_init(&full[i], 1);
-  hbuf[lane] = kInf, hbuf[32 + lane] = kInf, hbuf[64 + lane] = kInf, hbuf[96 + lane] = kInf;
-  if (lane == 0) mbar_fence_init();
-  __syncwarp();
-  ChainCtx ch;
-  if (!decode_chain(p, blockIdx.x * kPairWarps + warp, ch)) return;
-
-  const int len = ch.len;
-  const int nstages = (len + K - 1) / K;
-  const long long ibase = (long long)ch.img * p.H * p.W;
-  const int pix0 = ch.h0 * p.W + ch.w0;
-  const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
-  const float* U = p.unary + ibase * L;
-  const float* Mr = p.msg_read + ibase * L;
-
-  auto issue_stage = [&](int s) {  // copies of stage s into slot s % NS (all lanes call)
-    if (s >= nstages) return;
-    const int slot = s % NS;
-    const int np = len - s * K < K ? len - s * K : K;
-    float* T = tiles + slot * tile_floats;
-    if (lane == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&full[slot], (unsigned)(np * A * L) * 4u);
-    }
-    __syncwarp();
-    if (contiguous) {
-      const int first = ch.pstep == 1 ? pix0 + s * K : pix0 - (s * K + np - 1);
-      if (lane < A) {
-        const int sid = p.agg ? (lane == 1 ? ch.dir : ch.inv) : lane - 1;
-        const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * L;
-        bulk_g2s(T + lane * K * L, src, (unsigned)(np * L) * 4u, &full[slot]);
-      }
-    } else {
-      for (int q = lane; q < np * A; q += 32) {
-        const int k = q / A, a = q - k * A;
-        const int px = pix0 + (s * K + k) * ch.pstep;
-        const int sid = p.agg ? (a == 1 ? ch.dir : ch.inv) : a - 1;
-        const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * L;
-        bulk_g2s(T + (a * K + k) * L, src, (unsigned)L * 4u, &full[slot]);
-      }
-    }
-  };
-
-  const int c0 = 2 * lane;          // labels c0, c0 + 1 (L is a multiple of four: both or none exist)
-  const bool act = c0 < L;
-  const int lc0 = act ? c0 : L - 2;  // idle lanes shadow the last pair: loads need no predicate
-  float cr0[64], cr1[64];
-#pragma unroll
-  for (int f = 0; f < 64; ++f) {
-    cr0[f] = (act && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c0, f) : 0.f;
-    cr1[f] = (act && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c0 + 1, f) : 0.f;
-  }
-  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * L + c0;
-  const float* E = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
-  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * L + c0 : nullptr;
-  uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
-  const int dir_off = (p.agg ? 1 : 1 + ch.dir) * K * L, inv_off = (p.agg ? 2 : 1 + ch.inv) * K * L;
-  const float rho = p.rho;
-  auto load_e = [&](int s) -> float {  // lane k < K: weight of chain pixel s*K + k
-    const int j = s * K + lane;
-    return (E && lane < K && j < len && j >= 1) ? E[pix0 + j * ch.pstep] : 1.f;
-  };
-  // The 64 candidates are evaluated as two halves of 32 (the second wins ties: highest index), so
-  // that only 32 sums are alive next to the 128 context registers.
-  auto eval_label = [&](const float* hb, const float (&cr)[64], float e, float& best, int& bi) {
-    float ba, bb;
-    int ia, ib;
-    minplus_regrow<32, TRAIN, 64, 0>(hb, cr, e, ba, ia);
-    minplus_regrow<32, TRAIN, 64, 32>(hb + 32, cr, e, bb, ib);
-    best = fminf(ba, bb);
-    bi = bb <= ba ? ib + 32 : ia;
-  };
-
-  for (int s = 0; s < NS; ++s) issue_stage(s);
-  if (lane < K) etile[lane] = load_e(0);
-  float e_next = load_e(1);
-  float uu0 = 0.f, uu1 = 0.f, r0 = 0.f, r1 = 0.f;
-  int po = pix0 * L;             // element offset of the current pixel's label row
-  const int postep = ch.pstep * L;
-  int px = pix0;
-  for (int s = 0; s < nstages; ++s) {
-    const int slot = s % NS;
-    if (!mbar_wait(&full[slot], (s / NS) & 1)) {
-      if (lane == 0) atomicExch(p.status, 131);
-      return;
-    }
-    const int np = len - s * K < K ? len - s * K : K;
-    const float* T = tiles + slot * tile_floats + lc0;
-    const float* et = etile + (s & 1) * K;
-    const bool flip = contiguous && ch.pstep == -1;
-    __syncwarp();
-    for (int k = 0; k < np; ++k) {
-      const float* t = T + (flip ? np - 1 - k : k) * L;
-      float2 v = *reinterpret_cast<const float2*>(t);
-      if (!p.agg)
-        for (int a = 1; a <= D; ++a) {
-          const float2 x = *reinterpret_cast<const float2*>(t + a * K * L);
-          v.x += x.x, v.y += x.y;
-        }
-      const float2 md = *reinterpret_cast<const float2*>(t + dir_off);
-      const float2 mi = *reinterpret_cast<const float2*>(t + inv_off);
-      const float un0 = fmaf(v.x - md.x, rho, -mi.x);
-      const float un1 = fmaf(v.y - md.y, rho, -mi.y);
-      if (s + k > 0) {
-        const float e = et[k];
-        float* hb = hbuf + ((s * K + k) & 1) * 64;
-        if (act) *reinterpret_cast<float2*>(hb + c0) = make_float2(fmaf(rho, r0, uu0), fmaf(rho, r1, uu1));
-        __syncwarp();
-        float b0, b1;
-        int i0, i1;
-        eval_label(hb, cr0, e, b0, i0);
-        eval_label(hb, cr1, e, b1, i1);
-        const float x0 = act ? b0 : kInf, x1 = act ? b1 : kInf;
-        const float m = warp_min(fminf(x0, x1));
-        r0 = b0 - m;
-        r1 = b1 - m;
-        if (act) *reinterpret_cast<float2*>(Mw + po) = make_float2(r0, r1);
-        if (TRAIN) {
-          const unsigned bal0 = __ballot_sync(0xffffffffu, x0 == m);
-          const unsigned bal1 = __ballot_sync(0xffffffffu, x1 == m);
-          const int n0 = 2 * (31 - __clz(bal0));      // -2 when no even label attains the minimum
-          const int n1 = 2 * (31 - __clz(bal1)) + 1;  // -1 when no odd label does
-          if (act) *reinterpret_cast<uchar2*>(MI + po) = make_uchar2((unsigned char)i0, (unsigned char)i1);
-          if (lane == 0) NI[px] = (uint8_t)(n0 > n1 ? n0 : n1);
-        }
-      }
-      uu0 = un0;
-      uu1 = un1;
-      po += postep;
-      px += ch.pstep;
-    }
-    if (lane < K) etile[((s + 1) & 1) * K + lane] = e_next;
-    e_next = load_e(s + 2);
-    __syncwarp();
-    issue_stage(s + NS);  // this warp refills the slot it has just consumed
-  }
-}
-
-// ------------------------------------------------------------------------------------------------
 // Context / edge-weight analysis (rank-1 contexts with L > 32 only).
 // ------------------------------------------------------------------------------------------------
 __global__ void analyze_ctx_kernel(const float* ctx, int L, CtxInfo* info) {
-  // Single thread: L <= 256 values.
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const float cmax = ctx[L - 1];
-  int R = L - 1;
-  while (R > 0 && ctx[R - 1] == cmax) --R;
+  // one warp, L <= 256 values
+  const int lane = threadIdx.x;
+  const float c0 = ctx[0], cmax = ctx[L - 1];
+  int last = -1;  // highest label below L - 1 whose value differs from cmax
+  for (int k = lane; k < L - 1; k += 32) last = ctx[k] == cmax ? last : k;
+  const int R = __reduce_max_sync(0xffffffffu, last) + 1;
   // Exactness of the windowed evaluation needs only ctx[k] <= cmax for every k < R (and weights
   // >= 0): candidates outside the window then cost at least h_min + w * cmax.
-  bool mono = true;
-  for (int k = 0; k < R; ++k) mono = mono && (ctx[k] <= cmax);
+  bool mono = true, zmin = true;
+  for (int k = lane; k < L; k += 32) {
+    mono = mono && (k >= R || ctx[k] <= cmax);
+    zmin = zmin && c0 <= ctx[k];
+  }
+  mono = __all_sync(0xffffffffu, mono);
+  zmin = __all_sync(0xffffffffu, zmin);
+  if (lane != 0) return;
   info->windowed = (mono && 2 * R - 1 < L) ? 1 : 0;
   info->R = R;
   info->cmax = cmax;
   info->ew_min_bits = 0x7fffffff;
+  info->zero_min = zmin ? 1 : 0;
 }
 
 __global__ void analyze_ew_kernel(const float* ew, long long n, CtxInfo* info) {
@@ -1055,13 +706,15 @@ aggregate_vec4_kernel(const float4* __restrict__ unary, const float4* __restrict
 // image, through a shared-memory tile so that both sides are coalesced.
 __global__ void __launch_bounds__(256)
 aggregate_lhw_kernel(const float* __restrict__ unary, const float* __restrict__ msg, float* __restrict__ cost,
-                     int L, long long HW, int D, long long slice, float factor, int min_a_dir) {
+                     int L, int ls, long long HW, int D, long long slice, float factor, int min_a_dir) {
   extern __shared__ float tile[];  // [L][33]
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long long b = blockIdx.y, p0 = blockIdx.x * 32ll;
   const int np = HW - p0 < 32 ? (int)(HW - p0) : 32;
-  const long long base = (b * HW + p0) * L;
-  for (int i = threadIdx.x; i < np * L; i += 256) {
+  const long long base = (b * HW + p0) * ls;
+  for (int i = threadIdx.x; i < np * ls; i += 256) {
+    const int px = i / ls, l = i - px * ls;
+    if (l >= L) continue;  // padding of the row
     float v = unary[base + i] * factor;
     if (min_a_dir) {
       float mm = msg[base + i];
@@ -1073,7 +726,6 @@ aggregate_lhw_kernel(const float* __restrict__ unary, const float* __restrict__ 
     } else {
       for (int k = 0; k < D; ++k) v += msg[k * slice + base + i];
     }
-    const int px = i / L, l = i - px * L;
     tile[l * 33 + px] = v;
   }
   __syncthreads();
@@ -1082,21 +734,84 @@ aggregate_lhw_kernel(const float* __restrict__ unary, const float* __restrict__ 
     if (tx < np) dst[(long long)l * HW + tx] = tile[l * 33 + tx];
 }
 
-__global__ void label_kernel(const float* __restrict__ cost, uint8_t* __restrict__ label,
-                             long long npix, int L) {
-  const long long px = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (px >= npix) return;
-  const float* c = cost + px * L;
-  float mv = c[0];
-  int ml = 0;
-  for (int l = 1; l < L; ++l) {
-    const float v = c[l];
-    if (v < mv) {
-      mv = v;
-      ml = l;
+// Labels of the current costs U*factor + sum_k M_k (or + min_k M_k): lowest label attaining the
+// minimum, as the reference's ascending strict-< scan (MPLayers/TRWP/TRWP_forward.cu:30-58).  G lanes
+// per pixel, VEC labels per lane and round; each input is read once and the costs themselves are
+// written only where the caller has a use for them (`cost` not null).
+template <int G, int VEC>
+__global__ void __launch_bounds__(256)
+aggregate_label_kernel(const float* __restrict__ unary, const float* __restrict__ msg, float* __restrict__ cost,
+                       uint8_t* __restrict__ label, long long npix, int L, int ls, int D, long long slice,
+                       float factor, int min_a_dir) {
+  const int lane = threadIdx.x & (G - 1);
+  const long long px = (blockIdx.x * 256ll + threadIdx.x) / G;
+  const bool live = px < npix;
+  const long long row = (live ? px : npix - 1) * ls;
+  float mv = 0.f;
+  int ml = -1;  // -1: no label seen yet
+  for (int l0 = lane * VEC; l0 < L; l0 += G * VEC) {
+    float v[VEC];
+    auto load = [&](const float* q, float (&x)[VEC]) {
+      if constexpr (VEC == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(q);
+        x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
+      } else {
+        x[0] = *q;
+      }
+    };
+    load(unary + row + l0, v);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) v[i] *= factor;
+    if (min_a_dir) {
+      float mm[VEC];
+      load(msg + row + l0, mm);
+      for (int k = 1; k < D; ++k) {
+        float x[VEC];
+        load(msg + k * slice + row + l0, x);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i)
+          if (x[i] < mm[i]) mm[i] = x[i];
+      }
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) v[i] += mm[i];
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < D; ++k) {
+        float x[VEC];
+        load(msg + k * slice + row + l0, x);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) v[i] += x[i];
+      }
+    }
+    if (cost && live) {
+      if constexpr (VEC == 4) {
+        *reinterpret_cast<float4*>(cost + row + l0) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+        cost[row + l0] = v[0];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      // (a NaN counts at label 0 only, where the ascending scan starts from it)
+      if (l0 + i < L && ((ml < 0 && (v[i] == v[i] || l0 + i == 0)) || v[i] < mv)) {
+        mv = v[i];
+        ml = l0 + i;
+      }
     }
   }
-  label[px] = (uint8_t)ml;
+  // a lane without a label never wins; among the others the smaller value, then the lower label
+  bool nan0 = ml == 0 && mv != mv;
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, mv, o);
+    const int ol = __shfl_xor_sync(0xffffffffu, ml, o);
+    nan0 = nan0 || __shfl_xor_sync(0xffffffffu, (int)nan0, o);
+    if (ol >= 0 && (ml < 0 || ov < mv || (ov == mv && ol < ml))) {
+      mv = ov;
+      ml = ol;
+    }
+  }
+  if (live && lane == 0) label[px] = (uint8_t)(nan0 || ml < 0 ? 0 : ml);
 }
 
 template <typename K>
@@ -1106,22 +821,30 @@ cudaError_t ensure_smem(K kernel, size_t bytes) {
   return cudaSuccess;
 }
 
+// Rows of 16-byte multiples at 16-byte aligned bases (fwd_warp_kernel's V4 staging).
+bool rows_aligned(const FwdParams& p) {
+  return (p.ls & 3) == 0 && (((uintptr_t)p.unary | (uintptr_t)p.msg_read) & 15) == 0;
+}
+
 template <int LMAX, int DT, bool TRAIN>
 cudaError_t launch_warp_d(const FwdParams& p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
   const int wpb = total >= 148 * 32 ? 4 : 1;
   const size_t smem = (size_t)wpb * (kPF * ((p.agg ? 2 : p.D) + 2) * 32 + 64) * sizeof(float);
-  cudaError_t e = ensure_smem(fwd_warp_kernel<LMAX, DT, TRAIN>, smem);
-  if (e != cudaSuccess) return e;
-  ProfScope prof(kProfFwdSweep, st);
-  fwd_warp_kernel<LMAX, DT, TRAIN><<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
-  count_launch();
-  return cudaGetLastError();
+  auto go = [&](auto kernel) -> cudaError_t {
+    cudaError_t e = ensure_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
+    ProfScope prof(kProfFwdSweep, st);
+    kernel<<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
+    count_launch();
+    return cudaGetLastError();
+  };
+  return rows_aligned(p) ? go(fwd_warp_kernel<LMAX, DT, TRAIN, true>) : go(fwd_warp_kernel<LMAX, DT, TRAIN, false>);
 }
 
 template <int LMAX, bool TRAIN>
 cudaError_t launch_warp(const FwdParams& p, cudaStream_t st) {
-  if (p.agg) return launch_warp_d<LMAX, 0, TRAIN>(p, st);
+  if (p.agg) return launch_warp_d<LMAX, 2, TRAIN>(p, st);
   if (p.D == 4) return launch_warp_d<LMAX, 4, TRAIN>(p, st);
   if (p.D == 8) return launch_warp_d<LMAX, 8, TRAIN>(p, st);
   return launch_warp_d<LMAX, 0, TRAIN>(p, st);
@@ -1132,69 +855,12 @@ cudaError_t launch_warp_soft(const FwdParams& p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
   const int wpb = total >= 148 * 32 ? 4 : 1;
   const size_t smem = (size_t)wpb * (kPF * (p.D + 2) * 32 + 64 + 32 * 33) * sizeof(float);
-  cudaError_t e = ensure_smem(fwd_warp_kernel<LMAX, 0, TRAIN, true, EXACT>, smem);
+  cudaError_t e = ensure_smem(fwd_warp_kernel<LMAX, 0, TRAIN, false, true, EXACT>, smem);
   if (e != cudaSuccess) return e;
   ProfScope prof(kProfFwdSweep, st);
-  fwd_warp_kernel<LMAX, 0, TRAIN, true, EXACT><<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
+  fwd_warp_kernel<LMAX, 0, TRAIN, false, true, EXACT><<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
   count_launch();
   return cudaGetLastError();
-}
-
-size_t tma_smem_bytes(int L, int D, int stages) {
-  return ((size_t)stages * ((size_t)(D + 1) * kTK * 4 * L + 64) + 4 * 64) * sizeof(float) + 2 * stages * 8 + 16 + 128;
-}
-
-// Can direction `dir` of this problem use the bulk-copy kernel?  Needs 16-byte aligned row segments.
-bool tma_eligible(const FwdParams& p, int dir, int* stages) {
-  if (dir > 3 || p.L > 32 || (!p.agg && p.D != 4 && p.D != 8)) return false;
-  if ((p.W & 3) || (((long long)p.W * p.L) & 3)) return false;
-  const uintptr_t bits = (uintptr_t)p.unary | (uintptr_t)p.msg_read | (uintptr_t)p.ew;
-  if (bits & 15) return false;
-  int ns = tma_stage_override() ? tma_stage_override() : 4;
-  while (ns >= 2 && tma_smem_bytes(p.L, p.agg ? 2 : p.D, ns) > (ns >= 3 ? 110 : 200) * 1024) --ns;
-  if (ns < 2) return false;
-  *stages = ns;
-  return true;
-}
-
-template <int LMAX, int LT, int DT, bool TRAIN, bool VERT, bool FWD>
-cudaError_t launch_tma_v(FwdParams p, int dir, int stages, cudaStream_t st) {
-  p.dir0 = dir;
-  p.ndirs = 1;
-  p.tma_stages = stages;
-  const int groups = VERT ? p.nimg * (p.W >> 2) : (p.nimg * p.H + 3) >> 2;
-  const size_t smem = tma_smem_bytes(p.L, DT, stages);
-  cudaError_t e = ensure_smem(fwd_tma_kernel<LMAX, LT, DT, TRAIN, VERT, FWD>, smem);
-  if (e != cudaSuccess) return e;
-  TmaMaps maps{};
-  if (VERT) {
-    const unsigned long long inner = (unsigned long long)p.W * p.L, rows = (unsigned long long)p.nimg * p.H;
-    bool ok = encode_tmap_2d(&maps.a, p.unary, inner, rows, 4 * p.L, kTK) &&
-              encode_tmap_2d(&maps.b, p.msg_read, inner, rows * p.D, 4 * p.L, kTK);
-    if (ok && p.ew) ok = encode_tmap_2d(&maps.c, p.ew, (unsigned long long)p.W, rows * p.D, 4, kTK);
-    if (!ok) return cudaErrorNotSupported;
-  }
-  ProfScope prof(kProfFwdSweep, st);
-  fwd_tma_kernel<LMAX, LT, DT, TRAIN, VERT, FWD><<<groups, 160, smem, st>>>(p, maps);
-  count_launch();
-  return cudaGetLastError();
-}
-
-template <int LMAX, int LT, int DT, bool TRAIN>
-cudaError_t launch_tma_d(const FwdParams& p, int dir, int stages, cudaStream_t st) {
-  switch (dir) {
-    case 0: return launch_tma_v<LMAX, LT, DT, TRAIN, false, true>(p, dir, stages, st);
-    case 1: return launch_tma_v<LMAX, LT, DT, TRAIN, false, false>(p, dir, stages, st);
-    case 2: return launch_tma_v<LMAX, LT, DT, TRAIN, true, true>(p, dir, stages, st);
-    default: return launch_tma_v<LMAX, LT, DT, TRAIN, true, false>(p, dir, stages, st);
-  }
-}
-
-template <int LMAX, int LT, bool TRAIN>
-cudaError_t launch_tma(const FwdParams& p, int dir, int stages, cudaStream_t st) {
-  if (p.agg) return launch_tma_d<LMAX, LT, 2, TRAIN>(p, dir, stages, st);
-  if (p.D == 4) return launch_tma_d<LMAX, LT, 4, TRAIN>(p, dir, stages, st);
-  return launch_tma_d<LMAX, LT, 8, TRAIN>(p, dir, stages, st);
 }
 
 template <int MODE, bool TRAIN>
@@ -1217,7 +883,7 @@ cudaError_t launch_cta_tma(FwdParams p, cudaStream_t st) {
   const int A = (p.agg ? 2 : p.D) + 1;
   int K = 16, NS = 3;
   auto bytes = [&](int k, int ns) {
-    return ((size_t)ns * A * k * p.L + 2 * k + 2 * NT + 32) * sizeof(float) + 2 * ns * 8 + 16;
+    return ((size_t)ns * A * k * p.ls + 2 * k + 2 * NT + 32) * sizeof(float) + 2 * ns * 8 + 16;
   };
   while (K > 4 && bytes(K, NS) > 100 * 1024) K >>= 1;
   if (bytes(K, NS) > 100 * 1024) NS = 2;
@@ -1258,16 +924,16 @@ template <bool TRAIN>
 __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(128) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = p.L, D = p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
+  const int L = p.L, LR = p.ls, D = p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   float* ctab = smem;  // [64][kPairRS]
   for (int i = threadIdx.x; i < 64 * kPairRS; i += blockDim.x) {
     const int c = i / kPairRS, f = i - c * kPairRS;
     ctab[i] = (c < L && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c, f) : 0.f;
   }
-  const int tile_floats = A * K * L;
+  const int tile_floats = A * K * LR;
   const int per_warp = NS * tile_floats + 2 * 64 + 2 * K + 2 * NS + 2;
   float* wbase = smem + 64 * kPairRS + warp * ((per_warp + 3) & ~3);
-  float* tiles = wbase;                               // [NS][A][K][L]
+  float* tiles = wbase;                               // [NS][A][K][LR]
   float* hbuf = tiles + NS * tile_floats;             // [2][64]
   float* etile = hbuf + 128;                          // [2][K]
   unsigned long long* full = reinterpret_cast<unsigned long long*>(etile + 2 * K + ((2 * K) & 1));
@@ -1284,8 +950,8 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
   const long long ibase = (long long)ch.img * p.H * p.W;
   const int pix0 = ch.h0 * p.W + ch.w0;
   const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
-  const float* U = p.unary + ibase * L;
-  const float* Mr = p.msg_read + ibase * L;
+  const float* U = p.unary + ibase * LR;
+  const float* Mr = p.msg_read + ibase * LR;
 
   auto issue_stage = [&](int s) {
     if (s >= nstages) return;
@@ -1294,23 +960,23 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
     float* T = tiles + slot * tile_floats;
     if (lane == 0) {
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&full[slot], (unsigned)(np * A * L) * 4u);
+      mbar_arrive_expect_tx(&full[slot], (unsigned)(np * A * LR) * 4u);
     }
     __syncwarp();
     if (contiguous) {
       const int first = ch.pstep == 1 ? pix0 + s * K : pix0 - (s * K + np - 1);
       if (lane < A) {
         const int sid = p.agg ? (lane == 1 ? ch.dir : ch.inv) : lane - 1;
-        const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * L;
-        bulk_g2s(T + lane * K * L, src, (unsigned)(np * L) * 4u, &full[slot]);
+        const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * LR;
+        bulk_g2s(T + lane * K * LR, src, (unsigned)(np * LR) * 4u, &full[slot]);
       }
     } else {
       for (int q = lane; q < np * A; q += 32) {
         const int k = q / A, a = q - k * A;
         const int px = pix0 + (s * K + k) * ch.pstep;
         const int sid = p.agg ? (a == 1 ? ch.dir : ch.inv) : a - 1;
-        const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * L;
-        bulk_g2s(T + (a * K + k) * L, src, (unsigned)L * 4u, &full[slot]);
+        const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * LR;
+        bulk_g2s(T + (a * K + k) * LR, src, (unsigned)LR * 4u, &full[slot]);
       }
     }
   };
@@ -1320,11 +986,11 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
   const int lbc = actb ? lb : la;         // loads of a missing second label repeat the first
   const float* rowa = ctab + la * kPairRS;
   const float* rowb = ctab + lbc * kPairRS;
-  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * L;
+  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * LR;
   const float* E = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
-  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * L : nullptr;
+  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
-  const int dir_off = (p.agg ? 1 : 1 + ch.dir) * K * L, inv_off = (p.agg ? 2 : 1 + ch.inv) * K * L;
+  const int dir_off = (p.agg ? 1 : 1 + ch.dir) * K * LR, inv_off = (p.agg ? 2 : 1 + ch.inv) * K * LR;
   const float rho = p.rho;
   auto load_e = [&](int s) -> float {
     const int j = s * K + lane;
@@ -1345,9 +1011,9 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
   float uu0 = 0.f, uu1 = 0.f, r0 = 0.f, r1 = 0.f;
   // rows of the current chain pixel, moved by one pixel per step (the stage depth is a launch
   // parameter: nothing of it folds into immediates)
-  const int postep = ch.pstep * L, KL = K * L;
-  float* mwa = Mw + (long long)pix0 * L + la;
-  uint8_t* mia = TRAIN ? MI + (long long)pix0 * L + la : nullptr;
+  const int postep = ch.pstep * LR, KL = K * LR;
+  float* mwa = Mw + (long long)pix0 * LR + la;
+  uint8_t* mia = TRAIN ? MI + (long long)pix0 * LR + la : nullptr;
   uint8_t* nip = TRAIN ? NI + pix0 : nullptr;
   int hpar = 0;
   bool first = true;
@@ -1362,8 +1028,8 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
     const float* T = tiles + slot * tile_floats;
     const float* et = etile + (s & 1) * K;
     __syncwarp();
-    const float* t = T + (flip ? np - 1 : 0) * L;
-    const int tstep = flip ? -L : L;
+    const float* t = T + (flip ? np - 1 : 0) * LR;
+    const int tstep = flip ? -LR : LR;
     for (int k = 0; k < np; ++k, t += tstep, mwa += postep, hpar ^= 64) {
       float va = t[la], vb = t[lbc];
       if (!p.agg)
@@ -1410,11 +1076,11 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
 }
 
 template <bool TRAIN>
-cudaError_t launch_pair_smem(FwdParams p, cudaStream_t st) {
+cudaError_t launch_pair(FwdParams p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
   const int A = (p.agg ? 2 : p.D) + 1;
   int K = 4, NS = 3;
-  auto per_warp = [&](int k, int ns) { return ((ns * A * k * p.L + 128 + 2 * k + 2 * ns + 2) + 3) & ~3; };
+  auto per_warp = [&](int k, int ns) { return ((ns * A * k * p.ls + 128 + 2 * k + 2 * ns + 2) + 3) & ~3; };
   auto bytes = [&](int k) { return ((size_t)64 * kPairRS + (size_t)kPairSWarps * per_warp(k, NS)) * sizeof(float); };
   while (K > 1 && bytes(K) > 72 * 1024) K >>= 1;
   p.tma_k = K;
@@ -1428,30 +1094,9 @@ cudaError_t launch_pair_smem(FwdParams p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <bool TRAIN>
-cudaError_t launch_pair(FwdParams p, cudaStream_t st) {
-  // default: context rows in shared memory (three CTAs of four chains per SM); MPL_PAIR_REG=1 selects
-  // the variant that keeps both rows of a lane in registers (comparison knob)
-  if (!(getenv("MPL_PAIR_REG") && getenv("MPL_PAIR_REG")[0] == '1')) return launch_pair_smem<TRAIN>(p, st);
-  const int total = p.chain_off[p.ndirs];
-  const int A = (p.agg ? 2 : p.D) + 1;
-  int K = 8, NS = 3;
-  auto per_warp = [&](int k, int ns) { return ((ns * A * k * p.L + 128 + 2 * k + 2 * ns + 2) + 3) & ~3; };
-  while (K > 2 && (size_t)kPairWarps * per_warp(K, NS) * sizeof(float) > 100 * 1024) K >>= 1;
-  p.tma_k = K;
-  p.tma_stages = NS;
-  const size_t smem = (size_t)kPairWarps * per_warp(K, NS) * sizeof(float);
-  cudaError_t e = ensure_smem(fwd_pair_kernel<TRAIN>, smem);
-  if (e != cudaSuccess) return e;
-  ProfScope prof(kProfFwdSweep, st);
-  fwd_pair_kernel<TRAIN><<<(total + kPairWarps - 1) / kPairWarps, kPairWarps * 32, smem, st>>>(p);
-  count_launch();
-  return cudaGetLastError();
-}
-
 // Label rows of 16-byte multiples at 16-byte aligned bases: the bulk-copy CTA kernel applies.
 bool cta_tma_eligible(const FwdParams& p) {
-  if (p.L & 3) return false;
+  if (p.ls & 3) return false;
   return (((uintptr_t)p.unary | (uintptr_t)p.msg_read) & 15) == 0;
 }
 
@@ -1476,6 +1121,40 @@ cudaError_t launch_analyze(const float* ctx, int L, int rank, const float* ew, l
   return cudaGetLastError();
 }
 
+// Does this sweep (L > 32) run on the several-labels-per-lane kernel?  It evaluates at most 31
+// candidates per label against the pair kernel's 64: 2.0 against 7.2 ms for a 512 x 512 x 64
+// training forward.
+static bool wide_eligible(const FwdParams& p, bool train) {
+  static const bool no_wide_train = [] {  // MPL_NO_WIDE_TRAIN=1: tuning / comparison knob
+    const char* e = getenv("MPL_NO_WIDE_TRAIN");
+    return e && e[0] == '1';
+  }();
+  return p.L > 32 && p.L <= 256 && p.ctx_rank == 1 && (!train || !no_wide_train) && p.host_windowed &&
+         p.host_R <= 16 && cta_tma_eligible(p) && (p.agg || p.D != 2);
+}
+
+bool forward_skips_zero_slices(const FwdParams& p, bool train) { return wide_eligible(p, train); }
+
+__global__ void zero_chain_starts_kernel(const __grid_constant__ FwdParams p, float* a, float* b) {
+  const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (g >= p.chain_off[p.ndirs]) return;
+  ChainCtx ch;
+  decode_chain(p, g, ch);  // its return value only says whether the chain has a second pixel
+  const long long o = ch.dir * p.slice + ((long long)ch.img * p.H * p.W + ch.h0 * p.W + ch.w0) * p.ls;
+  for (int l = lane; l < p.ls; l += 32) {
+    a[o + l] = 0.f;
+    if (b) b[o + l] = 0.f;
+  }
+}
+
+cudaError_t launch_zero_chain_starts(const FwdParams& p, float* a, float* b, cudaStream_t st) {
+  const int total = p.chain_off[p.ndirs];
+  ProfScope prof(kProfElementwise, st);
+  zero_chain_starts_kernel<<<(total + 7) / 8, 256, 0, st>>>(p, a, b);
+  count_launch();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st) {
   if (p.chain_off[p.ndirs] == 0) return cudaSuccess;
   if (p.L <= 32) {
@@ -1488,9 +1167,8 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
     const bool few_chains = (p.ndirs > 1 && (long long)p.nimg * (p.H < p.W ? p.H : p.W) < 256) || p.parts > 1;
     for (int d = p.dir0; d < p.dir0 + p.ndirs && !few_chains; ++d) {
       int stages = 0;
-      if (d != first_generic || !tma_eligible(p, d, &stages)) break;
-      cudaError_t e = p.L == 21 ? (train ? launch_tma<21, 21, true>(p, d, stages, st) : launch_tma<21, 21, false>(p, d, stages, st))
-                                : (train ? launch_tma<32, 0, true>(p, d, stages, st) : launch_tma<32, 0, false>(p, d, stages, st));
+      if (d != first_generic || !forward_tma_eligible(p, d, &stages)) break;
+      const cudaError_t e = launch_forward_tma(p, d, stages, train, st);
       if (e != cudaSuccess) return e;
       first_generic = d + 1;
     }
@@ -1501,19 +1179,11 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
     rest.ndirs = nrest;
     for (int i = 0; i <= nrest; ++i) rest.chain_off[i] = p.chain_off[first_generic - p.dir0 + i] - base;
     for (int i = 0; i < nrest; ++i) rest.chain_begin[i] = p.chain_begin[first_generic - p.dir0 + i];
-    if (p.L == 21) return train ? launch_warp<21, true>(rest, st) : launch_warp<21, false>(rest, st);
+    if (p.L <= 16) return train ? launch_warp<16, true>(rest, st) : launch_warp<16, false>(rest, st);
+    if (p.L <= 21) return train ? launch_warp<21, true>(rest, st) : launch_warp<21, false>(rest, st);
     return train ? launch_warp<32, true>(rest, st) : launch_warp<32, false>(rest, st);
   }
-  // windowed rank-1 context: warp-per-chain kernel, inference and training (at most 31 candidates per
-  // label against the pair kernel's 64: 2.0 against 7.2 ms for a 512 x 512 x 64 training forward)
-  static const bool no_wide_train = [] {  // MPL_NO_WIDE_TRAIN=1: tuning / comparison knob
-    const char* e = getenv("MPL_NO_WIDE_TRAIN");
-    return e && e[0] == '1';
-  }();
-  if (p.ctx_rank == 1 && (!train || !no_wide_train) && p.host_windowed && p.host_R <= 16 &&
-      p.L <= 256 && cta_tma_eligible(p) && (p.agg || p.D != 2)) {
-    return launch_forward_wide(p, train, st);
-  }
+  if (wide_eligible(p, train)) return launch_forward_wide(p, train, st);
   if (p.L <= 64 && cta_tma_eligible(p) && !pair_kernels_disabled())
     return train ? launch_pair<true>(p, st) : launch_pair<false>(p, st);
   if (p.ctx_rank == 1) return train ? launch_cta_any<1, true>(p, st) : launch_cta_any<1, false>(p, st);
@@ -1542,7 +1212,7 @@ cudaError_t launch_forward_soft_sweep(const FwdParams& p, bool train, cudaStream
 // ------------------------------------------------------------------------------------------------
 template <int MODE>
 __global__ void lhw_to_hwl_kernel(const float* __restrict__ in, float* __restrict__ out, uint8_t* __restrict__ amax,
-                                  int L, long long HW) {
+                                  int L, int ls, long long HW) {
   extern __shared__ float tile[];  // [L][33]
   __shared__ float mx[32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -1564,26 +1234,26 @@ __global__ void lhw_to_hwl_kernel(const float* __restrict__ in, float* __restric
     }
     __syncthreads();
   }
-  float* dst = out + (b * HW + p0) * L;
-  for (int i = threadIdx.x; i < np * L; i += 256) {
-    const int px = i / L, l = i - px * L;
-    const float v = tile[l * 33 + px];
+  float* dst = out + (b * HW + p0) * ls;
+  for (int i = threadIdx.x; i < np * ls; i += 256) {
+    const int px = i / ls, l = i - px * ls;
+    const float v = l < L ? tile[l * 33 + px] : 0.f;
     dst[i] = MODE == 1 ? mx[px] - v : (MODE == 3 ? v : -v);
   }
 }
 
 template <int MODE>
 __global__ void hwl_to_lhw_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                  const uint8_t* __restrict__ amax, int L, long long HW) {
+                                  const uint8_t* __restrict__ amax, int L, int ls, long long HW) {
   extern __shared__ float tile[];  // [L][33]
   __shared__ float sm[32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long long b = blockIdx.y, p0 = blockIdx.x * 32ll;
   const int np = HW - p0 < 32 ? (int)(HW - p0) : 32;
-  const float* src = in + (b * HW + p0) * L;
-  for (int i = threadIdx.x; i < np * L; i += 256) {
-    const int px = i / L, l = i - px * L;
-    tile[l * 33 + px] = src[i];
+  const float* src = in + (b * HW + p0) * ls;
+  for (int i = threadIdx.x; i < np * ls; i += 256) {
+    const int px = i / ls, l = i - px * ls;
+    if (l < L) tile[l * 33 + px] = src[i];
   }
   __syncthreads();
   if (MODE == 2) {
@@ -1603,18 +1273,18 @@ __global__ void hwl_to_lhw_kernel(const float* __restrict__ in, float* __restric
     }
 }
 
-cudaError_t launch_layout(int kind, const float* in, float* out, uint8_t* amax, int B, int L, long long HW,
+cudaError_t launch_layout(int kind, const float* in, float* out, uint8_t* amax, int B, int L, int ls, long long HW,
                           cudaStream_t st) {
   const dim3 grid((unsigned)((HW + 31) / 32), (unsigned)B);
   const size_t smem = (size_t)L * 33 * sizeof(float);
   ProfScope prof(kProfElementwise, st);
   switch (kind) {
-    case 0: lhw_to_hwl_kernel<0><<<grid, 256, smem, st>>>(in, out, amax, L, HW); break;
-    case 1: lhw_to_hwl_kernel<1><<<grid, 256, smem, st>>>(in, out, amax, L, HW); break;
-    case 2: hwl_to_lhw_kernel<0><<<grid, 256, smem, st>>>(in, out, amax, L, HW); break;
-    case 4: lhw_to_hwl_kernel<3><<<grid, 256, smem, st>>>(in, out, amax, L, HW); break;
-    case 5: hwl_to_lhw_kernel<3><<<grid, 256, smem, st>>>(in, out, amax, L, HW); break;
-    default: hwl_to_lhw_kernel<2><<<grid, 256, smem, st>>>(in, out, amax, L, HW); break;
+    case 0: lhw_to_hwl_kernel<0><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
+    case 1: lhw_to_hwl_kernel<1><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
+    case 2: hwl_to_lhw_kernel<0><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
+    case 4: lhw_to_hwl_kernel<3><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
+    case 5: hwl_to_lhw_kernel<3><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
+    default: hwl_to_lhw_kernel<2><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
   }
   count_launch();
   return cudaGetLastError();
@@ -1681,16 +1351,31 @@ cudaError_t launch_energy(const float* unary, const float* ctx, const float* ew,
 }
 
 cudaError_t launch_aggregate(const float* unary, const float* msg, float* cost, uint8_t* label,
-                             long long npix, int L, int D, long long slice, float factor,
+                             long long npix, int L, int ls, int D, long long slice, float factor,
                              int min_a_dir, cudaStream_t st) {
-  const long long n = npix * L;
-  long long blocks = (n + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
+  const long long n = npix * ls;
   ProfScope prof(kProfElementwise, st);
-  const bool vec4 = n % 4 == 0 && slice % 4 == 0 &&
-                    ((reinterpret_cast<uintptr_t>(unary) | reinterpret_cast<uintptr_t>(msg) |
-                      reinterpret_cast<uintptr_t>(cost)) & 15) == 0;
-  if (vec4) {
+  const bool aligned = ((reinterpret_cast<uintptr_t>(unary) | reinterpret_cast<uintptr_t>(msg) |
+                         reinterpret_cast<uintptr_t>(cost)) & 15) == 0;
+  if (label) {
+    auto go = [&](auto kernel, int g) {
+      kernel<<<(unsigned)((npix * g + 255) / 256), 256, 0, st>>>(unary, msg, cost, label, npix, L, ls, D, slice,
+                                                                 factor, min_a_dir);
+    };
+    if (aligned && (ls & 3) == 0) {
+      if (L <= 16) {
+        go(aggregate_label_kernel<4, 4>, 4);
+      } else if (L <= 32) {
+        go(aggregate_label_kernel<8, 4>, 8);
+      } else if (L <= 64) {
+        go(aggregate_label_kernel<16, 4>, 16);
+      } else {
+        go(aggregate_label_kernel<32, 4>, 32);
+      }
+    } else {
+      go(aggregate_label_kernel<32, 1>, 32);
+    }
+  } else if (aligned && n % 4 == 0 && slice % 4 == 0) {
     long long b4 = (n / 4 + 255) / 256;
     if (b4 > 148 * 16) b4 = 148 * 16;
     aggregate_vec4_kernel<<<(int)b4, 256, 0, st>>>(reinterpret_cast<const float4*>(unary),
@@ -1698,23 +1383,21 @@ cudaError_t launch_aggregate(const float* unary, const float* msg, float* cost, 
                                                    reinterpret_cast<float4*>(cost), n / 4, D, slice / 4, factor,
                                                    min_a_dir);
   } else {
+    long long blocks = (n + 255) / 256;
+    if (blocks > 148 * 32) blocks = 148 * 32;
     aggregate_kernel<<<(int)blocks, 256, 0, st>>>(unary, msg, cost, n, D, slice, factor, min_a_dir);
   }
   count_launch();
-  if (label) {
-    label_kernel<<<(int)((npix + 127) / 128), 128, 0, st>>>(cost, label, npix, L);
-    count_launch();
-  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_aggregate_lhw(const float* unary, const float* msg, float* cost, int nimg, int L,
+cudaError_t launch_aggregate_lhw(const float* unary, const float* msg, float* cost, int nimg, int L, int ls,
                                  long long HW, int D, long long slice, float factor, int min_a_dir,
                                  cudaStream_t st) {
   const dim3 grid((unsigned)((HW + 31) / 32), (unsigned)nimg);
   const size_t smem = (size_t)L * 33 * sizeof(float);
   ProfScope prof(kProfElementwise, st);
-  aggregate_lhw_kernel<<<grid, 256, smem, st>>>(unary, msg, cost, L, HW, D, slice, factor, min_a_dir);
+  aggregate_lhw_kernel<<<grid, 256, smem, st>>>(unary, msg, cost, L, ls, HW, D, slice, factor, min_a_dir);
   count_launch();
   return cudaGetLastError();
 }

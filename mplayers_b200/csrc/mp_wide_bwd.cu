@@ -20,8 +20,8 @@ constexpr int kWNS = 2;  // stages in flight per warp
 // [kWNS][K][L] bytes, product tile [16][33], t and index-as-float windows [2][2][LP + 2G], the
 // chain's label-context gradient table by SIGNED offset c - f [2L], the far scatter buffer [LP],
 // kWNS mbarriers.
-__host__ __device__ inline int bwd_wide_floats(int L, int lp, int g, int K, int na) {
-  return kWNS * na * K * L + kWNS * K * L / 4 + 16 * 33 + 4 * (lp + 2 * g) + ((2 * L + 3) & ~3) + lp + 2 * kWNS + 2;
+__host__ __device__ inline int bwd_wide_floats(int L, int ls, int lp, int g, int K, int na) {
+  return kWNS * na * K * ls + kWNS * K * ls / 4 + 16 * 33 + 4 * (lp + 2 * g) + ((2 * L + 3) & ~3) + lp + 2 * kWNS + 2;
 }
 
 // Two adjacent floats added to global memory with one reduction (8-byte aligned address).
@@ -62,11 +62,11 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
   constexpr int NWV = (LPT + 2 * G) / 2;  // float2 loads covering a lane's window
   extern __shared__ __align__(128) float smem[];
   const int lane = threadIdx.x;
-  const int L = p.L, K = p.tma_k;
+  const int L = p.L, LR = p.ls, K = p.tma_k;
   float* ring = smem;                                        // [kWNS][NA][K][L]
-  const int stage_floats = NA * K * L;
+  const int stage_floats = NA * K * LR;
   uint8_t* itile = reinterpret_cast<uint8_t*>(ring + kWNS * stage_floats);  // [kWNS][K][L]
-  float* dtile = ring + kWNS * stage_floats + kWNS * K * L / 4;             // [16][33]
+  float* dtile = ring + kWNS * stage_floats + kWNS * K * LR / 4;             // [16][33]
   float* tbuf = dtile + 16 * 33;                             // [2][WB]
   float* ibuf = tbuf + 2 * WB;                               // [2][WB] argmin as float
   float* acc = ibuf + 2 * WB;                                // [2L] label-context gradient of the chain, cell L + c - f
@@ -93,14 +93,14 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
   const bool whole = nl == LPT;
 
   const long long ibase = (long long)ch.img * p.H * p.W;
-  float* DMr = p.dm_read + (long long)dir * p.slice + ibase * L;  // dM_dir, or P_dir
-  float* DMa = p.dm_acc + ibase * L;
-  float* DU = p.dunary + ibase * L;                               // dU, or C
+  float* DMr = p.dm_read + (long long)dir * p.slice + ibase * LR;  // dM_dir, or P_dir
+  float* DMa = p.dm_acc + ibase * LR;
+  float* DU = p.dunary + ibase * LR;                               // dU, or C
   const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
   float* DE = p.dew ? p.dew + (long long)dir * p.pslice + ibase : nullptr;
-  const uint8_t* MI = p.min_idx + (long long)dir * p.slice + ibase * L;
+  const uint8_t* MI = p.min_idx + (long long)dir * p.slice + ibase * LR;
   const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
-  const int len = ch.len, pstep = ch.pstep, ostep = pstep * L;
+  const int len = ch.len, pstep = ch.pstep, ostep = pstep * LR;
   const int pixl = ch.h0 * p.W + ch.w0 + (len - 1) * pstep;  // last pixel of the chain
   const float rho = p.rho;
   const int nsteps = len - 1;               // steps with a predecessor pixel
@@ -122,19 +122,19 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
       float* T = ring + slot * stage_floats;
       if (lane == 0) {
         fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&full[slot], (unsigned)(rows * NA * L) * 4u);
+        mbar_arrive_expect_tx(&full[slot], (unsigned)(rows * NA * LR) * 4u);
       }
       __syncwarp();
       if (contiguous) {
         const int first = pstep == 1 ? pixl - (s0 + rows - 1) : pixl + s0;
         if (lane < NA)
-          bulk_g2s(T + lane * K * L, (CP && lane == 0 ? DU : DMr) + (long long)first * L,
-                   (unsigned)(rows * L) * 4u, &full[slot]);
+          bulk_g2s(T + lane * K * LR, (CP && lane == 0 ? DU : DMr) + (long long)first * LR,
+                   (unsigned)(rows * LR) * 4u, &full[slot]);
       } else {
         for (int q = lane; q < rows * NA; q += 32) {
           const int u = q / NA, a = q - u * NA;
           const int px = pixl - (s0 + u) * pstep;
-          bulk_g2s(T + (a * K + u) * L, (CP && a == 0 ? DU : DMr) + (long long)px * L, (unsigned)L * 4u,
+          bulk_g2s(T + (a * K + u) * LR, (CP && a == 0 ? DU : DMr) + (long long)px * LR, (unsigned)LR * 4u,
                    &full[slot]);
         }
       }
@@ -142,9 +142,9 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
     // argmin indices of the steps with a predecessor
     for (int u = 0; u < K; ++u) {
       if (s0 + u >= nsteps) break;
-      uint8_t* dst = itile + (slot * K + u) * L;
-      const uint8_t* src = MI + (long long)(pixl - (s0 + u) * pstep) * L;
-      for (int j = 4 * lane; j < L; j += 128)
+      uint8_t* dst = itile + (slot * K + u) * LR;
+      const uint8_t* src = MI + (long long)(pixl - (s0 + u) * pstep) * LR;
+      for (int j = 4 * lane; j < LR; j += 128)
         cp_async4(reinterpret_cast<float*>(dst + j), reinterpret_cast<const float*>(src + j));
     }
     cp_async_commit();
@@ -171,9 +171,9 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
 #pragma unroll
   for (int k = 0; k < RW; ++k) ack[k] = 0.f;  // near offsets of the label-context gradient (this lane's share)
   // output pointers of the current pixel (label c0), moved by one pixel per step
-  float* pA = (CP ? DU : DMa + (long long)dir * p.slice) + (long long)pixl * L + c0;  // C, or the scatter field
-  float* pB = DMr + (long long)pixl * L + c0;                                         // P_dir
-  float* pI = DMa + (long long)inv * p.slice + (long long)pixl * L + c0;              // P_inv
+  float* pA = (CP ? DU : DMa + (long long)dir * p.slice) + (long long)pixl * LR + c0;  // C, or the scatter field
+  float* pB = DMr + (long long)pixl * LR + c0;                                         // P_dir
+  float* pI = DMa + (long long)inv * p.slice + (long long)pixl * LR + c0;              // P_inv
   const bool flip = contiguous && pstep == 1;
 
   // One step.  FULL (warp-uniform): all 32 * LPT labels exist, no per-label bounds tests.  FRONT: the
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
           const float2 a = reinterpret_cast<const float2*>(row)[v];
           x0[2 * v] = a.x, x0[2 * v + 1] = a.y;
           if (CP) {
-            const float2 c = reinterpret_cast<const float2*>(row + K * L)[v];
+            const float2 c = reinterpret_cast<const float2*>(row + K * LR)[v];
             x1[2 * v] = c.x, x1[2 * v + 1] = c.y;
           }
         }
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
         for (int i = 0; i < LPT; ++i) {
           if (i < nl) {
             x0[i] = row[i];
-            if (CP) x1[i] = row[K * L + i];
+            if (CP) x1[i] = row[K * LR + i];
           }
         }
       }
@@ -408,9 +408,9 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
     }
     __syncwarp();
     const int send = len - K * b < K ? len - K * b : K;
-    const float* row = ring + slot * stage_floats + (flip ? rows - 1 : 0) * L + c0;
-    const int rstep = flip ? -L : L;
-    const uint8_t* irow = itile + (slot * K) * L + c0;
+    const float* row = ring + slot * stage_floats + (flip ? rows - 1 : 0) * LR + c0;
+    const int rstep = flip ? -LR : LR;
+    const uint8_t* irow = itile + (slot * K) * LR + c0;
     float* drow = dtile + lane;
     for (int sl = 0; sl < send; ++sl) {
       const int s = K * b + sl;
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
         step(std::false_type{}, std::false_type{}, row, irow, drow, sl);
       }
       row += rstep;
-      irow += L;
+      irow += LR;
       drow += 33;
     }
     // edge-weight gradients of this block: lane j sums row j of the product tile
@@ -465,7 +465,7 @@ template <int LPT, int RW, int SCH>
 cudaError_t launch_bw(BwdParams p, int total, cudaStream_t st) {
   constexpr int LP = 32 * LPT, G = RW & ~1, NA = SCH == 1 ? 2 : 1;
   auto bytes = [&](int k) {
-    return ((size_t)bwd_wide_floats(p.L, LP, G, k, NA) + ((p.L + 3) & ~3) + 4) * sizeof(float);
+    return ((size_t)bwd_wide_floats(p.L, p.ls, LP, G, k, NA) + ((p.L + 3) & ~3) + 4) * sizeof(float);
   };
   // every chain of the launch resident at once where possible: the stage depth shrinks first
   const int per_sm = (total + 147) / 148;
@@ -507,13 +507,13 @@ cudaError_t launch_bw_l(const BwdParams& p, int total, cudaStream_t st) {
 
 }  // namespace
 
-bool bwd_wide_eligible(int L, int ctx_rank, int cp_scheme, const void* dunary, const void* dm_read,
+bool bwd_wide_eligible(int L, int ls, int ctx_rank, int cp_scheme, const void* dunary, const void* dm_read,
                        const void* dm_acc) {
   static const int min_l = [] {  // MPL_WIDE_BWD_MIN_L: tuning / comparison knob (first label count taken)
     const char* e = getenv("MPL_WIDE_BWD_MIN_L");
     return e ? atoi(e) : 33;
   }();
-  if (ctx_rank != 1 || L < min_l || L > 256 || (L & 3) || cp_scheme == 0) return false;
+  if (ctx_rank != 1 || L < min_l || L > 256 || (ls & 3) || cp_scheme == 0) return false;
   if (((uintptr_t)dunary | (uintptr_t)dm_read | (uintptr_t)dm_acc) & 15) return false;
   return !pair_kernels_disabled();
 }
