@@ -43,9 +43,11 @@ class TRWPSoftFunction(torch.autograd.Function):
         label_all = torch.zeros(n_iter, batch, cv, h, w, dtype=torch.uint8, device=dev) \
             if args.enable_saving_label else e8
         if is_training:
-            # entries of pixels without a predecessor are never written and stay 0, as in the reference
-            message_edge_label = unary.new_zeros(n_iter, n_dir, batch, cv, h, w, n_disp, n_disp)
-            cost_index = torch.zeros(n_iter, n_dir, batch, cv, h, w, dtype=torch.uint8, device=dev)
+            # Entries of pixels without a predecessor are 0, as in the reference.  Up to 32 labels the sweeps
+            # write them too (clearing the whole 2.3 GB of a 256 x 256 x 21 training step took 0.62 of 11.3 ms).
+            alloc = torch.empty if n_disp <= 32 else torch.zeros
+            message_edge_label = alloc(n_iter, n_dir, batch, cv, h, w, n_disp, n_disp, dtype=torch.float32, device=dev)
+            cost_index = alloc(n_iter, n_dir, batch, cv, h, w, dtype=torch.uint8, device=dev)
         else:
             message_edge_label, cost_index = e0, e8
         _TRWP.forward_soft(rho, int(n_iter), unary, label_context, ew, message, message_edge_label,
@@ -53,12 +55,16 @@ class TRWPSoftFunction(torch.autograd.Function):
         ctx.intermediate_results = rho, message_edge_label, cost_index, label_context, ew, enable_edge_weights
         ctx.norm_index_override = _norm_index_override(args, cost_index, n_disp)
         ctx.mark_non_differentiable(label_all, message_edge_label, cost_index)
+        # no zero gradients for the outputs that have none: the edge values' would be as large as they are
+        ctx.set_materialize_grads(False)
         return cost_final, label_all, message_edge_label, cost_index
 
     @staticmethod
     def backward(ctx, dcost_final, dlabel_all, dmessage_edge_label, dcost_index):
         rho, message_edge_label, cost_index, label_context, ew, enable_edge_weights = ctx.intermediate_results
         del ctx.intermediate_results
+        if dcost_final is None:
+            return None, None, None, None
         if cost_index.numel() == 0:
             raise RuntimeError("backward needs the edge values saved by a training-mode forward "
                                "(args.training was False)")

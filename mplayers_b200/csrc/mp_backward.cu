@@ -835,227 +835,6 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
   }
 }
 
-// ------------------------------------------------------------------------------------------------
-// Soft (expected-value) TRWP backward, L <= 32: one warp per chain, lane = label c, C + P scheme.
-// Per step the softmin weights of every label are recomputed from the saved edge values,
-//   d(value[c][f]) = t[c] * w[c][f] * (1 - value[c][f] + message[c]),
-// the scatter q[f] = sum_c d(value[c][f]) goes through a shared-memory transpose and is carried to
-// the predecessor pixel in a register; the label-context gradient of row c lives in registers of
-// lane c for the whole chain (diagonal included, as in the reference,
-// MPLayers/TRWP_hard_soft/TRWP_backward_soft.cu:100-127).
-// ------------------------------------------------------------------------------------------------
-constexpr int kSoftPF = 4;  // pixels staged ahead (power of two)
-
-__host__ __device__ inline int bwd_soft_slot_floats(int L) {
-  // L*L edge values copied as the 16-byte aligned superset of their (4-byte aligned) tile: up to 3
-  // floats of slack in front, rounded up to 16 bytes; then the C and P_dir rows (32 floats each)
-  return ((L * L + 6) & ~3) + 64;
-}
-__host__ __device__ inline int bwd_soft_warp_floats(int L) {
-  // ring of kSoftPF slots, transpose tile [32][33], kSoftPF mbarriers (2 floats each)
-  return kSoftPF * bwd_soft_slot_floats(L) + 32 * 33 + 3 + 2 * kSoftPF;
-}
-
-template <int LMAX, bool EXACT>  // EXACT: L == LMAX, every "f < L" test folds away
-__global__ void __launch_bounds__(128, 1) bwd_soft_kernel(const __grid_constant__ BwdParams p) {
-  extern __shared__ __align__(16) float smem[];
-  const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = blockIdx.x * wpb + warp;
-  BChain ch;
-  if (!decode_bchain(p, g, ch)) return;
-  const int L = EXACT ? LMAX : p.L, dir = ch.dir, inv = dir ^ 1;
-  const int n2 = L * L, slot_floats = bwd_soft_slot_floats(L);
-  float* ring = smem + warp * ((bwd_soft_warp_floats(L) + 3) & ~3);   // [kSoftPF][slot_floats]
-  float* tile = ring + kSoftPF * slot_floats;            // [32][33]
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(
-      ring + kSoftPF * slot_floats + ((32 * 33 + 1) & ~1));
-  if (lane == 0) {
-    for (int i = 0; i < kSoftPF; ++i) mbar_init(&full[i], 1);
-    mbar_fence_init();
-  }
-  __syncwarp();
-  const bool act = lane < L;
-  const int lc = act ? lane : L - 1;
-  const bool l2r = (dir & 1) == 0;
-
-  float cr[LMAX], acc[LMAX];
-#pragma unroll
-  for (int f = 0; f < LMAX; ++f) {
-    cr[f] = (act && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, lane, f) : 0.f;
-    acc[f] = 0.f;
-  }
-  const long long ibase = (long long)ch.img * p.H * p.W;
-  float* C = p.dunary + ibase * L + lc;                                   // common part of dM_k
-  float* Pd = p.dm_read + (long long)dir * p.slice + ibase * L + lc;      // P_dir
-  float* Pi = p.dm_read + (long long)inv * p.slice + ibase * L + lc;      // P_inv
-  const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
-  float* DE = p.dew ? p.dew + (long long)dir * p.pslice + ibase : nullptr;
-  const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
-  const float* EL = p.edge_label + ((long long)dir * p.pslice + ibase) * n2;
-  const int len = ch.len, pstep = ch.pstep;
-  const int pixl = ch.h0 * p.W + ch.w0 + (len - 1) * pstep;  // last pixel of the chain
-  const float rho = p.rho;
-
-  // Staging of step s (pixel pixl - s*pstep), kSoftPF steps ahead: its L*L edge values by ONE bulk
-  // copy of the 16-byte aligned superset of the tile (the tile itself is only 4-byte aligned; the
-  // consumer skips the slack), completion on the warp's own mbarrier; its C and P_dir rows by
-  // 4-byte cp.async.  Nothing in the step loop loads from global memory into a register except the
-  // per-block scalars.  A superset that would reach past the end of the saved tensor (the very
-  // last pixel) is copied element by element instead.
-  auto tile_src = [&](int s, unsigned& off_floats, unsigned& bytes, bool& bulk) -> const float* {
-    const float* src = EL + (long long)(pixl - s * pstep) * n2;
-    const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-    off_floats = (unsigned)(a & 15) >> 2;
-    bytes = (unsigned)((off_floats + n2) * 4 + 15) & ~15u;
-    const float* al = src - off_floats;
-    bulk = reinterpret_cast<uintptr_t>(al) + bytes <= reinterpret_cast<uintptr_t>(p.edge_label_end);
-    return bulk ? al : src;
-  };
-  auto issue = [&](int s) {
-    if (s < len) {
-      const int pxs = pixl - s * pstep;
-      const int slot = s & (kSoftPF - 1);
-      float* dst = ring + slot * slot_floats;
-      if (s < len - 1) {
-        unsigned off, bytes;
-        bool bulk;
-        const float* src = tile_src(s, off, bytes, bulk);
-        if (lane == 0) {
-          fence_proxy_async_smem();
-          mbar_arrive_expect_tx(&full[slot], bulk ? bytes : 0u);
-          if (bulk) bulk_g2s(dst, src, bytes, &full[slot]);
-        }
-        if (!bulk)
-          for (int i = lane; i < n2; i += 32) cp_async4(dst + i, src + i);
-      }
-      if (act) {
-        cp_async4(dst + slot_floats - 64 + lane, C + pxs * L);
-        cp_async4(dst + slot_floats - 32 + lane, Pd + pxs * L);
-      }
-    }
-    cp_async_commit();
-  };
-  auto load_blk = [&](int b, float& eb, int& nb) {  // lane l: scalars of step 32*b + l
-    const int s = 32 * b + lane;
-    eb = 1.f;
-    nb = 0;
-    if (s < len - 1) {
-      const int pxs = pixl - s * pstep;
-      if (E) eb = E[pxs];
-      nb = NI[pxs];
-    }
-  };
-
-#pragma unroll
-  for (int s = 0; s < kSoftPF; ++s) issue(s);
-  float e_cur, e_nxt;
-  int n_cur, n_nxt;
-  load_blk(0, e_cur, n_cur);
-  load_blk(1, e_nxt, n_nxt);
-
-  float q = 0.f;
-  int px = pixl;
-  for (int s = 0; s < len; ++s) {
-    if ((s & 31) == 0 && s) {
-      e_cur = e_nxt;
-      n_cur = n_nxt;
-      load_blk((s >> 5) + 1, e_nxt, n_nxt);
-    }
-    cp_async_wait<kSoftPF - 1>();
-    const float* sl = ring + (s & (kSoftPF - 1)) * slot_floats;
-    const float* ev = sl;   // edge values of this pixel inside the slot
-    if (s < len - 1) {
-      unsigned off, bytes;
-      bool bulk;
-      tile_src(s, off, bytes, bulk);
-      if (!mbar_wait(&full[s & (kSoftPF - 1)], (s / kSoftPF) & 1)) {
-        if (lane == 0) atomicExch(p.status, 151);
-        return;
-      }
-      ev = sl + (bulk ? off : 0u);
-    }
-    __syncwarp();
-    const int of = px * L;
-    const float c_old = sl[slot_floats - 64 + lc];
-    const float x0 = c_old + sl[slot_floats - 32 + lc];   // C + P_dir of this pixel
-    const float rq = rho * q;
-    float qn = 0.f;
-    if (s < len - 1) {
-      const float e = __shfl_sync(0xffffffffu, e_cur, s & 31);
-      const int n = __shfl_sync(0xffffffffu, n_cur, s & 31);
-      float d[LMAX];
-#pragma unroll
-      for (int f = 0; f < LMAX; ++f) d[f] = (f < L) ? (l2r ? ev[f * L + lc] : ev[lc * L + f]) : kInf;
-      float t = act ? x0 + rq : 0.f;
-      const float S = warp_sum(t);
-      t = (lane == n) ? t - S : t;
-      // softmin weights of row c
-      float m = d[0];
-#pragma unroll
-      for (int f = 1; f < LMAX; ++f) m = fminf(m, d[f]);
-      float ex[LMAX], se = 0.f, ms = 0.f;
-#pragma unroll
-      for (int f = 0; f < LMAX; ++f) {
-        ex[f] = (f < L) ? __expf(m - d[f]) : 0.f;
-        se += ex[f];
-      }
-      const float inv_se = 1.f / se;
-#pragma unroll
-      for (int f = 0; f < LMAX; ++f) {
-        ex[f] *= inv_se;   // now the weight of candidate f
-        ms = (f < L) ? fmaf(ex[f], d[f], ms) : ms;
-      }
-      float de = 0.f;
-#pragma unroll
-      for (int f = 0; f < LMAX; ++f) {
-        const float dd = (f < L && act) ? t * ex[f] * (1.f - d[f] + ms) : 0.f;
-        tile[lane * 33 + f] = dd;
-        de = fmaf(cr[f], dd, de);
-        acc[f] = fmaf(e, dd, acc[f]);
-      }
-      de = warp_sum(de);
-      if (DE && lane == 0) atomicAdd(DE + px, de);
-      __syncwarp();
-      if (act) {
-        float qa = 0.f, qb = 0.f;
-        int c = 0;
-        for (; c + 1 < L; c += 2) {
-          qa += tile[c * 33 + lane];
-          qb += tile[(c + 1) * 33 + lane];
-        }
-        if (c < L) qa += tile[c * 33 + lane];
-        qn = qa + qb;
-      }
-    }
-    if (act) {
-      const float cnew = c_old + rq;  // dU and every dM_k (k != dir, inv) receive rho*q
-      C[of] = cnew;
-      Pd[of] = -cnew;                 // dM_dir = C + P_dir = 0 after its sweep
-      atomicAdd(Pi + of, -q);
-    }
-    __syncwarp();
-    issue(s + kSoftPF);
-    q = qn;
-    px -= pstep;
-  }
-  cp_async_wait<0>();
-
-  // flush the label-context gradient of this chain (row c = lane)
-  float* part = p.dctx_part + (long long)(g % p.n_slots) * (p.ctx_rank == 2 ? L * L : L);
-  if (act) {
-#pragma unroll
-    for (int f = 0; f < LMAX; ++f) {
-      if (f < L && acc[f] != 0.f) {
-        if (p.ctx_rank == 2) {
-          atomicAdd(part + lane * L + f, acc[f]);
-        } else {
-          atomicAdd(part + (lane > f ? lane - f : f - lane), acc[f]);
-        }
-      }
-    }
-  }
-}
-
 constexpr int kPFB = 8;  // CTA kernel: pixels of dM_d staged ahead (power of two)
 
 // ------------------------------------------------------------------------------------------------
@@ -1548,35 +1327,6 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
     }
     bwd_cta_kernel<<<total, NT, smem, st>>>(p);
   }
-  count_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_backward_soft_sweep(const BwdParams& p0, cudaStream_t st) {
-  BwdParams p = p0;
-  p.ndirs = 1;
-  p.parts = 0;
-  p.chain_begin[0] = 0;
-  p.chain_off[0] = 0;
-  p.chain_off[1] = make_geom(p.dir, p.H, p.W).n_chains * p.nimg;
-  const int total = p.chain_off[1];
-  if (total == 0) return cudaSuccess;
-  if (p.cp_scheme != 1) return cudaErrorNotSupported;
-  if (p.L > 32) return launch_backward_soft_cta(p, total, st);  // one CTA per chain, up to 64 labels
-  const int wpb = 4;
-  const size_t smem = (size_t)wpb * ((bwd_soft_warp_floats(p.L) + 3) & ~3) * sizeof(float);
-  auto go = [&](auto kernel) -> cudaError_t {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
-    kernel<<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
-    return cudaSuccess;
-  };
-  ProfScope prof(kProfBwdSweep, st);
-  cudaError_t e = p.L == 21 ? go(bwd_soft_kernel<21, true>)
-                  : p.L < 21 ? go(bwd_soft_kernel<21, false>) : go(bwd_soft_kernel<32, false>);
-  if (e != cudaSuccess) return e;
   count_launch();
   return cudaGetLastError();
 }

@@ -36,52 +36,6 @@ __device__ __forceinline__ float uu_from_ring(const float* slot, int rs, int col
   return fmaf(s, rho, -slot[(1 + inv) * rs + col]);
 }
 
-// Sum of 32 values in the order of a shuffle-down tree over a warp (x[i] += x[i + 16], then 8, 4,
-// 2, 1; lane 0 holds the total): the order in which the reference's soft kernels reduce a row
-// (MPLayers/TRWP_hard_soft/TRWP_soft.cuh:45-71), so sums agree with them bit for bit.
-__device__ __forceinline__ float tree32_sum(float (&x)[32]) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int i = 0; i < off; ++i) x[i] = __fadd_rn(x[i], x[i + off]);
-  return x[0];
-}
-
-// Soft (expected-value) step of label c = this thread: val[f] = e*ctx(c,f) + h[f], weights
-// softmin_f(val), message = sum_f weight * val (MPLayers/TRWP_hard_soft/TRWP_forward_soft.cu:55-92).
-// Same intrinsics and operation order as the reference: __expf(-val + min), (w * val) / sum.
-template <int LMAX>
-__device__ __forceinline__ float soft_regrow(const float* hb, const float (&cr)[LMAX], float e, int L,
-                                             float (&val)[LMAX]) {
-  constexpr int NV = (LMAX + 3) / 4;
-  float hv[NV * 4];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const float4 t = reinterpret_cast<const float4*>(hb)[q];
-    hv[4 * q] = t.x, hv[4 * q + 1] = t.y, hv[4 * q + 2] = t.z, hv[4 * q + 3] = t.w;
-  }
-#pragma unroll
-  for (int f = 0; f < LMAX; ++f) val[f] = fmaf(e, cr[f], hv[f]);   // +inf beyond L
-  const float m = min_tree<LMAX>(val);
-  float ex[32], sf[32];
-#pragma unroll
-  for (int f = 0; f < 32; ++f) ex[f] = (f < LMAX && f < L) ? __expf(-val[f < LMAX ? f : 0] + m) : 0.f;
-#pragma unroll
-  for (int f = 0; f < 32; ++f) sf[f] = ex[f];
-  const float se = tree32_sum(sf);
-  // (w * val) / se for every f with ONE correctly rounded reciprocal: q0 = a*r, q = q0 + (a - se*q0)*r
-  // is the correctly rounded quotient (Markstein), i.e. the same bits as the IEEE division the
-  // reference performs per element; checked against __fdiv_rn on 3e10 random operand pairs.
-  const float rs = __frcp_rn(se);
-#pragma unroll
-  for (int f = 0; f < 32; ++f) {
-    const float a = __fmul_rn(ex[f], val[f < LMAX ? f : 0]);
-    const float q0 = __fmul_rn(a, rs);
-    sf[f] = (f < LMAX && f < L) ? __fmaf_rn(__fmaf_rn(-se, q0, a), rs, q0) : 0.f;
-  }
-  return tree32_sum(sf);
-}
-
 // ------------------------------------------------------------------------------------------------
 // L <= 32: one warp per chain.  DT = compile-time direction count (0: read it from the params).
 // ------------------------------------------------------------------------------------------------
@@ -94,21 +48,17 @@ __device__ __forceinline__ float soft_regrow(const float* hb, const float (&cr)[
 // and messages are then copied in 16-byte pieces, lane q piece q of their concatenation: one
 // copy instruction for 21 labels and four directions (30 pieces) where the 4-byte form, which also
 // serves unaligned rows, needs one per row and keeps every lane's address arithmetic in the step.
-// SOFT: the soft (expected-value) message instead of the minimum; in training it saves the L x L
-// edge values of every pixel (entry [f][c] for even directions, [c][f] for odd ones, as the
-// reference does, MPLayers/TRWP_hard_soft/TRWP_forward_soft.cu:50-59) and no argmin indices.
-// EXACT: the label count equals LMAX (lets the compiler drop every "f < L" test; used by the soft path).
-template <int LMAX, int DT, bool TRAIN, bool V4 = false, bool SOFT = false, bool EXACT = false>
+template <int LMAX, int DT, bool TRAIN, bool V4>
 __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
   if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
   constexpr bool AGG = DT == 2;
-  const int L = EXACT ? LMAX : p.L, LR = SOFT ? L : p.ls;
+  const int L = p.L, LR = p.ls;
   const int D = DT ? DT : p.D, rows = D + 2;  // D = staged message slices
   const int slot_floats = rows * 32;
-  float* ring = smem + warp * (kPF * slot_floats + 64 + (SOFT ? 32 * 33 : 0));
+  float* ring = smem + warp * (kPF * slot_floats + 64);
   float* hbuf = ring + kPF * slot_floats;
   float* ring_lane = ring + lane;
   const bool act = lane < L;
@@ -132,18 +82,8 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
   float* Mwl = p.msg_write + (long long)ch.dir * p.slice + ibase * LR + lc;
   const bool has_e = p.ew != nullptr;
   const float* E = has_e ? p.ew + (long long)ch.dir * p.pslice + ibase : p.unary;
-  uint8_t* MIl = (TRAIN && !SOFT) ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR + lc : nullptr;
+  uint8_t* MIl = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR + lc : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
-  float* EL = (TRAIN && SOFT) ? p.edge_label + ((long long)ch.dir * p.pslice + ibase) * L * L : nullptr;
-  const bool l2r = (ch.dir & 1) == 0;  // layout of the saved edge values
-  // flat element lane + 32k of a pixel's [c][f] table -> its place in the padded shared tile
-  constexpr int kFlat = SOFT ? (LMAX * LMAX + 31) / 32 : 1;
-  int toff[kFlat];
-#pragma unroll
-  for (int k = 0; k < kFlat; ++k) {
-    const int i = lane + 32 * k, c = i / L;
-    toff[k] = c * 33 + (i - c * L);
-  }
   const int len = ch.len;
   const int ostep = ch.pstep * LR;
   const int dir_row = AGG ? 32 : (1 + ch.dir) * 32, inv_row = AGG ? 64 : (1 + ch.inv) * 32;
@@ -223,45 +163,17 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
     // the message slice in place).
     const float uu_next = uu_of(sl + lc);
     float m_col = 0.f;
-    if constexpr (!SOFT && !TRAIN) m_col = warp_min(act ? fmaf(e, e >= 0.f ? colmin : colmax, hb[lane]) : kInf);
+    if constexpr (!TRAIN) m_col = warp_min(act ? fmaf(e, e >= 0.f ? colmin : colmax, hb[lane]) : kInf);
     float best;
     int bi = 0;
-    if constexpr (SOFT) {
-      float val[LMAX];
-      best = soft_regrow<LMAX>(hb, cr, e, L, val);
-      if (TRAIN) {
-        float* el = EL + (long long)px * L * L;
-        if (l2r) {   // entry [f][c]: lanes are consecutive in memory for every f
-          if (act) {
-#pragma unroll
-            for (int f = 0; f < LMAX; ++f)
-              if (f < L) el[f * L + lane] = val[f];
-          }
-        } else {     // entry [c][f]: through a shared-memory tile so that the stores are coalesced
-          float* tile = hbuf + 64;   // [L][33], private to the warp
-          __syncwarp();
-          if (act) {
-#pragma unroll
-            for (int f = 0; f < LMAX; ++f)
-              if (f < L) tile[lane * 33 + f] = val[f];
-          }
-          __syncwarp();
-          const int n2 = L * L;
-#pragma unroll
-          for (int k = 0; k < kFlat; ++k)
-            if (lane + 32 * k < n2) el[lane + 32 * k] = tile[toff[k]];
-        }
-      }
-    } else {
-      minplus_regrow<LMAX, TRAIN>(hb, cr, e, best, bi);
-    }
+    minplus_regrow<LMAX, TRAIN>(hb, cr, e, best, bi);
     // the minimum over the labels, known before the candidates (see fwd_tma_kernel)
-    const float m = SOFT || TRAIN ? warp_min(act ? best : kInf) : m_col;
+    const float m = TRAIN ? warp_min(act ? best : kInf) : m_col;
     r = best - m;
     if (act) Mwl[of] = r;
     if (TRAIN) {
       const unsigned bal = __ballot_sync(0xffffffffu, act && best == m);
-      if (!SOFT && act) MIl[of] = (uint8_t)bi;
+      if (act) MIl[of] = (uint8_t)bi;
       if (lane == 0) NI[px] = (uint8_t)(31 - __clz(bal));
     }
     __syncwarp();  // every lane has read the slot that is refilled next
@@ -850,19 +762,6 @@ cudaError_t launch_warp(const FwdParams& p, cudaStream_t st) {
   return launch_warp_d<LMAX, 0, TRAIN>(p, st);
 }
 
-template <int LMAX, bool TRAIN, bool EXACT>
-cudaError_t launch_warp_soft(const FwdParams& p, cudaStream_t st) {
-  const int total = p.chain_off[p.ndirs];
-  const int wpb = total >= 148 * 32 ? 4 : 1;
-  const size_t smem = (size_t)wpb * (kPF * (p.D + 2) * 32 + 64 + 32 * 33) * sizeof(float);
-  cudaError_t e = ensure_smem(fwd_warp_kernel<LMAX, 0, TRAIN, false, true, EXACT>, smem);
-  if (e != cudaSuccess) return e;
-  ProfScope prof(kProfFwdSweep, st);
-  fwd_warp_kernel<LMAX, 0, TRAIN, false, true, EXACT><<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
-  count_launch();
-  return cudaGetLastError();
-}
-
 template <int MODE, bool TRAIN>
 cudaError_t launch_cta(const FwdParams& p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
@@ -1189,15 +1088,6 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
   if (p.ctx_rank == 1) return train ? launch_cta_any<1, true>(p, st) : launch_cta_any<1, false>(p, st);
   if (p.L <= 64) return train ? launch_cta_any<2, true>(p, st) : launch_cta_any<2, false>(p, st);
   return train ? launch_cta_any<0, true>(p, st) : launch_cta_any<0, false>(p, st);
-}
-
-// Soft TRWP sweep of the directions described by p (L <= 32 only: one warp per chain).
-cudaError_t launch_forward_soft_sweep(const FwdParams& p, bool train, cudaStream_t st) {
-  if (p.chain_off[p.ndirs] == 0) return cudaSuccess;
-  if (p.L > 32) return launch_forward_soft_cta(p, train, st);  // one CTA per chain, up to 64 labels
-  if (p.L == 21) return train ? launch_warp_soft<21, true, true>(p, st) : launch_warp_soft<21, false, true>(p, st);
-  if (p.L < 21) return train ? launch_warp_soft<21, true, false>(p, st) : launch_warp_soft<21, false, false>(p, st);
-  return train ? launch_warp_soft<32, true, false>(p, st) : launch_warp_soft<32, false, false>(p, st);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -13,8 +13,9 @@
 //   * backward: everything but the t vector is known before the sweep arrives.  Worker warps turn the saved
 //     edge values into the factors G[c][f] = w[c][f] * (1 - v[c][f] + message[c]) several pixels ahead;
 //     the one walker warp is left with t, q' = G^T t and the label-context gradient.
-// 256 x 256, 21 labels: forward sweep 212 -> MEAS_F us, backward sweep 314 -> MEAS_B us.
+// 256 x 256, 21 labels: forward sweep 212 -> 124 us, backward sweep 314 -> 129 us.
 #include <cstdlib>
+#include <type_traits>
 
 #include "mp_common.cuh"
 #include "mp_minplus.cuh"
@@ -46,7 +47,8 @@ __device__ __forceinline__ float quad_tree_sum(const float (&x)[N]) {
 
 // NW = warps that evaluate rows (8 labels each), 2 * NW candidates per lane; one more warp stages the inputs
 // and stores the messages.  Two buffers of everything that crosses warps, one barrier per step.
-template <int NW, bool TRAIN>
+// LT = compile-time label count (0: from the params), L2R = even direction (layout of the saved values).
+template <int NW, int LT, bool TRAIN, bool L2R>
 __global__ void __launch_bounds__((NW + 1) * 32) fwd_soft_kernel(const __grid_constant__ FwdParams p) {
   constexpr int N = 2 * NW;
   extern __shared__ __align__(16) float smem[];
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) fwd_soft_kernel(const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
   const bool steps = decode_chain(p, blockIdx.x, ch);  // false: a single pixel
-  const int L = p.L, D = p.D, rows = D + 2;
+  const int L = LT ? LT : p.L, D = p.D, rows = D + 2;
   const long long ibase = (long long)ch.img * p.H * p.W;
   const int pix0 = ch.h0 * p.W + ch.w0, len = ch.len;
   float* EL = TRAIN ? p.edge_label + ((long long)ch.dir * p.pslice + ibase) * L * L : nullptr;
@@ -135,12 +137,11 @@ __global__ void __launch_bounds__((NW + 1) * 32) fwd_soft_kernel(const __grid_co
   }
 
   const int k = lane & 3, c = warp * 8 + (lane >> 2), cc = c < L ? c : L - 1;
-  const bool l2r = (ch.dir & 1) == 0;  // layout of the saved edge values
   float cr[N];
 #pragma unroll
   for (int j = 0; j < N; ++j) cr[j] = k + 4 * j < L ? ctx_value(p.ctx, p.ctx_rank, L, cc, k + 4 * j) : 0.f;
   // saved entry (c, k + 4j): [f][c] for even directions, [c][f] for odd ones
-  const int eo = l2r ? k * L + c : c * L + k, es = l2r ? 4 * L : 4;
+  const int eo = L2R ? k * L + c : c * L + k, es = L2R ? 4 * L : 4;
   float* el = TRAIN ? EL + (long long)pix0 * L * L + eo : nullptr;
   const long long estep = (long long)ch.pstep * L * L;
   __syncthreads();
@@ -196,7 +197,8 @@ __global__ void __launch_bounds__((NW + 1) * 32) fwd_soft_kernel(const __grid_co
 // ------------------------------------------------------------------------------------------------
 // Backward.  C + P bookkeeping (BwdParams::cp_scheme == 1).  Step s visits chain pixel len - 1 - s.
 // ------------------------------------------------------------------------------------------------
-constexpr int kWorkers = 4;
+// workers per chain (256 x 256 x 21 training step: 2 -> 5.52 ms, 3 -> 5.26, 4 -> 5.38, 6 -> 5.39)
+constexpr int kWorkers = 3;
 constexpr int kGS = 33;  // row stride of a factor table: conflict-free along rows and columns
 
 // One pixel between a worker and the walker: factors G[LMAX][kGS], then rows of 32: old C, C + P_dir,
@@ -213,7 +215,9 @@ __host__ __device__ inline int soft_edge_floats(int L) {
   return (L * L + 6) & ~3;
 }
 
-template <int LMAX>
+// LMAX = label count rounded up to a multiple of four, LT = the label count where it is known at compile time
+// (0: from the params), L2R = even direction (layout of the saved values).
+template <int LMAX, int LT, bool L2R>
 __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __grid_constant__ BwdParams p) {
   using S = SoftSlot<LMAX>;
   constexpr int NS = 2 * kWorkers;  // slots: worker w fills w and w + kWorkers in turn
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __g
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   BChain ch;
   decode_bchain(p, blockIdx.x, ch);
-  const int L = p.L, dir = ch.dir, inv = dir ^ 1, n2 = L * L, edge_floats = soft_edge_floats(L);
+  const int L = LT ? LT : p.L, dir = ch.dir, inv = dir ^ 1, n2 = L * L, edge_floats = soft_edge_floats(L);
   float* slots = smem;                          // [NS][S::kFloats]
   float* edges = smem + NS * S::kFloats;        // [NS][edge_floats]
   for (int i = threadIdx.x; i < NS * S::kFloats; i += blockDim.x) slots[i] = 0.f;  // rows and columns beyond L
@@ -250,13 +254,13 @@ __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __g
   if (warp > 0) {
     // ---------------------------------- worker: lane = label c ----------------------------------
     const int w = warp - 1;
-    const bool l2r = (dir & 1) == 0;
+    constexpr int LC = LT ? LT : LMAX;  // candidates evaluated
     const float* E = p.ew ? p.ew + (long long)dir * p.pslice + ibase : nullptr;
     const uint8_t* NI = p.norm_idx + (long long)dir * p.pslice + ibase;
     const float* EL = p.edge_label + ((long long)dir * p.pslice + ibase) * n2;
-    float cr[LMAX];
+    float cr[LC];
 #pragma unroll
-    for (int f = 0; f < LMAX; ++f) cr[f] = (act && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, lane, f) : 0.f;
+    for (int f = 0; f < LC; ++f) cr[f] = (act && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, lane, f) : 0.f;
     // The L*L edge values of a pixel come by ONE bulk copy of the 16-byte aligned superset of their tile.  A
     // superset that would reach past the end of the saved tensor (the very last pixel) is copied
     // element by element instead.
@@ -319,19 +323,19 @@ __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __g
         unsigned off, bytes;
         tile_src(s, off, bytes);
         const float* ev = edges + slot * edge_floats + off;
-        float d[LMAX];
+        float d[LC];
 #pragma unroll
-        for (int f = 0; f < LMAX; ++f) d[f] = (f < L) ? (l2r ? ev[f * L + lc] : ev[lc * L + f]) : kInf;
-        const float m = min_tree<LMAX>(d);
-        float ex[LMAX], sa = 0.f, sb = 0.f, ma = 0.f, mb = 0.f;
+        for (int f = 0; f < LC; ++f) d[f] = (f < L) ? (L2R ? ev[f * L + lc] : ev[lc * L + f]) : kInf;
+        const float m = min_tree<LC>(d);
+        float ex[LC], sa = 0.f, sb = 0.f, ma = 0.f, mb = 0.f;
 #pragma unroll
-        for (int f = 0; f < LMAX; ++f) {
+        for (int f = 0; f < LC; ++f) {
           ex[f] = (f < L) ? __expf(m - d[f]) : 0.f;
           if (f & 1) sb += ex[f]; else sa += ex[f];
         }
         const float inv_se = 1.f / (sa + sb);
 #pragma unroll
-        for (int f = 0; f < LMAX; ++f) {
+        for (int f = 0; f < LC; ++f) {
           ex[f] *= inv_se;   // the weight of candidate f
           if (f < L) {
             if (f & 1) mb = fmaf(ex[f], d[f], mb); else ma = fmaf(ex[f], d[f], ma);
@@ -340,14 +344,14 @@ __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __g
         const float ms = ma + mb;
         float ha = 0.f, ra = 0.f;
 #pragma unroll
-        for (int f = 0; f < LMAX; ++f) {
-          const float gv = (f < L && act) ? ex[f] * (1.f - d[f] + ms) : 0.f;
-          if (lane < LMAX) G[lane * kGS + f] = gv;
+        for (int f = 0; f < LC; ++f) {
+          const float gv = f < L ? ex[f] * (1.f - d[f] + ms) : 0.f;
+          if (act) G[lane * kGS + f] = gv;  // rows and columns beyond L stay zero
           ha = fmaf(cr[f], gv, ha);
           ra += gv;
         }
-        G[S::kH + lane] = ha;
-        G[S::kR + lane] = ra;
+        G[S::kH + lane] = act ? ha : 0.f;
+        G[S::kR + lane] = act ? ra : 0.f;
         const float sx = warp_sum(x0);
         if (lane == 0) {
           G[S::kS] = sx;
@@ -455,6 +459,9 @@ __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __g
   }
 }
 
+template <int V>
+using Int = std::integral_constant<int, V>;
+
 template <typename K>
 cudaError_t soft_smem(K kernel, size_t bytes) {
   if (bytes <= 48 * 1024 - 8 * 1024) return cudaSuccess;  // next to the static part
@@ -477,10 +484,17 @@ cudaError_t launch_forward_soft_sweep(const FwdParams& p, bool train, cudaStream
     count_launch();
     return cudaGetLastError();
   };
-  if (p.L <= 8) return train ? go(fwd_soft_kernel<1, true>, 1) : go(fwd_soft_kernel<1, false>, 1);
-  if (p.L <= 16) return train ? go(fwd_soft_kernel<2, true>, 2) : go(fwd_soft_kernel<2, false>, 2);
-  if (p.L <= 24) return train ? go(fwd_soft_kernel<3, true>, 3) : go(fwd_soft_kernel<3, false>, 3);
-  return train ? go(fwd_soft_kernel<4, true>, 4) : go(fwd_soft_kernel<4, false>, 4);
+  auto pick = [&](auto nw, auto lt) -> cudaError_t {
+    constexpr int NW = decltype(nw)::value, LT = decltype(lt)::value;
+    if (!train) return go(fwd_soft_kernel<NW, LT, false, true>, NW);
+    return (p.dir0 & 1) == 0 ? go(fwd_soft_kernel<NW, LT, true, true>, NW) : go(fwd_soft_kernel<NW, LT, true, false>, NW);
+  };
+  // (the callers launch one direction at a time)
+  if (p.L <= 8) return pick(Int<1>{}, Int<0>{});
+  if (p.L <= 16) return pick(Int<2>{}, Int<0>{});
+  if (p.L == 21) return pick(Int<3>{}, Int<21>{});
+  if (p.L <= 24) return pick(Int<3>{}, Int<0>{});
+  return pick(Int<4>{}, Int<0>{});
 }
 
 cudaError_t launch_backward_soft_sweep(const BwdParams& p0, cudaStream_t st) {
@@ -503,10 +517,16 @@ cudaError_t launch_backward_soft_sweep(const BwdParams& p0, cudaStream_t st) {
     count_launch();
     return cudaGetLastError();
   };
-  if (p.L <= 8) return go(bwd_soft_kernel<8>, SoftSlot<8>::kFloats);
-  if (p.L <= 16) return go(bwd_soft_kernel<16>, SoftSlot<16>::kFloats);
-  if (p.L <= 24) return go(bwd_soft_kernel<24>, SoftSlot<24>::kFloats);
-  return go(bwd_soft_kernel<32>, SoftSlot<32>::kFloats);
+  auto pick = [&](auto lmax, auto lt) -> cudaError_t {
+    constexpr int LM = decltype(lmax)::value, LT = decltype(lt)::value;
+    return (p.dir & 1) == 0 ? go(bwd_soft_kernel<LM, LT, true>, SoftSlot<LM>::kFloats)
+                            : go(bwd_soft_kernel<LM, LT, false>, SoftSlot<LM>::kFloats);
+  };
+  if (p.L <= 8) return pick(Int<8>{}, Int<0>{});
+  if (p.L <= 16) return pick(Int<16>{}, Int<0>{});
+  if (p.L == 21) return pick(Int<24>{}, Int<21>{});
+  if (p.L <= 24) return pick(Int<24>{}, Int<0>{});
+  return pick(Int<32>{}, Int<0>{});
 }
 
 }  // namespace mpl
