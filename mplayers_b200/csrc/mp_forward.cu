@@ -799,31 +799,37 @@ cudaError_t launch_cta_tma(FwdParams p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Variant with the context rows in shared memory (one [64][68] table per CTA; row stride 68 makes
-// the per-lane 16-byte row reads conflict-free): 164 registers instead of 255, so three chains
-// per SM sub-partition instead of two.  Lane l owns labels l and l + 32.  It is bound by shared
-// memory bandwidth (every step reads both 64-float rows of every lane: 16 KB per warp and step)
-// and still ~8 % faster than the register variant, which is bound by issue latency at two
-// warps per sub-partition.
-constexpr int kPairSWarps = 4;
+// 32 < L <= 64, rows of 16-byte multiples, any context: one WARP per chain, two labels per lane (l and l + 32).
+// No block barrier (the CTA-per-chain kernel needs two per step and two warps per chain).  Every warp
+// stages its own inputs: lane-parallel cp.async.bulk copies (one per array and stage for horizontal chains, one
+// label row per pixel otherwise) into a private ring, completion on the warp's own mbarriers, refilled by
+// the warp itself as soon as it has consumed a stage.
+//
+// Both context rows of a lane are in registers.  Training finds the argmin in two levels: candidates are
+// taken in groups of eight, the highest group attaining the minimum is kept with the running minimum, and
+// only its eight candidates are evaluated again (from a [64][68] table in shared memory, row stride 68: no
+// systematic bank conflicts) to find the label -- 16 flags per label instead of 64.  What bounds a step is the
+// dependent work of two warps per scheduler: 253 registers, eight chains per SM.  Measured on 1024 x 1024 x 64,
+// eight directions, 10 iterations, forward and backward: rows in shared memory and 64 flags per label 145.5
+// ms (bound by 16 KB of shared-memory reads per step), the same with two levels 144.4, this form 137.7;
+// two chains per warp sharing the reads 148.8 - 155, sharing the registers 163.
+constexpr int kPairWarps = 4;
 constexpr int kPairRS = 68;
 
-template <bool TRAIN>
-__device__ __forceinline__ void minplus_rows32(const float* hb, const float* crow, float e, float& best, int& bi) {
-  float cr[32];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float4 t = reinterpret_cast<const float4*>(crow)[q];
-    cr[4 * q] = t.x, cr[4 * q + 1] = t.y, cr[4 * q + 2] = t.z, cr[4 * q + 3] = t.w;
-  }
-  minplus_regrow<32, TRAIN>(hb, cr, e, best, bi);
+// Eight candidates e*ctx + h, two per packed multiply-add.
+__device__ __forceinline__ void pair_cand8(const float* c, const float4& h0, const float4& h1, float e, float (&v)[8]) {
+  ffma2(v[0], v[1], e, e, c[0], c[1], h0.x, h0.y);
+  ffma2(v[2], v[3], e, e, c[2], c[3], h0.z, h0.w);
+  ffma2(v[4], v[5], e, e, c[4], c[5], h1.x, h1.y);
+  ffma2(v[6], v[7], e, e, c[6], c[7], h1.z, h1.w);
 }
 
 template <bool TRAIN>
-__global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(const __grid_constant__ FwdParams p) {
+__global__ void __launch_bounds__(kPairWarps * 32, 2) fwd_pair_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(128) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = p.L, LR = p.ls, D = p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
+  const bool first_it = p.first != 0;  // zero messages (aggregate mode): only the unaries are staged
+  const int L = p.L, LR = p.ls, D = first_it ? 0 : p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   float* ctab = smem;  // [64][kPairRS]
   for (int i = threadIdx.x; i < 64 * kPairRS; i += blockDim.x) {
     const int c = i / kPairRS, f = i - c * kPairRS;
@@ -842,7 +848,7 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
   if (lane == 0) mbar_fence_init();
   __syncthreads();
   ChainCtx ch;
-  if (!decode_chain(p, blockIdx.x * kPairSWarps + warp, ch)) return;
+  if (!decode_chain(p, blockIdx.x * kPairWarps + warp, ch)) return;
 
   const int len = ch.len;
   const int nstages = (len + K - 1) / K;
@@ -895,13 +901,18 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
     const int j = s * K + lane;
     return (E && lane < K && j < len && j >= 1) ? E[pix0 + j * ch.pstep] : 1.f;
   };
-  auto eval_label = [&](const float* hb, const float* row, float e, float& best, int& bi) {
-    float ba, bb;
-    int ia, ib;
-    minplus_rows32<TRAIN>(hb, row, e, ba, ia);
-    minplus_rows32<TRAIN>(hb + 32, row + 32, e, bb, ib);
-    best = fminf(ba, bb);
-    bi = bb <= ba ? ib + 32 : ia;   // the later half wins ties: highest index
+  float ca[64], cb[64];  // the rows of labels la and lb
+#pragma unroll
+  for (int f = 0; f < 64; ++f) ca[f] = rowa[f], cb[f] = rowb[f];
+  // highest label attaining `best` among the eight of group g (a NaN minimum equals nothing: stay in the group)
+  auto label_in_group = [&](const float* hb, const float* row, float e, int g, float best) {
+    const float4* h = reinterpret_cast<const float4*>(hb) + 2 * g;
+    const float4* r4 = reinterpret_cast<const float4*>(row) + 2 * g;
+    const float4 x = r4[0], y = r4[1];
+    const float c[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    float v[8];
+    pair_cand8(c, h[0], h[1], e, v);
+    return 8 * g + (highest_equal<8>(v, best) & 7);
   };
 
   for (int s = 0; s < NS; ++s) issue_stage(s);
@@ -933,18 +944,36 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
       float va = t[la], vb = t[lbc];
       if (!p.agg)
         for (int a = 1; a <= D; ++a) va += t[a * KL + la], vb += t[a * KL + lbc];
-      const float un0 = fmaf(va - t[dir_off + la], rho, -t[inv_off + la]);
-      const float un1 = fmaf(vb - t[dir_off + lbc], rho, -t[inv_off + lbc]);
+      float un0, un1;
+      if (first_it) {
+        un0 = va * rho, un1 = vb * rho;
+      } else {
+        un0 = fmaf(va - t[dir_off + la], rho, -t[inv_off + la]);
+        un1 = fmaf(vb - t[dir_off + lbc], rho, -t[inv_off + lbc]);
+      }
       if (!first) {
         const float e = et[k];
         float* hb = hbuf + hpar;
         hb[la] = fmaf(rho, r0, uu0);
         if (actb) hb[lb] = fmaf(rho, r1, uu1);
         __syncwarp();
-        float b0, b1;
-        int i0, i1;
-        eval_label(hb, rowa, e, b0, i0);
-        eval_label(hb, rowb, e, b1, i1);
+        float b0 = kInf, b1 = kInf;
+        int g0 = 0, g1 = 0;  // highest group of eight attaining the minimum so far
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const float4 h0 = reinterpret_cast<const float4*>(hb)[2 * g], h1 = reinterpret_cast<const float4*>(hb)[2 * g + 1];
+          float v[8];
+          pair_cand8(ca + 8 * g, h0, h1, e, v);
+          const float m0 = min_tree<8>(v);
+          pair_cand8(cb + 8 * g, h0, h1, e, v);
+          const float m1 = min_tree<8>(v);
+          if (g == 0) {
+            b0 = m0, b1 = m1;
+          } else {
+            if (TRAIN) g0 = m0 <= b0 ? g : g0, g1 = m1 <= b1 ? g : g1;
+            b0 = fminf(b0, m0), b1 = fminf(b1, m1);
+          }
+        }
         const float x1 = actb ? b1 : kInf;
         const float m = warp_min(fminf(b0, x1));
         r0 = b0 - m;
@@ -954,7 +983,8 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
         if (TRAIN) {
           const unsigned bal0 = __ballot_sync(0xffffffffu, b0 == m);
           const unsigned bal1 = __ballot_sync(0xffffffffu, x1 == m);
-          mia[0] = (uint8_t)i0;
+          mia[0] = (uint8_t)label_in_group(hb, rowa, e, g0, b0);
+          const int i1 = label_in_group(hb, rowb, e, g1, b1);
           if (actb) mia[32] = (uint8_t)i1;
           if (lane == 0) *nip = (uint8_t)(bal1 ? 63 - __clz(bal1) : 31 - __clz(bal0));
         }
@@ -977,18 +1007,18 @@ __global__ void __launch_bounds__(kPairSWarps * 32, 3) fwd_pair_smem_kernel(cons
 template <bool TRAIN>
 cudaError_t launch_pair(FwdParams p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
-  const int A = (p.agg ? 2 : p.D) + 1;
+  const int A = (p.first ? 0 : p.agg ? 2 : p.D) + 1;
   int K = 4, NS = 3;
   auto per_warp = [&](int k, int ns) { return ((ns * A * k * p.ls + 128 + 2 * k + 2 * ns + 2) + 3) & ~3; };
-  auto bytes = [&](int k) { return ((size_t)64 * kPairRS + (size_t)kPairSWarps * per_warp(k, NS)) * sizeof(float); };
+  auto bytes = [&](int k) { return ((size_t)64 * kPairRS + (size_t)kPairWarps * per_warp(k, NS)) * sizeof(float); };
   while (K > 1 && bytes(K) > 72 * 1024) K >>= 1;
   p.tma_k = K;
   p.tma_stages = NS;
   const size_t smem = bytes(K);
-  cudaError_t e = ensure_smem(fwd_pair_smem_kernel<TRAIN>, smem);
+  cudaError_t e = ensure_smem(fwd_pair_kernel<TRAIN>, smem);
   if (e != cudaSuccess) return e;
   ProfScope prof(kProfFwdSweep, st);
-  fwd_pair_smem_kernel<TRAIN><<<(total + kPairSWarps - 1) / kPairSWarps, kPairSWarps * 32, smem, st>>>(p);
+  fwd_pair_kernel<TRAIN><<<(total + kPairWarps - 1) / kPairWarps, kPairWarps * 32, smem, st>>>(p);
   count_launch();
   return cudaGetLastError();
 }
@@ -1032,7 +1062,13 @@ static bool wide_eligible(const FwdParams& p, bool train) {
          p.host_R <= 16 && cta_tma_eligible(p) && (p.agg || p.D != 2);
 }
 
-bool forward_skips_zero_slices(const FwdParams& p, bool train) { return wide_eligible(p, train); }
+static bool pair_eligible(const FwdParams& p) {
+  return p.L > 32 && p.L <= 64 && cta_tma_eligible(p) && !pair_kernels_disabled();
+}
+
+bool forward_skips_zero_slices(const FwdParams& p, bool train) {
+  return wide_eligible(p, train) || (p.agg && pair_eligible(p));
+}
 
 __global__ void zero_chain_starts_kernel(const __grid_constant__ FwdParams p, float* a, float* b) {
   const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1083,8 +1119,7 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
     return train ? launch_warp<32, true>(rest, st) : launch_warp<32, false>(rest, st);
   }
   if (wide_eligible(p, train)) return launch_forward_wide(p, train, st);
-  if (p.L <= 64 && cta_tma_eligible(p) && !pair_kernels_disabled())
-    return train ? launch_pair<true>(p, st) : launch_pair<false>(p, st);
+  if (pair_eligible(p)) return train ? launch_pair<true>(p, st) : launch_pair<false>(p, st);
   if (p.ctx_rank == 1) return train ? launch_cta_any<1, true>(p, st) : launch_cta_any<1, false>(p, st);
   if (p.L <= 64) return train ? launch_cta_any<2, true>(p, st) : launch_cta_any<2, false>(p, st);
   return train ? launch_cta_any<0, true>(p, st) : launch_cta_any<0, false>(p, st);
