@@ -313,6 +313,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
 cudaError_t launch_analyze(const float* ctx, int L, int rank, const float* ew, long long n_ew,
                            CtxInfo* info, cudaStream_t st);
 cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st);
+// mp_wide_team.cu: several warps per chain, wide windows, no saved indices
+bool forward_team_eligible(const FwdParams& p);
+cudaError_t launch_forward_team(const FwdParams& p, cudaStream_t st);
 // mp_fwd_tma.cu
 bool forward_tma_eligible(const FwdParams& p, int dir, int* stages);
 cudaError_t launch_forward_tma(const FwdParams& p, int dir, int stages, bool train, cudaStream_t st);

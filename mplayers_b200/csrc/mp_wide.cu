@@ -9,7 +9,10 @@ cudaError_t launch_forward_wide_train(const FwdParams& p, cudaStream_t st);  // 
 // evaluation is exact (FwdParams::host_windowed) and that the staging alignment rules hold.
 // `train`: the sweep also saves the argmin and normalisation indices (FwdParams::min_idx / norm_idx).
 cudaError_t launch_forward_wide(const FwdParams& p, bool train, cudaStream_t st) {
-  return train ? launch_forward_wide_train(p, st) : launch_wide_l<false>(p, st);
+  if (train) return launch_forward_wide_train(p, st);
+  // (a first TRWP iteration leaves out the slices that are still zero: only fwd_wide_kernel has that form)
+  if (forward_team_eligible(p) && !(p.first && !p.agg && p.dir0 > 0)) return launch_forward_team(p, st);
+  return launch_wide_l<false>(p, st);
 }
 
 }  // namespace mpl
