@@ -307,10 +307,9 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
     if (rd != msg && p->n_iter > 0 && !p->messages_zero)
       MPL_CUDA(cudaMemcpyAsync(msg_update, msg, (size_t)D * d.slice * sizeof(float), cudaMemcpyDeviceToDevice, st));
   }
-  // With few labels and directions an ISGMR sweep sums U + sum_k M_k itself faster than a separate
-  // pass over all messages does (measured 5.13 -> 4.99 ms on 2x512x512, L = 21, D = 4); with
-  // 256 labels the extra staged rows cost more than the pass (28.4 -> 29.2 ms).
-  const bool use_agg = isgmr && !(L <= 32 && D <= 4);
+  fp.agg = 0;
+  set_dirs(fp, 0, D);
+  const bool use_agg = isgmr && !mpl::forward_sums_messages_itself(fp, train);
   // Zero start: messages known to be zero are neither written nor read where the sweeps can leave them
   // out (375 x 1242 x 128, eight directions, one iteration: 3.40 ms with them).  Either way the
   // pixels that no sweep visits -- the chains' first ones -- have to hold zeros in every buffer.
@@ -361,7 +360,7 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
     if (label_all) {
       const float* cur = isgmr ? rd : msg;  // after the swap `rd` holds this iteration's messages
       // the sums behind an iteration's labels are those the next iteration's sweeps start from
-      have_sums = isgmr && !(L <= 32 && D <= 4) && factor == 1.f && !p->enable_min_a_dir && it + 1 < p->n_iter;
+      have_sums = use_agg && factor == 1.f && !p->enable_min_a_dir && it + 1 < p->n_iter;
       MPL_CUDA(mpl::launch_aggregate(unary, cur, have_sums ? sums : nullptr, label_all + (long long)it * d.npix,
                                      d.npix, L, d.ls, D, d.slice, factor, p->enable_min_a_dir, st));
     }

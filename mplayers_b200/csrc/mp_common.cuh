@@ -319,6 +319,9 @@ cudaError_t launch_forward_team(const FwdParams& p, cudaStream_t st);
 // mp_fwd_tma.cu
 bool forward_tma_eligible(const FwdParams& p, int dir, int* stages);
 cudaError_t launch_forward_tma(const FwdParams& p, int dir, int stages, bool train, cudaStream_t st);
+// ISGMR: do the sweeps of p (agg == 0, all directions) sum U + sum_k M_k themselves faster than a separate pass
+// over the messages (aggregate mode) prepares it?
+bool forward_sums_messages_itself(const FwdParams& p, bool train);
 // Does a sweep described by p run without reading message slices that are known to be zero
 // (FwdParams::first)?  Those it would read otherwise have to hold zeros.
 bool forward_skips_zero_slices(const FwdParams& p, bool train);
