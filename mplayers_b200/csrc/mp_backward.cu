@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(128, 1) bwd_warp_kernel(const __grid_constant_
   // full (symmetric / Toeplitz) context table shared by the CTA
   float* ctab = smem;
   const int ctab_floats = (L * LS + 3) & ~3;
+  dependent_wait();
   for (int i = threadIdx.x; i < L * L; i += blockDim.x)
     ctab[(i / L) * LS + (i % L)] = ctx_value(p.ctx, p.ctx_rank, L, i / L, i % L);
   __syncthreads();
@@ -317,6 +318,7 @@ __global__ void __launch_bounds__(160, 1) bwd_tma_kernel(const __grid_constant__
     }
     mbar_fence_init();
   }
+  dependent_wait();
   for (int i = threadIdx.x; i < L * L; i += blockDim.x)
     ctab[(i / L) * LS + (i % L)] = ctx_value(p.ctx, p.ctx_rank, L, i / L, i % L);
   __syncthreads();
@@ -597,6 +599,7 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
   const int L = FULL ? 64 : p.L, LR = FULL ? 64 : p.ls, LS = L | 1;
   const int ctab_floats = (L * LS + 3) & ~3;
   float* ctab = smem;                              // [L][LS] full context table of the CTA
+  dependent_wait();
   for (int i = threadIdx.x; i < L * L; i += blockDim.x)
     ctab[(i / L) * LS + (i % L)] = ctx_value(p.ctx, p.ctx_rank, L, i / L, i % L);
   const int per_warp = (bwd_pair_floats(L, LR, p.ctx_rank, SCH) + 3) & ~3;
@@ -1030,6 +1033,7 @@ backward_init_lhw_kernel(const float* __restrict__ g, float* __restrict__ dunary
 // MPLayers/ISGMR/ISGMR_backward.cu:39-60, followed by SumMsgKernel and a copy, :482-483).
 __global__ void isgmr_combine_kernel(const float* __restrict__ q, float* __restrict__ dm,
                                      float* __restrict__ dunary, long long n, int D, float rho) {
+  dependent_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     float qv[16];
@@ -1148,8 +1152,7 @@ cudaError_t launch_bwd_tma(const BwdParams& p, cudaStream_t st) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    kernel<<<groups, 160, smem, st>>>(p, maps);
-    return cudaSuccess;
+    return launch_dependent(kernel, groups, 160, smem, st, p, maps);
   };
   if (qm) {
     if (vert) return rev ? go(bwd_tma_kernel<LT, PAD, true, true, true>) : go(bwd_tma_kernel<LT, PAD, true, false, true>);
@@ -1166,9 +1169,8 @@ cudaError_t launch_isgmr_combine(const float* q, float* dm, float* dunary, long 
   long long blocks = (n + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   ProfScope prof(kProfElementwise, st);
-  isgmr_combine_kernel<<<(int)blocks, 256, 0, st>>>(q, dm, dunary, n, D, rho);
   count_launch();
-  return cudaGetLastError();
+  return launch_dependent(isgmr_combine_kernel, (unsigned)blocks, 256, 0, st, q, dm, dunary, n, D, rho);
 }
 
 cudaError_t launch_isgmr_combine_total(const float* q_total, const float* q, float* dm, float* dunary, long long n,
@@ -1279,8 +1281,7 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
       }
-      kernel<<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
-      return cudaSuccess;
+      return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
     };
     // rows of 16-byte multiples at 16-byte aligned bases: staged in 16-byte pieces
     const bool v4 = (p.ls & 3) == 0 && (((uintptr_t)(p.cp_scheme == 1 ? p.dunary : nullptr) | (uintptr_t)p.dm_read) & 15) == 0;
@@ -1306,8 +1307,7 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
     auto go = [&](auto kernel) -> cudaError_t {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      kernel<<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
-      return cudaSuccess;
+      return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
     };
     cudaError_t e;
     if (L == 64) {

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
+  dependent_wait();
   if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
   constexpr bool AGG = DT == 2;
   const int L = p.L, LR = p.ls;
@@ -589,6 +590,7 @@ __global__ void aggregate_kernel(const float* __restrict__ unary, const float* _
 __global__ void __launch_bounds__(256)
 aggregate_vec4_kernel(const float4* __restrict__ unary, const float4* __restrict__ msg, float4* __restrict__ cost,
                       long long n4, int D, long long slice4, float factor, int min_a_dir) {
+  dependent_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4;
        i += (long long)gridDim.x * blockDim.x) {
     const float4 u = unary[i];
@@ -694,6 +696,7 @@ __global__ void __launch_bounds__(256)
 aggregate_label_kernel(const float* __restrict__ unary, const float* __restrict__ msg, float* __restrict__ cost,
                        uint8_t* __restrict__ label, long long npix, int L, int ls, int D, long long slice,
                        float factor, int min_a_dir) {
+  dependent_wait();
   const int lane = threadIdx.x & (G - 1);
   const long long px = (blockIdx.x * 256ll + threadIdx.x) / G;
   const bool live = px < npix;
@@ -786,9 +789,8 @@ cudaError_t launch_warp_d(const FwdParams& p, cudaStream_t st) {
     cudaError_t e = ensure_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfFwdSweep, st);
-    kernel<<<(total + wpb - 1) / wpb, wpb * 32, smem, st>>>(p);
     count_launch();
-    return cudaGetLastError();
+    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
   };
   return rows_aligned(p) ? go(fwd_warp_kernel<LMAX, DT, TRAIN, true>) : go(fwd_warp_kernel<LMAX, DT, TRAIN, false>);
 }
@@ -870,6 +872,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2) fwd_pair_kernel(const __gr
   const bool first_it = p.first != 0;  // zero messages (aggregate mode): only the unaries are staged
   const int L = p.L, LR = p.ls, D = first_it ? 0 : p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   float* ctab = smem;  // [64][kPairRS]
+  dependent_wait();
   for (int i = threadIdx.x; i < 64 * kPairRS; i += blockDim.x) {
     const int c = i / kPairRS, f = i - c * kPairRS;
     ctab[i] = (c < L && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c, f) : 0.f;
@@ -1057,9 +1060,8 @@ cudaError_t launch_pair(FwdParams p, cudaStream_t st) {
   cudaError_t e = ensure_smem(fwd_pair_kernel<TRAIN>, smem);
   if (e != cudaSuccess) return e;
   ProfScope prof(kProfFwdSweep, st);
-  fwd_pair_kernel<TRAIN><<<(total + kPairWarps - 1) / kPairWarps, kPairWarps * 32, smem, st>>>(p);
   count_launch();
-  return cudaGetLastError();
+  return launch_dependent(fwd_pair_kernel<TRAIN>, (total + kPairWarps - 1) / kPairWarps, kPairWarps * 32, smem, st, p);
 }
 
 // Label rows of 16-byte multiples at 16-byte aligned bases: the bulk-copy CTA kernel applies.
@@ -1359,8 +1361,8 @@ cudaError_t launch_aggregate(const float* unary, const float* msg, float* cost, 
                          reinterpret_cast<uintptr_t>(cost)) & 15) == 0;
   if (label) {
     auto go = [&](auto kernel, int g) {
-      kernel<<<(unsigned)((npix * g + 255) / 256), 256, 0, st>>>(unary, msg, cost, label, npix, L, ls, D, slice,
-                                                                 factor, min_a_dir);
+      launch_dependent(kernel, (unsigned)((npix * g + 255) / 256), 256, 0, st, unary, msg, cost, label, npix, L, ls, D,
+                       slice, factor, min_a_dir);
     };
     if (aligned && (ls & 3) == 0) {
       if (L <= 16) {
@@ -1378,10 +1380,9 @@ cudaError_t launch_aggregate(const float* unary, const float* msg, float* cost, 
   } else if (aligned && n % 4 == 0 && slice % 4 == 0) {
     long long b4 = (n / 4 + 255) / 256;
     if (b4 > 148 * 16) b4 = 148 * 16;
-    aggregate_vec4_kernel<<<(int)b4, 256, 0, st>>>(reinterpret_cast<const float4*>(unary),
-                                                   reinterpret_cast<const float4*>(msg),
-                                                   reinterpret_cast<float4*>(cost), n / 4, D, slice / 4, factor,
-                                                   min_a_dir);
+    launch_dependent(aggregate_vec4_kernel, (unsigned)b4, 256, 0, st, reinterpret_cast<const float4*>(unary),
+                     reinterpret_cast<const float4*>(msg), reinterpret_cast<float4*>(cost), n / 4, D, slice / 4, factor,
+                     min_a_dir);
   } else {
     long long blocks = (n + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;

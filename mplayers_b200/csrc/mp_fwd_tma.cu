@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     mbar_fence_init();
   }
   __syncthreads();
+  dependent_wait();
 
   if (warp == 4) {
     // ---------------------------------- producer ----------------------------------
@@ -330,9 +331,8 @@ cudaError_t launch_tma_v(FwdParams p, int dir, int stages, cudaStream_t st) {
     if (!ok) return cudaErrorNotSupported;
   }
   ProfScope prof(kProfFwdSweep, st);
-  fwd_tma_kernel<LMAX, LT, PAD, DT, TRAIN, VERT, FWD><<<groups, 160, smem, st>>>(p, maps);
   count_launch();
-  return cudaGetLastError();
+  return launch_dependent(fwd_tma_kernel<LMAX, LT, PAD, DT, TRAIN, VERT, FWD>, groups, 160, smem, st, p, maps);
 }
 
 template <int LMAX, int LT, bool PAD, int DT, bool TRAIN>

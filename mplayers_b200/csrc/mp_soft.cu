@@ -57,6 +57,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) fwd_soft_kernel(const __grid_co
   __shared__ float ebuf[2];                    // edge weight
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
+  dependent_wait();
   const bool steps = decode_chain(p, blockIdx.x, ch);  // false: a single pixel
   const int L = LT ? LT : p.L, D = p.D, rows = D + 2;
   const long long ibase = (long long)ch.img * p.H * p.W;
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__((kWorkers + 1) * 32) bwd_soft_kernel(const __g
     }
     mbar_fence_init();
   }
+  dependent_wait();
   if (warp == 0) tbuf[0][lane] = tbuf[1][lane] = etbuf[0][lane] = etbuf[1][lane] = 0.f;
   __syncthreads();
   const bool act = lane < L;
@@ -480,9 +482,8 @@ cudaError_t launch_forward_soft_sweep(const FwdParams& p, bool train, cudaStream
     cudaError_t e = soft_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfFwdSweep, st);
-    kernel<<<total, (nw + 1) * 32, smem, st>>>(p);
     count_launch();
-    return cudaGetLastError();
+    return launch_dependent(kernel, total, (nw + 1) * 32, smem, st, p);
   };
   auto pick = [&](auto nw, auto lt) -> cudaError_t {
     constexpr int NW = decltype(nw)::value, LT = decltype(lt)::value;
@@ -513,9 +514,8 @@ cudaError_t launch_backward_soft_sweep(const BwdParams& p0, cudaStream_t st) {
     cudaError_t e = soft_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfBwdSweep, st);
-    kernel<<<total, (kWorkers + 1) * 32, smem, st>>>(p);
     count_launch();
-    return cudaGetLastError();
+    return launch_dependent(kernel, total, (kWorkers + 1) * 32, smem, st, p);
   };
   auto pick = [&](auto lmax, auto lt) -> cudaError_t {
     constexpr int LM = decltype(lmax)::value, LT = decltype(lt)::value;

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
     for (int i = lane; i < 2 * (LP + 2 * G); i += 32) hwin[i] = kInf;  // guards and padding labels
   }
   __syncthreads();
+  dependent_wait();
   if (!valid || warp >= 2 * C) return;  // warps beyond 2C only pad the CTA (see launch_wide_d)
 
   // copies of stage s into its slot of the ring
@@ -444,9 +445,9 @@ cudaError_t launch_wide_s(FwdParams p, cudaStream_t st) {
                            (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   ProfScope prof(kProfFwdSweep, st);
-  fwd_wide_kernel<LPT, RW, DT, TRAIN, SELF><<<ctas, SELF ? C * 32 : C == 1 ? 96 : C * 64, smem, st>>>(p, maps);
   count_launch();
-  return cudaGetLastError();
+  return launch_dependent(fwd_wide_kernel<LPT, RW, DT, TRAIN, SELF>, ctas, SELF ? C * 32 : C == 1 ? 96 : C * 64, smem, st, p,
+                          maps);
 }
 
 template <int LPT, int RW, int DT, bool TRAIN>

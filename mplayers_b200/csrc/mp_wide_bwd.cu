@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
     for (int i = 0; i < kWNS; ++i) mbar_init(&full[i], 1);
     mbar_fence_init();
   }
+  dependent_wait();
   for (int i = lane; i < L; i += 32) {
     acc[i] = 0.f;
     acc[L + i] = 0.f;
@@ -482,8 +483,7 @@ cudaError_t launch_bw(BwdParams p, int total, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  kernel<<<total, 32, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(kernel, total, 32, smem, st, p);
 }
 
 template <int LPT, int SCH>

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
   const int L = p.L, LR = p.ls, D = DT == 1 ? 0 : DT ? DT : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
+  dependent_wait();
   if (!decode_chain(p, blockIdx.x, ch)) return;  // uniform for the CTA
   const int tile_floats = A * K * LR;
   float* tiles = smem;                                   // [NS][A][K][LR]
@@ -322,9 +323,8 @@ cudaError_t launch_team_d(FwdParams p, cudaStream_t st) {
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   ProfScope prof(kProfFwdSweep, st);
-  kernel<<<total, (TW + 1) * 32, smem, st>>>(p, maps);
   count_launch();
-  return cudaGetLastError();
+  return launch_dependent(kernel, total, (TW + 1) * 32, smem, st, p, maps);
 }
 
 template <int LPT, int TW>
