@@ -65,13 +65,15 @@ def _norm_index_override(args, cost_index, n_disp):
 
 class TRWPFunction(torch.autograd.Function):
     """pytorch/MP_module.py:17-86.  unary [B,cv,H,W,L]; label_context [L] or [L,L];
-    edge_weights [D,B,cv,H,W] or None.  Returns (cost_final [B,cv,H,W,L], label_all)."""
+    edge_weights [D,B,cv,H,W] or None.  Returns (cost_final [B,cv,H,W,L], label_all).  `n_disp` (not in the
+    reference): the label count where unary's label rows are padded (mpl_rows::label_stride)."""
     keep_diag = False
 
     @staticmethod
-    def forward(ctx, unary, label_context, edge_weights, args):
+    def forward(ctx, unary, label_context, edge_weights, args, n_disp=None):
         batch, cv, h, w, row = unary.size()   # row >= n_disp elements per pixel (padded label rows)
-        n_disp = _labels_in_row(args, row)
+        ctx.n_extra = 0 if n_disp is None else 1   # inputs beyond the reference's four
+        n_disp = n_disp or row
         rho, n_iter, n_dir, is_training = args.rho, args.mpnet_max_iter, args.mpnet_n_dirs, args.training
         unary = unary.contiguous()
         label_context = label_context.contiguous()
@@ -113,16 +115,17 @@ class TRWPFunction(torch.autograd.Function):
                        dlabel_context, dedge_weights, dmessage, _empty_f32(dcost_final.device),
                        keep_diag=ctx._forward_cls.keep_diag, context_window=ctx.context_window,
                        cost_labels_first=ctx.cost_labels_first, n_disp=ctx.n_disp)
-        return dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None
+        return (dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None) + (None,) * ctx.n_extra
 
 
 class ISGMRFunction(torch.autograd.Function):
     """pytorch/MP_module.py:89-161 (ISGMR and single-iteration SGM)."""
 
     @staticmethod
-    def forward(ctx, unary, label_context, edge_weights, args):
+    def forward(ctx, unary, label_context, edge_weights, args, n_disp=None):
         batch, cv, h, w, row = unary.size()   # row >= n_disp elements per pixel (padded label rows)
-        n_disp = _labels_in_row(args, row)
+        ctx.n_extra = 0 if n_disp is None else 1   # inputs beyond the reference's four
+        n_disp = n_disp or row
         rho, n_iter, n_dir, is_training = args.rho, args.mpnet_max_iter, args.mpnet_n_dirs, args.training
         unary = unary.contiguous()
         label_context = label_context.contiguous()
@@ -166,14 +169,7 @@ class ISGMRFunction(torch.autograd.Function):
                         dunary, dlabel_context, dedge_weights, dmessage,
                         _empty_f32(dcost_final.device), dmessage_tmp, context_window=ctx.context_window,
                         cost_labels_first=ctx.cost_labels_first, n_disp=ctx.n_disp)
-        return dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None
-
-
-def _labels_in_row(args, row):
-    """Label count of a call whose label rows have `row` elements; what the module said about padding
-    counts for one call."""
-    n_disp, args.labels_in_row = int(getattr(args, 'labels_in_row', 0) or row), 0
-    return n_disp
+        return (dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None) + (None,) * ctx.n_extra
 
 
 def _row_elements(args, unary, direction_comm=None):
@@ -281,7 +277,6 @@ class MPModule(torch.nn.Module):
         label_context = self._transformed_label_context()
         self.args.training = self.training
         self.args.cost_labels_first = False
-        self.args.labels_in_row = 0   # packed
         self.args.context_window = self._context_window(label_context, edge_weights)
         if self.args.mpnet_mrf_mode in {'ISGMR', 'SGM'}:
             cost_final, _ = ISGMRFunction.apply(unary, label_context, edge_weights, self.args)
@@ -299,16 +294,15 @@ class MPModule(torch.nn.Module):
         label_context = self._transformed_label_context()
         self.args.training = self.training
         self.args.cost_labels_first = True
-        self.args.labels_in_row = n_disp
         self.args.context_window = self._context_window(label_context, edge_weights)
         fn = ISGMRFunction if self.args.mpnet_mrf_mode in {'ISGMR', 'SGM'} else TRWPFunction
-        cost_final, _ = fn.apply(unary, label_context, edge_weights, self.args)
+        cost_final, _ = fn.apply(unary, label_context, edge_weights, self.args, n_disp)
         self.args.cost_labels_first = False
         return cost_final, label_context.unsqueeze(0)
 
     def forward(self, unary, edge_weights=None):
         # unary [B,cv,L,H,W]; edge_weights [B,D,H,W]
-        self.args.labels_in_row = unary.size(2)
+        n_disp = unary.size(2)
         unary = _glue.label_rows(unary, _row_elements(self.args, unary, self.direction_comm))
         edge_weights = edge_weights.unsqueeze(1).permute(2, 0, 1, 3, 4).contiguous() \
             if (edge_weights is not None) else edge_weights
@@ -330,9 +324,9 @@ class MPModule(torch.nn.Module):
             cost_final = _glue.labels_first(cost_final)
             cost_all = _empty_u8(unary.device)
         elif self.args.mpnet_mrf_mode in {'ISGMR', 'SGM'}:
-            cost_final, cost_all = ISGMRFunction.apply(unary, label_context, edge_weights, self.args)
+            cost_final, cost_all = ISGMRFunction.apply(unary, label_context, edge_weights, self.args, n_disp)
         elif self.args.mpnet_mrf_mode == 'TRWP':
-            cost_final, cost_all = TRWPFunction.apply(unary, label_context, edge_weights, self.args)
+            cost_final, cost_all = TRWPFunction.apply(unary, label_context, edge_weights, self.args, n_disp)
         else:
             assert False
         self.args.cost_labels_first = False

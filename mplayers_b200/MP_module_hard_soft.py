@@ -113,7 +113,7 @@ class MPModule(torch.nn.Module):
         self.args.msg_norm_index = msg_norm_index
         assert self.args.mpnet_mrf_mode == 'TRWP'
         soft = getattr(self.args, 'mpnet_enable_soft', False)   # the soft kernels take packed rows
-        self.args.labels_in_row = 0 if soft else unary.size(2)
+        n_disp = unary.size(2)
         unary = _glue.labels_last(unary) if soft else \
             _glue.label_rows(unary, _row_elements(self.args, unary))
         edge_weights = edge_weights.unsqueeze(1).permute(2, 0, 1, 3, 4).contiguous() \
@@ -141,7 +141,7 @@ class MPModule(torch.nn.Module):
         # the layer writes cost_final (and reads its gradient) with the labels first: no layout pass
         # on the way out (pytorch/MP_module_hard_soft.py permutes here)
         self.args.cost_labels_first = True
-        cost_final, cost_all = TRWPFunction.apply(unary, label_context, edge_weights, self.args)
+        cost_final, cost_all = TRWPFunction.apply(unary, label_context, edge_weights, self.args, n_disp)
         self.args.cost_labels_first = False
         label_context = label_context.unsqueeze(0)
         empty = torch.empty(0, dtype=torch.float32, device=unary.device)
