@@ -438,11 +438,15 @@ int backward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows
   const int cp = isgmr ? 2 : ((L <= 32 || pair_cp || wide_cp) ? 1 : 0);
   float* X = isgmr ? dmsg_update : dmsg;  // gradients of the messages the sweeps produced
   float* Y = isgmr ? dmsg : dmsg;         // gradients of the messages the sweeps read
+  // With C + P every slice P_k starts as zero; the several-labels-per-lane kernel writes each pair of slices
+  // where its first sweep (the pair's odd direction in the last iteration) comes across it instead.
+  const bool fresh_p = cp == 1 && L > 32 && wide_cp;
+  const int n_init = fresh_p ? 0 : D;
   if (p->cost_labels_first) {
     MPL_CUDA(mpl::launch_backward_init_lhw(dcost_final, dunary, X, (int)d.nimg, L, d.ls, (long long)p->height * p->width,
-                                           D, factor, cp == 1, st));
+                                           n_init, factor, cp == 1, st));
   } else {
-    MPL_CUDA(mpl::launch_backward_init(dcost_final, dunary, X, d.slice, D, factor, cp == 1, st));
+    MPL_CUDA(mpl::launch_backward_init(dcost_final, dunary, X, d.slice, n_init, factor, cp == 1, st));
   }
   int* status = ws_status(workspace);
   MPL_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
@@ -467,6 +471,7 @@ int backward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows
       for (int dir = D - 1; dir >= 0; --dir) {
         bp.dir = dir;
         bp.ndirs = 1;
+        bp.fresh = fresh_p && it == p->n_iter - 1 && (dir & 1);
         bp.dm_read = X;
         bp.dm_acc = Y;
         MPL_CUDA(mpl::launch_backward_sweep(bp, st));

@@ -160,6 +160,7 @@ struct BwdParams {
   // independent and run in one launch, and isgmr_combine_kernel afterwards forms
   // dM_k = rho*Q - rho*q_k - q_inv(k), dU += rho*Q with Q = sum_d q_d.
   int cp_scheme;
+  int fresh;              // cp_scheme 1, several-labels-per-lane kernel: P_dir and P_inv have not been written yet (they count as zero)
   int tma_stages;
   int tma_k;              // wide kernel: chain steps per stage
   int window;             // wide kernel: the caller's statement about a rank-1 context (mpl_problem::context_window), or 0
