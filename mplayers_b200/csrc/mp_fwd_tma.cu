@@ -30,6 +30,10 @@ cudaError_t ensure_smem(K kernel, size_t bytes) {
 // ------------------------------------------------------------------------------------------------
 constexpr int kTK = 16;
 
+__host__ __device__ constexpr bool tma_two_level(int lmax) { return lmax > 24; }
+// Floats of a warp's context table: row stride odd, a group of three may reach past the last row.
+__host__ __device__ constexpr int tma_table_floats(int lmax) { return (lmax * (lmax | 1) + 3 + 3) & ~3; }
+
 // LT = compile-time label count (0: runtime, up to LMAX = 32); FWD = the chain walks towards
 // increasing coordinates (directions 0 and 2).
 // PAD: the label rows are padded to a multiple of four (LT > 0 only).
@@ -41,6 +45,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   // pointer up by hand would hide its address space from the compiler and turn every shared
   // access into a slower generic one.)
   extern __shared__ __align__(128) float smem[];
+  constexpr bool kTwo = TRAIN && tma_two_level(LMAX);  // argmin in two levels, see `resolve`
   constexpr bool AGG = DT == 2;  // aggregate mode (see FwdParams::agg): arrays A, M_dir, M_inv
   constexpr int A = DT + 1;      // staged arrays: unary (or aggregate) + DT message slices
   constexpr int AE = A + 1;   // ... + edge weights
@@ -55,7 +60,9 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   float* tiles = smem;                                   // [NS][tile_floats]
   float* etiles = tiles + NS * tile_floats;              // [NS][64]
   float* hbufs = etiles + NS * 64;                       // [4][64]
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(hbufs + 4 * 64);  // [NS]
+  float* ctabs = hbufs + 4 * 64;                         // kTwo: [4][tma_table_floats(LMAX)]
+  unsigned long long* full =
+      reinterpret_cast<unsigned long long*>(ctabs + (kTwo ? 4 * tma_table_floats(LMAX) : 0));  // [NS]
   unsigned long long* empty = full + NS;                 // [NS]
 
   // the four chains of this CTA
@@ -196,12 +203,36 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   }
   // message of the current chain pixel from its predecessor's UU (in `uu`) and running message `r`;
   // TRAIN: the argmin of a pixel is resolved and stored one step later, between the exchange of the
-  // next pixel's h and its use, where the warp would wait for shared memory (`pval`, `pbest`, `pm`;
-  // 2 x 512 x 512 x 21, forward and backward: 4.84 -> 4.73 ms).
-  float pval[TRAIN ? LMAX : 1], pbest = 0.f, pm = 0.f;
-  auto resolve = [&]() {
+  // next pixel's h and its use, where the warp would wait for shared memory (2 x 512 x 512 x 21, forward
+  // and backward: 4.84 -> 4.73 ms).  With 32 candidates it is found in two levels: the minima of groups of
+  // three, which the minimum passes through anyway, tell the highest group attaining it, and that group's
+  // candidates are formed again from h and a context table in shared memory: 11 flags instead of 32
+  // (256 x 256, forward and backward: 28 labels 2.79 -> 2.60 ms; 12 labels 1.80 -> 1.82 and 21 labels at
+  // 2 x 512 x 512 4.62 -> 4.60 ms, where all candidates stay in registers instead).
+  constexpr int kCS = LMAX | 1;
+  constexpr int kKept = kTwo ? (LMAX + 2) / 3 : LMAX;  // group minima, or all candidates
+  float pval[TRAIN ? kKept : 1], pbest = 0.f, pm = 0.f, pe = 0.f;
+  float* ctab = ctabs + (kTwo ? wc * tma_table_floats(LMAX) : 0);
+  if constexpr (kTwo) {
+    for (int i = lane; i < tma_table_floats(LMAX); i += 32) ctab[i] = 0.f;
+    __syncwarp();
+#pragma unroll
+    for (int f = 0; f < LMAX; ++f)
+      if (act) ctab[lane * kCS + f] = cr[f];
+    __syncwarp();
+  }
+  auto resolve = [&](int par) {  // par: the h buffer of the pixel that is resolved
     if constexpr (TRAIN) {
-      const int bi = highest_equal<LMAX>(pval, pbest);
+      int bi = highest_equal<kKept>(pval, pbest);
+      if constexpr (kTwo) {
+        const int f0 = 3 * (bi & 15);  // (a NaN minimum equals nothing: any group)
+        const int at = f0 < LMAX ? f0 : 0;
+        const float* hp = hbuf + par * 32 + at;
+        const float* cp = ctab + lc * kCS + at;
+        const float v1 = fmaf(pe, cp[1], hp[1]);
+        const float v2 = LMAX % 3 == 2 && at + 2 >= LMAX ? kInf : fmaf(pe, cp[2], hp[2]);
+        bi = v2 == pbest ? at + 2 : v1 == pbest ? at + 1 : at;
+      }
       const unsigned bal = __ballot_sync(0xffffffffu, pbest == pm) & lmask;
       *mip = (uint8_t)bi;
       *nip = (uint8_t)(31 - __clz(bal));
@@ -227,15 +258,25 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     }
     const float uu_next = uu_at(t);
     if (TRAIN) {
-      if (pending) resolve();
+      if (pending) resolve(par ^ 1);
       mip += ostep;
       nip += pstep;
     }
-    float val[LMAX];
+    float val[LMAX], pnew[kTwo ? kKept : LMAX];
 #pragma unroll
     for (int f = 0; f + 1 < LMAX; f += 2) ffma2(val[f], val[f + 1], e, e, cr[f], cr[f + 1], hv[f], hv[f + 1]);
     if (LMAX & 1) val[LMAX - 1] = fmaf(e, cr[LMAX - 1], hv[LMAX - 1]);
-    const float best = min_tree<LMAX>(val);
+    float best;
+    if constexpr (kTwo) {
+#pragma unroll
+      for (int i = 0; i < kKept; ++i)
+        pnew[i] = 3 * i + 2 < LMAX   ? min3f(val[3 * i], val[3 * i + 1 < LMAX ? 3 * i + 1 : 0], val[3 * i + 2 < LMAX ? 3 * i + 2 : 0])
+                  : 3 * i + 1 < LMAX ? fminf(val[3 * i], val[3 * i + 1 < LMAX ? 3 * i + 1 : 0])
+                                     : val[3 * i];
+      best = min_tree<kKept>(pnew);
+    } else {
+      best = min_tree<LMAX>(val);
+    }
     if constexpr (TRAIN) m = warp_min(best);
     r = best - m;
     // Unpredicated stores: idle lanes hold the same values as lane L-1 and write the same
@@ -243,9 +284,10 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     *mw = r;
     if constexpr (TRAIN) {
 #pragma unroll
-      for (int f = 0; f < LMAX; ++f) pval[f] = val[f];
+      for (int i = 0; i < kKept; ++i) pval[i] = kTwo ? pnew[i] : val[i];
       pbest = best;
       pm = m;
+      pe = e;
     }
     uu = uu_next;
   };
@@ -289,11 +331,12 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[slot]);
   }
-  if (len > 1) resolve();
+  if (len > 1) resolve((len - 1) & 1);  // (stages hold an even number of pixels)
 }
 
-size_t tma_smem_bytes(int ls, int D, int stages) {
-  return ((size_t)stages * ((size_t)(D + 1) * kTK * 4 * ls + 64) + 4 * 64) * sizeof(float) + 2 * stages * 8 + 16 + 128;
+size_t tma_smem_bytes(int L, int ls, int D, int stages) {  // with the training tables of the 32-label form
+  const int table = L > 16 && L != 21 ? tma_table_floats(32) : 0;
+  return ((size_t)stages * ((size_t)(D + 1) * kTK * 4 * ls + 64) + 4 * 64 + 4 * table) * sizeof(float) + 2 * stages * 8 + 16 + 128;
 }
 
 }  // namespace
@@ -305,7 +348,7 @@ bool forward_tma_eligible(const FwdParams& p, int dir, int* stages) {
   const uintptr_t bits = (uintptr_t)p.unary | (uintptr_t)p.msg_read | (uintptr_t)p.ew;
   if (bits & 15) return false;
   int ns = tma_stage_override() ? tma_stage_override() : 4;
-  while (ns >= 2 && tma_smem_bytes(p.ls, p.agg ? 2 : p.D, ns) > (ns >= 3 ? 110 : 200) * 1024) --ns;
+  while (ns >= 2 && tma_smem_bytes(p.L, p.ls, p.agg ? 2 : p.D, ns) > (ns >= 3 ? 110 : 200) * 1024) --ns;
   if (ns < 2) return false;
   *stages = ns;
   return true;
@@ -319,7 +362,7 @@ cudaError_t launch_tma_v(FwdParams p, int dir, int stages, cudaStream_t st) {
   p.ndirs = 1;
   p.tma_stages = stages;
   const int groups = VERT ? p.nimg * (p.W >> 2) : (p.nimg * p.H + 3) >> 2;
-  const size_t smem = tma_smem_bytes(p.ls, DT, stages);
+  const size_t smem = tma_smem_bytes(p.L, p.ls, DT, stages);
   cudaError_t e = ensure_smem(fwd_tma_kernel<LMAX, LT, PAD, DT, TRAIN, VERT, FWD>, smem);
   if (e != cudaSuccess) return e;
   TmaMaps maps{};

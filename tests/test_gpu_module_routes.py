@@ -1,0 +1,84 @@
+"""Routes of the module calls and of wide-window inference against the general paths, bit for bit."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+import cases
+import gpu_runner as g
+from mplayers_b200 import MP_module
+from mplayers_b200.glue import mp_on_scores
+
+pytestmark = pytest.mark.gpu
+
+
+def _wide_context(L, R, lift):
+    """Quadratic up to offset R, then flat; `lift` > 0 makes offset 0 dearer than offset 1."""
+    k = np.minimum(np.arange(L), R).astype(np.float64)
+    c = 0.02 * k * k
+    c[0] = lift
+    return c.astype(np.float32)
+
+
+@pytest.mark.parametrize("mode,D,H,W,L,R,I,lift", [
+    ("ISGMR", 4, 9, 8, 36, 9, 2, 0.0),      # two warps of two labels per lane, fewest labels
+    ("ISGMR", 4, 11, 13, 128, 15, 3, 0.0),  # the last count of that form
+    ("ISGMR", 4, 6, 9, 132, 16, 2, 0.0),    # four warps: few chains, more than 128 labels
+    ("ISGMR", 4, 130, 120, 132, 12, 2, 0.0),  # two warps of four labels per lane, partly filled lanes
+    ("ISGMR", 8, 20, 18, 256, 15, 2, 0.1),  # aggregate mode; the smallest value not at offset 0
+    ("TRWP", 4, 17, 10, 192, 10, 3, 0.0),
+    ("TRWP", 8, 9, 12, 68, 15, 2, 0.1),
+    ("TRWP", 6, 9, 12, 100, 12, 2, 0.0),    # direction count without an instance of its own
+])
+def test_wide_window_teams(mode, D, H, W, L, R, I, lift):
+    rng = np.random.default_rng(L * 7 + R)
+    unary = (3 * rng.standard_normal((1, 1, H, W, L))).astype(np.float32)
+    ctx = _wide_context(L, R, lift)
+    for ew in (None, rng.uniform(0.0, 1.4, size=(D, 1, 1, H, W)).astype(np.float32)):
+        want = g.forward(mode, unary, ctx, ew, D, I, training=False, context_window=-1)   # every candidate
+        got = g.forward(mode, unary, ctx, ew, D, I, training=False, context_window=R)
+        assert np.array_equal(got["cost"], want["cost"])
+        assert np.array_equal(got["msg"], want["msg"])
+
+
+def _args(mode, D, I, L, train):
+    return types.SimpleNamespace(mpnet_mrf_mode=mode, mpnet_max_iter=I, mpnet_n_dirs=D, n_classes=L,
+                                 mpnet_smoothness_train="on" if train else None, mpnet_term_weight=1.0,
+                                 mpnet_diag_value=0.0, enable_symmetric=True)
+
+
+@pytest.mark.parametrize("mode,D,H,W,L", [("TRWP", 4, 9, 11, 21), ("TRWP", 4, 8, 12, 21), ("ISGMR", 8, 7, 8, 50),
+                                          ("ISGMR", 8, 6, 9, 13)])
+def test_labels_last_memory_and_scores(mode, D, H, W, L):
+    rng = np.random.default_rng(L + W)
+    rows = torch.from_numpy(rng.standard_normal((1, 1, H, W, L)).astype(np.float32)).cuda()
+    ctx = torch.from_numpy(cases.make_context("sym2d", L, rng)).cuda()
+    ew = torch.from_numpy(rng.uniform(0.3, 1.4, size=(1, D, H, W)).astype(np.float32)).cuda()
+    up = torch.from_numpy(rng.uniform(size=(1, 1, L, H, W)).astype(np.float32)).cuda()
+    layer = MP_module.MPModule(_args(mode, D, 2, L, True))
+    layer.set_label_context(torch.nn.Parameter(ctx), None, None)
+    layer.train()
+
+    def run(u):
+        u = u.detach().requires_grad_(True)
+        out = layer(u, edge_weights=ew)[0]
+        return out.detach(), torch.autograd.grad(out, u, up)[0]
+    planes = rows.permute(0, 1, 4, 2, 3)                 # labels last in memory
+    a, b = run(planes), run(planes.contiguous())
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    # the layer on scores: costs = max - scores, result negated
+    scores = rows[:, 0].permute(0, 3, 1, 2).contiguous()
+    costs = (scores.amax(1, keepdim=True) - scores).unsqueeze(1)
+    want = -layer(costs, edge_weights=ew)[0].squeeze(1)
+    assert torch.equal(mp_on_scores(layer, scores, ew)[0], want)
+
+
+@pytest.mark.parametrize("L", [2, 5, 16, 17, 32, 36, 64, 67, 132, 256])
+def test_labels_of_iterations(L):
+    """Lowest label among equal minima, across lanes and rounds; costs quantised so that most minima tie."""
+    rng = np.random.default_rng(L)
+    unary = rng.integers(0, 3, size=(1, 1, 5, 7, L)).astype(np.float32)
+    ctx = cases.make_context("potts2d", L, rng)
+    got = g.forward("TRWP", unary, ctx, None, 4, 1, training=False, save_labels=True)
+    assert np.array_equal(got["label_all"][0], got["cost"].argmin(-1).astype(np.uint8))
