@@ -733,6 +733,7 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
         const float* row = T + (flip ? rows - 1 - u : u) * LR + half * hl;
         float sa = 0.f, sb = 0.f;
         int c = lane >= hn ? lane - hn : lane;  // rotated start: lanes hit distinct banks
+        if (!FULL && c >= hn) c -= hn;          // (33 labels: the second half has 15)
 #pragma unroll 4
         for (int i = 0; i + 1 < hn; i += 2) {
           sa += CP ? row[c] + row[c + kPB * LR] : row[c];

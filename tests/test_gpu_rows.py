@@ -98,6 +98,14 @@ def test_padded_rows_and_zero_start(mode, D, B, H, W, L, I, kind, ewk):
             assert rel_err(got["dew"], ref["dew"]) < 1e-5, row
 
 
+@pytest.mark.parametrize("L", [33, 34, 35, 37, 63])
+@pytest.mark.parametrize("mode,D,I", [("TRWP", 4, 2), ("ISGMR", 4, 2), ("ISGMR", 8, 3)])
+def test_blocks_of_two_labels_per_lane(mode, D, I, L):
+    """33 .. 64 labels with a table: the backward works in blocks of 16 steps and sums a row of gradients in two halves,
+    the upper one of 15 labels at the least.  Chains of more than two blocks, and of one and a bit."""
+    test_padded_rows_and_zero_start(mode, D, 1, 18, 35, L, I, "sym2d", True)
+
+
 def test_rejects_bad_row_strides():
     e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
     for row, n in ((23, 21), (28, 21), (21, 22)):   # no multiple of 4; not the next one; too few elements
