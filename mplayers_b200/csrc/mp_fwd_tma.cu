@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
         const float v1 = fmaf(pe, cp[1], hp[1]);
         const float v2 = LMAX % 3 == 2 && at + 2 >= LMAX ? kInf : fmaf(pe, cp[2], hp[2]);
         bi = v2 == pbest ? at + 2 : v1 == pbest ? at + 1 : at;
+        __syncwarp();  // the next step writes this h buffer before its own barrier
       }
       const unsigned bal = __ballot_sync(0xffffffffu, pbest == pm) & lmask;
       *mip = (uint8_t)bi;
