@@ -134,8 +134,9 @@ def lib():
         L.mpl_static_scratch_status.restype = ctypes.c_int
         L.mpl_static_scratch_status.argtypes = [ctypes.POINTER(ctypes.c_int32)]
         L.mpl_workspace_status_offset.restype = sz
-        L.mpl_selftest_bounded_wait.restype = ctypes.c_int
-        L.mpl_selftest_bounded_wait.argtypes = [vp, sz, ctypes.c_int64, vp]
+        for fn in (L.mpl_selftest_bounded_wait, L.mpl_selftest_team_wait):
+            fn.restype = ctypes.c_int
+            fn.argtypes = [vp, sz, ctypes.c_int64, vp]
         L.mpl_last_error.restype = ctypes.c_char_p
         L.mpl_kernel_launches.restype = ctypes.c_int64
         L.mpl_version.restype = ctypes.c_int32

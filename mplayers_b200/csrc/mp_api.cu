@@ -1042,6 +1042,34 @@ __global__ void selftest_wait_kernel(int* status, long long limit_cycles) {
     if (threadIdx.x == 0) atomicExch(status, 901);
   }
 }
+
+// Two warps that meet at a named barrier every stage; in the second stage the wait of warp 1 gives up and the one of
+// warp 0 does not.  Both must leave behind that stage's barrier: code 902, moved on to 903 by warp 0.
+__global__ void __launch_bounds__(64) selftest_team_wait_kernel(int* status, long long limit_cycles) {
+  __shared__ unsigned long long bar[2];
+  __shared__ int words[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const mpl::StageExit quit{words};
+  if (threadIdx.x == 0) {
+    mpl::mbar_init(&bar[0], 1);
+    mpl::mbar_init(&bar[1], 1);
+    mpl::mbar_fence_init();
+    quit.init();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) mpl::mbar_arrive(&bar[0]);
+  for (int s = 0; s < 4; ++s) {
+    if (!mpl::mbar_wait(&bar[s > 0 ? warp : 0], 0, limit_cycles) && lane == 0) {
+      atomicExch(status, 902);
+      quit.give_up(s);
+    }
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    if (quit.left(s)) {
+      if (warp == 0 && lane == 0) atomicCAS(status, 902, 903);
+      return;
+    }
+  }
+}
 }  // namespace
 
 extern "C" {
@@ -1053,6 +1081,18 @@ int mpl_selftest_bounded_wait(void* workspace, size_t workspace_bytes, int64_t l
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   MPL_CUDA(cudaMemsetAsync(ws_status(workspace), 0, sizeof(int), st));
   selftest_wait_kernel<<<1, 32, 0, st>>>(ws_status(workspace), (long long)limit_cycles);
+  mpl::count_launch();
+  MPL_CUDA(cudaGetLastError());
+  return MPL_OK;
+}
+
+int mpl_selftest_team_wait(void* workspace, size_t workspace_bytes, int64_t limit_cycles, void* stream) {
+  if (!workspace || workspace_bytes < 256) return fail(MPL_ERR_INVALID, "workspace of at least 256 bytes needed");
+  if (limit_cycles < 1 || limit_cycles > 2000000000ll)
+    return fail(MPL_ERR_INVALID, "limit_cycles=%lld outside 1..2e9", (long long)limit_cycles);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  MPL_CUDA(cudaMemsetAsync(ws_status(workspace), 0, sizeof(int), st));
+  selftest_team_wait_kernel<<<1, 64, 0, st>>>(ws_status(workspace), (long long)limit_cycles);
   mpl::count_launch();
   MPL_CUDA(cudaGetLastError());
   return MPL_OK;

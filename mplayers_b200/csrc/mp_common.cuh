@@ -266,6 +266,18 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     if (clock64() - t0 > limit) return false;
   }
 }
+// Warps that meet at a named barrier every step may not lose one of them to a bounded wait that gave up: the others
+// would wait at the next barrier without a limit.  The warp records the fact, takes part in the barriers of its
+// stage on whatever the tile holds (the status word says that the outputs are worthless), and behind the
+// last one all warps read the record and leave together.  Two words in turn, by the parity of the
+// stage: a warp that reads late never sees what a partner records in the next stage.
+struct StageExit {
+  volatile int* word;  // [2] in shared memory
+  __device__ __forceinline__ void init() const { word[0] = word[1] = 0; }  // one thread, before a barrier
+  __device__ __forceinline__ void give_up(int stage) const { word[stage & 1] = 1; }
+  __device__ __forceinline__ bool left(int stage) const { return word[stage & 1] != 0; }  // behind the stage's last barrier
+};
+
 // Tensor maps of the vertical-direction kernels (2-D tiled TMA: one copy brings kTK image rows of
 // a four-pixel-wide column group).  Passed as a __grid_constant__ kernel parameter.
 struct alignas(64) TmaMaps {

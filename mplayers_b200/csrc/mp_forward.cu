@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   int* redB_i = reinterpret_cast<int*>(redB_v + 8);
   unsigned long long* full = reinterpret_cast<unsigned long long*>(redA_v + 32);  // [NS]
   unsigned long long* empty = full + NS;                                          // [NS]
+  const StageExit quit{reinterpret_cast<int*>(empty + NS)};
   const bool act = c < L;
 
   const int len = ch.len;
@@ -422,6 +423,7 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
       mbar_init(&empty[i], 1);
     }
     mbar_fence_init();
+    quit.init();
   }
   CtaCtx<MODE> cc;
   if (!producer) {
@@ -481,8 +483,8 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   for (int s = 0; s < nstages; ++s) {
     const int slot = s % NS;
     if (!mbar_wait(&full[slot], (s / NS) & 1)) {
-      if (c == 0) atomicExch(p.status, 112);
-      return;
+      atomicExch(p.status, 112);
+      quit.give_up(s);
     }
     const int np = len - s * K < K ? len - s * K : K;
     const float* T = tiles + slot * tile_floats;
@@ -521,6 +523,7 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
     if (c < K) etile[((s + 1) & 1) * K + c] = e_next;
     e_next = load_e(s + 2);
     cta_sync(NT);  // every consumer is done with the tile
+    if (quit.left(s)) return;
     if (c == 0) mbar_arrive(&empty[slot]);
   }
 }

@@ -46,6 +46,19 @@ def test_bounded_wait_gives_up_and_reports(monkeypatch):
     assert np.array_equal(got["cost"], want["cost"])
 
 
+def test_warps_that_share_barriers_leave_together():
+    """One warp's wait gives up, its partner's does not: neither may be left waiting at their next barrier."""
+    from mplayers_b200 import _lib
+    ws = _lib.workspace(256, torch.device("cuda"))
+    rc = _lib.lib().mpl_selftest_team_wait(ctypes.c_void_p(ws.data_ptr()), ws.numel(), 200_000,
+                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, _lib.lib().mpl_last_error().decode()
+    torch.cuda.synchronize()
+    st = ctypes.c_int32(-1)
+    assert _lib.lib().mpl_workspace_status(ctypes.c_void_p(ws.data_ptr()), ctypes.byref(st)) == 0
+    assert st.value == 903
+
+
 def test_deferred_check_raises_one_call_later(monkeypatch):
     from mplayers_b200 import _lib
     monkeypatch.delenv("MPL_CHECK_STATUS", raising=False)
