@@ -358,7 +358,8 @@ int mpl_trwp_backward_static(const mpl_problem* p, const float* context, const f
  * mpl_selftest_bounded_wait launches one warp that waits, with a limit of `limit_cycles` clocks, on
  * an mbarrier nothing ever arrives at, so that the give-up path (status code 901) can be exercised
  * without a fault, a trap or an unbounded spin.  mpl_selftest_team_wait does the same with two warps that meet at
- * a barrier every stage, of which one gives up: both leave together (status code 903). */
+ * a barrier every stage, of which one gives up, in the two forms the sweeps use: neither warp is left behind
+ * (the word counts to 4). */
 int mpl_workspace_status(const void* workspace, int32_t* status);
 int mpl_forward_status(const void* workspace, int32_t* status);
 int mpl_static_scratch_status(int32_t* status);

@@ -1043,32 +1043,34 @@ __global__ void selftest_wait_kernel(int* status, long long limit_cycles) {
   }
 }
 
-// Two warps that meet at a named barrier every stage; in the second stage the wait of warp 1 gives up and the one of
-// warp 0 does not.  Both must leave behind that stage's barrier: code 902, moved on to 903 by warp 0.
-__global__ void __launch_bounds__(64) selftest_team_wait_kernel(int* status, long long limit_cycles) {
+// Two warps that meet at a barrier every stage; in the second stage the wait of warp 1 gives up and the one of warp 0
+// does not.  VOTE: both leave at that stage's barrier (barrier_all); else warp 0 walks to the end
+// (barrier_drain).  Warp 1 moves the code from `code` - 1 to `code`, warp 0 on by one when it gets away.
+template <bool VOTE>
+__global__ void __launch_bounds__(64) selftest_team_wait_kernel(int* status, int code, long long limit_cycles) {
   __shared__ unsigned long long bar[2];
-  __shared__ int words[2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const mpl::StageExit quit{words};
   if (threadIdx.x == 0) {
     mpl::mbar_init(&bar[0], 1);
     mpl::mbar_init(&bar[1], 1);
     mpl::mbar_fence_init();
-    quit.init();
   }
   __syncthreads();
   if (threadIdx.x == 0) mpl::mbar_arrive(&bar[0]);
-  for (int s = 0; s < 4; ++s) {
-    if (!mpl::mbar_wait(&bar[s > 0 ? warp : 0], 0, limit_cycles) && lane == 0) {
-      atomicExch(status, 902);
-      quit.give_up(s);
-    }
-    asm volatile("bar.sync 1, 64;" ::: "memory");
-    if (quit.left(s)) {
-      if (warp == 0 && lane == 0) atomicCAS(status, 902, 903);
-      return;
+  constexpr int kStages = 4;
+  for (int s = 0; s < kStages; ++s) {
+    const bool ok = __all_sync(0xffffffffu, mpl::mbar_wait(&bar[s > 0 ? warp : 0], 0, limit_cycles));
+    if (!ok && lane == 0) atomicCAS(status, code - 1, code);
+    if (VOTE) {
+      if (!mpl::barrier_all(64, ok)) break;
+    } else if (ok) {
+      mpl::barrier_drain(64, 1);
+    } else {
+      mpl::barrier_drain(64, kStages - s);
+      break;
     }
   }
+  if (warp == 0 && lane == 0) atomicCAS(status, code, code + 1);
 }
 }  // namespace
 
@@ -1092,8 +1094,9 @@ int mpl_selftest_team_wait(void* workspace, size_t workspace_bytes, int64_t limi
     return fail(MPL_ERR_INVALID, "limit_cycles=%lld outside 1..2e9", (long long)limit_cycles);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   MPL_CUDA(cudaMemsetAsync(ws_status(workspace), 0, sizeof(int), st));
-  selftest_team_wait_kernel<<<1, 64, 0, st>>>(ws_status(workspace), (long long)limit_cycles);
-  mpl::count_launch();
+  selftest_team_wait_kernel<true><<<1, 64, 0, st>>>(ws_status(workspace), 1, (long long)limit_cycles);
+  selftest_team_wait_kernel<false><<<1, 64, 0, st>>>(ws_status(workspace), 3, (long long)limit_cycles);
+  mpl::count_launch(2);
   MPL_CUDA(cudaGetLastError());
   return MPL_OK;
 }

@@ -266,17 +266,27 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     if (clock64() - t0 > limit) return false;
   }
 }
-// Warps that meet at a named barrier every step may not lose one of them to a bounded wait that gave up: the others
-// would wait at the next barrier without a limit.  The warp records the fact, takes part in the barriers of its
-// stage on whatever the tile holds (the status word says that the outputs are worthless), and behind the
-// last one all warps read the record and leave together.  Two words in turn, by the parity of the
-// stage: a warp that reads late never sees what a partner records in the next stage.
-struct StageExit {
-  volatile int* word;  // [2] in shared memory
-  __device__ __forceinline__ void init() const { word[0] = word[1] = 0; }  // one thread, before a barrier
-  __device__ __forceinline__ void give_up(int stage) const { word[stage & 1] = 1; }
-  __device__ __forceinline__ bool left(int stage) const { return word[stage & 1] != 0; }  // behind the stage's last barrier
-};
+// Warps that meet at named barriers every step may not lose one of them to a bounded wait that gave up: the others
+// would wait at their next barrier without a limit.  Two ways out, chosen by what they cost the kernel:
+//   * barrier_all: named barrier 1 over `nthreads` threads, true in all of them if `ok` holds in all of them.  The
+//     last barrier of a stage carries the outcome of its wait, and all leave there together.
+//   * barrier_drain: the warp that gives up (all of its lanes) takes part in the `n` barriers that remain of
+//     its chain and then leaves.
+__device__ __forceinline__ bool barrier_all(int nthreads, bool ok) {
+  unsigned all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "bar.red.and.pred p, 1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(all)
+      : "r"((unsigned)ok), "r"(nthreads)
+      : "memory");
+  return all != 0;
+}
+__device__ __forceinline__ void barrier_drain(int nthreads, int n) {
+  for (; n > 0; --n) asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+}
 
 // Tensor maps of the vertical-direction kernels (2-D tiled TMA: one copy brings kTK image rows of
 // a four-pixel-wide column group).  Passed as a __grid_constant__ kernel parameter.

@@ -408,7 +408,6 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   int* redB_i = reinterpret_cast<int*>(redB_v + 8);
   unsigned long long* full = reinterpret_cast<unsigned long long*>(redA_v + 32);  // [NS]
   unsigned long long* empty = full + NS;                                          // [NS]
-  const StageExit quit{reinterpret_cast<int*>(empty + NS)};
   const bool act = c < L;
 
   const int len = ch.len;
@@ -423,7 +422,6 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
       mbar_init(&empty[i], 1);
     }
     mbar_fence_init();
-    quit.init();
   }
   CtaCtx<MODE> cc;
   if (!producer) {
@@ -482,10 +480,7 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   float uu = 0.f, r = 0.f;
   for (int s = 0; s < nstages; ++s) {
     const int slot = s % NS;
-    if (!mbar_wait(&full[slot], (s / NS) & 1)) {
-      atomicExch(p.status, 112);
-      quit.give_up(s);
-    }
+    const bool ok = mbar_wait(&full[slot], (s / NS) & 1);
     const int np = len - s * K < K ? len - s * K : K;
     const float* T = tiles + slot * tile_floats;
     const float* et = etile + (s & 1) * K;
@@ -522,8 +517,10 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
     }
     if (c < K) etile[((s + 1) & 1) * K + c] = e_next;
     e_next = load_e(s + 2);
-    cta_sync(NT);  // every consumer is done with the tile
-    if (quit.left(s)) return;
+    if (!barrier_all(NT, ok)) {  // every consumer is done with the tile
+      if (c == 0) atomicExch(p.status, 112);
+      return;
+    }
     if (c == 0) mbar_arrive(&empty[slot]);
   }
 }

@@ -20,7 +20,7 @@ namespace {
 constexpr int kRW = 16;  // window half-width (candidates |c - f| < kRW)
 constexpr int kG = 16;   // guard band (floats) on both sides of the h buffer
 
-// Shared memory of a chain: staging ring, two h buffers with guards, edge weights, reductions, barriers, StageExit.
+// Shared memory of a chain: staging ring, two h buffers with guards, edge weights, reductions, barriers.
 __host__ __device__ inline size_t team_bytes(int ns, int A, int k, int ls, int lp, int tw) {
   const size_t b = ((size_t)ns * A * k * ls + 2 * (lp + 2 * kG) + 2 * k + 4 * tw + 2) * sizeof(float) + 2 * ns * 8 + 16;
   return (b + 127) & ~(size_t)127;
@@ -54,7 +54,6 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
   float* redb = redh + 2 * TW;                           // [2][TW] smallest message of each warp
   unsigned long long* full = reinterpret_cast<unsigned long long*>(redb + 2 * TW);
   unsigned long long* empty = full + NS;
-  const StageExit quit{reinterpret_cast<int*>(empty + NS)};
   const int len = ch.len;
   const int nstages = (len + K - 1) / K;
   const long long ibase = (long long)ch.img * p.H * p.W;
@@ -67,7 +66,6 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
       mbar_init(&empty[i], TW);
     }
     mbar_fence_init();
-    quit.init();
   }
   for (int i = threadIdx.x; i < 2 * (LP + 2 * kG); i += blockDim.x) hwin[i] = kInf;  // guards and padding labels
   __syncthreads();
@@ -148,11 +146,11 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
   bool first = true;  // chain pixel 0 only provides inputs
   for (int s = 0; s < nstages; ++s) {
     const int slot = s % NS;
-    if (!mbar_wait(&full[slot], (s / NS) & 1)) {
-      if (lane == 0) {
-        atomicExch(p.status, 122);
-        quit.give_up(s);
-      }
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], (s / NS) & 1))) {
+      if (lane == 0) atomicExch(p.status, 122);
+      const int steps = len - (s > 0 ? s * K : 1);  // left of the chain: one or two barriers each, and one a stage
+      barrier_drain(TW * 32, nstages - s + (zero_min ? steps : 2 * steps));
+      return;
     }
     const int np = len - s * K < K ? len - s * K : K;
     const float* et = etile + (s & 1) * K;
@@ -285,7 +283,6 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
       e_next = load_e(s + 2);
     }
     team_sync<TW>();
-    if (quit.left(s)) return;
     if (lane == 0) mbar_arrive(&empty[slot]);
   }
 }
