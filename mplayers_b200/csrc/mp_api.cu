@@ -308,6 +308,8 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
       MPL_CUDA(cudaMemcpyAsync(msg_update, msg, (size_t)D * d.slice * sizeof(float), cudaMemcpyDeviceToDevice, st));
   }
   fp.agg = 0;
+  fp.msg_read = rd;
+  fp.msg_write = wr;
   set_dirs(fp, 0, D);
   const bool use_agg = isgmr && !mpl::forward_sums_messages_itself(fp, train);
   // Zero start: messages known to be zero are neither written nor read where the sweeps can leave them
@@ -316,7 +318,6 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
   bool skip_zero = false;
   if (p->messages_zero) {
     fp.agg = use_agg ? 1 : 0;
-    fp.msg_read = rd;
     skip_zero = p->n_iter > 0 && mpl::forward_skips_zero_slices(fp, train);
     if (!skip_zero) MPL_CUDA(cudaMemsetAsync(rd, 0, (size_t)D * d.slice * sizeof(float), st));
     // (directions beyond 3 of a TRWP iteration read all slices)

@@ -1093,14 +1093,14 @@ cudaError_t launch_analyze(const float* ctx, int L, int rank, const float* ew, l
 
 // Does this sweep (L > 32) run on the several-labels-per-lane kernel?  It evaluates at most 31
 // candidates per label against the pair kernel's 64: 2.0 against 7.2 ms for a 512 x 512 x 64
-// training forward.
+// training forward.  It stores messages in 8-byte pieces, the other kernels for these sizes one by one.
 static bool wide_eligible(const FwdParams& p, bool train) {
   static const bool no_wide_train = [] {  // MPL_NO_WIDE_TRAIN=1: tuning / comparison knob
     const char* e = getenv("MPL_NO_WIDE_TRAIN");
     return e && e[0] == '1';
   }();
   return p.L > 32 && p.L <= 256 && p.ctx_rank == 1 && (!train || !no_wide_train) && p.host_windowed &&
-         p.host_R <= 16 && cta_tma_eligible(p) && (p.agg || p.D != 2);
+         p.host_R <= 16 && cta_tma_eligible(p) && ((uintptr_t)p.msg_write & 7) == 0 && (p.agg || p.D != 2);
 }
 
 static bool pair_eligible(const FwdParams& p) {

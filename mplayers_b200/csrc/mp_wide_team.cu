@@ -340,9 +340,10 @@ cudaError_t launch_team(const FwdParams& p, cudaStream_t st) {
 
 }  // namespace
 
-// Few enough chains that they do not fill the schedulers one warp each; more are left to fwd_wide_kernel.
+// Few enough chains that they do not fill the schedulers one warp each; more are left to fwd_wide_kernel, and so are
+// message buffers that do not take 16-byte stores (ISGMR writes another buffer than the one it stages).
 bool forward_team_eligible(const FwdParams& p) {
-  return p.host_R > 8 && p.chain_off[p.ndirs] < 148 * 16;
+  return p.host_R > 8 && p.chain_off[p.ndirs] < 148 * 16 && ((uintptr_t)p.msg_write & 15) == 0;
 }
 
 cudaError_t launch_forward_team(const FwdParams& p, cudaStream_t st) {

@@ -7,7 +7,7 @@ import torch
 
 import cases
 import gpu_runner as g
-from mplayers_b200 import MP_module
+from mplayers_b200 import ISGMR, MP_module
 from mplayers_b200.glue import mp_on_scores
 
 pytestmark = pytest.mark.gpu
@@ -40,6 +40,34 @@ def test_wide_window_teams(mode, D, H, W, L, R, I, lift):
         got = g.forward(mode, unary, ctx, ew, D, I, training=False, context_window=R)
         assert np.array_equal(got["cost"], want["cost"])
         assert np.array_equal(got["msg"], want["msg"])
+
+
+@pytest.mark.parametrize("shift", [1, 2])
+@pytest.mark.parametrize("I", [1, 2])
+def test_message_buffer_off_the_alignment(I, shift):
+    """ISGMR writes one message buffer while it stages the other: one that takes no 16-byte stores (8 bytes off), or no
+    8-byte ones (4 bytes off), goes to kernels that store smaller pieces."""
+    D, H, W, L, R = 4, 11, 13, 256, 15   # four labels per lane, several warps per chain
+    rng = np.random.default_rng(shift)
+    unary = (3 * rng.standard_normal((1, 1, H, W, L))).astype(np.float32)
+    ctx = _wide_context(L, R, 0.0)
+    u, c = torch.from_numpy(unary).cuda(), torch.from_numpy(ctx).cuda()
+    e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
+    for training in (False, True):
+        want = g.forward("ISGMR", unary, ctx, None, D, I, training=training, context_window=R)
+        for zero in (False, True):
+            first, other = torch.zeros(D, 1, 1, H, W, L, device="cuda"), torch.zeros(shift + D * H * W * L, device="cuda")
+            other = other[shift:].view(first.shape)
+            # the buffer written by the first iteration is the second one for an even count
+            msg, mu = (other, first) if I % 2 else (first, other)
+            cost = torch.empty_like(u)
+            mi = torch.zeros(I, D, 1, 1, H, W, L, dtype=torch.uint8, device="cuda") if training else e8
+            ni = torch.zeros(I, D, 1, 1, H, W, dtype=torch.uint8, device="cuda") if training else e8
+            ISGMR.forward(0, 1.0, I, 0, u, c, e0, msg, cost, mi, ni, e0, mu, e8, context_window=R, messages_zero=zero)
+            assert np.array_equal(cost.cpu().numpy(), want["cost"])
+            assert np.array_equal(msg.cpu().numpy(), want["msg"])
+            if training:
+                assert np.array_equal(mi.cpu().numpy(), want["min_idx"])
 
 
 def _args(mode, D, I, L, train):
