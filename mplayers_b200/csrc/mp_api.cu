@@ -510,6 +510,9 @@ int32_t mpl_label_stride(const mpl_problem* p, int32_t isgmr) {
   Dims d;
   if (validate(p, &d) != MPL_OK) return 0;
   const int L = p->n_disp, padded = (L + 3) & ~3;
+  const mpl_rows rows{padded, 0};
+  const Problem q = with_rows(p, &rows);
+  if (validate(&q, &d) != MPL_OK) return L;  // too many elements with the padding
   if (L > 32) return padded;
   // up to 32 labels: the axis directions of an image whose width is a multiple of 4 have aligned row
   // segments whatever L is; everything else goes through kernels that stage one label row per

@@ -75,6 +75,19 @@ def test_workspace_sizes():
     assert lib.mpl_workspace_status_offset() == 64
 
 
+@pytest.mark.parametrize("h,w,n", [(7800, 7800, 33), (9999, 10001, 21)])
+def test_proposed_label_stride_is_one_a_call_accepts(h, w, n):
+    """Packed rows fit the kernels' 2^31 elements per image here, padded ones do not."""
+    lib = _lib.lib()
+    padded = (n + 3) & ~3
+    assert h * w * n < 2 ** 31 <= h * w * padded
+    p = _prob(height=h, width=w, n_disp=n)
+    for isgmr in (0, 1):
+        assert lib.mpl_label_stride(ctypes.byref(p), isgmr) == n
+    p = _prob(height=h // 2, width=w, n_disp=n)
+    assert lib.mpl_label_stride(ctypes.byref(p), 0) == padded
+
+
 @pytest.mark.parametrize("hw", [(1, 1), (1, 7), (5, 1), (2, 3), (6, 7), (13, 4)])
 def test_chains_partition_the_image(hw):
     H, W = hw
