@@ -91,8 +91,8 @@ typedef struct mpl_rows {
                                whose values do not matter on input and are unspecified on output.
                                Rows of 16-byte multiples let label counts that are no multiple of 4 take
                                the bulk-copy and several-labels-per-lane kernels (mpl_label_stride
-                               proposes a value).  A padded forward call needs a larger workspace
-                               (mpl_forward_workspace_bytes_rows), where the per-iteration sums are kept:
+                               proposes a value).  A padded ISGMR forward call needs a larger workspace
+                               (mpl_forward_workspace_bytes_mode), where the per-iteration sums are kept:
                                a labels-first cost_final has no padding. */
   int32_t messages_zero;    /* forward calls: 1 = the iterations start from zero messages whatever `msg` (and
                                `msg_update`) hold, which then need not be initialised; on return `msg` is
@@ -110,9 +110,12 @@ int mpl_analyze_context(const mpl_problem* p, const float* context, const float*
  * fastest; n_disp where packed rows are as good.  0 if `p` is invalid. */
 int32_t mpl_label_stride(const mpl_problem* p, int32_t isgmr);
 
-/* Bytes of device scratch the forward / backward entry points need for `p` (never 0). */
+/* Bytes of device scratch the forward / backward entry points need for `p` (never 0).  The per-iteration sums of a
+ * padded call are only formed by mpl_isgmr_* (isgmr = 1), and not in a first iteration from zero
+ * messages; mpl_forward_workspace_bytes_rows is enough for either mode. */
 size_t mpl_forward_workspace_bytes(const mpl_problem* p);
 size_t mpl_forward_workspace_bytes_rows(const mpl_problem* p, const mpl_rows* rows);
+size_t mpl_forward_workspace_bytes_mode(const mpl_problem* p, const mpl_rows* rows, int32_t isgmr);
 size_t mpl_backward_workspace_bytes(const mpl_problem* p);
 
 /* TRWP forward.  Replaces TRWP.forward of the reference extension

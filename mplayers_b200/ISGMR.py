@@ -29,7 +29,7 @@ def forward(enable_sgm, rho, n_iter, enable_min_a_dir, unary, context, edge_weig
                     context_window=context_window, cost_labels_first=cost_labels_first, n_disp=n_disp)
     rows = _lib.Rows(unary.size(-1), int(bool(messages_zero)))
     with torch.cuda.device(dev):
-        nbytes = _lib.lib().mpl_forward_workspace_bytes_rows(ctypes.byref(prob), ctypes.byref(rows))
+        nbytes = _lib.lib().mpl_forward_workspace_bytes_mode(ctypes.byref(prob), ctypes.byref(rows), 1)
         ws = _lib.workspace(nbytes, dev)
         _lib.check(_lib.lib().mpl_isgmr_forward_rows(
             ctypes.byref(prob), ctypes.byref(rows), _lib.ptr(unary), _lib.ptr(context), _lib.ptr(edge_weights),

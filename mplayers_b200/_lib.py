@@ -63,6 +63,8 @@ def lib():
         rp = ctypes.POINTER(Rows)
         L.mpl_forward_workspace_bytes_rows.restype = sz
         L.mpl_forward_workspace_bytes_rows.argtypes = [pp, rp]
+        L.mpl_forward_workspace_bytes_mode.restype = sz
+        L.mpl_forward_workspace_bytes_mode.argtypes = [pp, rp, i32]
         for name, n_ptr in (("trwp_forward", 9), ("trwp_backward", 10), ("isgmr_forward", 10), ("isgmr_backward", 11)):
             fn = getattr(L, "mpl_%s_rows" % name)
             fn.restype = ctypes.c_int

@@ -281,9 +281,9 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
     return fail(MPL_ERR_INVALID, "NULL tensor pointer");
   if ((msg_min_index == nullptr) != (msg_norm_index == nullptr))
     return fail(MPL_ERR_INVALID, "msg_min_index and msg_norm_index must both be given or both be NULL");
-  if (!workspace || workspace_bytes < mpl_forward_workspace_bytes_rows(p, rows))
+  if (!workspace || workspace_bytes < mpl_forward_workspace_bytes_mode(p, rows, isgmr))
     return fail(MPL_ERR_INVALID, "workspace too small: %zu < %zu", workspace_bytes,
-                mpl_forward_workspace_bytes_rows(p, rows));
+                mpl_forward_workspace_bytes_mode(p, rows, isgmr));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool train = msg_min_index != nullptr;
   const int D = p->n_dir, L = p->n_disp;
@@ -522,12 +522,18 @@ int32_t mpl_label_stride(const mpl_problem* p, int32_t isgmr) {
   return row_staged ? padded : L;
 }
 
-size_t mpl_forward_workspace_bytes_rows(const mpl_problem* p, const mpl_rows* rows) {
+size_t mpl_forward_workspace_bytes_mode(const mpl_problem* p, const mpl_rows* rows, int32_t isgmr) {
   Dims d;
   if (!p) return kTablesOffset;
   const Problem q = with_rows(p, rows);
-  if (validate(&q, &d) != MPL_OK || d.ls == p->n_disp) return kTablesOffset;
-  return kTablesOffset + (size_t)d.slice * sizeof(float);  // header + per-iteration sums
+  if (validate(&q, &d) != MPL_OK) return kTablesOffset;
+  // header + per-iteration sums, which only ISGMR forms, from the first iteration whose messages are not zero on
+  const bool sums = isgmr && d.ls != p->n_disp && p->n_iter > (q.messages_zero ? 1 : 0);
+  return kTablesOffset + (sums ? (size_t)d.slice * sizeof(float) : 0);
+}
+
+size_t mpl_forward_workspace_bytes_rows(const mpl_problem* p, const mpl_rows* rows) {
+  return mpl_forward_workspace_bytes_mode(p, rows, 1);
 }
 
 size_t mpl_forward_workspace_bytes(const mpl_problem* p) { return mpl_forward_workspace_bytes_rows(p, nullptr); }

@@ -75,6 +75,25 @@ def test_workspace_sizes():
     assert lib.mpl_workspace_status_offset() == 64
 
 
+@pytest.mark.parametrize("isgmr,n_iter,zero,row,sums", [
+    (0, 3, 0, 24, False), (0, 3, 1, 24, False),   # TRWP forms no sums
+    (1, 3, 0, 24, True), (1, 3, 1, 24, True), (1, 1, 0, 24, True),
+    (1, 1, 1, 24, False),                         # one iteration from zero messages starts from the unaries
+    (1, 0, 0, 24, False), (1, 3, 0, 21, False),   # packed rows: the sums live in cost_final
+])
+def test_forward_workspace_holds_sums_only_where_they_are_formed(isgmr, n_iter, zero, row, sums):
+    lib = _lib.lib()
+    p, rows = _prob(batch=2, height=50, width=61, n_iter=n_iter), _lib.Rows(row, zero)
+    need = 256 + (2 * 50 * 61 * row * 4 if sums else 0)
+    assert lib.mpl_forward_workspace_bytes_mode(ctypes.byref(p), ctypes.byref(rows), isgmr) == need
+    assert lib.mpl_forward_workspace_bytes_rows(ctypes.byref(p), ctypes.byref(rows)) >= need
+    one = ctypes.c_void_p(16)   # never dereferenced: validation fails first
+    fn = lib.mpl_isgmr_forward_rows if isgmr else lib.mpl_trwp_forward_rows
+    ptrs = [one, one, None, one] + ([one] if isgmr else []) + [one, None, None, None, one]
+    assert fn(ctypes.byref(p), ctypes.byref(rows), *ptrs, need - 1, None) == 1
+    assert "workspace too small" in lib.mpl_last_error().decode()
+
+
 @pytest.mark.parametrize("h,w,n", [(7800, 7800, 33), (9999, 10001, 21)])
 def test_proposed_label_stride_is_one_a_call_accepts(h, w, n):
     """Packed rows fit the kernels' 2^31 elements per image here, padded ones do not."""
