@@ -107,7 +107,8 @@ int mpl_analyze_context(const mpl_problem* p, const float* context, const float*
                         int32_t* window, void* workspace, size_t workspace_bytes, void* stream);
 
 /* The mpl_rows::label_stride with which mpl_trwp_* (isgmr = 0) or mpl_isgmr_* (isgmr = 1) calls of `p` run
- * fastest; n_disp where packed rows are as good.  0 if `p` is invalid. */
+ * fastest; n_disp where packed rows are as good, where the padding would take more than 8 GiB, and where a padded
+ * image would exceed 2^31 elements.  0 if `p` is invalid. */
 int32_t mpl_label_stride(const mpl_problem* p, int32_t isgmr);
 
 /* Bytes of device scratch the forward / backward entry points need for `p` (never 0).  The per-iteration sums of a

@@ -94,6 +94,14 @@ def test_forward_workspace_holds_sums_only_where_they_are_formed(isgmr, n_iter, 
     assert "workspace too small" in lib.mpl_last_error().decode()
 
 
+@pytest.mark.parametrize("n,batch,stride", [(1, 1, 4), (1, 700, 1), (2, 1, 4), (2, 700, 2), (21, 1, 24), (21, 700, 21),
+                                            (33, 1, 36), (33, 700, 33), (64, 700, 64)])
+def test_padding_of_label_rows_is_bounded(n, batch, stride):
+    """Rows are padded where that takes a few GB at most: 700 images of 499 x 501 pixels would take 9 or 13 GiB more."""
+    p = _prob(batch=batch, height=499, width=501, n_disp=n)
+    assert _lib.lib().mpl_label_stride(ctypes.byref(p), 0) == stride
+
+
 @pytest.mark.parametrize("h,w,n", [(7800, 7800, 33), (9999, 10001, 21)])
 def test_proposed_label_stride_is_one_a_call_accepts(h, w, n):
     """Packed rows fit the kernels' 2^31 elements per image here, padded ones do not."""
