@@ -72,7 +72,6 @@ class TRWPFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, unary, label_context, edge_weights, args, n_disp=None):
         batch, cv, h, w, row = unary.size()   # row >= n_disp elements per pixel (padded label rows)
-        ctx.n_extra = 0 if n_disp is None else 1   # inputs beyond the reference's four
         n_disp = n_disp or row
         rho, n_iter, n_dir, is_training = args.rho, args.mpnet_max_iter, args.mpnet_n_dirs, args.training
         unary = unary.contiguous()
@@ -115,7 +114,7 @@ class TRWPFunction(torch.autograd.Function):
                        dlabel_context, dedge_weights, dmessage, _empty_f32(dcost_final.device),
                        keep_diag=ctx._forward_cls.keep_diag, context_window=ctx.context_window,
                        cost_labels_first=ctx.cost_labels_first, n_disp=ctx.n_disp)
-        return (dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None) + (None,) * ctx.n_extra
+        return dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None, None
 
 
 class ISGMRFunction(torch.autograd.Function):
@@ -124,7 +123,6 @@ class ISGMRFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, unary, label_context, edge_weights, args, n_disp=None):
         batch, cv, h, w, row = unary.size()   # row >= n_disp elements per pixel (padded label rows)
-        ctx.n_extra = 0 if n_disp is None else 1   # inputs beyond the reference's four
         n_disp = n_disp or row
         rho, n_iter, n_dir, is_training = args.rho, args.mpnet_max_iter, args.mpnet_n_dirs, args.training
         unary = unary.contiguous()
@@ -169,7 +167,7 @@ class ISGMRFunction(torch.autograd.Function):
                         dunary, dlabel_context, dedge_weights, dmessage,
                         _empty_f32(dcost_final.device), dmessage_tmp, context_window=ctx.context_window,
                         cost_labels_first=ctx.cost_labels_first, n_disp=ctx.n_disp)
-        return (dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None) + (None,) * ctx.n_extra
+        return dunary, dlabel_context, (dedge_weights if enable_edge_weights else None), None, None
 
 
 def _row_elements(args, unary, direction_comm=None):

@@ -110,3 +110,21 @@ def test_labels_of_iterations(L):
     ctx = cases.make_context("potts2d", L, rng)
     got = g.forward("TRWP", unary, ctx, None, 4, 1, training=False, save_labels=True)
     assert np.array_equal(got["label_all"][0], got["cost"].argmin(-1).astype(np.uint8))
+
+
+@pytest.mark.parametrize("mode", ["TRWP", "ISGMR"])
+def test_label_count_argument_given_as_none(mode):
+    """The label count is an optional argument of the autograd functions: passing its default changes nothing."""
+    L, D, H, W = 7, 4, 5, 8
+    rng = np.random.default_rng(3)
+    u = torch.from_numpy(rng.standard_normal((1, 1, H, W, L)).astype(np.float32)).cuda().requires_grad_(True)
+    c = torch.from_numpy(cases.make_context("sym2d", L, rng)).cuda().requires_grad_(True)
+    args = types.SimpleNamespace(rho=0.5, mpnet_max_iter=2, mpnet_n_dirs=D, training=True, enable_min_a_dir=False,
+                                 enable_sgm=False, enable_saving_label=False, msg_norm_index=None)
+    fn = MP_module.TRWPFunction if mode == "TRWP" else MP_module.ISGMRFunction
+    got = []
+    for extra in ((), (None,), (L,)):
+        cost = fn.apply(u, c, None, args, *extra)[0]
+        got.append([cost.detach()] + list(torch.autograd.grad(cost, (u, c), torch.ones_like(cost))))
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
