@@ -63,11 +63,11 @@ class TRWPSoftFunction(torch.autograd.Function):
     def backward(ctx, dcost_final, dlabel_all, dmessage_edge_label, dcost_index):
         rho, message_edge_label, cost_index, label_context, ew, enable_edge_weights = ctx.intermediate_results
         del ctx.intermediate_results
-        if dcost_final is None:
-            return None, None, None, None
         if cost_index.numel() == 0:
             raise RuntimeError("backward needs the edge values saved by a training-mode forward "
                                "(args.training was False)")
+        if dcost_final is None:   # the consumer of the costs had no gradient to give
+            dcost_final = message_edge_label.new_zeros(*cost_index.shape[2:], message_edge_label.size(-1))
         if ctx.norm_index_override is not None:
             cost_index = ctx.norm_index_override
         dcost_final = dcost_final.contiguous()

@@ -7,7 +7,7 @@ import torch
 
 import cases
 import gpu_runner as g
-from mplayers_b200 import ISGMR, MP_module
+from mplayers_b200 import ISGMR, MP_module, MP_module_hard_soft
 from mplayers_b200.glue import mp_on_scores
 
 pytestmark = pytest.mark.gpu
@@ -128,3 +128,27 @@ def test_label_count_argument_given_as_none(mode):
         got.append([cost.detach()] + list(torch.autograd.grad(cost, (u, c), torch.ones_like(cost))))
     for other in got[1:]:
         assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+
+
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_costs_without_a_gradient():
+    """A consumer of the costs that hands back no gradient: zeros, from every autograd function."""
+    L, H, W = 5, 6, 8
+    u = torch.rand(1, 1, H, W, L, device="cuda", requires_grad=True)
+    c = torch.rand(L, L, device="cuda", requires_grad=True)
+    ew = torch.rand(4, 1, 1, H, W, device="cuda", requires_grad=True)
+    args = types.SimpleNamespace(rho=0.5, mpnet_max_iter=2, mpnet_n_dirs=4, training=True, enable_min_a_dir=False,
+                                 enable_sgm=False, enable_saving_label=False, msg_norm_index=None)
+    for fn in (MP_module.TRWPFunction, MP_module.ISGMRFunction, MP_module_hard_soft.TRWPSoftFunction):
+        out = _NoGradient.apply(fn.apply(u, c, ew, args)[0])
+        for grad in torch.autograd.grad(out.sum(), (u, c, ew)):
+            assert torch.equal(grad, torch.zeros_like(grad)), fn
