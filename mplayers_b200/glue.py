@@ -175,7 +175,7 @@ def label_rows(x, row):
 
 def labels_last(x):
     """[B,cv,L,H,W] -> contiguous [B,cv,H,W,L] (kernel for float32 tensors within its limits, torch otherwise)."""
-    if x.dim() == 5 and x.permute(0, 1, 3, 4, 2).is_contiguous():
+    if x.dim() == 5 and x.permute(0, 1, 3, 4, 2).is_contiguous() and x.data_ptr() % 16 == 0:
         return x.permute(0, 1, 3, 4, 2)   # labels last in memory already (compute_all_terms' volume)
     if x.dtype == torch.float32 and x.is_cuda and x.dim() == 5 and x.size(2) <= 256 and x.size(0) * x.size(1) <= 65535:
         return LabelsLast.apply(x)

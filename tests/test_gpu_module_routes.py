@@ -8,6 +8,7 @@ import torch
 import cases
 import gpu_runner as g
 from mplayers_b200 import ISGMR, MP_module, MP_module_hard_soft
+from mplayers_b200 import glue
 from mplayers_b200.glue import mp_on_scores
 
 pytestmark = pytest.mark.gpu
@@ -152,3 +153,13 @@ def test_costs_without_a_gradient():
         out = _NoGradient.apply(fn.apply(u, c, ew, args)[0])
         for grad in torch.autograd.grad(out.sum(), (u, c, ew)):
             assert torch.equal(grad, torch.zeros_like(grad)), fn
+
+
+def test_labels_last_memory_off_the_alignment():
+    """A volume whose labels are last in memory is used as it is only where the 16-byte staging of the sweeps can."""
+    buf = torch.rand(1 + 8 * 12 * 21, device="cuda")
+    x = buf[1:].view(1, 1, 8, 12, 21).permute(0, 1, 4, 2, 3)
+    y = glue.labels_last(x)
+    assert y.data_ptr() % 16 == 0 and torch.equal(y, x.permute(0, 1, 3, 4, 2))
+    aligned = buf[:-1].view(1, 1, 8, 12, 21).permute(0, 1, 4, 2, 3)
+    assert glue.labels_last(aligned).data_ptr() == buf.data_ptr()
