@@ -366,7 +366,7 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
 bool forward_team_eligible(const FwdParams& p);
 cudaError_t launch_forward_team(const FwdParams& p, cudaStream_t st);
 // mp_fwd_tma.cu
-bool forward_tma_eligible(const FwdParams& p, int dir, int* stages);
+bool forward_tma_eligible(const FwdParams& p, int dir, bool train, int* stages);
 cudaError_t launch_forward_tma(const FwdParams& p, int dir, int stages, bool train, cudaStream_t st);
 // ISGMR: do the sweeps of p (agg == 0, all directions) sum U + sum_k M_k themselves faster than a separate pass
 // over the messages (aggregate mode) prepares it?

@@ -1150,7 +1150,7 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
     const bool few_chains = (p.ndirs > 1 && (long long)p.nimg * (p.H < p.W ? p.H : p.W) < 256) || p.parts > 1;
     for (int d = p.dir0; d < p.dir0 + p.ndirs && !few_chains; ++d) {
       int stages = 0;
-      if (d != first_generic || !forward_tma_eligible(p, d, &stages)) break;
+      if (d != first_generic || !forward_tma_eligible(p, d, train, &stages)) break;
       const cudaError_t e = launch_forward_tma(p, d, stages, train, st);
       if (e != cudaSuccess) return e;
       first_generic = d + 1;

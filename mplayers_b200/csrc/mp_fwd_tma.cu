@@ -335,21 +335,21 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   if (len > 1) resolve((len - 1) & 1);  // (stages hold an even number of pixels)
 }
 
-size_t tma_smem_bytes(int L, int ls, int D, int stages) {  // with the training tables of the 32-label form
-  const int table = L > 16 && L != 21 ? tma_table_floats(32) : 0;
+size_t tma_smem_bytes(int L, int ls, int D, int stages, bool train) {  // with the training tables of the 32-label form
+  const int table = train && L > 16 && L != 21 ? tma_table_floats(32) : 0;
   return ((size_t)stages * ((size_t)(D + 1) * kTK * 4 * ls + 64) + 4 * 64 + 4 * table) * sizeof(float) + 2 * stages * 8 + 16 + 128;
 }
 
 }  // namespace
 
 // Can direction `dir` of this problem use the bulk-copy kernel?  Needs 16-byte aligned row segments.
-bool forward_tma_eligible(const FwdParams& p, int dir, int* stages) {
+bool forward_tma_eligible(const FwdParams& p, int dir, bool train, int* stages) {
   if (dir > 3 || p.L > 32 || (!p.agg && p.D != 4 && p.D != 8)) return false;
   if (p.W & 3) return false;
   const uintptr_t bits = (uintptr_t)p.unary | (uintptr_t)p.msg_read | (uintptr_t)p.ew;
   if (bits & 15) return false;
   int ns = tma_stage_override() ? tma_stage_override() : 4;
-  while (ns >= 2 && tma_smem_bytes(p.L, p.ls, p.agg ? 2 : p.D, ns) > (ns >= 3 ? 110 : 200) * 1024) --ns;
+  while (ns >= 2 && tma_smem_bytes(p.L, p.ls, p.agg ? 2 : p.D, ns, train) > (ns >= 3 ? 110 : 200) * 1024) --ns;
   if (ns < 2) return false;
   *stages = ns;
   return true;
@@ -363,7 +363,7 @@ cudaError_t launch_tma_v(FwdParams p, int dir, int stages, cudaStream_t st) {
   p.ndirs = 1;
   p.tma_stages = stages;
   const int groups = VERT ? p.nimg * (p.W >> 2) : (p.nimg * p.H + 3) >> 2;
-  const size_t smem = tma_smem_bytes(p.L, p.ls, DT, stages);
+  const size_t smem = tma_smem_bytes(p.L, p.ls, DT, stages, TRAIN);
   cudaError_t e = ensure_smem(fwd_tma_kernel<LMAX, LT, PAD, DT, TRAIN, VERT, FWD>, smem);
   if (e != cudaSuccess) return e;
   TmaMaps maps{};
