@@ -7,7 +7,7 @@ import torch
 
 import cases
 import gpu_runner as g
-from mplayers_b200 import ISGMR, MP_module, MP_module_hard_soft
+from mplayers_b200 import ISGMR, TRWP, MP_module, MP_module_hard_soft
 from mplayers_b200 import glue
 from mplayers_b200.glue import mp_on_scores
 
@@ -163,3 +163,38 @@ def test_labels_last_memory_off_the_alignment():
     assert y.data_ptr() % 16 == 0 and torch.equal(y, x.permute(0, 1, 3, 4, 2))
     aligned = buf[:-1].view(1, 1, 8, 12, 21).permute(0, 1, 4, 2, 3)
     assert glue.labels_last(aligned).data_ptr() == buf.data_ptr()
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("mode,D,H,W,L,R,I", [
+    ("ISGMR", 4, 11, 13, 128, 15, 1),      # the unaries alone, both forms of the first iteration's buffers
+    ("ISGMR", 4, 6, 9, 132, 9, 2),
+    ("ISGMR", 4, 130, 120, 132, 12, 2),
+    ("ISGMR", 8, 20, 18, 256, 16, 3),
+    ("ISGMR", 8, 1000, 9, 36, 10, 2),      # enough chains for one warp each
+    ("TRWP", 4, 17, 10, 192, 10, 3),       # directions 1 .. 3 of the first iteration: what exists so far
+    ("TRWP", 6, 9, 12, 100, 12, 2),        # slices beyond direction 3 hold zeros
+    ("TRWP", 8, 9, 12, 68, 16, 2),
+])
+def test_wide_window_zero_start(mode, D, H, W, L, R, I, training):
+    """Messages known to be zero, in buffers of NaN, against the same call on given zeros."""
+    rng = np.random.default_rng(L * 3 + R + D)
+    unary = (3 * rng.standard_normal((1, 1, H, W, L))).astype(np.float32)
+    ctx = _wide_context(L, R, 0.0)
+    want = g.forward(mode, unary, ctx, None, D, I, training=training, context_window=R)
+    u, c = torch.from_numpy(unary).cuda(), torch.from_numpy(ctx).cuda()
+    e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
+    msg, mu = (torch.full((D, 1, 1, H, W, L), float("nan"), device="cuda") for _ in range(2))
+    cost = torch.empty_like(u)
+    mi = torch.zeros(I, D, 1, 1, H, W, L, dtype=torch.uint8, device="cuda") if training else e8
+    ni = torch.zeros(I, D, 1, 1, H, W, dtype=torch.uint8, device="cuda") if training else e8
+    kw = dict(context_window=R, messages_zero=True)
+    if mode == "TRWP":
+        TRWP.forward(0.5, I, 0, u, c, e0, msg, cost, mi, ni, e0, e8, **kw)
+    else:
+        ISGMR.forward(0, 1.0, I, 0, u, c, e0, msg, cost, mi, ni, e0, mu, e8, **kw)
+    assert np.array_equal(cost.cpu().numpy(), want["cost"])
+    assert np.array_equal(msg.cpu().numpy(), want["msg"])
+    if training:
+        assert np.array_equal(mi.cpu().numpy(), want["min_idx"])
+        assert np.array_equal(ni.cpu().numpy(), want["norm_idx"])
