@@ -199,40 +199,43 @@ def step_bytes(cfg, batch, train):
 
 def dominant_kernel(cfg, kind):
     """Name of the sweep kernel the workload spends its time in (see mplayers_b200/csrc)."""
-    L = cfg["unary"].shape[2]
-    pair = 32 < L <= 64 and L % 4 == 0
+    B, _, L, H, W = cfg["unary"].shape
+    ctx = cfg["label_context"]
     if cfg.get("soft"):
-        return "bwd_soft_kernel" if kind == "bwd" else "fwd_warp_kernel<soft>"
-    if kind == "bwd":
-        if L <= 32:
-            return "bwd_tma_kernel"
-        if cfg["label_context"].dim() == 1 and 32 < L <= 256 and L % 4 == 0:
-            return "bwd_wide_kernel"
-        return "bwd_pair_kernel" if pair else "bwd_cta_kernel"
+        return "bwd_soft_kernel" if kind == "bwd" else "fwd_soft_kernel"
     if L <= 32:
-        return "fwd_tma_kernel"
-    if (not cfg["training"] or L > 64) and cfg["label_context"].dim() == 1 and L % 4 == 0:
-        return "fwd_wide_kernel"
-    if pair:
-        return "fwd_pair_smem_kernel"
-    return "fwd_cta_tma_kernel" if L % 4 == 0 else "fwd_cta_kernel"
+        return "bwd_tma_kernel" if kind == "bwd" else "fwd_tma_kernel"
+    if ctx.dim() == 1 and L <= 256:
+        if kind == "bwd":
+            return "bwd_wide_kernel"
+        # wide windows, no indices, chains that do not fill the schedulers one warp each
+        differs = (ctx != ctx[-1]).nonzero()
+        window = int(differs.max()) + 1 if len(differs) else 0
+        per_direction = [H, H, W, W] + [H + W - 1] * (cfg["n_dir"] - 4)
+        chains = B * (sum(per_direction) if cfg["mode"] == "ISGMR" else max(per_direction[:4]))
+        team = not cfg["training"] and window > 8 and chains < 148 * 16
+        return "fwd_wide_team_kernel" if team else "fwd_wide_kernel"
+    if L <= 64:
+        return "bwd_pair_kernel" if kind == "bwd" else "fwd_pair_kernel"
+    return "bwd_cta_kernel" if kind == "bwd" else "fwd_cta_tma_kernel"
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the sweep kernels, from the ncu
-# captures summarised under profiles/ (same workload, one GPU); None where no capture exists.
+# dram__bytes_read.sum + dram__bytes_write.sum of a launch of the sweep kernels, averaged over the launches of a step
+# (the first iteration, from zero messages, and the first backward sweeps of a pair of slices move less than the others);
+# from the ncu captures summarised in profiles/sweep_kernels_counters.md; None where no capture exists.
 NCU_TRAFFIC = {
-    ("seg_trwp_train", "bwd"): 149.3e6 + 80.9e6,
-    ("seg_trwp_train", "fwd"): 222.4e6 + 33.9e6,
-    ("stereo_trwp_infer", "fwd"): 1788.5e6 + 338.6e6,
-    ("stereo_trwp_train", "bwd"): 1163.8e6 + 1017.2e6,
-    ("denoise_isgmr_infer", "fwd"): 728.4e6 + 245.6e6,
-    # captured on the 384 x 384 copy of the workload (a full-size launch is too large to replay under
-    # the profiler); traffic is proportional to the pixel count, so the full-size figures are those
-    # times (1024 / 384)^2
-    ("large_isgmr_train_384", "fwd"): 748.7e6 + 354.4e6,
-    ("large_isgmr_train_384", "bwd"): 426.3e6 + 299.6e6,
-    ("large_isgmr_train", "fwd"): (748.7e6 + 354.4e6) * (1024 / 384) ** 2,
-    ("large_isgmr_train", "bwd"): (426.3e6 + 299.6e6) * (1024 / 384) ** 2,
+    ("seg_trwp_train", "bwd"): 149.7e6 + 78.3e6,
+    ("seg_trwp_train", "fwd"): 222.4e6 + 30.4e6,
+    ("stereo_trwp_infer", "fwd"): 1491.8e6 + 334.3e6,
+    ("stereo_trwp_train", "fwd"): 1491.9e6 + 420.4e6,
+    ("stereo_trwp_train", "bwd"): 1044.2e6 + 1012.8e6,
+    ("denoise_isgmr_infer", "fwd"): 1143.8e6 + 250.6e6,
+    # captured on the 384 x 384 copy of the workload; traffic is proportional to the pixel count, so the
+    # full-size figures are those of ten iterations times (1024 / 384)^2
+    ("large_isgmr_train_384", "fwd"): 591.8e6 + 342.9e6,
+    ("large_isgmr_train_384", "bwd"): 454.3e6 + 316.8e6,
+    ("large_isgmr_train", "fwd"): (681.8e6 + 346.2e6) * (1024 / 384) ** 2,
+    ("large_isgmr_train", "bwd"): (452.7e6 + 314.9e6) * (1024 / 384) ** 2,
 }
 
 
