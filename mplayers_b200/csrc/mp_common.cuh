@@ -313,9 +313,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 
 // Programmatic dependent launch: the launch of a sweep is prepared while the previous kernel of the stream still
 // runs, its CTAs start as that one's exit and wait in dependent_wait() until it has completed and its
-// writes are visible.  A call has dozens of short launches: 64 x 64 x 21 training 739 -> 645 us, 288 x 384 x 16
-// with 50 iterations 6.88 -> 6.24 ms.  (No early trigger: CTAs scheduled next to the whole running grid end
-// up unevenly spread over the SMs, 64 x 64 x 21 then took 811 us.)  A kernel launched with
+// writes are visible.  A call has dozens of short launches: 288 x 384 x 16 with 50
+// iterations 6.88 -> 6.24 ms.  (64 x 64 x 21 training, 40 sweeps of 63 steps, is within the spread of its repetitions,
+// 650 - 710 us either way.  No early trigger: CTAs scheduled next to the whole running grid end up
+// unevenly spread over the SMs, 64 x 64 x 21 then took 811 us.)  A kernel launched with
 // launch_dependent() must call dependent_wait() in every thread before it touches global memory or
 // returns: a grid that ended without waiting would let the one after it start too early.
 __device__ __forceinline__ void dependent_wait() {
@@ -391,7 +392,7 @@ cudaError_t launch_aggregate_lhw(const float* unary, const float* msg, float* co
 cudaError_t launch_backward_init_lhw(const float* dcost, float* dunary, float* dm, int nimg, int L, int ls, long long HW,
                                      int D, float factor, int cp_scheme, cudaStream_t st);
 cudaError_t launch_backward_sweep(const BwdParams& p, cudaStream_t st);
-// mp_wide_bwd.cu: rank-1 context, 32 < L <= 256, L % 4 == 0, schemes 1 and 2
+// mp_wide_bwd.cu: rank-1 context, 32 < L <= 256, rows of 16-byte multiples (ls % 4 == 0), schemes 1 and 2
 bool bwd_wide_eligible(int L, int ls, int ctx_rank, int cp_scheme, const void* dunary, const void* dm_read,
                        const void* dm_acc);
 cudaError_t launch_backward_wide(const BwdParams& p, int total, cudaStream_t st);

@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(256) fwd_cta_kernel(const __grid_constant__ Fw
   cp_async_wait<0>();
 }
 
-// CTA-per-chain kernel with bulk-copy staging, for L % 4 == 0 (every pixel's label row is then
+// CTA-per-chain kernel with bulk-copy staging, for rows of 16-byte multiples (every pixel's label row is then
 // 16-byte aligned, in any direction).  The last warp of the CTA is the producer: per stage of K
 // chain pixels it issues, for each of the D+1 input arrays, either one cp.async.bulk of K*L floats
 // (horizontal chains are contiguous) or K copies of one label row each (all other directions);

@@ -209,14 +209,6 @@ __device__ __forceinline__ void minplus_regrow(const float* hb, const float (&cr
   if (TRAIN) bi = highest_equal<LMAX>(val, best);
 }
 
-// The argmin index alone, for a minimum that is already known (recomputes the candidates).
-template <int LMAX>
-__device__ __forceinline__ int minplus_index(const float* hb, const float (&cr)[LMAX], float e, float best) {
-  float val[LMAX];
-  minplus_vals<LMAX>(hb, cr, e, val);
-  return highest_equal<LMAX>(val, best);
-}
-
 // q[f] = sum over labels c whose saved argmin is f of t[c], for f = `me`; fixed summation order
 // (interleaved partial sums).  tb / ib: the t values and argmin indices (stored as floats)
 // of all labels of this pixel in shared memory.  One compare-to-flag plus one fused multiply-add

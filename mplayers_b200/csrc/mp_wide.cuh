@@ -1,5 +1,5 @@
 // Forward sweep (inference, and training with saved indices) with a rank-1 context that saturates
-// inside a window (truncated linear / quadratic, Potts), 32 < L <= 256, L % 4 == 0: one warp per
+// inside a window (truncated linear / quadratic, Potts), 32 < L <= 256, rows of 16-byte multiples: one warp per
 // chain, several labels per lane.  Replaces, for those problems, the reference's chain kernels
 // (MPLayers/TRWP/TRWP_forward.cu:82-376) with their one thread per label and L block barriers
 // per step.

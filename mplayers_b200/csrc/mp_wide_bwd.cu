@@ -1,4 +1,4 @@
-// Backward sweep for a rank-1 context with 32 < L <= 256 labels, L % 4 == 0 (learning a truncated
+// Backward sweep for a rank-1 context with 32 < L <= 256 labels in rows of 16-byte multiples (learning a truncated
 // linear / quadratic function on stereo- or denoising-sized label sets): one WARP per chain, LPT
 // consecutive labels per lane, schemes 1 (C + P bookkeeping, TRWP) and 2 (scatter field, ISGMR).
 // Replaces, for those problems, the reference's backward chain kernels with one thread per label,
