@@ -59,8 +59,9 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
 
   float* tiles = smem;                                   // [NS][tile_floats]
   float* etiles = tiles + NS * tile_floats;              // [NS][64]
-  float* hbufs = etiles + NS * 64;                       // [4][64]
-  float* ctabs = hbufs + 4 * 64;                         // kTwo: [4][tma_table_floats(LMAX)]
+  constexpr int kH = kTwo ? 96 : 64;                     // floats of a warp's h buffers: three or two of 32
+  float* hbufs = etiles + NS * 64;                       // [4][kH]
+  float* ctabs = hbufs + 4 * kH;                         // kTwo: [4][tma_table_floats(LMAX)]
   unsigned long long* full =
       reinterpret_cast<unsigned long long*>(ctabs + (kTwo ? 4 * tma_table_floats(LMAX) : 0));  // [NS]
   unsigned long long* empty = full + NS;                 // [NS]
@@ -160,8 +161,8 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   float* Mwl = p.msg_write + (long long)dir * p.slice + ibase * LR + lc;
   uint8_t* MIl = TRAIN ? p.min_idx + (long long)dir * p.slice + ibase * LR + lc : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)dir * p.pslice + ibase : nullptr;
-  float* hbuf = hbufs + wc * 64;
-  for (int i = lane; i < 64; i += 32) hbuf[i] = kInf;  // labels >= L (LMAX > L) never win
+  float* hbuf = hbufs + wc * kH;
+  for (int i = lane; i < kH; i += 32) hbuf[i] = kInf;  // labels >= L (LMAX > L) never win
   if (!has_e)  // no edge weights: the producer copies none, every staged weight reads as 1
     for (int i = lane; i < NS * 64; i += 32) etiles[i] = 1.f;
   __syncwarp();
@@ -221,18 +222,21 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
       if (act) ctab[lane * kCS + f] = cr[f];
     __syncwarp();
   }
-  auto resolve = [&](int par) {  // par: the h buffer of the pixel that is resolved
+  // kTwo: h of the pixel that is resolved, of the current one, of the next one.  A pixel's h is read once more behind the
+  // next step's barrier, so the buffer written before the barrier after that has to be a third one (two buffers and one
+  // more warp barrier a step: 512 x 512 x 28, forward and backward, 3.20 ms against 3.18).
+  float *hprev = hbuf, *hcur = hbuf + 32, *hnext = hbuf + 64;
+  auto resolve = [&]() {
     if constexpr (TRAIN) {
       int bi = highest_equal<kKept>(pval, pbest);
       if constexpr (kTwo) {
         const int f0 = 3 * (bi & 15);  // (a NaN minimum equals nothing: any group)
         const int at = f0 < LMAX ? f0 : 0;
-        const float* hp = hbuf + par * 32 + at;
+        const float* hp = hprev + at;
         const float* cp = ctab + lc * kCS + at;
         const float v1 = fmaf(pe, cp[1], hp[1]);
         const float v2 = LMAX % 3 == 2 && at + 2 >= LMAX ? kInf : fmaf(pe, cp[2], hp[2]);
         bi = v2 == pbest ? at + 2 : v1 == pbest ? at + 1 : at;
-        __syncwarp();  // the next step writes this h buffer before its own barrier
       }
       const unsigned bal = __ballot_sync(0xffffffffu, pbest == pm) & lmask;
       *mip = (uint8_t)bi;
@@ -240,7 +244,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     }
   };
   auto step = [&](const float* t, float e, int par, bool pending) {
-    float* hb = hbuf + par * 32;
+    float* hb = kTwo ? hcur : hbuf + par * 32;
     const float h = fmaf(rho, r, uu);
     if (LT == 0 || LMAX != LT) {
       if (act) hb[lane] = h;
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     }
     const float uu_next = uu_at(t);
     if (TRAIN) {
-      if (pending) resolve(par ^ 1);
+      if (pending) resolve();
       mip += ostep;
       nip += pstep;
     }
@@ -289,6 +293,10 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
       pbest = best;
       pm = m;
       pe = e;
+    }
+    if constexpr (kTwo) {
+      float* const free_buf = hprev;
+      hprev = hcur, hcur = hnext, hnext = free_buf;
     }
     uu = uu_next;
   };
@@ -332,12 +340,12 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[slot]);
   }
-  if (len > 1) resolve((len - 1) & 1);  // (stages hold an even number of pixels)
+  if (len > 1) resolve();
 }
 
 size_t tma_smem_bytes(int L, int ls, int D, int stages, bool train) {  // with the training tables of the 32-label form
   const int table = train && L > 16 && L != 21 ? tma_table_floats(32) : 0;
-  return ((size_t)stages * ((size_t)(D + 1) * kTK * 4 * ls + 64) + 4 * 64 + 4 * table) * sizeof(float) + 2 * stages * 8 + 16 + 128;
+  return ((size_t)stages * ((size_t)(D + 1) * kTK * 4 * ls + 64) + 4 * (table ? 96 : 64) + 4 * table) * sizeof(float) + 2 * stages * 8 + 16 + 128;
 }
 
 }  // namespace
