@@ -366,6 +366,9 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
 // mp_wide_team.cu: several warps per chain, wide windows, no saved indices
 bool forward_team_eligible(const FwdParams& p);
 cudaError_t launch_forward_team(const FwdParams& p, cudaStream_t st);
+// mp_wide_many.cu: many chains, windows of up to eight offsets, aggregate mode, no saved indices
+bool forward_many_eligible(const FwdParams& p);
+cudaError_t launch_forward_many(const FwdParams& p, cudaStream_t st);
 // mp_fwd_tma.cu
 bool forward_tma_eligible(const FwdParams& p, int dir, bool train, int* stages);
 cudaError_t launch_forward_tma(const FwdParams& p, int dir, int stages, bool train, cudaStream_t st);

@@ -12,6 +12,7 @@ cudaError_t launch_forward_wide(const FwdParams& p, bool train, cudaStream_t st)
   if (train) return launch_forward_wide_train(p, st);
   // (a first TRWP iteration leaves out the slices that are still zero: only fwd_wide_kernel has that form)
   if (forward_team_eligible(p) && !(p.first && !p.agg && p.dir0 > 0)) return launch_forward_team(p, st);
+  if (forward_many_eligible(p)) return launch_forward_many(p, st);
   return launch_wide_l<false>(p, st);
 }
 

@@ -1,0 +1,57 @@
+"""Sweep kernels that leave out candidates, share a warp between chains or read sums of earlier sweeps, at the sizes and
+contexts where they can go wrong.  Forward results and saved indices have to be the oracle's bit for bit
+(its arithmetic is followed operation by operation); gradients sum in another order and are held
+to the tolerances of helpers.assert_grad_close."""
+import numpy as np
+import pytest
+
+import gpu_runner as g
+import test_gpu_rows as rows
+from helpers import assert_grad_close
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _same_forward(mode, unary, ctx, ew, D, I, training=True, **kw):
+    want = oracle.forward(mode, unary, ctx, ew, D, I, msg_init=kw["msg_init"]) if "msg_init" in kw \
+        else oracle.forward(mode, unary, ctx, ew, D, I)
+    got = g.forward(mode, unary, ctx, ew, D, I, training=training, **kw)
+    for k in ("cost", "msg") + (("min_idx", "norm_idx") if training else ()):
+        assert np.array_equal(got[k], want[k]), k
+    return want
+
+
+def _truncated(kind, R, L):
+    """Saturates at offset R; "quantised" costs tie often, "dip" is not smallest at offset 0."""
+    k = np.arange(L, dtype=np.float64)
+    c = np.minimum(k, R) if kind != "quadratic" else np.minimum(k, R) ** 2
+    if kind == "dip":
+        c[0] = 0.5
+        c[1:R] = 0.25
+    return c.astype(np.float32)
+
+
+@pytest.mark.parametrize("L", [36, 52, 64])
+@pytest.mark.parametrize("R,kind,I", [(1, "linear", 2), (2, "linear", 3), (3, "dip", 2), (4, "quadratic", 2)])
+def test_two_chains_per_warp(L, R, kind, I):
+    """Chains of one image in eight directions, diagonal ones of different length next to each other."""
+    rng = np.random.default_rng(L + R)
+    shape = (2, 1, 61, 98, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _truncated(kind, R, L)
+    ew = rng.uniform(0.0, 1.4, (8,) + shape[:-1]).astype(np.float32)
+    _same_forward("ISGMR", unary, ctx, ew, 8, I, training=False)
+
+
+@pytest.mark.parametrize("L,R,I", [(68, 3, 2), (128, 8, 1), (132, 2, 2), (256, 6, 1)])
+def test_one_chain_per_warp_and_two_pieces(L, R, I):
+    rng = np.random.default_rng(L + R)
+    shape = (2, 1, 61, 98, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _truncated("linear", R, L)
+    ew = rng.uniform(0.0, 1.4, (8,) + shape[:-1]).astype(np.float32)
+    _same_forward("ISGMR", unary, ctx, ew, 8, I, training=False)
+
+
+@pytest.mark.parametrize("L", [35, 50, 99, 137])
+def test_many_chains_padded(L):
+    rows.test_padded_rows_and_zero_start("ISGMR", 8, 2, 61, 98, L, 2, "tl1d", False)
