@@ -330,6 +330,9 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
     if (p->n_iter == 0 && rd != msg) MPL_CUDA(cudaMemsetAsync(msg, 0, (size_t)D * d.slice * sizeof(float), st));
   }
   bool have_sums = false;
+  // TRWP with four directions: `cost_final` holds the sums its sweeps of directions 2 and 3 start from
+  set_dirs(fp, 0, 1);
+  const bool prefix = !isgmr && d.ls == L && ((uintptr_t)cost_final & 15) == 0 && mpl::forward_takes_prefix(fp, train);
   for (int it = 0; it < p->n_iter; ++it) {
     fp.min_idx = train ? msg_min_index + (long long)it * D * d.slice : nullptr;
     fp.norm_idx = train ? msg_norm_index + (long long)it * D * d.npix : nullptr;
@@ -355,6 +358,9 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
     } else {
       for (int dir = 0; dir < D; ++dir) {  // later directions see earlier ones' new messages
         set_dirs(fp, dir, 1);
+        fp.prefix_out = prefix && dir == 1 ? cost_final : nullptr;
+        fp.unary = prefix && dir >= 2 ? cost_final : unary;
+        fp.slice0 = prefix && dir >= 2 ? 2 : 0;
         MPL_CUDA(mpl::launch_forward_sweep(fp, train, st));
       }
     }

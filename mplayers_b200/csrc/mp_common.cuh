@@ -119,6 +119,9 @@ struct FwdParams {
   // below `dir0`, which earlier sweeps of the iteration have written.  Only where
   // forward_skips_zero_slices() says so; other launches read slices that hold zeros.
   int first;
+  // TRWP, four directions, kernels with several labels per lane (forward_takes_prefix()): sums P = (U + M_0) + M_1 of an iteration.
+  float* prefix_out;      // direction 1 writes them here (or nullptr)
+  int slice0;             // 2: `unary` holds them and the sweep (direction 2 or 3) stages slices 2 and 3 only; else 0
   int host_windowed;      // host copy of the context analysis (rank-1, L > 32): windowed path is exact
   int host_R;             //   ... and its window half-width
   int dir0, ndirs;        // this launch covers directions dir0 .. dir0+ndirs-1
@@ -378,6 +381,8 @@ bool forward_sums_messages_itself(const FwdParams& p, bool train);
 // Does a sweep described by p run without reading message slices that are known to be zero
 // (FwdParams::first)?  Those it would read otherwise have to hold zeros.
 bool forward_skips_zero_slices(const FwdParams& p, bool train);
+// Can the sweeps of this TRWP call work through FwdParams::prefix_out?
+bool forward_takes_prefix(const FwdParams& p, bool train);
 // Zeroes the rows of the chains' first pixels in the D slices of `a` and (if not null) `b`: they have no
 // predecessor, so no sweep writes them.  p describes all directions.
 cudaError_t launch_zero_chain_starts(const FwdParams& p, float* a, float* b, cudaStream_t st);

@@ -1118,6 +1118,11 @@ bool forward_skips_zero_slices(const FwdParams& p, bool train) {
   return wide_eligible(p, train) || (p.agg && pair_eligible(p));
 }
 
+bool forward_takes_prefix(const FwdParams& p, bool train) {
+  // (every pixel has to lie on a chain that is walked; the several-warps kernel, which wide windows may take, does not know P)
+  return p.D == 4 && !p.agg && p.W > 1 && wide_eligible(p, train) && (train || p.host_R <= 8);
+}
+
 __global__ void zero_chain_starts_kernel(const __grid_constant__ FwdParams p, float* a, float* b) {
   const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (g >= p.chain_off[p.ndirs]) return;

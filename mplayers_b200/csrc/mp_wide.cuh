@@ -65,9 +65,18 @@ __device__ __forceinline__ int warp_max_i32(int v) {
 // (FwdParams::agg; arrays A, M_dir, M_inv); 1, -1, -2, -3: first iteration from zero messages
 // (FwdParams::first), where only what differs from zero is staged -- the unaries alone (1: every
 // direction of ISGMR, direction 0 of TRWP), or the unaries and the slices 0 .. dir - 1 that the
-// iteration's earlier TRWP sweeps have written (-dir).
+// iteration's earlier TRWP sweeps have written (-dir).  3, 5, -5: TRWP with four directions through the sums P = (U + M_0) +
+// M_1, which the additions of every sweep start with and which directions 2 and 3 leave as they are.  5 and -5 are 4 and -1
+// in a sweep of direction 1 that also writes P (FwdParams::prefix_out); 3 stages P (as FwdParams::unary) and the two
+// slices from FwdParams::slice0 = 2 on, and a first iteration's directions 2 and 3 are 1 and -1 over P.  21 volumes
+// instead of 24 per iteration, 11 instead of 14 in the first; the order of the additions stays.
 // SELF: no producer warps, each consumer stages its own inputs (a compile-time switch: as a run-time one
 // it cost the other launches 3 to 12 %).
+// Staged message slices of a mode DT (-1: FwdParams::D).
+__host__ __device__ constexpr int wide_slices(int dt) {
+  return dt == 1 ? 0 : dt == 3 ? 2 : dt == 5 ? 4 : dt == -5 ? 1 : dt < 0 ? -dt : dt ? dt : -1;
+}
+
 template <int LPT, int RW, int DT, bool TRAIN, bool SELF>
 __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __grid_constant__ FwdParams p,
                                                                        const __grid_constant__ TmaMaps maps) {
@@ -76,7 +85,9 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   constexpr int G = ((RW - 1 + 3) / 4) * 4;      // guard band (floats) on both sides of the window buffer
   constexpr int NWV = (LPT + 2 * G) / 2;         // float2 loads covering a lane's window
   constexpr bool AGG = DT == 2;  // aggregate mode (FwdParams::agg): arrays A, M_dir, M_inv
-  const int L = p.L, LR = p.ls, D = DT == 1 ? 0 : DT < 0 ? -DT : DT ? DT : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
+  constexpr bool PREFIX = DT == 5 || DT == -5;
+  constexpr int DC = wide_slices(DT);
+  const int L = p.L, LR = p.ls, D = DC >= 0 ? DC : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Warps 0..C-1 are the consumers of the CTA's C chains, warps C..2C-1 their producers.
   constexpr int C = wide_chains_per_cta(LPT, RW);
@@ -131,7 +142,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
         const int y0 = ch.img * p.H + (ch.dir == 2 ? s * K : p.H - (s + 1) * K);
         tma_load_2d(T, &maps.a, ch.w0 * LR, y0, &full[slot]);
         for (int a = 1; a < A; ++a) {
-          const int sid = AGG ? (a == 1 ? ch.dir : ch.inv) : a - 1;
+          const int sid = AGG ? (a == 1 ? ch.dir : ch.inv) : p.slice0 + a - 1;
           tma_load_2d(T + a * K * LR, &maps.b, ch.w0 * LR, sid * p.nimg * p.H + y0, &full[slot]);
         }
       }
@@ -145,7 +156,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
     if (contiguous) {
       const int first = ch.pstep == 1 ? pix0 + s * K : pix0 - (s * K + np - 1);
       if (lane < A) {
-        const int sid = AGG ? (lane == 1 ? ch.dir : ch.inv) : lane - 1;
+        const int sid = AGG ? (lane == 1 ? ch.dir : ch.inv) : p.slice0 + lane - 1;
         const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * LR;
         bulk_g2s(T + lane * K * LR, src, (unsigned)(np * LR) * 4u, &full[slot]);
       }
@@ -153,7 +164,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
       for (int q = lane; q < np * A; q += 32) {
         const int k = q / A, a = q - k * A;
         const int px = pix0 + (s * K + k) * ch.pstep;
-        const int sid = AGG ? (a == 1 ? ch.dir : ch.inv) : a - 1;
+        const int sid = AGG ? (a == 1 ? ch.dir : ch.inv) : p.slice0 + a - 1;
         const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * LR;
         bulk_g2s(T + (a * K + k) * LR, src, (unsigned)LR * 4u, &full[slot]);
       }
@@ -192,8 +203,8 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   const float* E = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
   const int c0 = lane * LPT;                    // first label of this lane
   const int nl = L - c0 < 0 ? 0 : (L - c0 < LPT ? L - c0 : LPT);  // labels of this lane that exist
-  const int dir_off = (AGG ? 1 : 1 + ch.dir) * K * LR, inv_off = (AGG ? 2 : 1 + ch.inv) * K * LR;
-  constexpr bool has_inv = DT < 0 ? (-DT & 1) != 0 : DT != 1;   // is M_inv among the staged slices?
+  const int dir_off = (AGG ? 1 : 1 + ch.dir - p.slice0) * K * LR, inv_off = (AGG ? 2 : 1 + ch.inv - p.slice0) * K * LR;
+  constexpr bool has_inv = DT < 0 ? (DC & 1) != 0 : DT != 1;   // is M_inv among the staged slices?
   constexpr bool has_dir = DT != 1 && DT >= 0;                  // is M_dir?
   const float rho = p.rho;
   auto load_e = [&](int s) -> float {  // lane k < K: weight of chain pixel s*K + k
@@ -210,6 +221,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   const int KL = K * LR;
   const int ostep = ch.pstep * LR;
   float* out = Mw + (long long)pix0 * LR + c0;                       // message row of the current pixel
+  float* pfx = PREFIX ? p.prefix_out + (ibase + pix0) * LR + c0 : nullptr;  // its row of P
   uint8_t* idxp = TRAIN ? MI + (long long)pix0 * LR + c0 : nullptr;  // its argmin indices
   uint8_t* nrmp = TRAIN ? NI + pix0 : nullptr;                      // its normalisation index
   int hpar = 0;                                                     // which window buffer the pixel writes
@@ -233,6 +245,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
     for (int k = 0; k < np; ++k, t += tstep, out += ostep, hpar ^= 1) {
       // inputs of this pixel -> UU (reference order of the additions), LPT labels per lane
       float un[LPT];
+      float pv[LPT], pm[LPT];  // PREFIX: U + M_0, and M_1 as it is at the chain's first pixel, which no sweep writes
       if (nl == LPT) {
         float v[LPT], md[LPT], mi[LPT];
 #pragma unroll
@@ -245,12 +258,17 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
           mi[2 * q] = z.x, mi[2 * q + 1] = z.y;
         }
 #pragma unroll
-        for (int a = 1; a <= (DT == 1 ? 0 : DT < 0 ? -DT : DT ? DT : 16); ++a) {
+        for (int a = 1; a <= (DC >= 0 ? DC : 16); ++a) {
           if (a <= D && !AGG) {
 #pragma unroll
             for (int q = 0; q < LPT / 2; ++q) {
               const float2 x = reinterpret_cast<const float2*>(t + a * KL)[q];
+              if (PREFIX && a == 2) pm[2 * q] = x.x, pm[2 * q + 1] = x.y;
               v[2 * q] += x.x, v[2 * q + 1] += x.y;
+            }
+            if (PREFIX && a == 1) {
+#pragma unroll
+              for (int i = 0; i < LPT; ++i) pv[i] = v[i], pm[i] = 0.f;
             }
           }
         }
@@ -263,7 +281,10 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
           if (i < nl) {
             float sum = t[i];
             if (!AGG)
-              for (int a = 1; a <= D; ++a) sum += t[a * KL + i];
+              for (int a = 1; a <= D; ++a) {
+                sum += t[a * KL + i];
+                if (PREFIX && a == 1) pv[i] = sum, pm[i] = D > 1 ? t[2 * KL + i] : 0.f;
+              }
             if (has_dir) sum -= t[dir_off + i];
             un[i] = fmaf(sum, rho, has_inv ? -t[inv_off + i] : -0.f);
           }
@@ -377,6 +398,19 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
             if (i < nl) out[i] = r[i];
         }
       }
+      if constexpr (PREFIX) {
+        if (nl == LPT) {
+#pragma unroll
+          for (int q = 0; q < LPT / 2; ++q)
+            reinterpret_cast<float2*>(pfx)[q] = make_float2(pv[2 * q] + (first ? pm[2 * q] : r[2 * q]),
+                                                            pv[2 * q + 1] + (first ? pm[2 * q + 1] : r[2 * q + 1]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < LPT; ++i)
+            if (i < nl) pfx[i] = pv[i] + (first ? pm[i] : r[i]);
+        }
+        pfx += ostep;
+      }
 #pragma unroll
       for (int i = 0; i < LPT; ++i) uu[i] = un[i];
       first = false;
@@ -400,7 +434,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
 template <int LPT, int RW, int DT, bool TRAIN, bool SELF>
 cudaError_t launch_wide_s(FwdParams p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
-  const int A = (DT == 1 ? 0 : DT < 0 ? -DT : p.agg ? 2 : p.D) + 1;
+  const int A = (wide_slices(DT) >= 0 ? wide_slices(DT) : p.D) + 1;
   constexpr int G = ((RW - 1 + 3) / 4) * 4;
   int K = 8, NS = 3;
   auto bytes = [&](int k, int ns) { return wide_chain_bytes(ns, A, k, p.ls, LPT, G); };
@@ -465,12 +499,15 @@ template <int LPT, int RW, bool TRAIN>
 cudaError_t launch_wide(const FwdParams& p, cudaStream_t st) {
   if (p.first) {  // (directions beyond 3 of a TRWP iteration read every slice: those above 3 hold zeros)
     if (p.agg || p.dir0 == 0) return launch_wide_d<LPT, RW, 1, TRAIN>(p, st);
-    if (p.dir0 == 1) return launch_wide_d<LPT, RW, -1, TRAIN>(p, st);
+    if (p.slice0 == 2) return p.dir0 == 2 ? launch_wide_d<LPT, RW, 1, TRAIN>(p, st) : launch_wide_d<LPT, RW, -1, TRAIN>(p, st);
+    if (p.dir0 == 1) return p.prefix_out ? launch_wide_d<LPT, RW, -5, TRAIN>(p, st) : launch_wide_d<LPT, RW, -1, TRAIN>(p, st);
     if (p.dir0 == 2) return launch_wide_d<LPT, RW, -2, TRAIN>(p, st);
     if (p.dir0 == 3) return launch_wide_d<LPT, RW, -3, TRAIN>(p, st);
   }
   if (p.agg) return launch_wide_d<LPT, RW, 2, TRAIN>(p, st);
   if (p.D == 2) return cudaErrorNotSupported;  // DT == 2 is reserved for the aggregate mode
+  if (p.slice0 == 2) return launch_wide_d<LPT, RW, 3, TRAIN>(p, st);
+  if (p.prefix_out) return launch_wide_d<LPT, RW, 5, TRAIN>(p, st);
   if (p.D == 4) return launch_wide_d<LPT, RW, 4, TRAIN>(p, st);
   if (p.D == 8) return launch_wide_d<LPT, RW, 8, TRAIN>(p, st);
   return launch_wide_d<LPT, RW, 0, TRAIN>(p, st);

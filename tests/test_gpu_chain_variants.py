@@ -55,3 +55,18 @@ def test_one_chain_per_warp_and_two_pieces(L, R, I):
 @pytest.mark.parametrize("L", [35, 50, 99, 137])
 def test_many_chains_padded(L):
     rows.test_padded_rows_and_zero_start("ISGMR", 8, 2, 61, 98, L, 2, "tl1d", False)
+
+
+@pytest.mark.parametrize("L,R,H,W", [(64, 2, 9, 14), (128, 4, 8, 11), (192, 2, 7, 12), (256, 7, 6, 9), (64, 3, 9, 1),
+                                     (64, 3, 1, 9)])
+@pytest.mark.parametrize("given", [False, True])
+def test_sums_of_two_directions(L, R, H, W, given):
+    """TRWP with four directions: directions 2 and 3 start from the sums that direction 1 wrote, from given messages too
+    (those at the chains' first pixels stay as they are)."""
+    rng = np.random.default_rng(L + W)
+    shape = (2, 1, H, W, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _truncated("linear", R, L)
+    ew = rng.uniform(0.1, 1.4, (4,) + shape[:-1]).astype(np.float32)
+    kw = {"msg_init": rng.uniform(0, 1, (4,) + shape).astype(np.float32)} if given else {}
+    _same_forward("TRWP", unary, ctx, ew, 4, 3, **kw)
+    _same_forward("TRWP", unary, ctx, ew, 4, 2, training=False, **kw)
