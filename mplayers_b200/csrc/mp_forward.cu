@@ -840,228 +840,241 @@ cudaError_t launch_cta_tma(FwdParams p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// 32 < L <= 64, rows of 16-byte multiples, any context: one WARP per chain, two labels per lane (l and l + 32).
-// No block barrier (the CTA-per-chain kernel needs two per step and two warps per chain).  Every warp
-// stages its own inputs: lane-parallel cp.async.bulk copies (one per array and stage for horizontal chains, one
-// label row per pixel otherwise) into a private ring, completion on the warp's own mbarriers, refilled by
-// the warp itself as soon as it has consumed a stage.
+// 32 < L <= 64, rows of 16-byte multiples, any context: one WARP per chain, two labels per lane (2l and 2l + 1), no
+// block barrier (the CTA-per-chain kernel needs two per step and two warps per chain).
 //
-// Both context rows of a lane are in registers.  Training finds the argmin in two levels: candidates are
-// taken in groups of eight, the highest group attaining the minimum is kept with the running minimum, and
-// only its eight candidates are evaluated again (from a [64][68] table in shared memory, row stride 68: no
-// systematic bank conflicts) to find the label -- 16 flags per label instead of 64.  What bounds a step is the
-// dependent work of two warps per scheduler: 253 registers, eight chains per SM.  Measured on 1024 x 1024 x 64,
-// eight directions, 10 iterations, forward and backward: rows in shared memory and 64 flags per label 145.5
-// ms (bound by 16 KB of shared-memory reads per step), the same with two levels 144.4, this form 137.7;
-// two chains per warp sharing the reads 148.8 - 155, sharing the registers 163.
-constexpr int kPairWarps = 4;
-constexpr int kPairRS = 68;
+// A step evaluates only the candidates that can be a minimum.  fma is monotone in each operand, rounding included:
+// with hmin = h[g] the smallest h, every label c has a candidate fma(e, ctx(c,g), hmin) <= fma(e, hi, hmin) =: top,
+// hi the largest entry of the table (e >= 0; for e < 0 the ends of the intervals change places), while the
+// candidates of f for the labels c != f are at least fma(e, low, h[f]), low the smallest entry of column f off the
+// diagonal.  Where that exceeds top, f is no minimum of theirs and not equal to one, so the argmin among
+// equal candidates stays what it is; the candidate of f for itself is always evaluated.  The same argument gives the
+// minimum over all labels before the candidates: min_f fma(e, column minimum, h[f]).  A comparison with a NaN keeps
+// the label, and a table with a NaN excludes nothing.  The labels in question are written to a list, ascending
+// (h and the offset of the label's context row), and every lane runs through it for its two labels.  Random 64 x 64
+// table, eight directions: 35 of 64 labels in the first iteration, 13 in the third, 8 from the sixth on.
+//
+// Every lane stages its own labels, 8 bytes per array and pixel, kPairRing pixels ahead: no barrier and no copy per row
+// (bulk copies of 256-byte rows, one per array and pixel off the horizontal directions, cost 100 instructions a step).
+constexpr int kPairCtx = 64 * 64;      // floats of the table
+constexpr int kPairBounds = 5 * 64;    // per label: smallest, largest entry of the column, the same without the diagonal, the diagonal
+constexpr int kPairList = 68;          // entries of a list: 64 and four that never win
+constexpr int kPairRing = 8;           // pixels (power of two)
 
-// Eight candidates e*ctx + h, two per packed multiply-add.
-__device__ __forceinline__ void pair_cand8(const float* c, const float4& h0, const float4& h1, float e, float (&v)[8]) {
-  ffma2(v[0], v[1], e, e, c[0], c[1], h0.x, h0.y);
-  ffma2(v[2], v[3], e, e, c[2], c[3], h0.z, h0.w);
-  ffma2(v[4], v[5], e, e, c[4], c[5], h1.x, h1.y);
-  ffma2(v[6], v[7], e, e, c[6], c[7], h1.z, h1.w);
-}
+__host__ __device__ inline int pair_warp_floats(int A) { return kPairRing * (A * 64 + 4) + 2 * 2 * kPairList; }
 
-template <bool TRAIN>
-__global__ void __launch_bounds__(kPairWarps * 32, 2) fwd_pair_kernel(const __grid_constant__ FwdParams p) {
+// MODE 0: the unaries and p.D message slices are staged; 1: aggregate mode (FwdParams::agg); 2: zero messages
+// (FwdParams::first, aggregate mode), only the unaries.  FULL: 64 labels in rows of 64, messages and indices aligned to pairs.
+template <int MODE, bool TRAIN, bool FULL>
+__global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(128) float smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool first_it = p.first != 0;  // zero messages (aggregate mode): only the unaries are staged
-  const int L = p.L, LR = p.ls, D = first_it ? 0 : p.agg ? 2 : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
-  float* ctab = smem;  // [64][kPairRS]
+  const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr bool AGG = MODE == 1;
+  const int L = FULL ? 64 : p.L, LR = FULL ? 64 : p.ls, D = MODE == 2 ? 0 : AGG ? 2 : p.D, A = D + 1;
+  float* ctab = smem;                // [64][64], row = label at the predecessor
+  float* btab = ctab + kPairCtx;     // [5][64]
   dependent_wait();
-  for (int i = threadIdx.x; i < 64 * kPairRS; i += blockDim.x) {
-    const int c = i / kPairRS, f = i - c * kPairRS;
+  for (int i = threadIdx.x; i < kPairCtx; i += blockDim.x) {
+    const int f = i >> 6, c = i & 63;
     ctab[i] = (c < L && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c, f) : 0.f;
   }
-  const int tile_floats = A * K * LR;
-  const int per_warp = NS * tile_floats + 2 * 64 + 2 * K + 2 * NS + 2;
-  float* wbase = smem + 64 * kPairRS + warp * ((per_warp + 3) & ~3);
-  float* tiles = wbase;                               // [NS][A][K][LR]
-  float* hbuf = tiles + NS * tile_floats;             // [2][64]
-  float* etile = hbuf + 128;                          // [2][K]
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(etile + 2 * K + ((2 * K) & 1));
-  if (lane == 0)
-    for (int i = 0; i < NS; ++i) mbar_init(&full[i], 1);
-  hbuf[lane] = kInf, hbuf[32 + lane] = kInf, hbuf[64 + lane] = kInf, hbuf[96 + lane] = kInf;
-  if (lane == 0) mbar_fence_init();
+  float* ring = btab + kPairBounds + warp * pair_warp_floats(A);  // [kPairRing][A][64] and 4 (the weight)
+  const int slot_floats = A * 64 + 4;
+  float2* list = reinterpret_cast<float2*>(ring + kPairRing * slot_floats);  // [2][kPairList], in turns
   __syncthreads();
+  bool nan = false;
+  if (threadIdx.x < 64) {
+    const int f = threadIdx.x;
+    float lo = kInf, hi = -kInf, olo = kInf, ohi = -kInf;
+    for (int c = 0; c < L && f < L; ++c) {
+      const float v = ctab[c * 64 + f];
+      nan |= v != v;
+      lo = fminf(lo, v), hi = fmaxf(hi, v);
+      if (c != f) olo = fminf(olo, v), ohi = fmaxf(ohi, v);
+    }
+    btab[f] = lo, btab[64 + f] = hi, btab[128 + f] = olo, btab[192 + f] = ohi, btab[256 + f] = f < L ? ctab[f * 65] : 0.f;
+  }
+  const bool any_nan = __syncthreads_or(nan);
   ChainCtx ch;
-  if (!decode_chain(p, blockIdx.x * kPairWarps + warp, ch)) return;
+  if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
 
   const int len = ch.len;
-  const int nstages = (len + K - 1) / K;
   const long long ibase = (long long)ch.img * p.H * p.W;
-  const int pix0 = ch.h0 * p.W + ch.w0;
-  const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
-  const float* U = p.unary + ibase * LR;
-  const float* Mr = p.msg_read + ibase * LR;
-
-  auto issue_stage = [&](int s) {
-    if (s >= nstages) return;
-    const int slot = s % NS;
-    const int np = len - s * K < K ? len - s * K : K;
-    float* T = tiles + slot * tile_floats;
-    if (lane == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&full[slot], (unsigned)(np * A * LR) * 4u);
-    }
-    __syncwarp();
-    if (contiguous) {
-      const int first = ch.pstep == 1 ? pix0 + s * K : pix0 - (s * K + np - 1);
-      if (lane < A) {
-        const int sid = p.agg ? (lane == 1 ? ch.dir : ch.inv) : lane - 1;
-        const float* src = (lane == 0 ? U : Mr + (long long)sid * p.slice) + (long long)first * LR;
-        bulk_g2s(T + lane * K * LR, src, (unsigned)(np * LR) * 4u, &full[slot]);
-      }
-    } else {
-      for (int q = lane; q < np * A; q += 32) {
-        const int k = q / A, a = q - k * A;
-        const int px = pix0 + (s * K + k) * ch.pstep;
-        const int sid = p.agg ? (a == 1 ? ch.dir : ch.inv) : a - 1;
-        const float* src = (a == 0 ? U : Mr + (long long)sid * p.slice) + (long long)px * LR;
-        bulk_g2s(T + (a * K + k) * LR, src, (unsigned)LR * 4u, &full[slot]);
-      }
-    }
-  };
-
-  const int la = lane, lb = lane + 32;
-  const bool actb = lb < L;               // la < L always (L > 32)
-  const int lbc = actb ? lb : la;         // loads of a missing second label repeat the first
-  const float* rowa = ctab + la * kPairRS;
-  const float* rowb = ctab + lbc * kPairRS;
-  float* Mw = p.msg_write + (long long)ch.dir * p.slice + ibase * LR;
-  const float* E = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
-  uint8_t* MI = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR : nullptr;
-  uint8_t* NI = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
-  const int dir_off = (p.agg ? 1 : 1 + ch.dir) * K * LR, inv_off = (p.agg ? 2 : 1 + ch.inv) * K * LR;
+  const int c0 = 2 * lane;
+  const bool act0 = FULL || c0 < L, act1 = FULL || c0 + 1 < L;
+  // bounds of the lane's labels (an inactive one has h = +inf and is never in the list)
+  const float* bt = btab + c0;
+  const float lo0 = act0 ? bt[0] : 0.f, lo1 = act1 ? bt[1] : 0.f, olo0 = bt[128], olo1 = bt[129];
+  const float hi0 = act0 ? bt[64] : 0.f, hi1 = act1 ? bt[65] : 0.f, ohi0 = bt[192], ohi1 = bt[193];
+  const float own0 = bt[256], own1 = bt[257];
+  // of the whole table
+  const float lo = any_nan ? -kInf : warp_min(fminf(act0 ? lo0 : kInf, act1 ? lo1 : kInf));
+  const float hi = any_nan ? kInf : -warp_min(fminf(act0 ? -hi0 : kInf, act1 ? -hi1 : kInf));
+  const char* crow = reinterpret_cast<const char*>(ctab + c0);  // + a list entry's offset: this lane's two context values
+  const unsigned below = (1u << lane) - 1u;
+  const int off0 = c0 * 256, off1 = off0 + 256, off_last = (L - 1) * 256;
   const float rho = p.rho;
-  auto load_e = [&](int s) -> float {
-    const int j = s * K + lane;
-    return (E && lane < K && j < len && j >= 1) ? E[pix0 + j * ch.pstep] : 1.f;
+
+  // Staging of chain pixel j (past the chain's end: the last one again, into slots nobody reads).  Everything that moves is a
+  // 32-bit offset into the image.
+  const int pix0 = ch.h0 * p.W + ch.w0, ostep = ch.pstep * LR;
+  const float* const Ub = p.unary + ibase * LR + c0;
+  const float* const Mb = p.msg_read + ibase * LR + c0;
+  const float* const Md = Mb + ch.dir * p.slice;
+  const float* const Mi = Mb + ch.inv * p.slice;
+  const float* const Eb = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
+  float* my_ring = ring + c0;
+  auto cp_async8 = [](float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
   };
-  float ca[64], cb[64];  // the rows of labels la and lb
-#pragma unroll
-  for (int f = 0; f < 64; ++f) ca[f] = rowa[f], cb[f] = rowb[f];
-  // highest label attaining `best` among the eight of group g (a NaN minimum equals nothing: stay in the group)
-  auto label_in_group = [&](const float* hb, const float* row, float e, int g, float best) {
-    const float4* h = reinterpret_cast<const float4*>(hb) + 2 * g;
-    const float4* r4 = reinterpret_cast<const float4*>(row) + 2 * g;
-    const float4 x = r4[0], y = r4[1];
-    const float c[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-    float v[8];
-    pair_cand8(c, h[0], h[1], e, v);
-    return 8 * g + (highest_equal<8>(v, best) & 7);
+  int ahead = 0, o_ahead = pix0 * LR, e_ahead = pix0;  // pixel that is staged next
+  auto issue = [&]() {
+    float* dst = my_ring + (ahead & (kPairRing - 1)) * slot_floats;
+    if (FULL || c0 < LR) {
+      cp_async8(dst, Ub + o_ahead);
+      if (AGG) {
+        cp_async8(dst + 64, Md + o_ahead);
+        cp_async8(dst + 128, Mi + o_ahead);
+      } else {
+        for (int k = 0; k < D; ++k) cp_async8(dst + (1 + k) * 64, Mb + k * p.slice + o_ahead);
+      }
+    }
+    if (Eb && lane == 0) cp_async4(dst + A * 64, Eb + e_ahead);
+    cp_async_commit();
+    ++ahead;
+    o_ahead += ahead < len ? ostep : 0;
+    e_ahead += ahead < len ? ch.pstep : 0;
+  };
+  const int dir_off = (AGG ? 1 : 1 + ch.dir) * 64, inv_off = (AGG ? 2 : 1 + ch.inv) * 64;
+  auto uu_of = [&](const float* t, float& u0, float& u1) {  // reference order of the additions
+    float2 v = *reinterpret_cast<const float2*>(t);
+    if (MODE == 0)
+      for (int a = 1; a <= D; ++a) {
+        const float2 x = *reinterpret_cast<const float2*>(t + a * 64);
+        v.x += x.x, v.y += x.y;
+      }
+    if (MODE == 2) {
+      u0 = v.x * rho, u1 = v.y * rho;
+    } else {
+      const float2 d = *reinterpret_cast<const float2*>(t + dir_off), i = *reinterpret_cast<const float2*>(t + inv_off);
+      u0 = fmaf(v.x - d.x, rho, -i.x);
+      u1 = fmaf(v.y - d.y, rho, -i.y);
+    }
   };
 
-  for (int s = 0; s < NS; ++s) issue_stage(s);
-  if (lane < K) etile[lane] = load_e(0);
-  float e_next = load_e(1);
-  float uu0 = 0.f, uu1 = 0.f, r0 = 0.f, r1 = 0.f;
-  // rows of the current chain pixel, moved by one pixel per step (the stage depth is a launch
-  // parameter: nothing of it folds into immediates)
-  const int postep = ch.pstep * LR, KL = K * LR;
-  float* mwa = Mw + (long long)pix0 * LR + la;
-  uint8_t* mia = TRAIN ? MI + (long long)pix0 * LR + la : nullptr;
-  uint8_t* nip = TRAIN ? NI + pix0 : nullptr;
-  int hpar = 0;
-  bool first = true;
-  const bool flip = contiguous && ch.pstep == -1;
-  for (int s = 0; s < nstages; ++s) {
-    const int slot = s % NS;
-    if (!mbar_wait(&full[slot], (s / NS) & 1)) {
-      if (lane == 0) atomicExch(p.status, 132);
-      return;
-    }
-    const int np = len - s * K < K ? len - s * K : K;
-    const float* T = tiles + slot * tile_floats;
-    const float* et = etile + (s & 1) * K;
+  float* const mw = p.msg_write + (long long)ch.dir * p.slice + ibase * LR + c0;
+  uint8_t* const mi = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR + c0 : nullptr;
+  uint8_t* const nip = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
+  int of = pix0 * LR, px = pix0;  // of the current pixel
+  // paired stores need 8-byte messages and 2-byte indices (rows are multiples of 16 bytes, of four indices)
+  const bool paired = FULL || (act1 && ((uintptr_t)mw & 7) == 0 && (!TRAIN || ((uintptr_t)mi & 1) == 0));
+  for (int j = 0; j < kPairRing - 1; ++j) issue();
+  cp_async_wait<kPairRing - 2>();
+  float uu0, uu1, r0 = 0.f, r1 = 0.f;
+  uu_of(my_ring, uu0, uu1);
+  float2* spare = list + kPairList;
+  for (int i = 1; i < len; ++i) {
+    issue();
+    of += ostep;
+    px += ch.pstep;
+    const float h0 = act0 ? fmaf(rho, r0, uu0) : kInf, h1 = act1 ? fmaf(rho, r1, uu1) : kInf;
+    const float hmin = warp_min(fminf(h0, h1));
+    cp_async_wait<kPairRing - 2>();
+    __syncwarp();  // the weight is lane 0's copy; the list two steps back has been read
+    const float* slot = ring + (i & (kPairRing - 1)) * slot_floats;
+    const float e = Eb ? slot[A * 64] : 1.f;
+    uu_of(slot + c0, uu0, uu1);
+    const bool up = e >= 0.f;
+    const float m = warp_min(fminf(fmaf(e, up ? lo0 : hi0, h0), fmaf(e, up ? lo1 : hi1, h1)));
+    const float top = fmaf(e, up ? hi : lo, hmin);
+    const bool live0 = act0 && !(fmaf(e, up ? olo0 : ohi0, h0) > top), live1 = act1 && !(fmaf(e, up ? olo1 : ohi1, h1) > top);
+    const unsigned even = __ballot_sync(0xffffffffu, live0), odd = __ballot_sync(0xffffffffu, live1);
+    const int n = __popc(even) + __popc(odd);
+    float2* at = list + __popc(even & below) + __popc(odd & below);
+    if (live0) *at = make_float2(h0, __int_as_float(off0));
+    if (live1) at[live0 ? 1 : 0] = make_float2(h1, __int_as_float(off1));
+    // the list is read four entries at a time: those behind it are +inf, which is a minimum only where all
+    // candidates are, and then the last label's
+    if (lane < 4) list[n + lane] = make_float2(kInf, __int_as_float(off_last));
     __syncwarp();
-    const float* t = T + (flip ? np - 1 : 0) * LR;
-    const int tstep = flip ? -LR : LR;
-    for (int k = 0; k < np; ++k, t += tstep, mwa += postep, hpar ^= 64) {
-      float va = t[la], vb = t[lbc];
-      if (!p.agg)
-        for (int a = 1; a <= D; ++a) va += t[a * KL + la], vb += t[a * KL + lbc];
-      float un0, un1;
-      if (first_it) {
-        un0 = va * rho, un1 = vb * rho;
-      } else {
-        un0 = fmaf(va - t[dir_off + la], rho, -t[inv_off + la]);
-        un1 = fmaf(vb - t[dir_off + lbc], rho, -t[inv_off + lbc]);
-      }
-      if (!first) {
-        const float e = et[k];
-        float* hb = hbuf + hpar;
-        hb[la] = fmaf(rho, r0, uu0);
-        if (actb) hb[lb] = fmaf(rho, r1, uu1);
-        __syncwarp();
-        float b0 = kInf, b1 = kInf;
-        int g0 = 0, g1 = 0;  // highest group of eight attaining the minimum so far
+    float b0 = kInf, b1 = kInf;
+    int i0 = 0, i1 = 0;  // offsets of the argmin's context rows: 256 * label
+    for (int j = 0; j < n; j += 4) {
+      const float4 x = reinterpret_cast<const float4*>(list + j)[0], y = reinterpret_cast<const float4*>(list + j)[1];
+      const float hf[4] = {x.x, x.z, y.x, y.z};
+      const int of[4] = {__float_as_int(x.y), __float_as_int(x.w), __float_as_int(y.y), __float_as_int(y.w)};
+      float v0[4], v1[4];
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const float4 h0 = reinterpret_cast<const float4*>(hb)[2 * g], h1 = reinterpret_cast<const float4*>(hb)[2 * g + 1];
-          float v[8];
-          pair_cand8(ca + 8 * g, h0, h1, e, v);
-          const float m0 = min_tree<8>(v);
-          pair_cand8(cb + 8 * g, h0, h1, e, v);
-          const float m1 = min_tree<8>(v);
-          if (g == 0) {
-            b0 = m0, b1 = m1;
-          } else {
-            if (TRAIN) g0 = m0 <= b0 ? g : g0, g1 = m1 <= b1 ? g : g1;
-            b0 = fminf(b0, m0), b1 = fminf(b1, m1);
-          }
-        }
-        const float x1 = actb ? b1 : kInf;
-        const float m = warp_min(fminf(b0, x1));
-        r0 = b0 - m;
-        r1 = b1 - m;
-        mwa[0] = r0;
-        if (actb) mwa[32] = r1;
-        if (TRAIN) {
-          const unsigned bal0 = __ballot_sync(0xffffffffu, b0 == m);
-          const unsigned bal1 = __ballot_sync(0xffffffffu, x1 == m);
-          mia[0] = (uint8_t)label_in_group(hb, rowa, e, g0, b0);
-          const int i1 = label_in_group(hb, rowb, e, g1, b1);
-          if (actb) mia[32] = (uint8_t)i1;
-          if (lane == 0) *nip = (uint8_t)(bal1 ? 63 - __clz(bal1) : 31 - __clz(bal0));
-        }
+      for (int q = 0; q < 4; ++q) {
+        const float2 c = *reinterpret_cast<const float2*>(crow + of[q]);
+        v0[q] = fmaf(e, c.x, hf[q]);
+        v1[q] = fmaf(e, c.y, hf[q]);
       }
-      uu0 = un0;
-      uu1 = un1;
-      first = false;
       if (TRAIN) {
-        mia += postep;
-        nip += ch.pstep;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          i0 = v0[q] <= b0 ? of[q] : i0, i1 = v1[q] <= b1 ? of[q] : i1;
+          b0 = fminf(b0, v0[q]);
+          b1 = fminf(b1, v1[q]);
+        }
+      } else {
+        b0 = min3f(min3f(b0, v0[0], v0[1]), v0[2], v0[3]);
+        b1 = min3f(min3f(b1, v1[0], v1[1]), v1[2], v1[3]);
       }
     }
-    if (lane < K) etile[((s + 1) & 1) * K + lane] = e_next;
-    e_next = load_e(s + 2);
-    __syncwarp();
-    issue_stage(s + NS);
+    {  // each label's candidate for itself
+      const float v0 = fmaf(e, own0, h0), v1 = fmaf(e, own1, h1);
+      if (TRAIN) {
+        i0 = v0 < b0 ? off0 : v0 == b0 ? max(i0, off0) : i0;
+        i1 = v1 < b1 ? off1 : v1 == b1 ? max(i1, off1) : i1;
+      }
+      b0 = fminf(b0, v0);
+      b1 = fminf(b1, v1);
+    }
+    r0 = b0 - m;
+    r1 = b1 - m;
+    if (paired) {
+      *reinterpret_cast<float2*>(mw + of) = make_float2(r0, r1);
+      if (TRAIN) *reinterpret_cast<unsigned short*>(mi + of) = (unsigned short)((i0 >> 8) | i1);
+    } else if (act0) {
+      mw[of] = r0;
+      if (act1) mw[of + 1] = r1;
+      if (TRAIN) {
+        mi[of] = (uint8_t)(i0 >> 8);
+        if (act1) mi[of + 1] = (uint8_t)(i1 >> 8);
+      }
+    }
+    if (TRAIN) {
+      const int n0 = 31 - __clz(__ballot_sync(0xffffffffu, act0 && b0 == m));
+      const int n1 = 31 - __clz(__ballot_sync(0xffffffffu, act1 && b1 == m));
+      if (lane == 0) nip[px] = (uint8_t)max(2 * n0, 2 * n1 + 1);
+    }
+    float2* const other = spare;
+    spare = list, list = other;
   }
+  cp_async_wait<0>();
 }
 
 template <bool TRAIN>
-cudaError_t launch_pair(FwdParams p, cudaStream_t st) {
+cudaError_t launch_pair(const FwdParams& p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
   const int A = (p.first ? 0 : p.agg ? 2 : p.D) + 1;
-  int K = 4, NS = 3;
-  auto per_warp = [&](int k, int ns) { return ((ns * A * k * p.ls + 128 + 2 * k + 2 * ns + 2) + 3) & ~3; };
-  auto bytes = [&](int k) { return ((size_t)64 * kPairRS + (size_t)kPairWarps * per_warp(k, NS)) * sizeof(float); };
-  while (K > 1 && bytes(K) > 72 * 1024) K >>= 1;
-  p.tma_k = K;
-  p.tma_stages = NS;
-  const size_t smem = bytes(K);
-  cudaError_t e = ensure_smem(fwd_pair_kernel<TRAIN>, smem);
-  if (e != cudaSuccess) return e;
-  ProfScope prof(kProfFwdSweep, st);
-  count_launch();
-  return launch_dependent(fwd_pair_kernel<TRAIN>, (total + kPairWarps - 1) / kPairWarps, kPairWarps * 32, smem, st, p);
+  // eight chains per CTA where they fill the SMs (24 warps each), else four, so that more SMs get some
+  const int wpb = total >= 148 * 16 && A <= 3 ? 8 : 4;
+  const size_t smem = (size_t)(kPairCtx + kPairBounds + pair_warp_floats(A) * wpb) * sizeof(float);
+  auto go = [&](auto kernel) -> cudaError_t {
+    cudaError_t e = ensure_smem(kernel, smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    ProfScope prof(kProfFwdSweep, st);
+    count_launch();
+    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
+  };
+  const bool full = p.L == 64 && p.ls == 64 && ((uintptr_t)p.msg_write & 7) == 0 && (!TRAIN || ((uintptr_t)p.min_idx & 1) == 0);
+  if (p.first) return full ? go(fwd_pair_kernel<2, TRAIN, true>) : go(fwd_pair_kernel<2, TRAIN, false>);
+  if (p.agg) return full ? go(fwd_pair_kernel<1, TRAIN, true>) : go(fwd_pair_kernel<1, TRAIN, false>);
+  return full ? go(fwd_pair_kernel<0, TRAIN, true>) : go(fwd_pair_kernel<0, TRAIN, false>);
 }
 
 // Label rows of 16-byte multiples at 16-byte aligned bases: the bulk-copy CTA kernel applies.

@@ -13,6 +13,30 @@ from oracle import oracle
 pytestmark = pytest.mark.gpu
 
 
+def _table(kind, L, rng):
+    if kind == "random":       # few candidates are live once messages have spread
+        a = rng.uniform(0.0, 1.0, (L, L))
+    elif kind == "potts":      # every column without its diagonal holds one value
+        a = np.ones((L, L))
+    elif kind == "zero":       # all candidates of a step are equal: all live, the highest label wins
+        a = np.zeros((L, L))
+    elif kind == "mixed":      # negative entries, a diagonal that is not the smallest
+        a = rng.uniform(-1.0, 1.0, (L, L))
+    elif kind == "ties":
+        a = rng.integers(1, 4, (L, L)).astype(float)
+    else:                      # "steep": costs of very different size
+        a = 10.0 ** rng.uniform(-6, 6, (L, L))
+    a = np.triu(a, 1)
+    d = rng.uniform(-0.5, 0.5, L) if kind == "mixed" else np.zeros(L)
+    return (a + a.T + np.diag(d)).astype(np.float32)
+
+
+def _unary(kind, shape, rng):
+    if kind in ("ties", "zero", "potts"):
+        return rng.integers(0, 4, shape).astype(np.float32)
+    return rng.standard_normal(shape).astype(np.float32)
+
+
 def _same_forward(mode, unary, ctx, ew, D, I, training=True, **kw):
     want = oracle.forward(mode, unary, ctx, ew, D, I, msg_init=kw["msg_init"]) if "msg_init" in kw \
         else oracle.forward(mode, unary, ctx, ew, D, I)
@@ -20,6 +44,31 @@ def _same_forward(mode, unary, ctx, ew, D, I, training=True, **kw):
     for k in ("cost", "msg") + (("min_idx", "norm_idx") if training else ()):
         assert np.array_equal(got[k], want[k]), k
     return want
+
+
+@pytest.mark.parametrize("kind", ["random", "potts", "zero", "mixed", "ties", "steep"])
+@pytest.mark.parametrize("mode,D,I,L,negative", [
+    ("ISGMR", 8, 2, 64, False),
+    ("ISGMR", 4, 3, 36, True),    # weights of both signs: the bounds change places
+    ("TRWP", 4, 2, 60, True),
+    ("TRWP", 8, 1, 40, False),
+])
+def test_live_labels(kind, mode, D, I, L, negative):
+    rng = np.random.default_rng(L + D)
+    shape = (1, 1, 13, 22, L)
+    ew = rng.uniform(-0.5 if negative else 0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    if kind in ("ties", "zero", "potts"):
+        ew = np.sign(ew) * 2.0 ** np.round(2 * np.abs(ew))
+    ctx, unary = _table(kind, L, rng), _unary(kind, shape, rng)
+    _same_forward(mode, unary, ctx, ew.astype(np.float32), D, I)
+    _same_forward(mode, unary, ctx, None, D, I, training=False)
+
+
+@pytest.mark.parametrize("L", [33, 34, 62, 63])
+def test_live_labels_odd_counts(L):
+    """Label counts that leave a lane with one label or none, on rows padded to a multiple of four."""
+    rows.test_padded_rows_and_zero_start("ISGMR", 8, 1, 12, 19, L, 3, "sym2d", True)
+    rows.test_padded_rows_and_zero_start("TRWP", 4, 1, 12, 19, L, 2, "sym2d", True)
 
 
 def _truncated(kind, R, L):
