@@ -1241,7 +1241,8 @@ cudaError_t launch_backward_init_lhw(const float* dcost, float* dunary, float* d
 cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
   BwdParams p = p0;
   if (p.ndirs < 1) p.ndirs = 1;
-  if (p.cp_scheme == 2 && p.L <= 32 && p.ndirs > 1 && p.parts <= 1 &&
+  const bool quad = bwd_quad_eligible(p) && !pair_kernels_disabled();
+  if (!quad && p.cp_scheme == 2 && p.L <= 32 && p.ndirs > 1 && p.parts <= 1 &&
       (long long)p.nimg * (p.H < p.W ? p.H : p.W) >= 256) {
     // ISGMR, L <= 32: the axis directions whose rows are 16-byte aligned go to the bulk-copy kernel
     // one by one (the sweeps are independent), the rest to one launch of the generic kernel.
@@ -1271,7 +1272,10 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
   if (total == 0) return cudaSuccess;
   const int L = p.L, LS = L | 1;
   ProfScope prof(kProfBwdSweep, st);
-  if (L <= 32 && p.parts <= 1 && bwd_tma_eligible(p)) {
+  if (quad) {
+    cudaError_t e = launch_backward_quad(p, total, st);
+    if (e != cudaSuccess) return e;
+  } else if (L <= 32 && p.parts <= 1 && bwd_tma_eligible(p)) {
     p.tma_stages = tma_stage_override() ? tma_stage_override() : 4;
     cudaError_t e = L == 21 && p.ls == 21   ? launch_bwd_tma<21, 21, false>(p, st)
                     : L == 21 && p.ls == 24 ? launch_bwd_tma<21, 21, true>(p, st)

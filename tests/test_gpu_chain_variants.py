@@ -71,6 +71,41 @@ def test_live_labels_odd_counts(L):
     rows.test_padded_rows_and_zero_start("TRWP", 4, 1, 12, 19, L, 2, "sym2d", True)
 
 
+@pytest.mark.parametrize("L,D,B,H,W", [
+    (64, 8, 2, 30, 41),     # diagonal chains of 1 .. 30 pixels share warps
+    (36, 8, 1, 35, 64),
+    (64, 4, 1, 150, 150),   # chains longer than the table of a warp is kept
+    (64, 4, 1, 3, 300),
+    (32, 8, 2, 30, 41),     # eight lanes per chain
+    (20, 8, 2, 30, 41),
+    (4, 4, 2, 150, 151),
+    (24, 8, 2, 30, 41),     # a 1-D context, whose table is folded
+])
+def test_backward_lanes_share_a_chain(L, D, B, H, W):
+    rng = np.random.default_rng(L + W)
+    shape = (B, 1, H, W, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _table("random", L, rng)
+    if L == 24:
+        ctx = _truncated("linear", 3, L)
+    ew = rng.uniform(0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    want = _same_forward("ISGMR", unary, ctx, ew, D, 2)
+    dcost = rng.uniform(-1, 1, shape).astype(np.float32)
+    ref = oracle.backward("ISGMR", ctx, ew, dcost, want["min_idx"], want["norm_idx"])
+    got = g.backward("ISGMR", ctx, ew, dcost, want["min_idx"], want["norm_idx"])
+    again = g.backward("ISGMR", ctx, ew, dcost, want["min_idx"], want["norm_idx"])
+    for k in ("dunary", "dctx", "dew"):
+        assert_grad_close(got[k], ref[k], k)
+        assert np.array_equal(got[k], again[k]), k
+    none = g.backward("ISGMR", ctx, None, dcost, want["min_idx"], want["norm_idx"], keep_diag=True)
+    assert_grad_close(none["dctx"], oracle.backward("ISGMR", ctx, None, dcost, want["min_idx"], want["norm_idx"],
+                                                    keep_diag=True)["dctx"], "dctx")
+
+
+@pytest.mark.parametrize("L", [5, 21, 31, 33, 38, 63])
+def test_backward_lanes_share_a_chain_padded(L):
+    rows.test_padded_rows_and_zero_start("ISGMR", 8, 2, 30, 41, L, 2, "sym2d", True)
+
+
 def _truncated(kind, R, L):
     """Saturates at offset R; "quantised" costs tie often, "dip" is not smallest at offset 0."""
     k = np.arange(L, dtype=np.float64)
