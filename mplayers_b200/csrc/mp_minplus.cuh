@@ -209,6 +209,67 @@ __device__ __forceinline__ void minplus_regrow(const float* hb, const float (&cr
   if (TRAIN) bi = highest_equal<LMAX>(val, best);
 }
 
+// A rank-1 context that stays at its last value from offset R <= 4 on, below which it is nowhere larger (truncated
+// linear and quadratic functions, Potts): with e >= 0 the candidates of a label are those of its neighbours up to
+// R - 1 away and the one of the smallest h at the last value.
+struct NarrowWindow {
+  int R;           // 0: the context is no such one
+  float c[4];      // its values at offsets 0 .. 3
+  float least;     // smallest value of the lane's column of the label-by-label table
+  float last;
+};
+
+__device__ __forceinline__ NarrowWindow narrow_window(const float* ctx, int rank, int L, int lane) {
+  const int lc = lane < L ? lane : L - 1;
+  NarrowWindow w;
+  w.R = 0;
+  w.last = w.least = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w.c[k] = 0.f;
+  if (rank != 1) return w;
+  w.last = __ldg(ctx + L - 1);
+  const float mine = __ldg(ctx + lc);
+  const unsigned other = __ballot_sync(0xffffffffu, mine != w.last), above = __ballot_sync(0xffffffffu, !(mine <= w.last));
+  const int R = other ? 32 - __clz(other) : 1;
+  w.R = above == 0 && R <= 4 ? R : 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w.c[k] = __ldg(ctx + (k < L ? k : L - 1));
+  const int reach = max(lc, L - 1 - lc);  // furthest offset of the label
+  w.least = kInf;
+  for (int k = 0; k <= reach; ++k) w.least = fminf(w.least, __ldg(ctx + k));
+  return w;
+}
+
+// The step through such a window of up to RW offsets (those from R to RW - 1 hold the last value: exact as well).  Neighbours
+// come by shuffle (idle lanes repeat the last label, lc); a label outside 0 .. L - 1 counts as +inf.  The highest index among equal candidates: inside the window the
+// highest offset; outside it candidates are equal to the saturated minimum gv, and the highest label whose
+// saturated candidate is gv stands for all of them (its window candidate is no larger).
+template <int RW, bool TRAIN>
+__device__ __forceinline__ void minplus_narrow(const NarrowWindow& w, float h, float e, int L, int lc,
+                                               unsigned lmask, float& best, int& bi, float& m) {
+  const float hmin = warp_min(h);
+  m = warp_min(fmaf(e, w.least, h));  // fma is monotone (a uniform branch around this reduction: 28 -> 36 us a sweep)
+  const float gv = fmaf(e, w.last, hmin);
+  float cand[2 * RW];
+  cand[0] = gv;
+  cand[RW] = fmaf(e, w.c[0], h);
+#pragma unroll
+  for (int k = 1; k < RW; ++k) {
+    const float dn = __shfl_sync(0xffffffffu, h, lc - k), up = __shfl_sync(0xffffffffu, h, lc + k);
+    cand[RW - k] = lc >= k ? fmaf(e, w.c[k], dn) : kInf;
+    cand[RW + k] = lc + k < L ? fmaf(e, w.c[k], up) : kInf;
+  }
+  best = min_tree<2 * RW>(cand);
+  if (TRAIN) {
+    const unsigned sat = __ballot_sync(0xffffffffu, fmaf(e, w.last, h) == gv) & lmask;
+    const int fstar = 31 - __clz(sat);
+    int fw = -1;
+#pragma unroll
+    for (int k = 1 - RW; k < RW; ++k) fw = cand[RW + k] == best ? lc + k : fw;
+    bi = gv == best ? max(fstar, fw) : fw;
+  }
+}
+
 // q[f] = sum over labels c whose saved argmin is f of t[c], for f = `me`; fixed summation order
 // (interleaved partial sums).  tb / ib: the t values and argmin indices (stored as floats)
 // of all labels of this pixel in shared memory.  One compare-to-flag plus one fused multiply-add

@@ -116,6 +116,29 @@ def _truncated(kind, R, L):
     return c.astype(np.float32)
 
 
+@pytest.mark.parametrize("kind", ["linear", "quadratic", "dip"])
+@pytest.mark.parametrize("mode,D,B,H,W,L,R", [
+    ("TRWP", 4, 1, 19, 36, 16, 2),     # tiled copies
+    ("TRWP", 4, 1, 18, 17, 13, 2),     # one row per pixel
+    ("TRWP", 8, 1, 12, 20, 21, 4),
+    ("ISGMR", 8, 8, 33, 36, 32, 3),
+    ("ISGMR", 8, 1, 12, 13, 31, 1),
+    ("ISGMR", 4, 8, 32, 36, 2, 1),
+    ("TRWP", 4, 1, 20, 24, 24, 6),     # wider than a narrow window
+])
+def test_narrow_windows(kind, mode, D, B, H, W, L, R):
+    rng = np.random.default_rng(L + R)
+    shape = (B, 1, H, W, L)
+    ctx = _truncated(kind, R, L)
+    unary = rng.integers(0, 6, shape).astype(np.float32) / 2
+    ew = rng.choice([0.0, 0.5, 1.0, 2.0], (D,) + shape[:-1]).astype(np.float32)
+    _same_forward(mode, unary, ctx, ew, D, 2)
+    _same_forward(mode, unary, ctx, None, D, 2, training=False)
+    ew[:, :, :, H // 2:, W // 3] = -1.0    # stages and steps with a negative weight evaluate every candidate
+    _same_forward(mode, unary, ctx, ew, D, 2)
+    _same_forward(mode, unary, ctx, ew, D, 2, training=False)
+
+
 @pytest.mark.parametrize("L", [36, 52, 64])
 @pytest.mark.parametrize("R,kind,I", [(1, "linear", 2), (2, "linear", 3), (3, "dip", 2), (4, "quadratic", 2)])
 def test_two_chains_per_warp(L, R, kind, I):
