@@ -96,7 +96,8 @@ typedef struct mpl_rows {
                                a labels-first cost_final has no padding. */
   int32_t messages_zero;    /* forward calls: 1 = the iterations start from zero messages whatever `msg` (and
                                `msg_update`) hold, which then need not be initialised; on return `msg` is
-                               complete.  Ignored by backward calls. */
+                               complete.  2 = the same, and the caller does not need the messages: what
+                               `msg` holds on return is undefined.  Ignored by backward calls. */
 } mpl_rows;
 
 /* Analyses a rank-1 context (and the edge weights, may be NULL) for mpl_problem::context_window:

@@ -86,7 +86,7 @@ class TRWPFunction(torch.autograd.Function):
         _TRWP.forward(rho, int(n_iter), int(args.enable_min_a_dir), unary, label_context, ew, message,
                       cost_final, message_index, cost_index, _empty_f32(unary.device), label_all,
                       context_window=int(getattr(args, "context_window", 0) or 0), cost_labels_first=lf,
-                      n_disp=n_disp, messages_zero=True)
+                      n_disp=n_disp, messages_zero=True, messages_needed=False)
         ctx.cost_labels_first = lf
         ctx.n_disp = n_disp
         ctx.intermediate_results = rho, message_index, cost_index, label_context, ew, enable_edge_weights

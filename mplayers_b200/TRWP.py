@@ -27,13 +27,14 @@ def _problem(n_iter, msg_shape, context, rho, enable_min_a_dir=0, enable_sgm=0, 
 
 def forward(rho, n_iter, enable_min_a_dir, unary, context, edge_weights, msg, cost_final,
             msg_min_index, msg_norm_index, unary_update, label_all, context_window=0, cost_labels_first=False, n_disp=0,
-            messages_zero=False):
+            messages_zero=False, messages_needed=True):
     """`context_window` (keyword, not in the reference's signature): see mpl_problem::context_window;
     0 lets the library find out by itself, which makes an inference call with a rank-1 context and
     more than 32 labels wait for the stream once.  `cost_labels_first` (keyword): cost_final is
     [B,cv,L,H,W] instead of [B,cv,H,W,L] (mpl_problem::cost_labels_first).  `n_disp` (keyword): the label
     count where the label rows of the labels-last tensors are padded (mpl_rows::label_stride);
-    `messages_zero` (keyword): start from zero messages, `msg` need not be initialised."""
+    `messages_zero` (keyword): start from zero messages, `msg` need not be initialised; with
+    `messages_needed` = False besides, `msg` is scratch whose contents on return are undefined."""
     dev = unary.device
     for t, n in ((unary, "unary"), (context, "context"), (edge_weights, "edge_weights"), (msg, "msg"),
                  (cost_final, "cost_final")):
@@ -45,7 +46,7 @@ def forward(rho, n_iter, enable_min_a_dir, unary, context, edge_weights, msg, co
         raise RuntimeError("msg must be [D,B,cv,H,W,L] matching unary [B,cv,H,W,L]")
     prob = _problem(n_iter, tuple(msg.shape), context, rho, enable_min_a_dir, context_window=context_window,
                     cost_labels_first=cost_labels_first, n_disp=n_disp)
-    rows = _lib.Rows(unary.size(-1), int(bool(messages_zero)))
+    rows = _lib.Rows(unary.size(-1), (1 if messages_needed else 2) if messages_zero else 0)
     with torch.cuda.device(dev):
         nbytes = _lib.lib().mpl_forward_workspace_bytes_mode(ctypes.byref(prob), ctypes.byref(rows), 0)
         ws = _lib.workspace(nbytes, dev)

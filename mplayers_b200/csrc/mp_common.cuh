@@ -120,7 +120,7 @@ struct FwdParams {
   // forward_skips_zero_slices() says so; other launches read slices that hold zeros.
   int first;
   // TRWP, four directions, kernels with several labels per lane (forward_takes_prefix()): sums P = (U + M_0) + M_1 of an iteration.
-  float* prefix_out;      // direction 1 writes them here (or nullptr)
+  float* prefix_out;      // direction 1 writes them here, direction 3 the final costs instead of its messages (or nullptr)
   int slice0;             // 2: `unary` holds them and the sweep (direction 2 or 3) stages slices 2 and 3 only; else 0
   int host_windowed;      // host copy of the context analysis (rank-1, L > 32): windowed path is exact
   int host_R;             //   ... and its window half-width

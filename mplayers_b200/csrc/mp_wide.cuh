@@ -69,12 +69,14 @@ __device__ __forceinline__ int warp_max_i32(int v) {
 // M_1, which the additions of every sweep start with and which directions 2 and 3 leave as they are.  5 and -5 are 4 and -1
 // in a sweep of direction 1 that also writes P (FwdParams::prefix_out); 3 stages P (as FwdParams::unary) and the two
 // slices from FwdParams::slice0 = 2 on, and a first iteration's directions 2 and 3 are 1 and -1 over P.  21 volumes
-// instead of 24 per iteration, 11 instead of 14 in the first; the order of the additions stays.
+// instead of 24 per iteration, 11 instead of 14 in the first; the order of the additions stays.  6 and -6 are 3 and -1 over P
+// in the call's last sweep (direction 3) where nobody needs its messages: it stores the final costs (P + M_2) + M_3 in
+// FwdParams::prefix_out instead.
 // SELF: no producer warps, each consumer stages its own inputs (a compile-time switch: as a run-time one
 // it cost the other launches 3 to 12 %).
 // Staged message slices of a mode DT (-1: FwdParams::D).
 __host__ __device__ constexpr int wide_slices(int dt) {
-  return dt == 1 ? 0 : dt == 3 ? 2 : dt == 5 ? 4 : dt == -5 ? 1 : dt < 0 ? -dt : dt ? dt : -1;
+  return dt == 1 ? 0 : dt == 3 || dt == 6 ? 2 : dt == 5 ? 4 : dt == -5 || dt == -6 ? 1 : dt < 0 ? -dt : dt ? dt : -1;
 }
 
 template <int LPT, int RW, int DT, bool TRAIN, bool SELF>
@@ -85,7 +87,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   constexpr int G = ((RW - 1 + 3) / 4) * 4;      // guard band (floats) on both sides of the window buffer
   constexpr int NWV = (LPT + 2 * G) / 2;         // float2 loads covering a lane's window
   constexpr bool AGG = DT == 2;  // aggregate mode (FwdParams::agg): arrays A, M_dir, M_inv
-  constexpr bool PREFIX = DT == 5 || DT == -5;
+  constexpr bool FINAL = DT == 6 || DT == -6, PREFIX = DT == 5 || DT == -5 || FINAL;
   constexpr int DC = wide_slices(DT);
   const int L = p.L, LR = p.ls, D = DC >= 0 ? DC : p.D, A = D + 1, K = p.tma_k, NS = p.tma_stages;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   const int KL = K * LR;
   const int ostep = ch.pstep * LR;
   float* out = Mw + (long long)pix0 * LR + c0;                       // message row of the current pixel
-  float* pfx = PREFIX ? p.prefix_out + (ibase + pix0) * LR + c0 : nullptr;  // its row of P
+  float* pfx = PREFIX ? p.prefix_out + (ibase + pix0) * LR + c0 : nullptr;  // its row of P, or of the costs
   uint8_t* idxp = TRAIN ? MI + (long long)pix0 * LR + c0 : nullptr;  // its argmin indices
   uint8_t* nrmp = TRAIN ? NI + pix0 : nullptr;                      // its normalisation index
   int hpar = 0;                                                     // which window buffer the pixel writes
@@ -245,7 +247,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
     for (int k = 0; k < np; ++k, t += tstep, out += ostep, hpar ^= 1) {
       // inputs of this pixel -> UU (reference order of the additions), LPT labels per lane
       float un[LPT];
-      float pv[LPT], pm[LPT];  // PREFIX: U + M_0, and M_1 as it is at the chain's first pixel, which no sweep writes
+      float pv[LPT], pm[LPT];  // PREFIX: U + M_0 (P + M_2), and M_1 (M_3) as it is at the chain's first pixel, which no sweep writes
       if (nl == LPT) {
         float v[LPT], md[LPT], mi[LPT];
 #pragma unroll
@@ -389,7 +391,8 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
         }
 #pragma unroll
         for (int i = 0; i < LPT; ++i) r[i] = best[i] - m;
-        if (nl == LPT) {
+        if (FINAL) {
+        } else if (nl == LPT) {
 #pragma unroll
           for (int q = 0; q < LPT / 2; ++q) reinterpret_cast<float2*>(out)[q] = make_float2(r[2 * q], r[2 * q + 1]);
         } else {
@@ -499,6 +502,7 @@ template <int LPT, int RW, bool TRAIN>
 cudaError_t launch_wide(const FwdParams& p, cudaStream_t st) {
   if (p.first) {  // (directions beyond 3 of a TRWP iteration read every slice: those above 3 hold zeros)
     if (p.agg || p.dir0 == 0) return launch_wide_d<LPT, RW, 1, TRAIN>(p, st);
+    if (p.slice0 == 2 && p.prefix_out) return launch_wide_d<LPT, RW, -6, TRAIN>(p, st);
     if (p.slice0 == 2) return p.dir0 == 2 ? launch_wide_d<LPT, RW, 1, TRAIN>(p, st) : launch_wide_d<LPT, RW, -1, TRAIN>(p, st);
     if (p.dir0 == 1) return p.prefix_out ? launch_wide_d<LPT, RW, -5, TRAIN>(p, st) : launch_wide_d<LPT, RW, -1, TRAIN>(p, st);
     if (p.dir0 == 2) return launch_wide_d<LPT, RW, -2, TRAIN>(p, st);
@@ -506,7 +510,7 @@ cudaError_t launch_wide(const FwdParams& p, cudaStream_t st) {
   }
   if (p.agg) return launch_wide_d<LPT, RW, 2, TRAIN>(p, st);
   if (p.D == 2) return cudaErrorNotSupported;  // DT == 2 is reserved for the aggregate mode
-  if (p.slice0 == 2) return launch_wide_d<LPT, RW, 3, TRAIN>(p, st);
+  if (p.slice0 == 2) return p.prefix_out ? launch_wide_d<LPT, RW, 6, TRAIN>(p, st) : launch_wide_d<LPT, RW, 3, TRAIN>(p, st);
   if (p.prefix_out) return launch_wide_d<LPT, RW, 5, TRAIN>(p, st);
   if (p.D == 4) return launch_wide_d<LPT, RW, 4, TRAIN>(p, st);
   if (p.D == 8) return launch_wide_d<LPT, RW, 8, TRAIN>(p, st);

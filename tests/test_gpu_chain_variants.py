@@ -4,10 +4,12 @@ contexts where they can go wrong.  Forward results and saved indices have to be 
 to the tolerances of helpers.assert_grad_close."""
 import numpy as np
 import pytest
+import torch
 
 import gpu_runner as g
 import test_gpu_rows as rows
 from helpers import assert_grad_close
+from mplayers_b200 import TRWP
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -177,3 +179,25 @@ def test_sums_of_two_directions(L, R, H, W, given):
     kw = {"msg_init": rng.uniform(0, 1, (4,) + shape).astype(np.float32)} if given else {}
     _same_forward("TRWP", unary, ctx, ew, 4, 3, **kw)
     _same_forward("TRWP", unary, ctx, ew, 4, 2, training=False, **kw)
+
+
+@pytest.mark.parametrize("L,R,I", [(64, 3, 1), (128, 2, 3), (192, 2, 2), (200, 6, 2)])
+@pytest.mark.parametrize("labels_first", [False, True])
+def test_costs_from_the_last_sweep(L, R, I, labels_first):
+    """The caller does not need the messages: the last sweep stores the costs, in training too."""
+    rng = np.random.default_rng(L + I)
+    unary, ctx = rng.standard_normal((2, 1, 9, 14, L)).astype(np.float32), _truncated("linear", R, L)
+    want = oracle.forward("TRWP", unary, ctx, None, 4, I)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
+    for training in (False, True):
+        msg = torch.full((4,) + unary.shape, float("nan"), device="cuda")
+        cost = torch.full((2, 1, L, 9, 14) if labels_first else unary.shape, float("nan"), device="cuda")
+        mi = torch.zeros((I, 4) + unary.shape, dtype=torch.uint8, device="cuda") if training else e8
+        ni = torch.zeros((I, 4) + unary.shape[:-1], dtype=torch.uint8, device="cuda") if training else e8
+        TRWP.forward(0.5, I, 0, dev(unary), dev(ctx), e0, msg, cost, mi, ni, e0, e8, context_window=R,
+                     cost_labels_first=labels_first, messages_zero=True, messages_needed=False)
+        got = cost.cpu().numpy()
+        assert np.array_equal(np.moveaxis(got, 2, -1) if labels_first else got, want["cost"])
+        if training:
+            assert np.array_equal(mi.cpu().numpy(), want["min_idx"]) and np.array_equal(ni.cpu().numpy(), want["norm_idx"])
