@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
   const float* slot = ring;
   int px = pixl;
 
+#pragma unroll 1
   for (int s = 0; s < most; ++s, out -= ostep, px -= ch.pstep) {
     if ((s & 3) == 0) scalars((s >> 2) + 1, e_nxt, n_nxt);
     issue();

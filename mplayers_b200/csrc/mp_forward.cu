@@ -859,6 +859,215 @@ cudaError_t launch_cta_tma(FwdParams p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Up to 32 labels and many independent chains (all directions of an ISGMR iteration in one launch): one warp per chain, lane =
+// label, only the candidates that can be a minimum (see fwd_pair_kernel; class scores with a clear winner leave one to three
+// of 21).  With fewer chains than two per scheduler the kernels that evaluate all candidates are as fast: there a step
+// costs its dependent path, which the list of candidates does not shorten (2 x 512 x 512 x 21, TRWP, 1024 chains a sweep:
+// 90 us, through such a list 150).  2 x 256 x 256 x 21, eight directions, training: the axis directions one
+// launch after another and the diagonal ones 285 us per iteration, this kernel 225.
+constexpr int kLiveList = 36;   // entries: 32 and four that never win
+constexpr int kLiveRing = 8;    // pixels staged ahead (power of two)
+__host__ __device__ constexpr int live_warp_floats(int A) { return kLiveRing * (A * 32 + 4) + 2 * 2 * kLiveList; }
+
+// DT = staged message slices: 2 in aggregate mode (FwdParams::agg), else 0 (p.D of them).  V4: rows of 16-byte multiples (see
+// fwd_warp_kernel); in aggregate mode one copy instruction then stages a pixel.  R1: rank-1 context; where it has a
+// narrow window, steps with a weight >= 0 go through that.
+template <int DT, bool TRAIN, bool V4, bool R1>
+__global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant__ FwdParams p) {
+  extern __shared__ __align__(16) float smem[];
+  const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr bool AGG = DT == 2;
+  const int L = p.L, LR = p.ls, D = AGG ? 2 : p.D, A = D + 1;
+  float* ctab = smem;  // [32][32], row = label at the predecessor
+  dependent_wait();
+  for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
+    const int f = i >> 5, c = i & 31;
+    ctab[i] = (c < L && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c, f) : 0.f;
+  }
+  __syncthreads();
+  ChainCtx ch;
+  if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
+  float* ring = ctab + 32 * 32 + warp * live_warp_floats(A);  // [kLiveRing][A][32] and the weight
+  const int slot_floats = A * 32 + 4;
+  float2* list = reinterpret_cast<float2*>(ring + kLiveRing * slot_floats);  // [2][kLiveList], in turns
+  float2* spare = list + kLiveList;
+
+  const bool act = lane < L;
+  const int lc = act ? lane : 0;
+  // bounds of the lane's column and of the table, see fwd_pair_kernel
+  float lo = kInf, hi = -kInf, olo = kInf, ohi = -kInf;
+  bool nan = false;
+  for (int c = 0; c < L; ++c) {
+    const float v = ctab[c * 32 + lc];
+    nan |= v != v;
+    lo = fminf(lo, v), hi = fmaxf(hi, v);
+    if (c != lc) olo = fminf(olo, v), ohi = fmaxf(ohi, v);
+  }
+  const float own = ctab[lc * 33];
+  NarrowWindow window{};
+  if constexpr (R1) window = narrow_window(p.ctx, 1, L, lane);
+  nan = __any_sync(0xffffffffu, nan);
+  const float tab_lo = nan ? -kInf : warp_min(lo), tab_hi = nan ? kInf : -warp_min(-hi);
+  const char* crow = reinterpret_cast<const char*>(ctab + lane);  // + a list entry's offset: the lane's context value
+  const unsigned below = (1u << lane) - 1u, lmask = L >= 32 ? 0xffffffffu : (1u << L) - 1u;
+  const int off = lane * 128, off_last = (L - 1) * 128;
+  const float rho = p.rho;
+
+  // staging of chain pixel j (past the chain's end: the last one again, into slots nobody reads)
+  const int len = ch.len, pix0 = ch.h0 * p.W + ch.w0, ostep = ch.pstep * LR;
+  const long long ibase = (long long)ch.img * p.H * p.W;
+  constexpr int kRounds = V4 ? (AGG ? 1 : 5) : 1;   // pieces q = lane, lane + 32, ... of the A rows of LR / 4 pieces
+  const int nch = LR >> 2, npiece = A * nch;
+  const float* src[kRounds];
+  int dst_off[kRounds];
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    const int q = lane + 32 * k, a = V4 ? q / nch : 0, j = q - a * nch;
+    const int sid = AGG ? (a == 1 ? ch.dir : ch.inv) : a - 1;
+    src[k] = (a == 0 || q >= npiece ? p.unary : p.msg_read + sid * p.slice) + ibase * LR + (V4 ? 4 * j : lc);
+    dst_off[k] = V4 ? a * 32 + 4 * j : lane;
+  }
+  const float* Ms = p.msg_read + ibase * LR + lc;
+  const float* Eb = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) src[k] += pix0 * LR;
+  const float* Md = Ms + ch.dir * p.slice + pix0 * LR;
+  const float* Mi = Ms + ch.inv * p.slice + pix0 * LR;
+  Ms += pix0 * LR;
+  if (Eb) Eb += pix0;
+  const bool has_e = Eb != nullptr;
+  int ahead = 0;
+  auto issue = [&]() {
+    float* dst = ring + (ahead & (kLiveRing - 1)) * slot_floats;
+    if constexpr (V4) {
+#pragma unroll
+      for (int k = 0; k < kRounds; ++k)
+        if (lane + 32 * k < npiece) cp_async16(dst + dst_off[k], src[k]);
+    } else {
+      cp_async4(dst + lane, src[0]);
+      if (AGG) {
+        cp_async4(dst + 32 + lane, Md);
+        cp_async4(dst + 64 + lane, Mi);
+      } else {
+        for (int k = 0; k < D; ++k) cp_async4(dst + (1 + k) * 32 + lane, Ms + k * p.slice);
+      }
+    }
+    if (has_e && lane == 31) cp_async4(dst + A * 32, Eb);
+    cp_async_commit();
+    if (++ahead < len) {
+#pragma unroll
+      for (int k = 0; k < kRounds; ++k) src[k] += ostep;
+      if (!V4) {
+        if (AGG) {
+          Md += ostep, Mi += ostep;
+        } else {
+          Ms += ostep;
+        }
+      }
+      if (has_e) Eb += ch.pstep;
+    }
+  };
+  const int dir_off = (AGG ? 1 : 1 + ch.dir) * 32, inv_off = (AGG ? 2 : 1 + ch.inv) * 32;
+  auto uu_of = [&](const float* t) {  // reference order of the additions
+    float v = t[0];
+    if (!AGG)
+      for (int a = 1; a <= D; ++a) v += t[a * 32];
+    return fmaf(v - t[dir_off], rho, -t[inv_off]);
+  };
+  float* mw = p.msg_write + (long long)ch.dir * p.slice + (ibase + pix0) * LR + lane;
+  uint8_t* mi = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + (ibase + pix0) * LR + lane : nullptr;
+  uint8_t* nip = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase + pix0 : nullptr;
+  for (int j = 0; j < kLiveRing - 1; ++j) issue();
+  cp_async_wait<kLiveRing - 2>();
+  __syncwarp();
+  float uu = uu_of(ring + lc), r = 0.f;
+#pragma unroll 1
+  for (int i = 1; i < len; ++i) {
+    issue();
+    mw += ostep;
+    const float h = act ? fmaf(rho, r, uu) : kInf;
+    cp_async_wait<kLiveRing - 2>();
+    __syncwarp();  // every lane's copies; the list two steps back has been read
+    const float* slot = ring + (i & (kLiveRing - 1)) * slot_floats;
+    const float e = has_e ? slot[A * 32] : 1.f;
+    uu = uu_of(slot + lc);
+    float best = kInf, m;
+    int bi = 0;
+    const bool up = e >= 0.f;
+    if (R1 && window.R && up) {
+      if (window.R <= 2) {
+        minplus_narrow<2, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
+      } else {
+        minplus_narrow<4, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
+      }
+      bi <<= 7;
+    } else {
+      const float hmin = warp_min(h);
+      m = warp_min(act ? fmaf(e, up ? lo : hi, h) : kInf);
+      const float top = fmaf(e, up ? tab_hi : tab_lo, hmin);
+      const bool live = act && !(fmaf(e, up ? olo : ohi, h) > top);
+      const unsigned all = __ballot_sync(0xffffffffu, live);
+      const int n = __popc(all);
+      if (live) list[__popc(all & below)] = make_float2(h, __int_as_float(off));
+      if (lane < 4) list[n + lane] = make_float2(kInf, __int_as_float(off_last));  // read four at a time, see fwd_pair_kernel
+      __syncwarp();
+#pragma unroll 1
+      for (int j = 0; j < n; j += 4) {
+        const float4 x = reinterpret_cast<const float4*>(list + j)[0], y = reinterpret_cast<const float4*>(list + j)[1];
+        const float hf[4] = {x.x, x.z, y.x, y.z};
+        const int of[4] = {__float_as_int(x.y), __float_as_int(x.w), __float_as_int(y.y), __float_as_int(y.w)};
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = fmaf(e, *reinterpret_cast<const float*>(crow + of[q]), hf[q]);
+        if (TRAIN) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            bi = v[q] <= best ? of[q] : bi;
+            best = fminf(best, v[q]);
+          }
+        } else {
+          best = min3f(min3f(best, v[0], v[1]), v[2], v[3]);
+        }
+      }
+      const float v = fmaf(e, own, h);  // the label's candidate for itself
+      if (TRAIN) bi = v < best ? off : v == best ? max(bi, off) : bi;
+      best = fminf(best, v);
+    }
+    r = best - m;
+    if (act) *mw = r;
+    if (TRAIN) {
+      mi += ostep;
+      nip += ch.pstep;
+      if (act) *mi = (uint8_t)(bi >> 7);
+      const unsigned bal = __ballot_sync(0xffffffffu, best == m) & lmask;
+      if (lane == 0) *nip = (uint8_t)(31 - __clz(bal));
+    }
+    float2* const other = spare;
+    spare = list, list = other;
+  }
+  cp_async_wait<0>();
+}
+
+template <bool TRAIN>
+cudaError_t launch_live(const FwdParams& p, cudaStream_t st) {
+  const int total = p.chain_off[p.ndirs], wpb = total >= 148 * 32 ? 8 : 4;
+  const size_t smem = (size_t)(32 * 32 + live_warp_floats((p.agg ? 2 : p.D) + 1) * wpb) * sizeof(float);
+  auto go = [&](auto kernel) -> cudaError_t {
+    cudaError_t e = ensure_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
+    ProfScope prof(kProfFwdSweep, st);
+    count_launch();
+    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
+  };
+  const bool v4 = rows_aligned(p) && (p.agg ? 3 : p.D + 1) * (p.ls >> 2) <= (p.agg ? 32 : 160);
+  if (p.ctx_rank == 1) {
+    if (p.agg) return v4 ? go(fwd_live_kernel<2, TRAIN, true, true>) : go(fwd_live_kernel<2, TRAIN, false, true>);
+    return v4 ? go(fwd_live_kernel<0, TRAIN, true, true>) : go(fwd_live_kernel<0, TRAIN, false, true>);
+  }
+  if (p.agg) return v4 ? go(fwd_live_kernel<2, TRAIN, true, false>) : go(fwd_live_kernel<2, TRAIN, false, false>);
+  return v4 ? go(fwd_live_kernel<0, TRAIN, true, false>) : go(fwd_live_kernel<0, TRAIN, false, false>);
+}
+
 // 32 < L <= 64, rows of 16-byte multiples, any context: one WARP per chain, two labels per lane (2l and 2l + 1), no
 // block barrier (the CTA-per-chain kernel needs two per step and two warps per chain).
 //
@@ -934,35 +1143,38 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
   const int off0 = c0 * 256, off1 = off0 + 256, off_last = (L - 1) * 256;
   const float rho = p.rho;
 
-  // Staging of chain pixel j (past the chain's end: the last one again, into slots nobody reads).  Everything that moves is a
-  // 32-bit offset into the image.
+  // Staging of chain pixel j (past the chain's end: the last one again, into slots nobody reads).  Running pointers: 32-bit
+  // offsets to one base each were slower (1024 x 1024 x 64, eight directions: 2.99 -> 3.12 ms a launch).
   const int pix0 = ch.h0 * p.W + ch.w0, ostep = ch.pstep * LR;
-  const float* const Ub = p.unary + ibase * LR + c0;
-  const float* const Mb = p.msg_read + ibase * LR + c0;
-  const float* const Md = Mb + ch.dir * p.slice;
-  const float* const Mi = Mb + ch.inv * p.slice;
-  const float* const Eb = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase : nullptr;
+  const float* Us = p.unary + (ibase + pix0) * LR + c0;
+  const float* Ms = p.msg_read + (ibase + pix0) * LR + c0;
+  const float* Md = Ms + ch.dir * p.slice;
+  const float* Mi = Ms + ch.inv * p.slice;
+  const float* Es = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase + pix0 : nullptr;
   float* my_ring = ring + c0;
   auto cp_async8 = [](float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
   };
-  int ahead = 0, o_ahead = pix0 * LR, e_ahead = pix0;  // pixel that is staged next
+  int ahead = 0;  // pixel that is staged next
   auto issue = [&]() {
     float* dst = my_ring + (ahead & (kPairRing - 1)) * slot_floats;
     if (FULL || c0 < LR) {
-      cp_async8(dst, Ub + o_ahead);
+      cp_async8(dst, Us);
       if (AGG) {
-        cp_async8(dst + 64, Md + o_ahead);
-        cp_async8(dst + 128, Mi + o_ahead);
+        cp_async8(dst + 64, Md);
+        cp_async8(dst + 128, Mi);
       } else {
-        for (int k = 0; k < D; ++k) cp_async8(dst + (1 + k) * 64, Mb + k * p.slice + o_ahead);
+        for (int k = 0; k < D; ++k) cp_async8(dst + (1 + k) * 64, Ms + k * p.slice);
       }
     }
-    if (Eb && lane == 0) cp_async4(dst + A * 64, Eb + e_ahead);
+    if (Es && lane == 0) cp_async4(dst + A * 64, Es);
     cp_async_commit();
-    ++ahead;
-    o_ahead += ahead < len ? ostep : 0;
-    e_ahead += ahead < len ? ch.pstep : 0;
+    if (++ahead < len) {
+      Us += ostep;
+      if (AGG) Md += ostep, Mi += ostep;
+      if (MODE == 0) Ms += ostep;
+      if (Es) Es += ch.pstep;
+    }
   };
   const int dir_off = (AGG ? 1 : 1 + ch.dir) * 64, inv_off = (AGG ? 2 : 1 + ch.inv) * 64;
   auto uu_of = [&](const float* t, float& u0, float& u1) {  // reference order of the additions
@@ -981,10 +1193,9 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
     }
   };
 
-  float* const mw = p.msg_write + (long long)ch.dir * p.slice + ibase * LR + c0;
-  uint8_t* const mi = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + ibase * LR + c0 : nullptr;
-  uint8_t* const nip = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase : nullptr;
-  int of = pix0 * LR, px = pix0;  // of the current pixel
+  float* mw = p.msg_write + (long long)ch.dir * p.slice + (ibase + pix0) * LR + c0;
+  uint8_t* mi = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + (ibase + pix0) * LR + c0 : nullptr;
+  uint8_t* nip = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase + pix0 : nullptr;
   // paired stores need 8-byte messages and 2-byte indices (rows are multiples of 16 bytes, of four indices)
   const bool paired = FULL || (act1 && ((uintptr_t)mw & 7) == 0 && (!TRAIN || ((uintptr_t)mi & 1) == 0));
   for (int j = 0; j < kPairRing - 1; ++j) issue();
@@ -992,16 +1203,16 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
   float uu0, uu1, r0 = 0.f, r1 = 0.f;
   uu_of(my_ring, uu0, uu1);
   float2* spare = list + kPairList;
+#pragma unroll 1
   for (int i = 1; i < len; ++i) {
     issue();
-    of += ostep;
-    px += ch.pstep;
+    mw += ostep;
     const float h0 = act0 ? fmaf(rho, r0, uu0) : kInf, h1 = act1 ? fmaf(rho, r1, uu1) : kInf;
     const float hmin = warp_min(fminf(h0, h1));
     cp_async_wait<kPairRing - 2>();
     __syncwarp();  // the weight is lane 0's copy; the list two steps back has been read
     const float* slot = ring + (i & (kPairRing - 1)) * slot_floats;
-    const float e = Eb ? slot[A * 64] : 1.f;
+    const float e = Es ? slot[A * 64] : 1.f;
     uu_of(slot + c0, uu0, uu1);
     const bool up = e >= 0.f;
     const float m = warp_min(fminf(fmaf(e, up ? lo0 : hi0, h0), fmaf(e, up ? lo1 : hi1, h1)));
@@ -1018,6 +1229,7 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
     __syncwarp();
     float b0 = kInf, b1 = kInf;
     int i0 = 0, i1 = 0;  // offsets of the argmin's context rows: 256 * label
+#pragma unroll 1
     for (int j = 0; j < n; j += 4) {
       const float4 x = reinterpret_cast<const float4*>(list + j)[0], y = reinterpret_cast<const float4*>(list + j)[1];
       const float hf[4] = {x.x, x.z, y.x, y.z};
@@ -1052,21 +1264,23 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
     }
     r0 = b0 - m;
     r1 = b1 - m;
+    if (TRAIN) mi += ostep;
     if (paired) {
-      *reinterpret_cast<float2*>(mw + of) = make_float2(r0, r1);
-      if (TRAIN) *reinterpret_cast<unsigned short*>(mi + of) = (unsigned short)((i0 >> 8) | i1);
+      *reinterpret_cast<float2*>(mw) = make_float2(r0, r1);
+      if (TRAIN) *reinterpret_cast<unsigned short*>(mi) = (unsigned short)((i0 >> 8) | i1);
     } else if (act0) {
-      mw[of] = r0;
-      if (act1) mw[of + 1] = r1;
+      mw[0] = r0;
+      if (act1) mw[1] = r1;
       if (TRAIN) {
-        mi[of] = (uint8_t)(i0 >> 8);
-        if (act1) mi[of + 1] = (uint8_t)(i1 >> 8);
+        mi[0] = (uint8_t)(i0 >> 8);
+        if (act1) mi[1] = (uint8_t)(i1 >> 8);
       }
     }
     if (TRAIN) {
+      nip += ch.pstep;
       const int n0 = 31 - __clz(__ballot_sync(0xffffffffu, act0 && b0 == m));
       const int n1 = 31 - __clz(__ballot_sync(0xffffffffu, act1 && b1 == m));
-      if (lane == 0) nip[px] = (uint8_t)max(2 * n0, 2 * n1 + 1);
+      if (lane == 0) *nip = (uint8_t)max(2 * n0, 2 * n1 + 1);
     }
     float2* const other = spare;
     spare = list, list = other;
@@ -1177,6 +1391,7 @@ cudaError_t launch_zero_chain_starts(const FwdParams& p, float* a, float* b, cud
 
 cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st) {
   if (p.chain_off[p.ndirs] == 0) return cudaSuccess;
+  if (p.L <= 32 && p.ndirs > 1 && p.chain_off[p.ndirs] >= 148 * 8) return train ? launch_live<true>(p, st) : launch_live<false>(p, st);
   if (p.L <= 32) {
     // directions with aligned row segments go to the bulk-copy kernel (one launch each), the
     // remaining contiguous range of directions to the generic kernel

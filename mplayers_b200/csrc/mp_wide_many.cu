@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(kManyWarps * 32, P == 2 ? 4 : 6) fwd_wide_many
   int hpar = C * M::kWin;                 // to the other buffer
 
   // (past its end, the shorter of two chains repeats stale inputs without an effect)
+#pragma unroll 1
   for (int s = 1; s < most; ++s) {
     issue();
     out += ostep;

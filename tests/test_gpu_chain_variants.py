@@ -66,6 +66,20 @@ def test_live_labels(kind, mode, D, I, L, negative):
     _same_forward(mode, unary, ctx, None, D, I, training=False)
 
 
+@pytest.mark.parametrize("kind", ["random", "potts", "zero", "mixed", "ties", "steep"])
+@pytest.mark.parametrize("D,L,negative", [(8, 21, False), (8, 32, True), (8, 3, False), (4, 24, True)])
+def test_live_labels_up_to_32(kind, D, L, negative):
+    """Enough chains in a launch that they fill the schedulers."""
+    rng = np.random.default_rng(L + D)
+    shape = (10 if D == 4 else 4, 1, 33, 38, L)
+    ew = rng.uniform(-0.5 if negative else 0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    if kind in ("ties", "zero", "potts"):
+        ew = np.sign(ew) * 2.0 ** np.round(2 * np.abs(ew))
+    ctx, unary = _table(kind, L, rng), _unary(kind, shape, rng)
+    _same_forward("ISGMR", unary, ctx, ew.astype(np.float32), D, 2)
+    _same_forward("ISGMR", unary, ctx, None, D, 2, training=False)
+
+
 @pytest.mark.parametrize("L", [33, 34, 62, 63])
 def test_live_labels_odd_counts(L):
     """Label counts that leave a lane with one label or none, on rows padded to a multiple of four."""
