@@ -341,6 +341,17 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, uns
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Layout kernels: tiles of 128 pixels up to this label count (2 x 512 x 512 x 21: the four of a training step 218 us with
+// tiles of 32 pixels and one element per access, 130 us with these and four), of 32 pixels above.
+constexpr int kTileLabels = 32;
+// Position in a run of label rows -> pixel, without a division: i < 2^15, ls <= 256.
+struct RowIndex {
+  int ls;
+  unsigned magic;  // ceil(2^32 / ls); 0: rows of one element
+  explicit RowIndex(int stride) : ls(stride), magic(stride > 1 ? 0xffffffffu / stride + 1 : 0) {}
+  __device__ __forceinline__ int pixel(int i) const { return magic ? (int)__umulhi((unsigned)i, magic) : i; }
+};
+
 // MPL_NO_PAIR=1 keeps 32 < L <= 64 on the CTA-per-chain kernels (tuning / comparison knob).
 inline bool pair_kernels_disabled() {
   const char* e = getenv("MPL_NO_PAIR");

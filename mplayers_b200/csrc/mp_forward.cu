@@ -16,6 +16,7 @@
 // Arithmetic follows the reference order (see Appendix of the oracle header): UU = ((U + M_0 + ...
 // + M_{D-1}) - M_d) * rho - M_inv, candidate = fma(E, ctx, fma(rho, r, UU)); ties -> highest index.
 #include <cstdlib>
+#include <type_traits>
 
 #include "mp_common.cuh"
 #include "mp_minplus.cuh"
@@ -635,34 +636,59 @@ aggregate_vec4_kernel(const float4* __restrict__ unary, const float4* __restrict
 // The same sums written with the labels FIRST ([nimg, L, H*W] planes, the layout the reference's
 // module hands back after its permute, pytorch/MP_module.py:232): one block per 32 pixels of an
 // image, through a shared-memory tile so that both sides are coalesced.
+template <int TP>
 __global__ void __launch_bounds__(256)
 aggregate_lhw_kernel(const float* __restrict__ unary, const float* __restrict__ msg, float* __restrict__ cost,
-                     int L, int ls, long long HW, int D, long long slice, float factor, int min_a_dir) {
-  extern __shared__ float tile[];  // [L][33]
+                     int L, RowIndex ri, long long HW, int D, long long slice, float factor, int min_a_dir) {
+  extern __shared__ float tile[];  // [L][TP + 1]
+  constexpr int S = TP + 1;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long long b = blockIdx.y, p0 = blockIdx.x * 32ll;
-  const int np = HW - p0 < 32 ? (int)(HW - p0) : 32;
-  const long long base = (b * HW + p0) * ls;
-  for (int i = threadIdx.x; i < np * ls; i += 256) {
-    const int px = i / ls, l = i - px * ls;
-    if (l >= L) continue;  // padding of the row
-    float v = unary[base + i] * factor;
-    if (min_a_dir) {
-      float mm = msg[base + i];
-      for (int k = 1; k < D; ++k) {
-        const float x = msg[k * slice + base + i];
-        if (x < mm) mm = x;
+  const long long b = blockIdx.y, p0 = blockIdx.x * (long long)TP;
+  const int np = HW - p0 < TP ? (int)(HW - p0) : TP, n = np * ri.ls;
+  const long long base = (b * HW + p0) * ri.ls;
+  if (!min_a_dir && ((n | (int)base | (int)slice) & 3) == 0 &&
+      ((reinterpret_cast<uintptr_t>(unary) | reinterpret_cast<uintptr_t>(msg)) & 15) == 0) {
+#pragma unroll 2
+    for (int i = 4 * threadIdx.x; i < n; i += 1024) {  // four consecutive elements, of two pixels where a row ends
+      int px = ri.pixel(i), l = i - px * ri.ls;
+      const float4 u = *reinterpret_cast<const float4*>(unary + base + i);
+      float v[4] = {u.x * factor, u.y * factor, u.z * factor, u.w * factor};
+#pragma unroll 4
+      for (int k = 0; k < D; ++k) {
+        const float4 x = *reinterpret_cast<const float4*>(msg + k * slice + base + i);
+        v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w;
       }
-      v += mm;
-    } else {
-      for (int k = 0; k < D; ++k) v += msg[k * slice + base + i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (l < L) tile[l * S + px] = v[j];
+        if (++l == ri.ls) l = 0, ++px;
+      }
     }
-    tile[l * 33 + px] = v;
+  } else {
+    for (int i = threadIdx.x; i < n; i += 256) {
+      const int px = ri.pixel(i), l = i - px * ri.ls;
+      if (l >= L) continue;  // padding of the row
+      float v = unary[base + i] * factor;
+      if (min_a_dir) {
+        float mm = msg[base + i];
+        for (int k = 1; k < D; ++k) {
+          const float x = msg[k * slice + base + i];
+          if (x < mm) mm = x;
+        }
+        v += mm;
+      } else {
+        for (int k = 0; k < D; ++k) v += msg[k * slice + base + i];
+      }
+      tile[l * S + px] = v;
+    }
   }
   __syncthreads();
   float* dst = cost + b * L * HW + p0;
-  for (int l = ty; l < L; l += 8)
-    if (tx < np) dst[(long long)l * HW + tx] = tile[l * 33 + tx];
+#pragma unroll
+  for (int c = 0; c < TP; c += 32)
+    if (c + tx < np)
+#pragma unroll 4
+      for (int l = ty; l < L; l += 8) dst[(long long)l * HW + c + tx] = tile[l * S + c + tx];
 }
 
 // The same in 16-byte pieces (rows of 16-byte multiples, 16-byte aligned pointers): the D + 1 loads of a piece are
@@ -1435,111 +1461,131 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
 //   MODE 2 (backward of 1, direction hwl -> lhw): out[l] = -in[l] + (l == argmax) * sum_l in[l]
 //   MODE 3: out = in (the plain layout change of pytorch/MP_module.py:198,232)
 // ------------------------------------------------------------------------------------------------
-template <int MODE>
-__global__ void lhw_to_hwl_kernel(const float* __restrict__ in, float* __restrict__ out, uint8_t* __restrict__ amax,
-                                  int L, int ls, long long HW) {
-  extern __shared__ float tile[];  // [L][33]
-  __shared__ float mx[32];
+template <int MODE, int TP>
+__global__ void __launch_bounds__(256) lhw_to_hwl_kernel(const float* __restrict__ in, float* __restrict__ out, uint8_t* __restrict__ amax,
+                                  int L, RowIndex ri, long long HW) {
+  extern __shared__ float tile[];  // [L][TP + 1]
+  __shared__ float mx[TP];
+  constexpr int S = TP + 1;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  const long long b = blockIdx.y, p0 = blockIdx.x * 32ll;
-  const float* src = in + b * L * HW;
-  const int np = HW - p0 < 32 ? (int)(HW - p0) : 32;
-#pragma unroll 8
-  for (int l = ty; l < L; l += 8) tile[l * 33 + tx] = tx < np ? src[(long long)l * HW + p0 + tx] : 0.f;
+  const long long b = blockIdx.y, p0 = blockIdx.x * (long long)TP;
+  const float* src = in + b * L * HW + p0;
+  const int np = HW - p0 < TP ? (int)(HW - p0) : TP;
+#pragma unroll(TP == 32 ? 8 : 3)
+  for (int l = ty; l < L; l += 8)
+#pragma unroll
+    for (int c = 0; c < TP; c += 32) tile[l * S + c + tx] = c + tx < np ? src[(long long)l * HW + c + tx] : 0.f;
   __syncthreads();
   if (MODE == 1) {
-    if (ty == 0) {
-      float m = tile[tx];
+    if (threadIdx.x < TP) {
+      const int px = threadIdx.x;
+      float m = tile[px];
       int k = 0;
       for (int l = 1; l < L; ++l) {
-        const float v = tile[l * 33 + tx];
+        const float v = tile[l * S + px];
         if (v > m) m = v, k = l;
       }
-      mx[tx] = m;
-      if (tx < np) amax[b * HW + p0 + tx] = (uint8_t)k;
+      mx[px] = m;
+      if (px < np) amax[b * HW + p0 + px] = (uint8_t)k;
     }
     __syncthreads();
   }
-  float* dst = out + (b * HW + p0) * ls;
-  if ((ls & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {  // rows of 16-byte multiples: one store per four labels
-    const int row4 = ls >> 2;
+  float* dst = out + (b * HW + p0) * ri.ls;
+  auto value = [&](int l, int px) {
+    const float x = l < L ? tile[l * S + px] : 0.f;
+    return MODE == 1 ? mx[px] - x : (MODE == 3 ? x : -x);
+  };
+  const int n = np * ri.ls;
+  if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {  // one store per four consecutive elements
 #pragma unroll 4
-    for (int i = threadIdx.x; i < np * row4; i += 256) {
-      const int px = i / row4, l = 4 * (i - px * row4);
+    for (int i = 4 * threadIdx.x; i < n; i += 1024) {
+      int px = ri.pixel(i), l = i - px * ri.ls;
       float v[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float x = l + j < L ? tile[(l + j) * 33 + px] : 0.f;
-        v[j] = MODE == 1 ? mx[px] - x : (MODE == 3 ? x : -x);
+        v[j] = value(l, px);
+        if (++l == ri.ls) l = 0, ++px;
       }
-      *reinterpret_cast<float4*>(dst + 4 * i) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(dst + i) = make_float4(v[0], v[1], v[2], v[3]);
     }
     return;
   }
-  for (int i = threadIdx.x; i < np * ls; i += 256) {
-    const int px = i / ls, l = i - px * ls;
-    const float v = l < L ? tile[l * 33 + px] : 0.f;
-    dst[i] = MODE == 1 ? mx[px] - v : (MODE == 3 ? v : -v);
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const int px = ri.pixel(i);
+    dst[i] = value(i - px * ri.ls, px);
   }
 }
 
-template <int MODE>
-__global__ void hwl_to_lhw_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                  const uint8_t* __restrict__ amax, int L, int ls, long long HW) {
-  extern __shared__ float tile[];  // [L][33]
-  __shared__ float sm[32];
+template <int MODE, int TP>
+__global__ void __launch_bounds__(256) hwl_to_lhw_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                  const uint8_t* __restrict__ amax, int L, RowIndex ri, long long HW) {
+  extern __shared__ float tile[];  // [L][TP + 1]
+  __shared__ float sm[TP];
+  constexpr int S = TP + 1;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long long b = blockIdx.y, p0 = blockIdx.x * 32ll;
-  const int np = HW - p0 < 32 ? (int)(HW - p0) : 32;
-  const float* src = in + (b * HW + p0) * ls;
-  if ((ls & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
-    const int row4 = ls >> 2;
+  const long long b = blockIdx.y, p0 = blockIdx.x * (long long)TP;
+  const int np = HW - p0 < TP ? (int)(HW - p0) : TP;
+  const float* src = in + (b * HW + p0) * ri.ls;
+  const int n = np * ri.ls;
+  if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < np * row4; i += 256) {
-      const int px = i / row4, l = 4 * (i - px * row4);
-      const float4 x = *reinterpret_cast<const float4*>(src + 4 * i);
-      if (l < L) tile[l * 33 + px] = x.x;
-      if (l + 1 < L) tile[(l + 1) * 33 + px] = x.y;
-      if (l + 2 < L) tile[(l + 2) * 33 + px] = x.z;
-      if (l + 3 < L) tile[(l + 3) * 33 + px] = x.w;
+    for (int i = 4 * threadIdx.x; i < n; i += 1024) {
+      int px = ri.pixel(i), l = i - px * ri.ls;
+      const float4 x = *reinterpret_cast<const float4*>(src + i);
+      const float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (l < L) tile[l * S + px] = v[j];
+        if (++l == ri.ls) l = 0, ++px;
+      }
     }
   } else {
-    for (int i = threadIdx.x; i < np * ls; i += 256) {
-      const int px = i / ls, l = i - px * ls;
-      if (l < L) tile[l * 33 + px] = src[i];
+    for (int i = threadIdx.x; i < n; i += 256) {
+      const int px = ri.pixel(i), l = i - px * ri.ls;
+      if (l < L) tile[l * S + px] = src[i];
     }
   }
   __syncthreads();
   if (MODE == 2) {
-    if (ty == 0 && tx < np) {
+    if (threadIdx.x < np) {
       float s = 0.f;
-      for (int l = 0; l < L; ++l) s += tile[l * 33 + tx];
-      sm[tx] = s;
+      for (int l = 0; l < L; ++l) s += tile[l * S + threadIdx.x];
+      sm[threadIdx.x] = s;
     }
     __syncthreads();
   }
-  float* dst = out + b * L * HW;
-  const int k = (MODE == 2 && tx < np) ? (int)amax[b * HW + p0 + tx] : -1;
-  for (int l = ty; l < L; l += 8)
-    if (tx < np) {
-      const float v = tile[l * 33 + tx];
-      dst[(long long)l * HW + p0 + tx] = MODE == 3 ? v : -v + ((MODE == 2 && l == k) ? sm[tx] : 0.f);
+  float* dst = out + b * L * HW + p0;
+#pragma unroll
+  for (int c = 0; c < TP; c += 32) {
+    const int px = c + tx;
+    if (px >= np) continue;
+    const int k = MODE == 2 ? (int)amax[b * HW + p0 + px] : -1;
+#pragma unroll 4
+    for (int l = ty; l < L; l += 8) {
+      const float v = tile[l * S + px];
+      dst[(long long)l * HW + px] = MODE == 3 ? v : -v + ((MODE == 2 && l == k) ? sm[px] : 0.f);
     }
+  }
 }
 
 cudaError_t launch_layout(int kind, const float* in, float* out, uint8_t* amax, int B, int L, int ls, long long HW,
                           cudaStream_t st) {
-  const dim3 grid((unsigned)((HW + 31) / 32), (unsigned)B);
-  const size_t smem = (size_t)L * 33 * sizeof(float);
   ProfScope prof(kProfElementwise, st);
-  switch (kind) {
-    case 0: lhw_to_hwl_kernel<0><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
-    case 1: lhw_to_hwl_kernel<1><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
-    case 2: hwl_to_lhw_kernel<0><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
-    case 4: lhw_to_hwl_kernel<3><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
-    case 5: hwl_to_lhw_kernel<3><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
-    default: hwl_to_lhw_kernel<2><<<grid, 256, smem, st>>>(in, out, amax, L, ls, HW); break;
-  }
+  const RowIndex ri(ls);
+  auto go = [&](auto tp) {
+    constexpr int TP = decltype(tp)::value;
+    const dim3 grid((unsigned)((HW + TP - 1) / TP), (unsigned)B);
+    const size_t smem = (size_t)L * (TP + 1) * sizeof(float);
+    switch (kind) {
+      case 0: lhw_to_hwl_kernel<0, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
+      case 1: lhw_to_hwl_kernel<1, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
+      case 2: hwl_to_lhw_kernel<0, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
+      case 4: lhw_to_hwl_kernel<3, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
+      case 5: hwl_to_lhw_kernel<3, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
+      default: hwl_to_lhw_kernel<2, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
+    }
+  };
+  L <= kTileLabels ? go(std::integral_constant<int, 128>{}) : go(std::integral_constant<int, 32>{});
   count_launch();
   return cudaGetLastError();
 }
@@ -1659,7 +1705,13 @@ cudaError_t launch_aggregate_lhw(const float* unary, const float* msg, float* co
   } else if (vec4) {
     aggregate_lhw_vec4_kernel<0><<<grid, 256, smem, st>>>(unary, msg, cost, L, ls, HW, D, slice, factor);
   } else {
-    aggregate_lhw_kernel<<<grid, 256, smem, st>>>(unary, msg, cost, L, ls, HW, D, slice, factor, min_a_dir);
+    const RowIndex ri(ls);
+    auto go = [&](auto tp) {
+      constexpr int TP = decltype(tp)::value;
+      aggregate_lhw_kernel<TP><<<dim3((unsigned)((HW + TP - 1) / TP), (unsigned)nimg), 256, (size_t)L * (TP + 1) * sizeof(float), st>>>(
+          unary, msg, cost, L, ri, HW, D, slice, factor, min_a_dir);
+    };
+    L <= kTileLabels ? go(std::integral_constant<int, 128>{}) : go(std::integral_constant<int, 32>{});
   }
   count_launch();
   return cudaGetLastError();
