@@ -215,3 +215,13 @@ def test_costs_from_the_last_sweep(L, R, I, labels_first):
         assert np.array_equal(np.moveaxis(got, 2, -1) if labels_first else got, want["cost"])
         if training:
             assert np.array_equal(mi.cpu().numpy(), want["min_idx"]) and np.array_equal(ni.cpu().numpy(), want["norm_idx"])
+
+
+@pytest.mark.parametrize("L", [1, 2, 21, 32, 33, 255, 256])
+@pytest.mark.parametrize("H,W", [(8, 16), (3, 43), (1, 127), (5, 7), (4, 33)])
+def test_layout_tiles(L, H, W):
+    """Images of one tile, one pixel more, one less, and runs that are no multiple of four; data moves, bit for bit."""
+    from mplayers_b200 import glue
+    x = torch.from_numpy(np.random.default_rng(L + W).standard_normal((2, 1, L, H, W)).astype(np.float32)).cuda()
+    last = glue.labels_last(x)
+    assert torch.equal(last, x.permute(0, 1, 3, 4, 2)) and torch.equal(glue.labels_first(last), x)
