@@ -33,9 +33,24 @@ struct Quad {
   static constexpr int kRow = NT == 64 ? 80 : 32;  // floats of a chain's row of products, likewise
   static constexpr int kSlot = P * 128 + P * kIdx;                                  // floats of a ring slot
   static constexpr int kFloats = kTab + NT * 32 + C * kRow + kQRing * kSlot;        // of a warp
-  static constexpr int kWarps = NT == 64 ? 6 : 4;  // per CTA at most (64 labels: what fits an SM next to the context table)
+  // per CTA at most; 64 labels: what fits an SM next to the context table, 32: small ones spread the long chains
+  static constexpr int kWarps = NT == 64 ? 6 : 2;
   static_assert(kTab % 4 == 0 && kSlot % 4 == 0 && kFloats % 4 == 0, "16-byte alignment of the parts");
 };
+
+// Adds v[k] to the cell a[k] bytes behind `base`, k = 0 .. 3 in this order: where several are the same cell, each starts
+// from the result of the one before it, and the last one's store stays.
+__device__ __forceinline__ void add4(char* base, const unsigned (&a)[4], const float (&v)[4]) {
+  float x[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) x[k] = *reinterpret_cast<const float*>(base + a[k]);
+  x[0] += v[0];
+  x[1] = (a[1] == a[0] ? x[0] : x[1]) + v[1];
+  x[2] = (a[2] == a[1] ? x[1] : a[2] == a[0] ? x[0] : x[2]) + v[2];
+  x[3] = (a[3] == a[2] ? x[2] : a[3] == a[1] ? x[1] : a[3] == a[0] ? x[0] : x[3]) + v[3];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) *reinterpret_cast<float*>(base + a[k]) = x[k];
+}
 
 // FULL: all labels exist, in rows without padding.
 template <int G, int LN, bool FULL>
@@ -219,43 +234,28 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
 #pragma unroll
     for (int o = 1; o < G; o <<= 1) de += __shfl_xor_sync(0xffffffffu, de, o);
     if (DE && on && g == 0) atomicAdd(DE + px, de);
-    // Scatter into the lane's column, four labels at a time: where several go to the same cell, each starts from the
-    // result of the one before it, and the last one's store stays.
+    // scatter into the lane's column, four labels at a time
 #pragma unroll
     for (int u = 0; u < LN; u += 4) {
-      float* a[4];
-      float x[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) a[k] = reinterpret_cast<float*>(colb + cell[u + k]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) x[k] = *a[k];
-      x[0] += t[u];
-      x[1] = (cell[u + 1] == cell[u] ? x[0] : x[1]) + t[u + 1];
-      x[2] = (cell[u + 2] == cell[u + 1] ? x[1] : cell[u + 2] == cell[u] ? x[0] : x[2]) + t[u + 2];
-      x[3] = (cell[u + 3] == cell[u + 2] ? x[2] : cell[u + 3] == cell[u + 1] ? x[1] : cell[u + 3] == cell[u] ? x[0] : x[3]) + t[u + 3];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) *a[k] = x[k];
+      const unsigned a[4] = {cell[u], cell[u + 1], cell[u + 2], cell[u + 3]};
+      const float v[4] = {t[u], t[u + 1], t[u + 2], t[u + 3]};
+      add4(colb, a, v);
     }
     __syncwarp();
-    // the columns of the lane's labels, which are cleared for the next step
-#pragma unroll
-    for (int u = 0; u < LN; ++u) {
-      float4* a = reinterpret_cast<float4*>(colq + ((u >> 2) * 4 * G + (u & 3) << 7));
-      const float4 x = *a;
-      *a = make_float4(0.f, 0.f, 0.f, 0.f);
-      q[u] = (x.x + x.y) + (x.z + x.w);
-      if (G == 8) {
-        float4* b = reinterpret_cast<float4*>(colq2 + ((u >> 2) * 4 * G + (u & 3) << 7));
-        const float4 y = *b;
-        *b = make_float4(0.f, 0.f, 0.f, 0.f);
-        q[u] += (y.x + y.y) + (y.z + y.w);
-      }
-    }
-    // context gradient: the lane's labels of the chains one after the other, two chains at a time
+    // The columns of the lane's labels, which are cleared for the next step, and the context gradient: the lane's labels of
+    // the chains one after the other.  With 32 labels the loads of both come first, so that their latencies overlap
+    // (2 x 256 x 256 x 21, eight directions: 246 -> 214 us); with 64 labels that took 3.44 -> 3.61 ms at 1024 x 1024.
     const uint8_t* ib = islot + (slot - ring) * 4;
+    auto column = [&](int u, char* base) { return reinterpret_cast<float4*>(base + ((u >> 2) * 4 * G + (u & 3) << 7)); };
+    if constexpr (NT == 64) {
 #pragma unroll
-    for (int c = 0; c < Q::C; c += 2) {
-      if constexpr (NT == 64) {
+      for (int u = 0; u < LN; ++u) {
+        const float4 x = *column(u, colq);
+        *column(u, colq) = make_float4(0.f, 0.f, 0.f, 0.f);
+        q[u] = (x.x + x.y) + (x.z + x.w);
+      }
+#pragma unroll
+      for (int c = 0; c < Q::C; c += 2) {
         const float2 pa = *reinterpret_cast<const float2*>(prod + c * Q::kRow + 2 * lane);
         const float2 pb = *reinterpret_cast<const float2*>(prod + (c + 1) * Q::kRow + 2 * lane);
         const unsigned ia = *reinterpret_cast<const unsigned short*>(ib + 4 * G * c) & 0x3f3fu;
@@ -271,14 +271,22 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
         *a1 = ya1;
         *b0 = yb0;
         *b1 = yb1;
-      } else {
-        const float pa = prod[c * Q::kRow + lane], pb = prod[(c + 1) * Q::kRow + lane];
-        float* a = acc0 + (ib[4 * G * c] & 31);
-        float* b = acc0 + (ib[4 * G * (c + 1)] & 31);
-        const float xa = *a, xb = *b;
-        const float ya = xa + pa, yb = (a == b ? ya : xb) + pb;
-        *a = ya;
-        *b = yb;
+      }
+    } else {
+      static_assert(NT == 64 || Q::C == 4, "the four chains of a warp");
+      float pv[4];
+      unsigned off[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) pv[c] = prod[c * Q::kRow + lane], off[c] = (ib[4 * G * c] & 31) * 4;
+      float4 x[LN], y[LN];
+#pragma unroll
+      for (int u = 0; u < LN; ++u) x[u] = *column(u, colq), y[u] = *column(u, colq2);
+      add4(reinterpret_cast<char*>(acc0), off, pv);
+#pragma unroll
+      for (int u = 0; u < LN; ++u) {
+        *column(u, colq) = *column(u, colq2) = make_float4(0.f, 0.f, 0.f, 0.f);
+        q[u] = (x[u].x + x[u].y) + (x[u].z + x[u].w);
+        q[u] += (y[u].x + y[u].y) + (y[u].z + y[u].w);
       }
     }
     __syncwarp();  // products and indices are read: the next step may overwrite them
