@@ -1,4 +1,5 @@
-// Instances of fwd_tma_kernel for label-by-label tables, and the dispatch (mp_fwd_tma_rank1.cu: rank-1 contexts).
+// Instances of fwd_tma_kernel for label-by-label tables, and the dispatch (mp_fwd_tma_rank1.cu,
+// mp_fwd_tma_stride.cu: rank-1 contexts).
 #include "mp_fwd_tma.cuh"
 
 namespace mpl {

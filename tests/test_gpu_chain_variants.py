@@ -225,3 +225,17 @@ def test_layout_tiles(L, H, W):
     x = torch.from_numpy(np.random.default_rng(L + W).standard_normal((2, 1, L, H, W)).astype(np.float32)).cuda()
     last = glue.labels_last(x)
     assert torch.equal(last, x.permute(0, 1, 3, 4, 2)) and torch.equal(glue.labels_first(last), x)
+
+
+@pytest.mark.parametrize("R", [2, 12])     # inside a narrow window, all candidates
+@pytest.mark.parametrize("L", [4, 8, 12, 16, 20, 24, 28, 32])
+def test_row_strides(L, R):
+    rng = np.random.default_rng(L)
+    unary = rng.standard_normal((2, 1, 9, 20, L)).astype(np.float32)
+    ew = rng.uniform(0.2, 1.4, (4,) + unary.shape[:-1]).astype(np.float32)
+    _same_forward("TRWP", unary, _truncated("linear", min(R, L - 1), L), ew, 4, 2, training=False)
+
+
+@pytest.mark.parametrize("L", [1, 7, 10, 15, 18, 23, 27, 30])
+def test_row_strides_padded(L):
+    rows.test_padded_rows_and_zero_start("TRWP", 4, 2, 9, 20, L, 2, "tl1d", False)
