@@ -1324,7 +1324,7 @@ cudaError_t launch_backward_sweep(const BwdParams& p0, cudaStream_t st) {
   const int L = p.L, LS = L | 1;
   ProfScope prof(kProfBwdSweep, st);
   if (quad) {
-    cudaError_t e = launch_backward_quad(p, total, st);
+    cudaError_t e = launch_backward_quad(p, st);
     if (e != cudaSuccess) return e;
   } else if (L <= 32 && p.parts <= 1 && bwd_tma_eligible(p)) {
     p.tma_stages = tma_stage_override() ? tma_stage_override() : 4;

@@ -73,12 +73,12 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
   }
   for (int i = lane; i < Q::kFloats; i += 32) acc[i] = 0.f;  // the columns, and indices that no copy writes
   __syncthreads();
-  const int w = blockIdx.x * wpb + warp, total = p.chain_off[p.ndirs];
-  if (w * Q::C >= total) return;
+  const int w = blockIdx.x * wpb + warp;
+  if (w >= chain_units(p, Q::C)) return;
 
   const int j = lane / G, g = lane % G;
   BChain ch;
-  const bool have = decode_bchain(p, w * Q::C + j, ch);
+  const bool have = decode_bchain(p, chain_of_unit(p, Q::C, w, j), ch);
   const int len = have ? ch.len : 0, nsteps = len - 1;  // steps with a predecessor pixel
   if (!have) ch.dir = p.dir, ch.img = ch.h0 = ch.w0 = 0, ch.pstep = 0;
   int most = len;  // of the warp's chains
@@ -300,9 +300,9 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
 }
 
 template <int G, int LN>
-cudaError_t launch_quad(const BwdParams& p, int total, cudaStream_t st) {
+cudaError_t launch_quad(const BwdParams& p, cudaStream_t st) {
   using Q = Quad<G, LN>;
-  const int warps = (total + Q::C - 1) / Q::C;
+  const int warps = chain_units(p, Q::C);
   int wpb = (warps + 147) / 148;
   wpb = wpb > Q::kWarps ? Q::kWarps : wpb;
   const size_t smem = (size_t)(Q::kTab + wpb * Q::kFloats) * sizeof(float);
@@ -329,8 +329,8 @@ bool bwd_quad_eligible(const BwdParams& p) {
   return total >= (p.L > 32 ? 148 * 2 : 148 * 4);
 }
 
-cudaError_t launch_backward_quad(const BwdParams& p, int total, cudaStream_t st) {
-  return p.L > 32 ? launch_quad<4, 16>(p, total, st) : launch_quad<8, 4>(p, total, st);
+cudaError_t launch_backward_quad(const BwdParams& p, cudaStream_t st) {
+  return p.L > 32 ? launch_quad<4, 16>(p, st) : launch_quad<8, 4>(p, st);
 }
 
 }  // namespace mpl

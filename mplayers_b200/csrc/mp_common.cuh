@@ -417,7 +417,7 @@ bool bwd_wide_eligible(int L, int ls, int ctx_rank, int cp_scheme, const void* d
 cudaError_t launch_backward_wide(const BwdParams& p, int total, cudaStream_t st);
 // mp_bwd_quad.cu: rank-2 context, up to 64 labels, scheme 2, many chains
 bool bwd_quad_eligible(const BwdParams& p);
-cudaError_t launch_backward_quad(const BwdParams& p, int total, cudaStream_t st);
+cudaError_t launch_backward_quad(const BwdParams& p, cudaStream_t st);
 cudaError_t launch_isgmr_combine_total(const float* q_total, const float* q, float* dm, float* dunary, long long n,
                                        int dir0, int ndirs, float rho, cudaStream_t st);
 cudaError_t launch_forward_soft_sweep(const FwdParams& p, bool train, cudaStream_t st);

@@ -912,7 +912,7 @@ __global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant_
   }
   __syncthreads();
   ChainCtx ch;
-  if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
+  if (!decode_chain(p, chain_of_unit(p, wpb, blockIdx.x, warp), ch)) return;
   float* ring = ctab + 32 * 32 + warp * live_warp_floats(A);  // [kLiveRing][A][32] and the weight
   const int slot_floats = A * 32 + 4;
   float2* list = reinterpret_cast<float2*>(ring + kLiveRing * slot_floats);  // [2][kLiveList], in turns
@@ -1083,7 +1083,7 @@ cudaError_t launch_live(const FwdParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfFwdSweep, st);
     count_launch();
-    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
+    return launch_dependent(kernel, chain_units(p, wpb), wpb * 32, smem, st, p);
   };
   const bool v4 = rows_aligned(p) && (p.agg ? 3 : p.D + 1) * (p.ls >> 2) <= (p.agg ? 32 : 160);
   if (p.ctx_rank == 1) {
@@ -1150,7 +1150,7 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
   }
   const bool any_nan = __syncthreads_or(nan);
   ChainCtx ch;
-  if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
+  if (!decode_chain(p, chain_of_unit(p, wpb, blockIdx.x, warp), ch)) return;
 
   const int len = ch.len;
   const long long ibase = (long long)ch.img * p.H * p.W;
@@ -1328,7 +1328,7 @@ cudaError_t launch_pair(const FwdParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfFwdSweep, st);
     count_launch();
-    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
+    return launch_dependent(kernel, chain_units(p, wpb), wpb * 32, smem, st, p);
   };
   const bool full = p.L == 64 && p.ls == 64 && ((uintptr_t)p.msg_write & 7) == 0 && (!TRAIN || ((uintptr_t)p.min_idx & 1) == 0);
   if (p.first) return full ? go(fwd_pair_kernel<2, TRAIN, true>) : go(fwd_pair_kernel<2, TRAIN, false>);

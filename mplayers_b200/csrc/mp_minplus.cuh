@@ -60,6 +60,48 @@ __device__ __forceinline__ bool decode_bchain(const BwdParams& p, int g, BChain&
   return true;
 }
 
+// Order in which a launch over all directions takes its chains, `per` neighbours (a unit) at a time: the axis directions as
+// they are, then the diagonals of all directions and images by their length, longest first.  In the order of
+// chain_start a diagonal's long chains come after its short ones or start another run, and the last CTAs of a launch
+// are among the longest (1024 x 1024, bwd_quad_kernel's CTAs on 148 SMs: the last one ends after 1982 steps, of 1218 that an
+// even split takes; longest first 1311).  Per launch, eight directions,
+// training: 1024 x 1024 x 64 forward 2.96 -> 2.55 ms, backward 3.44 -> 2.36 ms; 2 x 256 x 256 x 21 forward 232 -> 189 us; inference at
+// 333 x 449 x 50 191 -> 183 us, at 375 x 1242 x 128 641 -> 622 us.  Other steps than by one pixel and launches over a part of the chains keep their order.
+__host__ __device__ inline int first_dir(const FwdParams& p) { return p.dir0; }
+__host__ __device__ inline int first_dir(const BwdParams& p) { return p.dir; }
+template <typename Params>
+__host__ __device__ inline bool longest_first(const Params& p) {
+  return p.parts <= 1 && first_dir(p) + p.ndirs > 4 && first_dir(p) + p.ndirs <= 8;
+}
+template <typename Params>
+__host__ __device__ inline int axis_dirs(const Params& p) {
+  return first_dir(p) < 4 ? 4 - first_dir(p) : 0;
+}
+template <typename Params>
+__host__ __device__ inline int chain_units(const Params& p, int per) {
+  if (!longest_first(p)) return (p.chain_off[p.ndirs] + per - 1) / per;
+  const int na = axis_dirs(p), n = p.H + p.W - 1;
+  return (p.chain_off[na] + per - 1) / per + (p.ndirs - na) * p.nimg * ((n + per - 1) / per);
+}
+// Chain j < per of a unit, as decode_chain and decode_bchain take it; the number of chains where there is none.
+template <typename Params>
+__device__ __forceinline__ int chain_of_unit(const Params& p, int per, int unit, int j) {
+  if (!longest_first(p)) return unit * per + j;
+  const int none = p.chain_off[p.ndirs], na = axis_dirs(p), axis = p.chain_off[na], axis_units = (axis + per - 1) / per;
+  if (unit < axis_units) return unit * per + j < axis ? unit * per + j : none;
+  const int H = p.H, W = p.W, n = H + W - 1, lists = (p.ndirs - na) * p.nimg;
+  const int y = unit - axis_units, list = y % lists, s = y / lists * per + j;  // s-th longest of a direction and image
+  if (s >= n) return none;
+  // chain_start: W chains from the first row (the r-th longest of them at column r or W - 1 - r), then those from rows 1 ..
+  // H - 1; min(H, W) pixels long at first, then in turns one pixel shorter
+  const int extra = W >= H ? W - H : 0, tall = W >= H ? 0 : H - W, plateau = extra + tall + 1, k = (s - plateau) >> 1;
+  const bool row = s < plateau ? tall == 0 || s == 0 : ((s - plateau) & 1) == 0;
+  const int at = s < plateau ? s : row ? extra + 1 + k : tall + 1 + k;  // rank in the row, or row of the start
+  int hs, ws;
+  dir_step(first_dir(p) + na + list / p.nimg, hs, ws);
+  return axis + list * n + (row ? (ws > 0 ? at : W - 1 - at) : W + at - 1);
+}
+
 __device__ __forceinline__ float min3f(float a, float b, float c) {
   float d;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));  // 3-input min (sm_100)

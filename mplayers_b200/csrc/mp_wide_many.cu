@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kManyWarps * 32, P == 2 ? 4 : 6) fwd_wide_many
   __syncwarp();
   dependent_wait();
   ChainCtx ch;
-  const bool valid = decode_chain(p, (blockIdx.x * kManyWarps + warp) * C + sub, ch);
+  const bool valid = decode_chain(p, chain_of_unit(p, kManyWarps * C, blockIdx.x, warp * C + sub), ch);
   if (!valid) ch.dir = p.dir0, ch.inv = ch.dir ^ 1, ch.img = ch.h0 = ch.w0 = ch.pstep = 0;
   const int len = valid ? ch.len : 0;
   const int most = C == 2 ? max(len, __shfl_xor_sync(0xffffffffu, len, 16)) : len;
@@ -192,7 +192,6 @@ __global__ void __launch_bounds__(kManyWarps * 32, P == 2 ? 4 : 6) fwd_wide_many
 
 template <int RW, int C, int P, bool FIRST>
 cudaError_t launch_many(const FwdParams& p, cudaStream_t st) {
-  const int total = p.chain_off[p.ndirs];
   const size_t smem = (size_t)Many<RW, C, P, FIRST>::kFloats * sizeof(float) * kManyWarps;
   auto kernel = fwd_wide_many_kernel<RW, C, P, FIRST>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -201,7 +200,7 @@ cudaError_t launch_many(const FwdParams& p, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   ProfScope prof(kProfFwdSweep, st);
   count_launch();
-  return launch_dependent(kernel, (total + C * kManyWarps - 1) / (C * kManyWarps), kManyWarps * 32, smem, st, p);
+  return launch_dependent(kernel, chain_units(p, C * kManyWarps), kManyWarps * 32, smem, st, p);
 }
 
 template <int RW, bool FIRST>

@@ -239,3 +239,18 @@ def test_row_strides(L, R):
 @pytest.mark.parametrize("L", [1, 7, 10, 15, 18, 23, 27, 30])
 def test_row_strides_padded(L):
     rows.test_padded_rows_and_zero_start("TRWP", 4, 2, 9, 20, L, 2, "tl1d", False)
+
+
+@pytest.mark.parametrize("L,B,H,W", [(20, 8, 1, 40), (20, 6, 40, 1), (32, 8, 7, 23), (32, 8, 23, 7), (64, 3, 19, 20), (64, 2, 41, 30),
+                                     (64, 12, 2, 9)])
+def test_longest_chains_first(L, B, H, W):
+    """Images much wider or higher than the other side, lines, and units of chains that end in mid direction."""
+    test_backward_lanes_share_a_chain(L, 8, B, H, W)
+
+
+@pytest.mark.parametrize("B,H,W", [(12, 7, 23), (12, 23, 7), (9, 1, 50), (8, 20, 21)])
+@pytest.mark.parametrize("L", [52, 132])
+def test_longest_chains_first_in_a_window(L, B, H, W):
+    rng = np.random.default_rng(L + W)
+    unary = rng.standard_normal((B, 1, H, W, L)).astype(np.float32)
+    _same_forward("ISGMR", unary, _truncated("linear", 2, L), None, 8, 2, training=False)
