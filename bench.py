@@ -203,7 +203,10 @@ def dominant_kernel(cfg, kind):
     ctx = cfg["label_context"]
     if cfg.get("soft"):
         return "bwd_soft_kernel" if kind == "bwd" else "fwd_soft_kernel"
+    many = cfg["mode"] == "ISGMR"   # the directions of an iteration in one launch (at the workloads' sizes)
     if L <= 32:
+        if many:
+            return "bwd_quad_kernel" if kind == "bwd" else "fwd_live_kernel"
         return "bwd_tma_kernel" if kind == "bwd" else "fwd_tma_kernel"
     if ctx.dim() == 1 and L <= 256:
         if kind == "bwd":
@@ -216,7 +219,9 @@ def dominant_kernel(cfg, kind):
         team = not cfg["training"] and window > 8 and chains < 148 * 16
         return "fwd_wide_team_kernel" if team else "fwd_wide_kernel"
     if L <= 64:
-        return "bwd_pair_kernel" if kind == "bwd" else "fwd_pair_kernel"
+        if kind == "bwd":
+            return "bwd_quad_kernel" if many else "bwd_pair_kernel"
+        return "fwd_pair_kernel"
     return "bwd_cta_kernel" if kind == "bwd" else "fwd_cta_tma_kernel"
 
 
@@ -226,16 +231,16 @@ def dominant_kernel(cfg, kind):
 NCU_TRAFFIC = {
     ("seg_trwp_train", "bwd"): 149.7e6 + 78.3e6,
     ("seg_trwp_train", "fwd"): 222.4e6 + 30.4e6,
-    ("stereo_trwp_infer", "fwd"): 1491.8e6 + 334.3e6,
-    ("stereo_trwp_train", "fwd"): 1491.9e6 + 420.4e6,
+    ("stereo_trwp_infer", "fwd"): 1133.4e6 + 412.1e6,
+    ("stereo_trwp_train", "fwd"): 1133.5e6 + 499.2e6,
     ("stereo_trwp_train", "bwd"): 1044.2e6 + 1012.8e6,
     ("denoise_isgmr_infer", "fwd"): 1143.8e6 + 250.6e6,
     # captured on the 384 x 384 copy of the workload; traffic is proportional to the pixel count, so the
     # full-size figures are those of ten iterations times (1024 / 384)^2
-    ("large_isgmr_train_384", "fwd"): 591.8e6 + 342.9e6,
-    ("large_isgmr_train_384", "bwd"): 454.3e6 + 316.8e6,
-    ("large_isgmr_train", "fwd"): (681.8e6 + 346.2e6) * (1024 / 384) ** 2,
-    ("large_isgmr_train", "bwd"): (452.7e6 + 314.9e6) * (1024 / 384) ** 2,
+    ("large_isgmr_train_384", "fwd"): 551.8e6 + 341.0e6,
+    ("large_isgmr_train_384", "bwd"): 406.8e6 + 284.2e6,
+    ("large_isgmr_train", "fwd"): (700.4e6 + 346.4e6) * (1024 / 384) ** 2,
+    ("large_isgmr_train", "bwd"): (406.6e6 + 283.7e6) * (1024 / 384) ** 2,
 }
 
 

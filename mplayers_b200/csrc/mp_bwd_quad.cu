@@ -8,8 +8,9 @@
 // per chain and step instead of about 400 with 64 labels.  The context gradient, whose table cannot be private to a
 // chain, is accumulated by the warp in a second layout of the same products, lane = one or two labels, chains one
 // after the other, into one table per warp.  Every sum has a fixed order, so the results are run-to-run
-// identical.  1024 x 1024 x 64, eight directions: 5.72 ms a launch with bwd_pair_kernel, 3.43 with this one; what
-// bounds it is latency (four cycles per instruction, six warps per SM: the tables).
+// identical.  1024 x 1024 x 64, eight directions: 5.72 ms a launch with bwd_pair_kernel, 3.43 with this one in
+// the order of the chains' start pixels, 2.36 with the longest chains first (chain_of_unit); what bounds it is latency (four
+// cycles per instruction, six warps per SM: the tables).
 #include "mp_common.cuh"
 #include "mp_minplus.cuh"
 

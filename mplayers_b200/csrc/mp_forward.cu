@@ -890,7 +890,8 @@ cudaError_t launch_cta_tma(FwdParams p, cudaStream_t st) {
 // of 21).  With fewer chains than two per scheduler the kernels that evaluate all candidates are as fast: there a step
 // costs its dependent path, which the list of candidates does not shorten (2 x 512 x 512 x 21, TRWP, 1024 chains a sweep:
 // 90 us, through such a list 150).  2 x 256 x 256 x 21, eight directions, training: the axis directions one
-// launch after another and the diagonal ones 285 us per iteration, this kernel 225.
+// launch after another and the diagonal ones 285 us per iteration, this kernel 225, with the
+// longest chains first 189.
 constexpr int kLiveList = 36;   // entries: 32 and four that never win
 constexpr int kLiveRing = 8;    // pixels staged ahead (power of two)
 __host__ __device__ constexpr int live_warp_floats(int A) { return kLiveRing * (A * 32 + 4) + 2 * 2 * kLiveList; }

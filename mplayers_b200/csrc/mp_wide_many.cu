@@ -7,7 +7,7 @@
 // directions; with up to 64 labels, everything that is paid per warp -- reductions, addresses, the loop -- buys two
 // labels per lane.  Here a lane stages its own labels, 16 bytes per array and pixel, kManyRing pixels ahead, and half a
 // warp is enough for 64 labels.  333 x 449 x 50, eight directions, window 4: 372 us a sweep with fwd_wide_kernel, 344
-// with two chains per warp on bulk copies, 192 in this form (152 at the copy rate).
+// with two chains per warp on bulk copies, 183 in this form (152 at the copy rate).
 #include "mp_common.cuh"
 #include "mp_minplus.cuh"
 
