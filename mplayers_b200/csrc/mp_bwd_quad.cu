@@ -319,15 +319,15 @@ cudaError_t launch_quad(const BwdParams& p, cudaStream_t st) {
 
 }  // namespace
 
-// Rank-1 contexts above 32 labels have a kernel that knows where their indices point (bwd_wide_kernel).  Below these numbers
-// of chains most schedulers would have no warp.
+// Rank-1 contexts above 32 labels have a kernel that knows where their indices point (bwd_wide_kernel).  A warp's step takes
+// 1.6 us with 64 labels however few warps there are, so a launch takes its longest chain times that, where the kernels of
+// one chain per warp take 0.94 ns per pixel and direction: these win below some 1700 directions x images x shorter sides
+// (384 x 384 x 64, eight directions, 3072: 1.10 ms with bwd_pair_kernel, 0.62 here; 93 x 213 x 45, 744: a training step of
+// five iterations 2.55 ms with this kernel, 1.97 before it).
 bool bwd_quad_eligible(const BwdParams& p) {
   if (p.cp_scheme != 2 || p.ndirs < 2 || p.L > 64 || (p.L > 32 && p.ctx_rank != 2) || (p.ls & 3)) return false;
   if ((((uintptr_t)p.dm_read | (uintptr_t)p.dm_acc) & 15) || ((uintptr_t)p.min_idx & 3)) return false;
-  long long total = 0;
-  for (int i = 0; i < p.ndirs; ++i) total += (long long)make_geom(p.dir + i, p.H, p.W).n_chains * p.nimg;
-  if (p.parts > 1) total /= p.parts;
-  return total >= (p.L > 32 ? 148 * 2 : 148 * 4);
+  return (long long)p.ndirs * p.nimg * (p.H < p.W ? p.H : p.W) >= 148 * 16 * (p.parts > 1 ? p.parts : 1);
 }
 
 cudaError_t launch_backward_quad(const BwdParams& p, cudaStream_t st) {

@@ -49,8 +49,7 @@ __device__ __forceinline__ float uu_from_ring(const float* slot, int rs, int col
 // and messages are then copied in 16-byte pieces, lane q piece q of their concatenation: one
 // copy instruction for 21 labels and four directions (30 pieces) where the 4-byte form, which also
 // serves unaligned rows, needs one per row and keeps every lane's address arithmetic in the step.
-// R1: rank-1 context; where it has a narrow window, steps with a weight >= 0 go through that.
-template <int LMAX, int DT, bool TRAIN, bool V4, bool R1>
+template <int LMAX, int DT, bool TRAIN, bool V4>
 __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -76,13 +75,6 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
 #pragma unroll
   for (int f = 0; f < LMAX; ++f) {
     if (f < L) colmin = fminf(colmin, cr[f]), colmax = fmaxf(colmax, cr[f]);
-  }
-
-  NarrowWindow window{};
-  unsigned lmask = 0xffffffffu;
-  if constexpr (R1) {
-    window = narrow_window(p.ctx, 1, L, lane);
-    lmask = L >= 32 ? 0xffffffffu : (1u << L) - 1u;
   }
 
   const long long ibase = (long long)ch.img * p.H * p.W;
@@ -172,22 +164,13 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
     // Old values at pixel i are consumed BEFORE the new message of pixel i is stored (TRWP updates
     // the message slice in place).
     const float uu_next = uu_of(sl + lc);
-    float m_col = 0.f, best;
+    float m_col = 0.f;
+    if constexpr (!TRAIN) m_col = warp_min(act ? fmaf(e, e >= 0.f ? colmin : colmax, hb[lane]) : kInf);
+    float best;
     int bi = 0;
-    const bool narrow = R1 && window.R && e >= 0.f;
-    if (narrow) {
-      const float h = hb[lane];
-      if (window.R <= 2) {
-        minplus_narrow<2, TRAIN>(window, h, e, L, lc, lmask, best, bi, m_col);
-      } else {
-        minplus_narrow<4, TRAIN>(window, h, e, L, lc, lmask, best, bi, m_col);
-      }
-    } else {
-      if constexpr (!TRAIN) m_col = warp_min(act ? fmaf(e, e >= 0.f ? colmin : colmax, hb[lane]) : kInf);
-      minplus_regrow<LMAX, TRAIN>(hb, cr, e, best, bi);
-    }
+    minplus_regrow<LMAX, TRAIN>(hb, cr, e, best, bi);
     // the minimum over the labels, known before the candidates (see fwd_tma_kernel)
-    const float m = TRAIN && !narrow ? warp_min(act ? best : kInf) : m_col;
+    const float m = TRAIN ? warp_min(act ? best : kInf) : m_col;
     r = best - m;
     if (act) Mwl[of] = r;
     if (TRAIN) {
@@ -835,9 +818,7 @@ cudaError_t launch_warp_d(const FwdParams& p, cudaStream_t st) {
     count_launch();
     return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
   };
-  if (p.ctx_rank == 1)
-    return rows_aligned(p) ? go(fwd_warp_kernel<LMAX, DT, TRAIN, true, true>) : go(fwd_warp_kernel<LMAX, DT, TRAIN, false, true>);
-  return rows_aligned(p) ? go(fwd_warp_kernel<LMAX, DT, TRAIN, true, false>) : go(fwd_warp_kernel<LMAX, DT, TRAIN, false, false>);
+  return rows_aligned(p) ? go(fwd_warp_kernel<LMAX, DT, TRAIN, true>) : go(fwd_warp_kernel<LMAX, DT, TRAIN, false>);
 }
 
 template <int LMAX, bool TRAIN>
@@ -1022,11 +1003,7 @@ __global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant_
     int bi = 0;
     const bool up = e >= 0.f;
     if (R1 && window.R && up) {
-      if (window.R <= 2) {
-        minplus_narrow<2, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
-      } else {
-        minplus_narrow<4, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
-      }
+      minplus_narrow<2, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
       bi <<= 7;
     } else {
       const float hmin = warp_min(h);

@@ -369,11 +369,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     if (R1 && window.R && __all_sync(0xffffffffu, lane >= npix || e0[lane * ek] >= 0.f)) {
       if (TRAIN && pend) resolve();
       pend = false;
-      if (window.R <= 2) {
-        narrow_stage(std::integral_constant<int, 2>{}, s, npix, t0, e0);
-      } else {
-        narrow_stage(std::integral_constant<int, 4>{}, s, npix, t0, e0);
-      }
+      narrow_stage(std::integral_constant<int, 2>{}, s, npix, t0, e0);
     } else if (s > 0 && npix == kTK) {
       // full stage: fully unrolled, every tile offset is an immediate
 #pragma unroll

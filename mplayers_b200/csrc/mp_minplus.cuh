@@ -251,12 +251,13 @@ __device__ __forceinline__ void minplus_regrow(const float* hb, const float (&cr
   if (TRAIN) bi = highest_equal<LMAX>(val, best);
 }
 
-// A rank-1 context that stays at its last value from offset R <= 4 on, below which it is nowhere larger (truncated
+// A rank-1 context that stays at its last value from offset R <= 2 on, below which it is nowhere larger (truncated
 // linear and quadratic functions, Potts): with e >= 0 the candidates of a label are those of its neighbours up to
-// R - 1 away and the one of the smallest h at the last value.
+// R - 1 away and the one of the smallest h at the last value.  (Windows of 3 and 4 take four more shuffles a step: 271 x 1163 x 21,
+// inference, window 3 through fwd_warp_kernel 4.6 -> 8.4 ms; they evaluate all candidates.)
 struct NarrowWindow {
   int R;           // 0: the context is no such one
-  float c[4];      // its values at offsets 0 .. 3
+  float c[2];      // its values at offsets 0, 1
   float least;     // smallest value of the lane's column of the label-by-label table
   float last;
 };
@@ -267,15 +268,15 @@ __device__ __forceinline__ NarrowWindow narrow_window(const float* ctx, int rank
   w.R = 0;
   w.last = w.least = 0.f;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) w.c[k] = 0.f;
+  for (int k = 0; k < 2; ++k) w.c[k] = 0.f;
   if (rank != 1) return w;
   w.last = __ldg(ctx + L - 1);
   const float mine = __ldg(ctx + lc);
   const unsigned other = __ballot_sync(0xffffffffu, mine != w.last), above = __ballot_sync(0xffffffffu, !(mine <= w.last));
   const int R = other ? 32 - __clz(other) : 1;
-  w.R = above == 0 && R <= 4 ? R : 0;
+  w.R = above == 0 && R <= 2 ? R : 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) w.c[k] = __ldg(ctx + (k < L ? k : L - 1));
+  for (int k = 0; k < 2; ++k) w.c[k] = __ldg(ctx + (k < L ? k : L - 1));
   const int reach = max(lc, L - 1 - lc);  // furthest offset of the label
   w.least = kInf;
   for (int k = 0; k <= reach; ++k) w.least = fminf(w.least, __ldg(ctx + k));

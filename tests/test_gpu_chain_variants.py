@@ -96,6 +96,9 @@ def test_live_labels_odd_counts(L):
     (20, 8, 2, 30, 41),
     (4, 4, 2, 150, 151),
     (24, 8, 2, 30, 41),     # a 1-D context, whose table is folded
+    # enough chains for the kernel (directions x images x shorter sides >= 2368), and just too few
+    (64, 8, 10, 30, 41), (64, 8, 9, 30, 41), (36, 8, 9, 35, 64), (64, 4, 4, 150, 150), (64, 4, 60, 10, 120),
+    (32, 8, 10, 30, 41), (20, 8, 10, 30, 41), (4, 4, 4, 150, 151), (24, 8, 10, 30, 41),
 ])
 def test_backward_lanes_share_a_chain(L, D, B, H, W):
     rng = np.random.default_rng(L + W)
@@ -119,7 +122,8 @@ def test_backward_lanes_share_a_chain(L, D, B, H, W):
 
 @pytest.mark.parametrize("L", [5, 21, 31, 33, 38, 63])
 def test_backward_lanes_share_a_chain_padded(L):
-    rows.test_padded_rows_and_zero_start("ISGMR", 8, 2, 30, 41, L, 2, "sym2d", True)
+    for B in (2, 10):
+        rows.test_padded_rows_and_zero_start("ISGMR", 8, B, 30, 41, L, 2, "sym2d", True)
 
 
 def _truncated(kind, R, L):
@@ -242,7 +246,7 @@ def test_row_strides_padded(L):
 
 
 @pytest.mark.parametrize("L,B,H,W", [(20, 8, 1, 40), (20, 6, 40, 1), (32, 8, 7, 23), (32, 8, 23, 7), (64, 3, 19, 20), (64, 2, 41, 30),
-                                     (64, 12, 2, 9)])
+                                     (64, 12, 2, 9), (64, 40, 8, 20), (20, 60, 17, 5), (32, 13, 23, 40), (36, 70, 11, 5)])
 def test_longest_chains_first(L, B, H, W):
     """Images much wider or higher than the other side, lines, and units of chains that end in mid direction."""
     test_backward_lanes_share_a_chain(L, 8, B, H, W)
