@@ -108,10 +108,11 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   const int nstages = (len + K - 1) / K;
   const long long ibase = (long long)ch.img * p.H * p.W;
   const int pix0 = ch.h0 * p.W + ch.w0;
-  const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
   // vertical chains (directions 2 / 3) with tensor maps from the launcher: one 2-D tiled TMA box
   // (L labels x K image rows of the chain's column) per array and stage instead of K row copies
   const bool boxed = p.tma_box != 0 && (ch.dir == 2 || ch.dir == 3);
+  // (the columns of an image one pixel wide are boxed too, although their pixels are adjacent in memory)
+  const bool contiguous = !boxed && (ch.pstep == 1 || ch.pstep == -1);
 
   if (!producer) {
     if (lane == 0) {

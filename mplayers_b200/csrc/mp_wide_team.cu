@@ -58,8 +58,8 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
   const int nstages = (len + K - 1) / K;
   const long long ibase = (long long)ch.img * p.H * p.W;
   const int pix0 = ch.h0 * p.W + ch.w0;
-  const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
   const bool boxed = p.tma_box != 0 && (ch.dir == 2 || ch.dir == 3);
+  const bool contiguous = !boxed && (ch.pstep == 1 || ch.pstep == -1);  // (see fwd_wide_kernel)
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
       mbar_init(&full[i], 1);

@@ -258,3 +258,14 @@ def test_longest_chains_first_in_a_window(L, B, H, W):
     rng = np.random.default_rng(L + W)
     unary = rng.standard_normal((B, 1, H, W, L)).astype(np.float32)
     _same_forward("ISGMR", unary, _truncated("linear", 2, L), None, 8, 2, training=False)
+
+
+@pytest.mark.parametrize("mode,D", [("TRWP", 4), ("TRWP", 8), ("ISGMR", 4), ("ISGMR", 8)])
+@pytest.mark.parametrize("L,R", [(64, 3), (36, 2), (128, 6), (192, 12), (256, 15)])
+@pytest.mark.parametrize("H", [2, 5, 8, 9, 11, 23])
+def test_images_of_one_column(mode, D, L, R, H):
+    """A column of such an image is contiguous in memory and copied in boxes of rows, of which the last may be a part."""
+    rng = np.random.default_rng(L + H)
+    unary, ctx = rng.standard_normal((2, 1, H, 1, L)).astype(np.float32), _truncated("linear", R, L)
+    _same_forward(mode, unary, ctx, None, D, 2)
+    _same_forward(mode, unary, ctx, None, D, 2, training=False)
