@@ -1369,8 +1369,10 @@ bool forward_skips_zero_slices(const FwdParams& p, bool train) {
 }
 
 bool forward_takes_prefix(const FwdParams& p, bool train) {
-  // (every pixel has to lie on a chain that is walked; the several-warps kernel, which wide windows may take, does not know P)
-  return p.D == 4 && !p.agg && p.W > 1 && wide_eligible(p, train) && (train || p.host_R <= 8);
+  // (every pixel has to lie on a chain that is walked, of direction 1, which writes P, and of direction 3, which may write the
+  // costs: images of one column or one row keep the final sums; the several-warps kernel, which wide windows may take,
+  // does not know P)
+  return p.D == 4 && !p.agg && p.W > 1 && p.H > 1 && wide_eligible(p, train) && (train || p.host_R <= 8);
 }
 
 __global__ void zero_chain_starts_kernel(const __grid_constant__ FwdParams p, float* a, float* b) {

@@ -2,6 +2,8 @@
 contexts where they can go wrong.  Forward results and saved indices have to be the oracle's bit for bit
 (its arithmetic is followed operation by operation); gradients sum in another order and are held
 to the tolerances of helpers.assert_grad_close."""
+import types
+
 import numpy as np
 import pytest
 import torch
@@ -9,7 +11,7 @@ import torch
 import gpu_runner as g
 import test_gpu_rows as rows
 from helpers import assert_grad_close
-from mplayers_b200 import TRWP
+from mplayers_b200 import MP_module, TRWP
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -269,3 +271,47 @@ def test_images_of_one_column(mode, D, L, R, H):
     unary, ctx = rng.standard_normal((2, 1, H, 1, L)).astype(np.float32), _truncated("linear", R, L)
     _same_forward(mode, unary, ctx, None, D, 2)
     _same_forward(mode, unary, ctx, None, D, 2, training=False)
+
+
+@pytest.mark.parametrize("H,W", [(1, 9), (9, 1), (1, 2), (2, 1), (2, 2), (1, 1), (37, 6)])
+@pytest.mark.parametrize("L,R,I,weights", [(64, 3, 1, False), (64, 2, 2, True), (36, 2, 1, True), (200, 4, 2, False)])
+@pytest.mark.parametrize("labels_first", [False, True])
+def test_costs_from_the_last_sweep_on_lines(H, W, L, R, I, weights, labels_first):
+    """Images of one row or column have chains of one pixel, which no sweep walks; 2 x 2 and a column of several stages
+    beside them, lanes with a part of their labels, weights."""
+    rng = np.random.default_rng(L + 10 * H + W)
+    unary, ctx = rng.standard_normal((2, 1, H, W, L)).astype(np.float32), _truncated("linear", R, L)
+    ew = rng.uniform(0.1, 1.4, (4,) + unary.shape[:-1]).astype(np.float32) if weights else None
+    want = oracle.forward("TRWP", unary, ctx, ew, 4, I)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
+    for training in (False, True):
+        msg = torch.full((4,) + unary.shape, float("nan"), device="cuda")
+        cost = torch.full((2, 1, L, H, W) if labels_first else unary.shape, float("nan"), device="cuda")
+        mi = torch.zeros((I, 4) + unary.shape, dtype=torch.uint8, device="cuda") if training else e8
+        ni = torch.zeros((I, 4) + unary.shape[:-1], dtype=torch.uint8, device="cuda") if training else e8
+        TRWP.forward(0.5, I, 0, dev(unary), dev(ctx), dev(ew) if weights else e0, msg, cost, mi, ni, e0, e8,
+                     context_window=R, cost_labels_first=labels_first, messages_zero=True, messages_needed=False)
+        got = cost.cpu().numpy()
+        assert np.array_equal(np.moveaxis(got, 2, -1) if labels_first else got, want["cost"])
+        if training:
+            assert np.array_equal(mi.cpu().numpy(), want["min_idx"]) and np.array_equal(ni.cpu().numpy(), want["norm_idx"])
+
+
+@pytest.mark.parametrize("H,W", [(1, 23), (23, 1), (4, 6)])
+@pytest.mark.parametrize("train", [False, True])
+def test_module_on_lines(H, W, train):
+    """The module asks for the costs with the labels first and for no messages."""
+    rng = np.random.default_rng(H + W)
+    unary, ctx = rng.standard_normal((1, 1, H, W, 64)).astype(np.float32), _truncated("linear", 3, 64)
+    want = oracle.forward("TRWP", unary, ctx, None, 4, 3)["cost"]
+    args = types.SimpleNamespace(mpnet_mrf_mode="TRWP", mpnet_max_iter=3, mpnet_n_dirs=4, n_classes=64,
+                                 mpnet_smoothness_train="on" if train else None, mpnet_term_weight=1.0, mpnet_diag_value=0.0,
+                                 enable_symmetric=True, mpnet_smoothness_mode="TL", mpnet_smoothness_trunct_value=-1,
+                                 mpnet_smoothness_trunct_loc=-1, enable_cuda=True)
+    layer = MP_module.MPModule(args)
+    layer.set_label_context(torch.nn.Parameter(torch.from_numpy(ctx).cuda(), requires_grad=train), None, None)
+    layer.train(train)
+    x = torch.from_numpy(np.ascontiguousarray(np.moveaxis(unary, -1, 2))).cuda().requires_grad_(train)
+    got = layer(x)[0].detach().cpu().numpy()
+    assert np.array_equal(np.moveaxis(got, 2, -1), want)
