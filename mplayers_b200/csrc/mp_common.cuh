@@ -231,6 +231,7 @@ __device__ __forceinline__ float float_from_order_bits(int b) {
 }
 
 constexpr float kInf = __builtin_huge_valf();
+constexpr float kNaN = __builtin_nanf("");
 
 // ---- mbarrier / bulk-copy (TMA) primitives; every wait is bounded --------------------------------
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }

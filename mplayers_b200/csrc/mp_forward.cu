@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant_
 
   for (int i = 1; i < len; ++i) {
     float* hb = hbuf + (i & 1) * 32;
-    hb[lane] = act ? fmaf(rho, r, uu) : kInf;
+    hb[lane] = act ? fmaf(rho, r, uu) : kNaN;  // labels >= L never win, nor equal the minimum
     cp_async_wait<kPF - 1>();  // everything staged for chain pixel i has landed
     __syncwarp();
     const float* sl = ring + (i & (kPF - 1)) * slot_floats;
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) fwd_cta_kernel(const __grid_constant__ Fw
   const bool act = c < L;
   CtaCtx<MODE> cc;
   cta_ctx_init<MODE>(p, cc, act, c, L, ctx1);
-  hbuf[c] = kInf;  // entries >= L stay +inf
+  hbuf[c] = kNaN;  // entries >= L never win, nor equal the minimum
   __syncthreads();
 
   const long long ibase = (long long)ch.img * p.H * p.W;
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(288) fwd_cta_tma_kernel(const __grid_constant_
   CtaCtx<MODE> cc;
   if (!producer) {
     cta_ctx_init<MODE>(p, cc, act, c, L, ctx1);
-    hbuf[c] = kInf;  // entries >= L stay +inf
+    hbuf[c] = kNaN;  // entries >= L never win, nor equal the minimum
   }
   __syncthreads();
 

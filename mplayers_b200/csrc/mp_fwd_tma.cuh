@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   uint8_t* MIl = TRAIN ? p.min_idx + (long long)dir * p.slice + ibase * LR + lc : nullptr;
   uint8_t* NI = TRAIN ? p.norm_idx + (long long)dir * p.pslice + ibase : nullptr;
   float* hbuf = hbufs + wc * kH;
-  for (int i = lane; i < kH; i += 32) hbuf[i] = kInf;  // labels >= L (LMAX > L) never win
+  for (int i = lane; i < kH; i += 32) hbuf[i] = kNaN;  // labels >= L (LMAX > L) never win, nor equal the minimum
   if (!has_e)  // no edge weights: the producer copies none, every staged weight reads as 1
     for (int i = lane; i < NS * 64; i += 32) etiles[i] = 1.f;
   __syncwarp();
@@ -236,12 +236,11 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     if constexpr (TRAIN) {
       int bi = highest_equal<kKept>(pval, pbest);
       if constexpr (kTwo) {
-        const int f0 = 3 * (bi & 15);  // (a NaN minimum equals nothing: any group)
-        const int at = f0 < LMAX ? f0 : 0;
+        const int at = 3 * bi;
         const float* hp = hprev + at;
         const float* cp = ctab + lc * kCS + at;
         const float v1 = fmaf(pe, cp[1], hp[1]);
-        const float v2 = LMAX % 3 == 2 && at + 2 >= LMAX ? kInf : fmaf(pe, cp[2], hp[2]);
+        const float v2 = LMAX % 3 == 2 && at + 2 >= LMAX ? kNaN : fmaf(pe, cp[2], hp[2]);
         bi = v2 == pbest ? at + 2 : v1 == pbest ? at + 1 : at;
       }
       const unsigned bal = __ballot_sync(0xffffffffu, pbest == pm) & lmask;

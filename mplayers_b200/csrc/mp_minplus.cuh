@@ -174,7 +174,9 @@ __device__ __forceinline__ void minplus_vals(const float* hb, const float (&cr)[
   if (LMAX & 1) val[LMAX - 1] = fmaf(e, cr[OFF + LMAX - 1], hv[LMAX - 1]);
 }
 
-// Highest f with val[f] == best (best must be the exact minimum of val, so at least one matches).
+// Highest f with val[f] == best.  best is the exact minimum of val, so at least one matches, unless all are NaN: then 0, for
+// the index is saved and the backward pass addresses a table with it.  (The accumulator of the first group starts
+// at 2^0, which stands for label 0 whether it matches or not.)
 template <int LMAX>
 __device__ __forceinline__ int highest_equal(const float (&val)[LMAX], float best) {
   // Sums of distinct powers of two are exact in any order, so each group of 24 labels is
@@ -183,14 +185,16 @@ __device__ __forceinline__ int highest_equal(const float (&val)[LMAX], float bes
   float acc[NA][4];
 #pragma unroll
   for (int a = 0; a < NA; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+  acc[0][0] = 1.f;
   if constexpr (LMAX <= 24) {
     // one group: scalar fmas (measured on the 21-label sweeps: 102.1 against 104.1 us; with 32
     // candidates the packed form below is the faster one, 7.4 against 8.1 ms on the 64-label sweeps)
 #pragma unroll
-    for (int f = 0; f < LMAX; ++f) acc[0][f & 3] = fmaf(eq_flag(val[f], best), pow2f(f), acc[0][f & 3]);
+    for (int f = 1; f < LMAX; ++f) acc[0][f & 3] = fmaf(eq_flag(val[f], best), pow2f(f), acc[0][f & 3]);
   } else {
+    acc[0][1] = eq_flag(val[1], best) * pow2f(1);
 #pragma unroll
-    for (int f = 0; f + 1 < LMAX; f += 2) {  // 24 is even: a pair never straddles two groups
+    for (int f = 2; f + 1 < LMAX; f += 2) {  // 24 is even: a pair never straddles two groups
       const int a = f / 24, j = f & 2;
       ffma2(acc[a][j], acc[a][j + 1], eq_flag(val[f], best), eq_flag(val[f + 1], best), pow2f(f % 24),
             pow2f((f + 1) % 24), acc[a][j], acc[a][j + 1]);
@@ -284,9 +288,10 @@ __device__ __forceinline__ NarrowWindow narrow_window(const float* ctx, int rank
 }
 
 // The step through such a window of up to RW offsets (those from R to RW - 1 hold the last value: exact as well).  Neighbours
-// come by shuffle (idle lanes repeat the last label, lc); a label outside 0 .. L - 1 counts as +inf.  The highest index among equal candidates: inside the window the
-// highest offset; outside it candidates are equal to the saturated minimum gv, and the highest label whose
-// saturated candidate is gv stands for all of them (its window candidate is no larger).
+// come by shuffle; the candidate of a label outside 0 .. L - 1 is NaN, which no minimum takes and nothing equals.  The highest
+// index among equal candidates: inside the window the highest offset; outside it candidates are equal to the saturated
+// minimum gv, and the highest label whose saturated candidate is gv stands for all of them (its window candidate is no
+// larger).  Where all candidates are NaN the index is 0.
 template <int RW, bool TRAIN>
 __device__ __forceinline__ void minplus_narrow(const NarrowWindow& w, float h, float e, int L, int lc,
                                                unsigned lmask, float& best, int& bi, float& m) {
@@ -299,14 +304,14 @@ __device__ __forceinline__ void minplus_narrow(const NarrowWindow& w, float h, f
 #pragma unroll
   for (int k = 1; k < RW; ++k) {
     const float dn = __shfl_sync(0xffffffffu, h, lc - k), up = __shfl_sync(0xffffffffu, h, lc + k);
-    cand[RW - k] = lc >= k ? fmaf(e, w.c[k], dn) : kInf;
-    cand[RW + k] = lc + k < L ? fmaf(e, w.c[k], up) : kInf;
+    cand[RW - k] = lc >= k ? fmaf(e, w.c[k], dn) : kNaN;
+    cand[RW + k] = lc + k < L ? fmaf(e, w.c[k], up) : kNaN;
   }
   best = min_tree<2 * RW>(cand);
   if (TRAIN) {
     const unsigned sat = __ballot_sync(0xffffffffu, fmaf(e, w.last, h) == gv) & lmask;
     const int fstar = 31 - __clz(sat);
-    int fw = -1;
+    int fw = 0;
 #pragma unroll
     for (int k = 1 - RW; k < RW; ++k) fw = cand[RW + k] == best ? lc + k : fw;
     bi = gv == best ? max(fstar, fw) : fw;

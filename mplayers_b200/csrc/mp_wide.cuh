@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
       }
       mbar_fence_init();
     }
-    for (int i = lane; i < 2 * (LP + 2 * G); i += 32) hwin[i] = kInf;  // guards and padding labels
+    for (int i = lane; i < 2 * (LP + 2 * G); i += 32) hwin[i] = kNaN;  // guards and padding labels: no minimum takes them, nothing equals them
   }
   __syncthreads();
   dependent_wait();
@@ -321,13 +321,13 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
         const float gv = fmaf(e, cmax, hmin);  // candidate through the saturated value
         int fstar = 0;                         // TRAIN: highest label whose saturated candidate equals gv
         if (TRAIN) {
-          int lf = -1;
+          int lf = 0;
 #pragma unroll
           for (int i = 0; i < LPT; ++i) lf = (i < nl && fmaf(e, cmax, hv[i]) == gv) ? c0 + i : lf;
           fstar = warp_max_i32(lf);
         }
         __syncwarp();
-        // window of this lane: labels c0 - G .. c0 + LPT + G - 1 (guards read +inf)
+        // window of this lane: labels c0 - G .. c0 + LPT + G - 1 (guards read NaN)
         float win[NWV * 2];
         if constexpr (LPT % 4 == 0) {
 #pragma unroll
@@ -355,8 +355,9 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
           best[i] = min_tree<2 * RW>(cand);
           if (i < nl) bl = fminf(bl, best[i]);
           if constexpr (TRAIN) {
-            // highest window offset attaining the minimum (candidates outside 0..L-1 read +inf)
-            int fw = -1;
+            // highest window offset attaining the minimum (candidates outside 0..L-1 are NaN); 0 where none does:
+            // then fstar is the index, or everything is NaN
+            int fw = 0;
             if constexpr (RW >= 8) {
               // many candidates: flags summed with weights 2^k on the full-rate pipe, the index is the
               // exponent of the sum (a compare and a select per candidate run at half rate)
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
 #pragma unroll
               for (int j = 0; j < 2 * RW - 1; ++j) wv[j] = cand[j + 1];
               const int hw = highest_equal_or_none<2 * RW - 1>(wv, best[i]);
-              fw = hw >= 0 ? c0 + i + hw - (RW - 1) : -1;
+              fw = hw >= 0 ? c0 + i + hw - (RW - 1) : 0;
             } else {
 #pragma unroll
               for (int kk = -(RW - 1); kk <= RW - 1; ++kk) fw = (cand[kk + RW] == best[i]) ? c0 + i + kk : fw;

@@ -315,3 +315,36 @@ def test_module_on_lines(H, W, train):
     x = torch.from_numpy(np.ascontiguousarray(np.moveaxis(unary, -1, 2))).cuda().requires_grad_(train)
     got = layer(x)[0].detach().cpu().numpy()
     assert np.array_equal(np.moveaxis(got, 2, -1), want)
+
+
+@pytest.mark.parametrize("bad", ["nan pixel", "inf pixel", "nan label", "nan table"])
+@pytest.mark.parametrize("mode,D,B,H,W,L,R", [    # R = 0: a label-by-label table
+    ("TRWP", 4, 2, 9, 20, 21, 0), ("TRWP", 4, 2, 9, 20, 13, 0), ("TRWP", 4, 2, 9, 20, 28, 0), ("TRWP", 4, 2, 9, 20, 30, 0),
+    ("TRWP", 4, 2, 9, 20, 31, 0), ("TRWP", 4, 2, 9, 20, 32, 0), ("TRWP", 4, 2, 9, 20, 1, 0),
+    ("TRWP", 4, 2, 9, 19, 21, 0), ("TRWP", 4, 2, 9, 19, 15, 0), ("TRWP", 4, 2, 9, 19, 29, 0),
+    ("TRWP", 4, 2, 9, 20, 21, 2), ("TRWP", 4, 2, 9, 20, 13, 2), ("TRWP", 4, 2, 9, 20, 32, 1),
+    ("ISGMR", 8, 4, 33, 38, 21, 0), ("ISGMR", 8, 4, 33, 38, 19, 2), ("ISGMR", 8, 4, 33, 38, 32, 2),
+    ("TRWP", 4, 1, 9, 14, 60, 0), ("ISGMR", 8, 1, 13, 22, 36, 0), ("ISGMR", 8, 3, 30, 41, 64, 0),
+    ("TRWP", 4, 1, 9, 14, 37, 0), ("TRWP", 4, 1, 9, 14, 100, 0), ("TRWP", 4, 1, 9, 14, 39, 30),
+    ("TRWP", 4, 1, 9, 14, 52, 2), ("TRWP", 4, 1, 9, 14, 100, 4), ("TRWP", 4, 1, 9, 14, 132, 7), ("ISGMR", 8, 1, 9, 14, 200, 14),
+    ("ISGMR", 4, 1, 9, 14, 64, 16),
+])
+def test_saved_argmin_is_a_label(bad, mode, D, B, H, W, L, R):
+    """The backward pass addresses tables with the saved argmin: it is a label also where nothing is a minimum (NaN) or
+    every candidate is infinite, in label counts that leave lanes idle too."""
+    rng = np.random.default_rng(L + W)
+    shape = (B, 1, H, W, L)
+    unary = rng.standard_normal(shape).astype(np.float32)
+    ctx = _truncated("linear", min(R, L - 1), L) if R else _table("random", L, rng)
+    if bad == "nan table":
+        if R:
+            ctx[0] = np.nan
+        else:
+            ctx[0, L - 1] = ctx[L - 1, 0] = np.nan
+    elif bad == "nan label":
+        unary[..., H // 2, W // 2, L // 2] = np.nan
+    else:
+        unary[..., H // 2, W // 2, :] = np.nan if bad == "nan pixel" else np.inf
+    ew = rng.uniform(0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    got = g.forward(mode, unary, ctx, ew, D, 2)
+    assert got["min_idx"].max() < L
