@@ -129,6 +129,7 @@ size_t mpl_backward_workspace_bytes(const mpl_problem* p);
  *   edge_weights   NULL = every weight is 1
  *   msg_min_index, msg_norm_index   both NULL = inference (nothing saved); both non-NULL = training
  *   label_all      NULL = do not save per-iteration labels
+ *   cost_final     without cost_labels_first it may be `unary` itself: the costs then replace the unaries at the end
  * The reference's `unary_update` scratch argument has no counterpart (the update is fused). */
 int mpl_trwp_forward(const mpl_problem* p, const float* unary, const float* context,
                      const float* edge_weights, float* msg, float* cost_final,

@@ -330,9 +330,12 @@ int forward_common(bool isgmr, const mpl_problem* problem, const mpl_rows* rows,
     if (p->n_iter == 0 && rd != msg) MPL_CUDA(cudaMemsetAsync(msg, 0, (size_t)D * d.slice * sizeof(float), st));
   }
   bool have_sums = false;
-  // TRWP with four directions: `cost_final` holds the sums its sweeps of directions 2 and 3 start from
+  // TRWP with four directions: `cost_final` holds the sums its sweeps of directions 2 and 3 start from (unless it is
+  // the unaries' own buffer: every iteration reads those)
   set_dirs(fp, 0, 1);
-  const bool prefix = !isgmr && d.ls == L && ((uintptr_t)cost_final & 15) == 0 && mpl::forward_takes_prefix(fp, train);
+  const uintptr_t volume = (uintptr_t)d.slice * sizeof(float), cost_at = (uintptr_t)cost_final, unary_at = (uintptr_t)unary;
+  const bool apart = cost_at + volume <= unary_at || unary_at + volume <= cost_at;
+  const bool prefix = !isgmr && apart && d.ls == L && (cost_at & 15) == 0 && mpl::forward_takes_prefix(fp, train);
   // ... and the last sweep stores the costs instead of messages that the caller does not need (375 x 1242 x 192, three
   // iterations: the sums of five volumes behind it were 387 us): in place of those sums, or, where the costs go there with
   // the labels first, in place of the messages.

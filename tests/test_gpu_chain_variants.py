@@ -348,3 +348,23 @@ def test_saved_argmin_is_a_label(bad, mode, D, B, H, W, L, R):
     ew = rng.uniform(0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
     got = g.forward(mode, unary, ctx, ew, D, 2)
     assert got["min_idx"].max() < L
+
+
+@pytest.mark.parametrize("L,R,I", [(64, 3, 2), (192, 2, 3), (128, 4, 1), (21, 2, 2)])
+@pytest.mark.parametrize("needed", [True, False])
+def test_costs_in_place_of_the_unaries(L, R, I, needed):
+    """TRWP may write the costs into the buffer that holds the unaries."""
+    rng = np.random.default_rng(L + I)
+    unary, ctx = rng.standard_normal((2, 1, 9, 14, L)).astype(np.float32), _truncated("linear", R, L)
+    want = oracle.forward("TRWP", unary, ctx, None, 4, I)
+    e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
+    for training in (False, True):
+        both = torch.from_numpy(unary).cuda()
+        msg = torch.zeros((4,) + unary.shape, device="cuda")
+        mi = torch.zeros((I, 4) + unary.shape, dtype=torch.uint8, device="cuda") if training else e8
+        ni = torch.zeros((I, 4) + unary.shape[:-1], dtype=torch.uint8, device="cuda") if training else e8
+        TRWP.forward(0.5, I, 0, both, torch.from_numpy(ctx).cuda(), e0, msg, both, mi, ni, e0, e8, messages_zero=True,
+                     messages_needed=needed)
+        assert np.array_equal(both.cpu().numpy(), want["cost"])
+        if training:
+            assert np.array_equal(mi.cpu().numpy(), want["min_idx"])
