@@ -345,12 +345,15 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, uns
 // Layout kernels: tiles of 128 pixels up to this label count (2 x 512 x 512 x 21: the four of a training step 218 us with
 // tiles of 32 pixels and one element per access, 130 us with these and four), of 32 pixels above.
 constexpr int kTileLabels = 32;
-// Position in a run of label rows -> pixel, without a division: i < 2^15, ls <= 256.
+// Position in a run of label rows -> pixel, without a division up to kMaxMagic elements per row: for the positions i of a
+// tile of 128 pixels i * (magic * ls - 2^32) stays below 2^32 up to 5792 (first wrong pixel at 5843), so the product's upper
+// half is exact.  The layout entry points take any stride; longer rows are divided.
 struct RowIndex {
+  static constexpr int kMaxMagic = 4096;
   int ls;
-  unsigned magic;  // ceil(2^32 / ls); 0: rows of one element
-  explicit RowIndex(int stride) : ls(stride), magic(stride > 1 ? 0xffffffffu / stride + 1 : 0) {}
-  __device__ __forceinline__ int pixel(int i) const { return magic ? (int)__umulhi((unsigned)i, magic) : i; }
+  unsigned magic;  // ceil(2^32 / ls); 0: rows of one element, or too long ones
+  explicit RowIndex(int stride) : ls(stride), magic(stride > 1 && stride <= kMaxMagic ? 0xffffffffu / stride + 1 : 0) {}
+  __device__ __forceinline__ int pixel(int i) const { return magic ? (int)__umulhi((unsigned)i, magic) : ls > 1 ? i / ls : i; }
 };
 
 // MPL_NO_PAIR=1 keeps 32 < L <= 64 on the CTA-per-chain kernels (tuning / comparison knob).

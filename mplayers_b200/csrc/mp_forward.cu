@@ -1565,7 +1565,7 @@ cudaError_t launch_layout(int kind, const float* in, float* out, uint8_t* amax, 
       default: hwl_to_lhw_kernel<2, TP><<<grid, 256, smem, st>>>(in, out, amax, L, ri, HW); break;
     }
   };
-  L <= kTileLabels ? go(std::integral_constant<int, 128>{}) : go(std::integral_constant<int, 32>{});
+  L <= kTileLabels && ls <= RowIndex::kMaxMagic ? go(std::integral_constant<int, 128>{}) : go(std::integral_constant<int, 32>{});
   count_launch();
   return cudaGetLastError();
 }

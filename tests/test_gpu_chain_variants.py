@@ -368,3 +368,17 @@ def test_costs_in_place_of_the_unaries(L, R, I, needed):
         assert np.array_equal(both.cpu().numpy(), want["cost"])
         if training:
             assert np.array_equal(mi.cpu().numpy(), want["min_idx"])
+
+
+@pytest.mark.parametrize("stride", [4096, 4100, 5843, 6001, 12000, 40000])
+@pytest.mark.parametrize("L", [3, 32, 40])
+def test_layout_of_long_rows(stride, L):
+    """The layout entry points take any row stride from the label count on."""
+    from mplayers_b200 import _lib
+    lib, H, W = _lib.lib(), 5, 53
+    x = torch.from_numpy(np.random.default_rng(L).standard_normal((2, L, H, W)).astype(np.float32)).cuda()
+    rows_, back = torch.full((2, H, W, stride), float("nan"), device="cuda"), torch.empty_like(x)
+    st = torch.cuda.current_stream().cuda_stream
+    assert lib.mpl_permute_lhw_to_rows(x.data_ptr(), rows_.data_ptr(), 2, L, H, W, stride, st) == 0
+    assert lib.mpl_permute_rows_to_lhw(rows_.data_ptr(), back.data_ptr(), 2, L, H, W, stride, st) == 0
+    assert torch.equal(rows_[..., :L], x.permute(0, 2, 3, 1)) and not rows_[..., L:].any() and torch.equal(back, x)
