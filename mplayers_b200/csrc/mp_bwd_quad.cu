@@ -97,8 +97,7 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
   const int pieces = LR >> 2;  // of four labels
   const int ostep = ch.pstep * LR;
 
-  // The lane's gradients and indices of the next step; past the chain's end its last slots are cleared, so that the steps
-  // the warp's longer chains still take add zeros.
+  // The lane's gradients and indices of the next step; past the chain's end its last slots are cleared.
   float* const ring_end = ring + kQRing * Q::kSlot;
   float* fill = ring;
   int ahead = 0;
@@ -190,7 +189,10 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
           *reinterpret_cast<float4*>(out + 4 * G * i) = make_float4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
     }
     const bool on = s < nsteps;
-    const float rq = on ? rho : 0.f;
+    if (s == nsteps) {  // the chain ends here: the steps the warp's longer chains still take add zeros, whatever q holds
+#pragma unroll
+      for (int i = 0; i < LN; ++i) q[i] = 0.f;
+    }
     const float e = __shfl_sync(0xffffffffu, e_cur, j * G + (s & 3));
     const int nn = __shfl_sync(0xffffffffu, n_cur, j * G + (s & 3)) - 4 * g;
     const int n = on ? nn : -1;  // (a lane's labels are at 0 .. 3, 4 G .. 4 G + 3, ...)
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int u = 4 * i + k;
-        t[u] = fmaf(rq, q[u], t[u]);
+        t[u] = fmaf(rho, q[u], t[u]);
         if (n == 4 * G * i + k) t[u] -= S;       // MPLayers/commonCUDA.cuh:131-145
         de = fmaf(*reinterpret_cast<const float*>(crow + (4 * G * i + k) * TS * 4 + f4[k]), t[u], de);
       }

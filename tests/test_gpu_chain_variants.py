@@ -382,3 +382,21 @@ def test_layout_of_long_rows(stride, L):
     assert lib.mpl_permute_lhw_to_rows(x.data_ptr(), rows_.data_ptr(), 2, L, H, W, stride, st) == 0
     assert lib.mpl_permute_rows_to_lhw(rows_.data_ptr(), back.data_ptr(), 2, L, H, W, stride, st) == 0
     assert torch.equal(rows_[..., :L], x.permute(0, 2, 3, 1)) and not rows_[..., L:].any() and torch.equal(back, x)
+
+
+@pytest.mark.parametrize("L,B,H,W", [(64, 10, 30, 41), (20, 10, 30, 41), (36, 10, 30, 41)])
+def test_infinite_gradient_stays_in_its_chains(L, B, H, W):
+    """A chain whose gradient ends infinite shares its warp with longer ones: the cells of the context gradient that it does
+    not touch stay finite."""
+    rng = np.random.default_rng(L)
+    shape = (B, 1, H, W, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _table("random", L, rng)
+    ew = rng.uniform(0.2, 1.0, (8,) + shape[:-1]).astype(np.float32)
+    want = _same_forward("ISGMR", unary, ctx, ew, 8, 1)
+    dcost = rng.uniform(-1, 1, shape).astype(np.float32)
+    dcost[3, 0, 0, 1, L // 2] = np.inf
+    ref = oracle.backward("ISGMR", ctx, ew, dcost, want["min_idx"], want["norm_idx"])["dctx"]
+    got = g.backward("ISGMR", ctx, ew, dcost, want["min_idx"], want["norm_idx"])["dctx"]
+    finite = np.isfinite(ref)   # (the oracle's normalisation sum takes what its chain has scattered too: a few cells more)
+    assert finite.any() and not finite.all()
+    assert_grad_close(got[finite], ref[finite], "dctx")
