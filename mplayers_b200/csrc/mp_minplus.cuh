@@ -268,22 +268,16 @@ struct NarrowWindow {
 
 __device__ __forceinline__ NarrowWindow narrow_window(const float* ctx, int rank, int L, int lane) {
   const int lc = lane < L ? lane : L - 1;
-  NarrowWindow w;
-  w.R = 0;
-  w.last = w.least = 0.f;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) w.c[k] = 0.f;
+  NarrowWindow w{};
   if (rank != 1) return w;
   w.last = __ldg(ctx + L - 1);
   const float mine = __ldg(ctx + lc);
+  w.c[0] = __ldg(ctx);
+  w.c[1] = __ldg(ctx + (L > 1 ? 1 : 0));
   const unsigned other = __ballot_sync(0xffffffffu, mine != w.last), above = __ballot_sync(0xffffffffu, !(mine <= w.last));
   const int R = other ? 32 - __clz(other) : 1;
   w.R = above == 0 && R <= 2 ? R : 0;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) w.c[k] = __ldg(ctx + (k < L ? k : L - 1));
-  const int reach = max(lc, L - 1 - lc);  // furthest offset of the label
-  w.least = kInf;
-  for (int k = 0; k <= reach; ++k) w.least = fminf(w.least, __ldg(ctx + k));
+  w.least = fminf(w.c[0], w.c[1]);  // (no value is larger than the last one, and every label has a neighbour)
   return w;
 }
 
