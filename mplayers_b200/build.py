@@ -10,7 +10,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmplayers_b200.so")
 SOURCES = ["mp_api.cu", "mp_forward.cu", "mp_fwd_tma.cu", "mp_fwd_tma_rank1.cu", "mp_fwd_tma_stride.cu", "mp_backward.cu", "mp_wide.cu", "mp_wide_train.cu", "mp_wide_team.cu",
-           "mp_wide_many.cu", "mp_wide_bwd.cu", "mp_bwd_quad.cu", "mp_soft.cu", "mp_soft_cta.cu", "mp_terms.cu", "mp_swbp.cu"]
+           "mp_wide_many.cu", "mp_pair_rows.cu", "mp_wide_bwd.cu", "mp_bwd_quad.cu", "mp_soft.cu", "mp_soft_cta.cu", "mp_terms.cu", "mp_swbp.cu"]
 HEADERS = [os.path.join(CSRC, "mp_common.cuh"), os.path.join(CSRC, "mp_minplus.cuh"), os.path.join(CSRC, "mp_wide.cuh"),
            os.path.join(CSRC, "mp_fwd_tma.cuh"),
            os.path.join(os.path.dirname(HERE), "include", "mplayers_b200.h")]

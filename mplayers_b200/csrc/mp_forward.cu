@@ -1095,14 +1095,14 @@ constexpr int kPairRing = 8;           // pixels (power of two)
 
 __host__ __device__ inline int pair_warp_floats(int A) { return kPairRing * (A * 64 + 4) + 2 * 2 * kPairList; }
 
-// MODE 0: the unaries and p.D message slices are staged; 1: aggregate mode (FwdParams::agg); 2: zero messages
-// (FwdParams::first, aggregate mode), only the unaries.  FULL: 64 labels in rows of 64, messages and indices aligned to pairs.
-template <int MODE, bool TRAIN, bool FULL>
+// In aggregate mode (FwdParams::agg) only: single directions go to fwd_rows_kernel (mp_pair_rows.cu).  FIRST: zero messages
+// (FwdParams::first), only the unaries are staged.  FULL: 64 labels in rows of 64, messages and indices aligned to pairs.
+template <bool FIRST, bool TRAIN, bool FULL>
 __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ __align__(128) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr bool AGG = MODE == 1;
-  const int L = FULL ? 64 : p.L, LR = FULL ? 64 : p.ls, D = MODE == 2 ? 0 : AGG ? 2 : p.D, A = D + 1;
+  constexpr int A = FIRST ? 1 : 3;
+  const int L = FULL ? 64 : p.L, LR = FULL ? 64 : p.ls;
   float* ctab = smem;                // [64][64], row = label at the predecessor
   float* btab = ctab + kPairCtx;     // [5][64]
   dependent_wait();
@@ -1151,9 +1151,8 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
   // offsets to one base each were slower (1024 x 1024 x 64, eight directions: 2.99 -> 3.12 ms a launch).
   const int pix0 = ch.h0 * p.W + ch.w0, ostep = ch.pstep * LR;
   const float* Us = p.unary + (ibase + pix0) * LR + c0;
-  const float* Ms = p.msg_read + (ibase + pix0) * LR + c0;
-  const float* Md = Ms + ch.dir * p.slice;
-  const float* Mi = Ms + ch.inv * p.slice;
+  const float* Md = p.msg_read + ch.dir * p.slice + (ibase + pix0) * LR + c0;
+  const float* Mi = p.msg_read + ch.inv * p.slice + (ibase + pix0) * LR + c0;
   const float* Es = p.ew ? p.ew + (long long)ch.dir * p.pslice + ibase + pix0 : nullptr;
   float* my_ring = ring + c0;
   auto cp_async8 = [](float* dst, const float* src) {
@@ -1164,39 +1163,29 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
     float* dst = my_ring + (ahead & (kPairRing - 1)) * slot_floats;
     if (FULL || c0 < LR) {
       cp_async8(dst, Us);
-      if (AGG) {
+      if (!FIRST) {
         cp_async8(dst + 64, Md);
         cp_async8(dst + 128, Mi);
-      } else {
-        for (int k = 0; k < D; ++k) cp_async8(dst + (1 + k) * 64, Ms + k * p.slice);
       }
     }
     if (Es && lane == 0) cp_async4(dst + A * 64, Es);
     cp_async_commit();
     if (++ahead < len) {
       Us += ostep;
-      if (AGG) Md += ostep, Mi += ostep;
-      if (MODE == 0) Ms += ostep;
+      if (!FIRST) Md += ostep, Mi += ostep;
       if (Es) Es += ch.pstep;
     }
   };
-  const int dir_off = (AGG ? 1 : 1 + ch.dir) * 64, inv_off = (AGG ? 2 : 1 + ch.inv) * 64;
   auto uu_of = [&](const float* t, float& u0, float& u1) {  // reference order of the additions
-    float2 v = *reinterpret_cast<const float2*>(t);
-    if (MODE == 0)
-      for (int a = 1; a <= D; ++a) {
-        const float2 x = *reinterpret_cast<const float2*>(t + a * 64);
-        v.x += x.x, v.y += x.y;
-      }
-    if (MODE == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(t);
+    if (FIRST) {
       u0 = v.x * rho, u1 = v.y * rho;
     } else {
-      const float2 d = *reinterpret_cast<const float2*>(t + dir_off), i = *reinterpret_cast<const float2*>(t + inv_off);
+      const float2 d = *reinterpret_cast<const float2*>(t + 64), i = *reinterpret_cast<const float2*>(t + 128);
       u0 = fmaf(v.x - d.x, rho, -i.x);
       u1 = fmaf(v.y - d.y, rho, -i.y);
     }
   };
-
   float* mw = p.msg_write + (long long)ch.dir * p.slice + (ibase + pix0) * LR + c0;
   uint8_t* mi = TRAIN ? p.min_idx + (long long)ch.dir * p.slice + (ibase + pix0) * LR + c0 : nullptr;
   uint8_t* nip = TRAIN ? p.norm_idx + (long long)ch.dir * p.pslice + ibase + pix0 : nullptr;
@@ -1295,9 +1284,9 @@ __global__ void __launch_bounds__(256, 3) fwd_pair_kernel(const __grid_constant_
 template <bool TRAIN>
 cudaError_t launch_pair(const FwdParams& p, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
-  const int A = (p.first ? 0 : p.agg ? 2 : p.D) + 1;
+  const int A = p.first ? 1 : 3;
   // eight chains per CTA where they fill the SMs (24 warps each), else four, so that more SMs get some
-  const int wpb = total >= 148 * 16 && A <= 3 ? 8 : 4;
+  const int wpb = total >= 148 * 16 ? 8 : 4;
   const size_t smem = (size_t)(kPairCtx + kPairBounds + pair_warp_floats(A) * wpb) * sizeof(float);
   auto go = [&](auto kernel) -> cudaError_t {
     cudaError_t e = ensure_smem(kernel, smem);
@@ -1309,9 +1298,8 @@ cudaError_t launch_pair(const FwdParams& p, cudaStream_t st) {
     return launch_dependent(kernel, chain_units(p, wpb), wpb * 32, smem, st, p);
   };
   const bool full = p.L == 64 && p.ls == 64 && ((uintptr_t)p.msg_write & 7) == 0 && (!TRAIN || ((uintptr_t)p.min_idx & 1) == 0);
-  if (p.first) return full ? go(fwd_pair_kernel<2, TRAIN, true>) : go(fwd_pair_kernel<2, TRAIN, false>);
-  if (p.agg) return full ? go(fwd_pair_kernel<1, TRAIN, true>) : go(fwd_pair_kernel<1, TRAIN, false>);
-  return full ? go(fwd_pair_kernel<0, TRAIN, true>) : go(fwd_pair_kernel<0, TRAIN, false>);
+  if (p.first) return full ? go(fwd_pair_kernel<true, TRAIN, true>) : go(fwd_pair_kernel<true, TRAIN, false>);
+  return full ? go(fwd_pair_kernel<false, TRAIN, true>) : go(fwd_pair_kernel<false, TRAIN, false>);
 }
 
 // Label rows of 16-byte multiples at 16-byte aligned bases: the bulk-copy CTA kernel applies.
@@ -1395,6 +1383,10 @@ cudaError_t launch_zero_chain_starts(const FwdParams& p, float* a, float* b, cud
   return cudaGetLastError();
 }
 
+// mp_pair_rows.cu: 33 .. 64 labels, chains that do not fill the schedulers
+bool forward_rows_wins(const FwdParams& p, bool train);
+cudaError_t launch_forward_rows(const FwdParams& p, bool train, cudaStream_t st);
+
 cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st) {
   if (p.chain_off[p.ndirs] == 0) return cudaSuccess;
   if (p.L <= 32 && p.ndirs > 1 && p.chain_off[p.ndirs] >= 148 * 8) return train ? launch_live<true>(p, st) : launch_live<false>(p, st);
@@ -1425,6 +1417,7 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
     return train ? launch_warp<32, true>(rest, st) : launch_warp<32, false>(rest, st);
   }
   if (wide_eligible(p, train)) return launch_forward_wide(p, train, st);
+  if (pair_eligible(p) && forward_rows_wins(p, train)) return launch_forward_rows(p, train, st);
   if (pair_eligible(p)) return train ? launch_pair<true>(p, st) : launch_pair<false>(p, st);
   if (p.ctx_rank == 1) return train ? launch_cta_any<1, true>(p, st) : launch_cta_any<1, false>(p, st);
   if (p.L <= 64) return train ? launch_cta_any<2, true>(p, st) : launch_cta_any<2, false>(p, st);

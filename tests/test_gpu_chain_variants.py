@@ -400,3 +400,43 @@ def test_infinite_gradient_stays_in_its_chains(L, B, H, W):
     finite = np.isfinite(ref)   # (the oracle's normalisation sum takes what its chain has scattered too: a few cells more)
     assert finite.any() and not finite.all()
     assert_grad_close(got[finite], ref[finite], "dctx")
+
+
+@pytest.mark.parametrize("kind", ["random", "potts", "zero", "mixed", "ties", "steep"])
+@pytest.mark.parametrize("D,B,H,W,L,I,negative", [
+    (8, 16, 13, 22, 64, 2, False),   # steps over the longest chain's: 1664, as far above the line as the test can be
+    (8, 4, 50, 52, 64, 1, True),     # 1600, on it
+    (8, 4, 49, 62, 36, 2, False),    # just below, elongated: every candidate
+    (8, 2, 48, 60, 48, 2, True),     # below, nearly square
+    (4, 40, 13, 20, 56, 2, True),
+    (4, 12, 30, 24, 40, 1, False),   # more chains than are resident in the other form
+    (4, 2, 9, 20, 38, 2, True),      # inference of few labels takes the list, training does not
+])
+def test_live_labels_of_many_chains(kind, D, B, H, W, L, I, negative):
+    """ISGMR on both sides of the line between the two 33 .. 64-label forms."""
+    rng = np.random.default_rng(L + D)
+    shape = (B, 1, H, W, L)
+    ew = rng.uniform(-0.5 if negative else 0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    if kind in ("ties", "zero", "potts"):
+        ew = np.sign(ew) * 2.0 ** np.round(2 * np.abs(ew))
+    ctx, unary = _table(kind, L, rng), _unary(kind, shape, rng)
+    _same_forward("ISGMR", unary, ctx, ew.astype(np.float32), D, I)
+    _same_forward("ISGMR", unary, ctx, None, D, I, training=False)
+
+
+@pytest.mark.parametrize("L", [33, 34, 41, 62, 63])
+@pytest.mark.parametrize("train", [False, True])
+def test_live_labels_of_many_chains_padded(L, train):
+    rows.test_padded_rows_and_zero_start("ISGMR", 8, 17, 12, 19, L, 2, "sym2d", train)
+    rows.test_padded_rows_and_zero_start("ISGMR", 4, 1, 8, 30, L, 3, "sym2d", train)
+
+
+@pytest.mark.parametrize("D,L,H,W", [(4, 64, 9, 26), (4, 44, 21, 8), (8, 64, 9, 13), (8, 33, 6, 17), (16, 60, 8, 9)])
+def test_every_candidate_from_registers(D, L, H, W):
+    """One direction in a launch; with many directions a stage is one or two pixels deep."""
+    rng = np.random.default_rng(L + D)
+    shape = (2, 1, H, W, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _table("mixed", L, rng)
+    ew = rng.uniform(-0.5, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    _same_forward("TRWP", unary, ctx, ew, D, 2)
+    _same_forward("TRWP", unary, ctx, None, D, 2, training=False)
