@@ -50,11 +50,12 @@ __device__ __forceinline__ float uu_from_ring(const float* slot, int rs, int col
 // copy instruction for 21 labels and four directions (30 pieces) where the 4-byte form, which also
 // serves unaligned rows, needs one per row and keeps every lane's address arithmetic in the step.
 template <int LMAX, int DT, bool TRAIN, bool V4>
-__global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant__ FwdParams p) {
+__global__ void __launch_bounds__(128, 1) fwd_warp_kernel(const __grid_constant__ FwdParams p, bool leave_narrow) {
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainCtx ch;
   dependent_wait();
+  if (leave_narrow && narrow_window(p.ctx, 1, p.L, lane).R) return;  // those are fwd_live_kernel's (see live_use)
   if (!decode_chain(p, blockIdx.x * wpb + warp, ch)) return;
   constexpr bool AGG = DT == 2;
   const int L = p.L, LR = p.ls;
@@ -807,7 +808,7 @@ bool rows_aligned(const FwdParams& p) {
 }
 
 template <int LMAX, int DT, bool TRAIN>
-cudaError_t launch_warp_d(const FwdParams& p, cudaStream_t st) {
+cudaError_t launch_warp_d(const FwdParams& p, bool leave_narrow, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs];
   const int wpb = total >= 148 * 32 ? 4 : 1;
   const size_t smem = (size_t)wpb * (kPF * ((p.agg ? 2 : p.D) + 2) * 32 + 64) * sizeof(float);
@@ -816,17 +817,17 @@ cudaError_t launch_warp_d(const FwdParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfFwdSweep, st);
     count_launch();
-    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p);
+    return launch_dependent(kernel, (total + wpb - 1) / wpb, wpb * 32, smem, st, p, leave_narrow);
   };
   return rows_aligned(p) ? go(fwd_warp_kernel<LMAX, DT, TRAIN, true>) : go(fwd_warp_kernel<LMAX, DT, TRAIN, false>);
 }
 
 template <int LMAX, bool TRAIN>
-cudaError_t launch_warp(const FwdParams& p, cudaStream_t st) {
-  if (p.agg) return launch_warp_d<LMAX, 2, TRAIN>(p, st);
-  if (p.D == 4) return launch_warp_d<LMAX, 4, TRAIN>(p, st);
-  if (p.D == 8) return launch_warp_d<LMAX, 8, TRAIN>(p, st);
-  return launch_warp_d<LMAX, 0, TRAIN>(p, st);
+cudaError_t launch_warp(const FwdParams& p, bool leave_narrow, cudaStream_t st) {
+  if (p.agg) return launch_warp_d<LMAX, 2, TRAIN>(p, leave_narrow, st);
+  if (p.D == 4) return launch_warp_d<LMAX, 4, TRAIN>(p, leave_narrow, st);
+  if (p.D == 8) return launch_warp_d<LMAX, 8, TRAIN>(p, leave_narrow, st);
+  return launch_warp_d<LMAX, 0, TRAIN>(p, leave_narrow, st);
 }
 
 template <int MODE, bool TRAIN>
@@ -866,12 +867,11 @@ cudaError_t launch_cta_tma(FwdParams p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Up to 32 labels and many independent chains (all directions of an ISGMR iteration in one launch): one warp per chain, lane =
+// Up to 32 labels and many independent chains (the directions of an ISGMR iteration in one launch): one warp per chain, lane =
 // label, only the candidates that can be a minimum (see fwd_pair_kernel; class scores with a clear winner leave one to three
-// of 21).  With fewer chains than two per scheduler the kernels that evaluate all candidates are as fast: there a step
-// costs its dependent path, which the list of candidates does not shorten (2 x 512 x 512 x 21, TRWP, 1024 chains a sweep:
-// 90 us, through such a list 150).  2 x 256 x 256 x 21, eight directions, training: the axis directions one
-// launch after another and the diagonal ones 285 us per iteration, this kernel 225, with the
+// of 21).  Where chains do not fill the schedulers a step costs its dependent path, which the list of candidates makes
+// longer, and which sizes take this kernel is live_use's to say.  2 x 256 x 256 x 21, eight directions, training: the axis
+// directions one launch after another and the diagonal ones 285 us per iteration, this kernel 225, with the
 // longest chains first 189.
 constexpr int kLiveList = 36;   // entries: 32 and four that never win
 constexpr int kLiveRing = 8;    // pixels staged ahead (power of two)
@@ -881,13 +881,18 @@ __host__ __device__ constexpr int live_warp_floats(int A) { return kLiveRing * (
 // fwd_warp_kernel); in aggregate mode one copy instruction then stages a pixel.  R1: rank-1 context; where it has a
 // narrow window, steps with a weight >= 0 go through that.
 template <int DT, bool TRAIN, bool V4, bool R1>
-__global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant__ FwdParams p) {
+__global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant__ FwdParams p, bool only_narrow) {
   extern __shared__ __align__(16) float smem[];
   const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr bool AGG = DT == 2;
   const int L = p.L, LR = p.ls, D = AGG ? 2 : p.D, A = D + 1;
   float* ctab = smem;  // [32][32], row = label at the predecessor
   dependent_wait();
+  NarrowWindow window{};
+  if constexpr (R1) {
+    window = narrow_window(p.ctx, 1, L, lane);
+    if (only_narrow && !window.R) return;  // fwd_warp_kernel's (see live_use)
+  }
   for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
     const int f = i >> 5, c = i & 31;
     ctab[i] = (c < L && f < L) ? ctx_value(p.ctx, p.ctx_rank, L, c, f) : 0.f;
@@ -912,8 +917,6 @@ __global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant_
     if (c != lc) olo = fminf(olo, v), ohi = fmaxf(ohi, v);
   }
   const float own = ctab[lc * 33];
-  NarrowWindow window{};
-  if constexpr (R1) window = narrow_window(p.ctx, 1, L, lane);
   nan = __any_sync(0xffffffffu, nan);
   const float tab_lo = nan ? -kInf : warp_min(lo), tab_hi = nan ? kInf : -warp_min(-hi);
   const char* crow = reinterpret_cast<const char*>(ctab + lane);  // + a list entry's offset: the lane's context value
@@ -1053,7 +1056,7 @@ __global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant_
 }
 
 template <bool TRAIN>
-cudaError_t launch_live(const FwdParams& p, cudaStream_t st) {
+cudaError_t launch_live(const FwdParams& p, bool only_narrow, cudaStream_t st) {
   const int total = p.chain_off[p.ndirs], wpb = total >= 148 * 32 ? 8 : 4;
   const size_t smem = (size_t)(32 * 32 + live_warp_floats((p.agg ? 2 : p.D) + 1) * wpb) * sizeof(float);
   auto go = [&](auto kernel) -> cudaError_t {
@@ -1061,7 +1064,7 @@ cudaError_t launch_live(const FwdParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     ProfScope prof(kProfFwdSweep, st);
     count_launch();
-    return launch_dependent(kernel, chain_units(p, wpb), wpb * 32, smem, st, p);
+    return launch_dependent(kernel, chain_units(p, wpb), wpb * 32, smem, st, p, only_narrow);
   };
   const bool v4 = rows_aligned(p) && (p.agg ? 3 : p.D + 1) * (p.ls >> 2) <= (p.agg ? 32 : 160);
   if (p.ctx_rank == 1) {
@@ -1383,23 +1386,61 @@ cudaError_t launch_zero_chain_starts(const FwdParams& p, float* a, float* b, cud
   return cudaGetLastError();
 }
 
+// Which launches over several directions, up to 32 labels, fwd_live_kernel takes: none, those whose rank-1 context has a
+// narrow window (the host does not know: both kernels are launched, and the one whose context it is not returns at once), all.
+// `axis_copies`: the other way is one launch of the bulk-copy kernel per axis direction and one of the generic kernel
+// over the diagonals, else one launch of the generic kernel.  `need`: steps of all directions over the longest chain's.
+// Time of the other way over this kernel's, random table unless said, 5 .. 16 / 21 / 27 .. 32 labels, inference (training):
+//   four directions: this kernel has no sums to read (five rows staged), the axis launches win: 512 x 512 .25 - .69 / .46 / .85,
+//     one launch too: 257 x 301 .41 / .43 / .47.  In training the axis launches of more than 21 labels lose (300 x 400 1.32, 512 x
+//     512 1.21, 2 x 256 x 256 1.27), but not where images are elongated (120 x 500 .63) or many (2 x 512 x 512 .76).
+//   diagonals, axis launches: 256 x 256 1.87 / 1.94 / 2.3, 512 x 512 1.30 / 1.37 / 1.61, 2 x 512 x 512 1.08 / 1.16 / 1.43, 1000 x 300 with
+//     a window of 4 1.01 / 1.05 / 1.26.
+//   diagonals, one launch: 101 x 131 .80 / .84 / .97 (.91 / .97 / 1.18), 151 x 203 .90 / .93 / 1.11 (.94 / 1.04 / 1.31), 201 x 303 .84 / .87 / 1.10
+//     (.88 / .97 / 1.33), 255 x 257 .98 / 1.03 / 1.31 (1.06 / 1.17 / 1.57), 401 x 403 .89 / .98 / 1.17 (1.06 / 1.23 / 1.60), 101 x 501 .66 / .68 / .83 (.81
+//     / .90 / 1.11), 201 x 601 .70 / .78 / .91 (.86 / .93 / 1.18), 301 x 1201 .93 / .98 / 1.17 (.99 / 1.13 / 1.47).  Windows up to 2: 101 x 131 1.00 / 1.08 / 1.30,
+//     201 x 601 1.00 / 1.09 / 1.21, 255 x 257 1.34 / 1.48 / 1.81, 101 x 501 .92 / .98 / 1.17; of 4: 101 x 131 .65 / .67 / .79 (.73 / .76 / .95),
+//     255 x 257 .85 / .92 / 1.14 (.91 / 1.01 / 1.36), 301 x 1201 .77 / .79 / .91 (.81 / .90 / 1.18).
+// Tables whose entries differ by far more than the unaries exclude little: 321 x 323, values to 40, .75 / .71 / .69.
+enum class LiveUse { kNone, kNarrow, kAll };
+static LiveUse live_use(const FwdParams& p, bool train, bool axis_copies) {
+  const int lo = p.H < p.W ? p.H : p.W, hi = p.H < p.W ? p.W : p.H;
+  const long long need = (long long)p.ndirs * p.nimg * lo / (p.parts > 1 ? p.parts : 1);
+  const bool many_labels = p.L > 21;
+  auto use = [](bool yes) { return yes ? LiveUse::kAll : LiveUse::kNone; };
+  if (p.dir0 + p.ndirs <= 4) return use(train && many_labels && axis_copies && need >= 1000 && need <= 2400);
+  if (axis_copies) return LiveUse::kAll;
+  if (p.ctx_rank == 2) {
+    if (train) return use(need >= (many_labels ? 800 : 2000));
+    return use(many_labels ? need >= 2400 || (need >= 1200 && hi <= 2 * lo) : p.L > 16 && need >= 2000 && 2 * hi <= 3 * lo);
+  }
+  if (train && many_labels && (need >= 2400 || (need >= 1600 && hi <= 2 * lo))) return LiveUse::kAll;
+  if (p.L > 16 && (train || many_labels) && need >= 2000 && 2 * hi <= 3 * lo) return LiveUse::kAll;
+  return need >= 800 && hi <= (p.L > 16 ? 5 : 4) * lo ? LiveUse::kNarrow : LiveUse::kNone;
+}
+
 // mp_pair_rows.cu: 33 .. 64 labels, chains that do not fill the schedulers
 bool forward_rows_wins(const FwdParams& p, bool train);
 cudaError_t launch_forward_rows(const FwdParams& p, bool train, cudaStream_t st);
 
 cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st) {
   if (p.chain_off[p.ndirs] == 0) return cudaSuccess;
-  if (p.L <= 32 && p.ndirs > 1 && p.chain_off[p.ndirs] >= 148 * 8) return train ? launch_live<true>(p, st) : launch_live<false>(p, st);
   if (p.L <= 32) {
+    int stages = 0;
+    // several independent directions (ISGMR) of a small problem: one launch of the generic kernel
+    // over all of them beats one small launch per direction
+    const bool few_chains = (p.ndirs > 1 && (long long)p.nimg * (p.H < p.W ? p.H : p.W) < 256) || p.parts > 1;
+    const LiveUse live = p.ndirs > 1 ? live_use(p, train, !few_chains && forward_tma_eligible(p, p.dir0, train, &stages)) : LiveUse::kNone;
+    if (live != LiveUse::kNone) {
+      const bool narrow = live == LiveUse::kNarrow;
+      const cudaError_t e = train ? launch_live<true>(p, narrow, st) : launch_live<false>(p, narrow, st);
+      if (e != cudaSuccess || !narrow) return e;
+    }
     // directions with aligned row segments go to the bulk-copy kernel (one launch each), the
     // remaining contiguous range of directions to the generic kernel
     FwdParams rest = p;
     int first_generic = p.dir0;
-    // several independent directions (ISGMR) of a small problem: one launch of the generic kernel
-    // over all of them beats one small launch per direction
-    const bool few_chains = (p.ndirs > 1 && (long long)p.nimg * (p.H < p.W ? p.H : p.W) < 256) || p.parts > 1;
     for (int d = p.dir0; d < p.dir0 + p.ndirs && !few_chains; ++d) {
-      int stages = 0;
       if (d != first_generic || !forward_tma_eligible(p, d, train, &stages)) break;
       const cudaError_t e = launch_forward_tma(p, d, stages, train, st);
       if (e != cudaSuccess) return e;
@@ -1412,9 +1453,10 @@ cudaError_t launch_forward_sweep(const FwdParams& p, bool train, cudaStream_t st
     rest.ndirs = nrest;
     for (int i = 0; i <= nrest; ++i) rest.chain_off[i] = p.chain_off[first_generic - p.dir0 + i] - base;
     for (int i = 0; i < nrest; ++i) rest.chain_begin[i] = p.chain_begin[first_generic - p.dir0 + i];
-    if (p.L <= 16) return train ? launch_warp<16, true>(rest, st) : launch_warp<16, false>(rest, st);
-    if (p.L <= 21) return train ? launch_warp<21, true>(rest, st) : launch_warp<21, false>(rest, st);
-    return train ? launch_warp<32, true>(rest, st) : launch_warp<32, false>(rest, st);
+    const bool leave = live == LiveUse::kNarrow;
+    if (p.L <= 16) return train ? launch_warp<16, true>(rest, leave, st) : launch_warp<16, false>(rest, leave, st);
+    if (p.L <= 21) return train ? launch_warp<21, true>(rest, leave, st) : launch_warp<21, false>(rest, leave, st);
+    return train ? launch_warp<32, true>(rest, leave, st) : launch_warp<32, false>(rest, leave, st);
   }
   if (wide_eligible(p, train)) return launch_forward_wide(p, train, st);
   if (pair_eligible(p) && forward_rows_wins(p, train)) return launch_forward_rows(p, train, st);

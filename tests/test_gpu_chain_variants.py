@@ -440,3 +440,51 @@ def test_every_candidate_from_registers(D, L, H, W):
     ew = rng.uniform(-0.5, 1.0, (D,) + shape[:-1]).astype(np.float32)
     _same_forward("TRWP", unary, ctx, ew, D, 2)
     _same_forward("TRWP", unary, ctx, None, D, 2, training=False)
+
+
+@pytest.mark.parametrize("kind", ["random", "potts", "zero", "mixed", "ties", "steep"])
+@pytest.mark.parametrize("D,B,H,W,L,negative", [
+    (8, 10, 33, 38, 21, False), (8, 10, 33, 38, 32, True), (8, 10, 33, 38, 17, False), (8, 8, 33, 38, 3, False),
+    (8, 8, 33, 36, 16, True),      # the other way would be one launch per axis direction
+    (4, 9, 33, 36, 24, True),      # four directions, training: five rows staged
+    (4, 19, 33, 36, 32, False),    # and too many of them
+    (8, 3, 33, 95, 29, False),     # 792 steps over the longest chain's, one below the line, and 816
+    (8, 3, 34, 95, 29, True),
+])
+def test_live_labels_up_to_32_by_size(kind, D, B, H, W, L, negative):
+    """Both sides of the lines between the forms of several directions in a launch."""
+    rng = np.random.default_rng(L + D)
+    shape = (B, 1, H, W, L)
+    ew = rng.uniform(-0.5 if negative else 0.2, 1.0, (D,) + shape[:-1]).astype(np.float32)
+    if kind in ("ties", "zero", "potts"):
+        ew = np.sign(ew) * 2.0 ** np.round(2 * np.abs(ew))
+    ctx, unary = _table(kind, L, rng), _unary(kind, shape, rng)
+    _same_forward("ISGMR", unary, ctx, ew.astype(np.float32), D, 2)
+    _same_forward("ISGMR", unary, ctx, None, D, 2, training=False)
+
+
+@pytest.mark.parametrize("kind", ["linear", "quadratic", "dip"])
+@pytest.mark.parametrize("R", [1, 2, 3])     # 3 is no narrow window
+@pytest.mark.parametrize("B,H,W,L", [
+    (4, 33, 38, 2), (4, 33, 38, 13), (4, 33, 38, 31), (4, 33, 38, 32),   # two kernels, one of which returns at once
+    (8, 33, 36, 13), (8, 33, 36, 32),                                     # this kernel for every context
+    (10, 33, 70, 28),
+])
+def test_narrow_windows_of_many_chains(kind, R, B, H, W, L):
+    rng = np.random.default_rng(L + R)
+    shape = (B, 1, H, W, L)
+    ctx = _truncated(kind, min(R, L - 1), L)
+    unary = rng.integers(0, 6, shape).astype(np.float32) / 2
+    ew = rng.choice([0.0, 0.5, 1.0, 2.0], (8,) + shape[:-1]).astype(np.float32)
+    _same_forward("ISGMR", unary, ctx, ew, 8, 2)
+    _same_forward("ISGMR", unary, ctx, None, 8, 2, training=False)
+    ew[:, :, :, H // 2:, W // 3] = -1.0    # steps with a negative weight evaluate a list of candidates
+    _same_forward("ISGMR", unary, ctx, ew, 8, 2)
+    _same_forward("ISGMR", unary, ctx, ew, 8, 2, training=False)
+
+
+@pytest.mark.parametrize("L", [2, 13, 21, 31])
+@pytest.mark.parametrize("train", [False, True])
+def test_narrow_windows_of_many_chains_padded(L, train):
+    rows.test_padded_rows_and_zero_start("ISGMR", 8, 4, 33, 38, L, 2, "tl1d", train)
+    rows.test_padded_rows_and_zero_start("ISGMR", 8, 10, 33, 38, L, 2, "tl1d", train)
