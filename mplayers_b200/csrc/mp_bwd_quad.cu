@@ -189,9 +189,9 @@ __global__ void __launch_bounds__(Quad<G, LN>::kWarps * 32, 1) bwd_quad_kernel(c
           *reinterpret_cast<float4*>(out + 4 * G * i) = make_float4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
     }
     const bool on = s < nsteps;
-    if (s == nsteps) {  // the chain ends here: the steps the warp's longer chains still take add zeros, whatever q holds
+    if (__any_sync(0xffffffffu, s == nsteps)) {  // a chain ends here: the steps the warp's longer ones still take add zeros
 #pragma unroll
-      for (int i = 0; i < LN; ++i) q[i] = 0.f;
+      for (int i = 0; i < LN; ++i) q[i] = on ? q[i] : 0.f;
     }
     const float e = __shfl_sync(0xffffffffu, e_cur, j * G + (s & 3));
     const int nn = __shfl_sync(0xffffffffu, n_cur, j * G + (s & 3)) - 4 * g;
@@ -325,11 +325,21 @@ cudaError_t launch_quad(const BwdParams& p, cudaStream_t st) {
 // 1.6 us with 64 labels however few warps there are, so a launch takes its longest chain times that, where the kernels of
 // one chain per warp take 0.94 ns per pixel and direction: these win below some 1700 directions x images x shorter sides
 // (384 x 384 x 64, eight directions, 3072: 1.10 ms with bwd_pair_kernel, 0.62 here; 93 x 213 x 45, 744: a training step of
-// five iterations 2.55 ms with this kernel, 1.97 before it).
+// five iterations 2.55 ms with this kernel, 1.97 before it).  In elongated images the diagonals are short and the long
+// rows or columns decide: the time of the other kernels over this one's, eight directions, 12 / 21 / 29 / 50 / 64 labels,
+// 303 x 605 (2424) .83 / .87 / .98 / 1.07 / 1.09, 301 x 1201 (2408) .75 / .78 / .88 / .92 / .97, against 321 x 323 (2568) 1.03 / 1.09 / 1.35 /
+// 1.44 / 1.43; 375 x 1242 (3000) .87 / .91, and a training call with 29 labels 4.73 ms without, 3.99 ms with this kernel.  Not so with 32
+// labels (1.30, 1.16, 1.56 and 1.37), nor where the other way is one launch per axis direction (1000 x 300, 2400: 1.05 / 1.07 / 1.59).
+// Up to eight labels the others have as little to do (375 x 499 x 4, 3000: .89; 511 x 513, 4088: 1.05).
 bool bwd_quad_eligible(const BwdParams& p) {
   if (p.cp_scheme != 2 || p.ndirs < 2 || p.L > 64 || (p.L > 32 && p.ctx_rank != 2) || (p.ls & 3)) return false;
   if ((((uintptr_t)p.dm_read | (uintptr_t)p.dm_acc) & 15) || ((uintptr_t)p.min_idx & 3)) return false;
-  return (long long)p.ndirs * p.nimg * (p.H < p.W ? p.H : p.W) >= 148 * 16 * (p.parts > 1 ? p.parts : 1);
+  const int lo = p.H < p.W ? p.H : p.W, hi = p.H < p.W ? p.W : p.H, parts = p.parts > 1 ? p.parts : 1;
+  const bool axis_launches = p.L <= 32 && parts == 1 && p.dir < 4 && (p.W & 3) == 0 && (long long)p.nimg * lo >= 256;
+  long long line = 148 * 16;
+  if (!axis_launches && p.L <= 8) line = 4000;
+  if (!axis_launches && p.L > 8 && p.L != 32 && 5 * hi > 8 * lo && !(p.L >= 44 && hi <= 2 * lo)) line = p.L <= 21 ? 4000 : 2800;
+  return (long long)p.ndirs * p.nimg * lo >= line * parts;
 }
 
 cudaError_t launch_backward_quad(const BwdParams& p, cudaStream_t st) {

@@ -488,3 +488,15 @@ def test_narrow_windows_of_many_chains(kind, R, B, H, W, L):
 def test_narrow_windows_of_many_chains_padded(L, train):
     rows.test_padded_rows_and_zero_start("ISGMR", 8, 4, 33, 38, L, 2, "tl1d", train)
     rows.test_padded_rows_and_zero_start("ISGMR", 8, 10, 33, 38, L, 2, "tl1d", train)
+
+
+@pytest.mark.parametrize("L,D,B,H,W", [
+    (21, 8, 17, 20, 45), (21, 8, 25, 20, 45),      # elongated: 2720 steps over the longest chain's, and 4000
+    (32, 8, 15, 20, 45), (28, 8, 18, 20, 45), (24, 8, 17, 20, 45),
+    (48, 8, 17, 20, 39), (40, 8, 17, 20, 45), (40, 8, 18, 20, 45),
+    (8, 8, 25, 20, 21), (8, 8, 24, 20, 21), (8, 8, 15, 20, 24),   # few labels; the last one against axis launches
+    (64, 8, 296, 1, 9), (64, 8, 296, 9, 1), (20, 8, 500, 1, 9), (20, 8, 500, 9, 1),   # lines
+])
+def test_backward_lanes_share_a_chain_by_size(L, D, B, H, W):
+    """Both sides of the lines between the backward forms, and images of one row or column above them."""
+    test_backward_lanes_share_a_chain(L, D, B, H, W)
