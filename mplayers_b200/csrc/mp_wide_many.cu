@@ -217,8 +217,13 @@ cudaError_t launch_many_r(const FwdParams& p, cudaStream_t st) {
 }  // namespace
 
 // The caller has checked that the windowed evaluation is exact and that 16-byte staging applies.  Messages are stored
-// in 16-byte pieces.  Below 148 x 12 chains the warps would not fill the schedulers.
+// in 16-byte pieces.  Below 148 x 12 chains the warps would not fill the schedulers.  With a window of more than four
+// offsets and 61 .. 64 labels, which leave fwd_wide_kernel no idle lane either, the long rows of an elongated image
+// decide (window 8, eight directions, 64 labels, a call with that kernel / with this one: 96 x 700 236 / 261 us, 130 x 700 260 / 285,
+// 200 x 1242 518 / 545, 375 x 1242 914 / 729, 240 x 320 207 / 177; 56 labels 292 / 269, 315 / 290, 610 / 556).
 bool forward_many_eligible(const FwdParams& p) {
+  const int lo = p.H < p.W ? p.H : p.W, hi = p.H < p.W ? p.W : p.H;
+  if (p.host_R > 4 && p.L > 60 && p.L <= 64 && hi > 2 * lo && (long long)p.ndirs * p.nimg * lo < 148 * 12) return false;
   return p.agg && p.host_R <= 8 && p.chain_off[p.ndirs] > 148 * 12 && ((uintptr_t)p.msg_write & 15) == 0;
 }
 
