@@ -1359,11 +1359,20 @@ bool forward_skips_zero_slices(const FwdParams& p, bool train) {
   return wide_eligible(p, train) || (p.agg && pair_eligible(p));
 }
 
+// Directions 2 and 3 then stage two volumes less each, but direction 1's rows, few and long where an image is low, store a
+// volume more, and lanes that have no or not all of their labels store it piece by piece.  Time of a call without the sums
+// over one with them, window 2 (training in brackets), 375 x 1242, 375 x 640, 300 x 400, 198 x 919, 96 x 640:
+//    36 labels .94 (.98), .95, .95, .92, .91 (.97)       64 labels 1.05 (1.01), 1.01 (1.00), 1.00, .98, .97 (.99)
+//    72 labels 1.12 (1.04), 1.01 (1.00), 1.00, .98, .96  100 labels 1.13 (1.04), 1.04 (1.01), 1.01, 1.00, .98
+//   128 labels 1.20 (1.04), 1.09, 1.06, 1.04, 1.00       156 labels 1.09 (1.01), 1.04, 1.05, 1.03 (1.00), .94 (.98)
+//   192 labels 1.25 (1.04), 1.15, 1.09, 1.17, 1.02       256 labels 1.16 (1.04), 1.16, 1.12, 1.15, 1.05
 bool forward_takes_prefix(const FwdParams& p, bool train) {
+  const long long height = (long long)p.nimg * p.H * p.L;
+  const bool pays = (p.L & 63) == 0 ? p.L >= 128 || height >= 22000 : p.L > 64 && height >= 27000;
   // (every pixel has to lie on a chain that is walked, of direction 1, which writes P, and of direction 3, which may write the
   // costs: images of one column or one row keep the final sums; the several-warps kernel, which wide windows may take,
   // does not know P)
-  return p.D == 4 && !p.agg && p.W > 1 && p.H > 1 && wide_eligible(p, train) && (train || p.host_R <= 8);
+  return pays && p.D == 4 && !p.agg && p.W > 1 && p.H > 1 && wide_eligible(p, train) && (train || p.host_R <= 8);
 }
 
 __global__ void zero_chain_starts_kernel(const __grid_constant__ FwdParams p, float* a, float* b) {

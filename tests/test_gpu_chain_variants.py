@@ -500,3 +500,36 @@ def test_narrow_windows_of_many_chains_padded(L, train):
 def test_backward_lanes_share_a_chain_by_size(L, D, B, H, W):
     """Both sides of the lines between the backward forms, and images of one row or column above them."""
     test_backward_lanes_share_a_chain(L, D, B, H, W)
+
+
+@pytest.mark.parametrize("L,R,B,H,W", [
+    (64, 3, 20, 18, 7), (64, 2, 19, 18, 7),        # images x rows x labels 23040 and 21888
+    (72, 2, 30, 13, 5), (72, 4, 28, 13, 5),        # lanes without labels: 28080 and 26208
+    (200, 6, 10, 14, 9), (200, 3, 9, 14, 9),       # lanes with a part of theirs: 28000 and 25200
+    (60, 2, 40, 20, 5),                            # none
+])
+def test_sums_of_two_directions_by_size(L, R, B, H, W):
+    """Both sides of the line above which TRWP goes through the sums of two directions; the costs with the labels first come
+    from the last sweep there."""
+    rng = np.random.default_rng(L + B)
+    shape = (B, 1, H, W, L)
+    unary, ctx = rng.standard_normal(shape).astype(np.float32), _truncated("linear", R, L)
+    ew = rng.uniform(0.1, 1.4, (4,) + shape[:-1]).astype(np.float32)
+    _same_forward("TRWP", unary, ctx, ew, 4, 2)
+    want = _same_forward("TRWP", unary, ctx, None, 4, 2, training=False)
+    e0, e8 = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.uint8, device="cuda")
+    msg = torch.full((4,) + shape, float("nan"), device="cuda")
+    cost = torch.full((B, 1, L, H, W), float("nan"), device="cuda")
+    TRWP.forward(0.5, 2, 0, torch.from_numpy(unary).cuda(), torch.from_numpy(ctx).cuda(), e0, msg, cost, e8, e8, e0, e8,
+                 context_window=R, cost_labels_first=True, messages_zero=True, messages_needed=False)
+    assert np.array_equal(np.moveaxis(cost.cpu().numpy(), 2, -1), want["cost"])
+
+
+@pytest.mark.parametrize("L,B", [(64, 4), (64, 12), (61, 4), (60, 4), (56, 4)])
+def test_many_chains_of_elongated_images(L, B):
+    """Windows of more than four offsets: below 1776 steps over the longest chain's and above, label counts at the line."""
+    rng = np.random.default_rng(L + B)
+    unary = rng.standard_normal((B, 1, 20, 60, L)).astype(np.float32)
+    _same_forward("ISGMR", unary, _truncated("linear", 6, L), None, 8, 2, training=False)
+    if L & 3:
+        rows.test_padded_rows_and_zero_start("ISGMR", 8, B, 20, 60, L, 2, "tq1d", False)
