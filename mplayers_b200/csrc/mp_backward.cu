@@ -767,7 +767,8 @@ __global__ void __launch_bounds__(256, 1) bwd_pair_kernel(const __grid_constant_
         float t0 = 0.f, t1 = 0.f, cv0 = 0.f, cv1 = 0.f;
         if (act) {
           const uchar2 fi = *reinterpret_cast<const uchar2*>(irow);
-          const int f0 = fi.x, f1 = act1 ? fi.y : 0;
+          int f0 = fi.x, f1 = act1 ? fi.y : 0;
+          if (p.ctx_rank == 1) f0 = min(f0, L - 1), f1 = min(f1, L - 1);  // (see load_idx of bwd_cta_kernel)
           t0 = x0.x + x1.x + rq0;
           t1 = x0.y + x1.y + rq1;
           t0 = (c0 == n) ? t0 - S : t0;  // MPLayers/commonCUDA.cuh:131-145
@@ -887,7 +888,8 @@ __global__ void __launch_bounds__(256) bwd_cta_kernel(const __grid_constant__ Bw
     cp_async_commit();
   };
   auto load_idx = [&](int s) -> int {
-    return (s < len - 1 && act) ? (int)MI[(long long)(pixl - s * ch.pstep) * LR + c] : -1;
+    // (a windowed sweep that saw only NaN saved no label: any byte)
+    return (s < len - 1 && act) ? min((int)MI[(long long)(pixl - s * ch.pstep) * LR + c], L - 1) : -1;
   };
   auto load_blk = [&](int b, float& eb, int& nb) {
     const int s = 32 * b + lane;

@@ -108,11 +108,10 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
   const int nstages = (len + K - 1) / K;
   const long long ibase = (long long)ch.img * p.H * p.W;
   const int pix0 = ch.h0 * p.W + ch.w0;
+  const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
   // vertical chains (directions 2 / 3) with tensor maps from the launcher: one 2-D tiled TMA box
   // (L labels x K image rows of the chain's column) per array and stage instead of K row copies
   const bool boxed = p.tma_box != 0 && (ch.dir == 2 || ch.dir == 3);
-  // (the columns of an image one pixel wide are boxed too, although their pixels are adjacent in memory)
-  const bool contiguous = !boxed && (ch.pstep == 1 || ch.pstep == -1);
 
   if (!producer) {
     if (lane == 0) {
@@ -122,7 +121,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
       }
       mbar_fence_init();
     }
-    for (int i = lane; i < 2 * (LP + 2 * G); i += 32) hwin[i] = kNaN;  // guards and padding labels: no minimum takes them, nothing equals them
+    for (int i = lane; i < 2 * (LP + 2 * G); i += 32) hwin[i] = kInf;  // guards and padding labels
   }
   __syncthreads();
   dependent_wait();
@@ -321,13 +320,13 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
         const float gv = fmaf(e, cmax, hmin);  // candidate through the saturated value
         int fstar = 0;                         // TRAIN: highest label whose saturated candidate equals gv
         if (TRAIN) {
-          int lf = 0;
+          int lf = -1;
 #pragma unroll
           for (int i = 0; i < LPT; ++i) lf = (i < nl && fmaf(e, cmax, hv[i]) == gv) ? c0 + i : lf;
           fstar = warp_max_i32(lf);
         }
         __syncwarp();
-        // window of this lane: labels c0 - G .. c0 + LPT + G - 1 (guards read NaN)
+        // window of this lane: labels c0 - G .. c0 + LPT + G - 1 (guards read +inf)
         float win[NWV * 2];
         if constexpr (LPT % 4 == 0) {
 #pragma unroll
@@ -355,9 +354,8 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
           best[i] = min_tree<2 * RW>(cand);
           if (i < nl) bl = fminf(bl, best[i]);
           if constexpr (TRAIN) {
-            // highest window offset attaining the minimum (candidates outside 0..L-1 are NaN); 0 where none does:
-            // then fstar is the index, or everything is NaN
-            int fw = 0;
+            // highest window offset attaining the minimum (candidates outside 0..L-1 read +inf)
+            int fw = -1;
             if constexpr (RW >= 8) {
               // many candidates: flags summed with weights 2^k on the full-rate pipe, the index is the
               // exponent of the sum (a compare and a select per candidate run at half rate)
@@ -365,7 +363,7 @@ __global__ void __launch_bounds__(kWideChains * 64, 1) fwd_wide_kernel(const __g
 #pragma unroll
               for (int j = 0; j < 2 * RW - 1; ++j) wv[j] = cand[j + 1];
               const int hw = highest_equal_or_none<2 * RW - 1>(wv, best[i]);
-              fw = hw >= 0 ? c0 + i + hw - (RW - 1) : 0;
+              fw = hw >= 0 ? c0 + i + hw - (RW - 1) : -1;
             } else {
 #pragma unroll
               for (int kk = -(RW - 1); kk <= RW - 1; ++kk) fw = (cand[kk + RW] == best[i]) ? c0 + i + kk : fw;
@@ -469,8 +467,8 @@ cudaError_t launch_wide_s(FwdParams p, cudaStream_t st) {
   // tensor maps for the vertical chains (box = one pixel's labels x K image rows); the box must
   // land 128-byte aligned in the staging ring
   TmaMaps maps{};
-  p.tma_box = 0;
-  if (p.dir0 <= 3 && p.dir0 + p.ndirs > 2 && ((size_t)K * p.ls * sizeof(float)) % 128 == 0 && p.ls <= 256) {
+  p.tma_box = 0;  // (the columns of an image one pixel wide are contiguous and copied as such)
+  if (p.W > 1 && p.dir0 <= 3 && p.dir0 + p.ndirs > 2 && ((size_t)K * p.ls * sizeof(float)) % 128 == 0 && p.ls <= 256) {
     const unsigned long long inner = (unsigned long long)p.W * p.ls, rows = (unsigned long long)p.nimg * p.H;
     if (encode_tmap_2d(&maps.a, p.unary, inner, rows, p.ls, K) &&
         (A == 1 || encode_tmap_2d(&maps.b, p.msg_read, inner, rows * p.D, p.ls, K)))

@@ -18,10 +18,10 @@ constexpr int kWNS = 2;  // stages in flight per warp
 
 // Floats of shared memory per warp: staged gradients [kWNS][NA][K][L], argmin indices
 // [kWNS][K][L] bytes, product tile [16][33], t and index-as-float windows [2][2][LP + 2G], the
-// chain's label-context gradient table by SIGNED offset c - f [2L], the far scatter buffer [LP],
+// chain's label-context gradient table by SIGNED offset c - f [256 + L], the far scatter buffer [LP],
 // kWNS mbarriers.
 __host__ __device__ inline int bwd_wide_floats(int L, int ls, int lp, int g, int K, int na) {
-  return kWNS * na * K * ls + kWNS * K * ls / 4 + 16 * 33 + 4 * (lp + 2 * g) + ((2 * L + 3) & ~3) + lp + 2 * kWNS + 2;
+  return kWNS * na * K * ls + kWNS * K * ls / 4 + 16 * 33 + 4 * (lp + 2 * g) + ((256 + L + 3) & ~3) + lp + 2 * kWNS + 2;
 }
 
 // Two adjacent floats added to global memory with one reduction (8-byte aligned address).
@@ -72,20 +72,18 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
   float* dtile = ring + kWNS * stage_floats + kWNS * K * LR / 4;             // [16][33]
   float* tbuf = dtile + 16 * 33;                             // [2][WB]
   float* ibuf = tbuf + 2 * WB;                               // [2][WB] argmin as float
-  float* acc = ibuf + 2 * WB;                                // [2L] label-context gradient of the chain, cell L + c - f
-  float* qfar = acc + ((2 * L + 3) & ~3);                    // [LP]
+  float* acc = ibuf + 2 * WB;                                // [256 + L] label-context gradient of the chain, cell 256 + c - f (an index
+                                                    // saved where all candidates were NaN may be any byte)
+  float* qfar = acc + ((256 + L + 3) & ~3);                    // [LP]
   unsigned long long* full = reinterpret_cast<unsigned long long*>(qfar + LP);
-  float* ctab = reinterpret_cast<float*>(full + kWNS + 1);   // [L] the context
+  float* ctab = reinterpret_cast<float*>(full + kWNS + 1);   // [256] the context
   if (lane == 0) {
     for (int i = 0; i < kWNS; ++i) mbar_init(&full[i], 1);
     mbar_fence_init();
   }
   dependent_wait();
-  for (int i = lane; i < L; i += 32) {
-    acc[i] = 0.f;
-    acc[L + i] = 0.f;
-    ctab[i] = __ldg(p.ctx + i);
-  }
+  for (int i = lane; i < 256 + L; i += 32) acc[i] = 0.f;
+  for (int i = lane; i < 256; i += 32) ctab[i] = i < L ? __ldg(p.ctx + i) : 0.f;
   for (int i = lane; i < 2 * WB; i += 32) tbuf[i] = 0.f, ibuf[i] = -1.f;
   for (int i = lane; i < LP; i += 32) qfar[i] = 0.f;
   __syncwarp();
@@ -324,7 +322,7 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
         bool left = false;
         // signed offset: distinct labels, distinct cells (lanes without a far label keep away: the
         // cells of labels that do not exist may lie outside the table)
-        float* cell = acc + (any ? L + c0 - tg : L);
+        float* cell = acc + (any ? 256 + c0 - tg : 256);
 #pragma unroll
         for (int i = 0; i < LPT; ++i) {
           const bool hit = pend[i] && f[i] == tg;
@@ -344,8 +342,9 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
 #pragma unroll
           for (int i = 0; i < LPT; ++i) {
             if (pend[i]) {
-              atomicAdd(qfar + f[i], t[i]);
-              atomicAdd(acc + (L + c0 + i - f[i]), e * t[i]);
+              const int fi = min(f[i], L - 1);
+              atomicAdd(qfar + fi, t[i]);
+              atomicAdd(acc + (256 + c0 + i - fi), e * t[i]);
             }
           }
           __syncwarp();
@@ -465,12 +464,12 @@ __global__ void __launch_bounds__(32, 8) bwd_wide_kernel(const __grid_constant__
 #pragma unroll
   for (int k = 0; k < RW; ++k) {
     const float v = warp_sum(ack[k]);
-    if (lane == 0 && k < L && (k > 0 || p.keep_diag)) acc[L + k] += v;
+    if (lane == 0 && k < L && (k > 0 || p.keep_diag)) acc[256 + k] += v;
   }
   __syncwarp();
   float* part = p.dctx_part + (long long)(blockIdx.x % p.n_slots) * L;
   for (int i = lane; i < L; i += 32) {
-    const float v = i > 0 ? acc[L + i] + acc[L - i] : acc[L];  // fold the two signs of the offset
+    const float v = i > 0 ? acc[256 + i] + acc[256 - i] : acc[256];  // fold the two signs of the offset
     if (v != 0.f) atomicAdd(part + i, v);
   }
 }
@@ -479,7 +478,7 @@ template <int LPT, int RW, int SCH>
 cudaError_t launch_bw(BwdParams p, int total, cudaStream_t st) {
   constexpr int LP = 32 * LPT, G = RW & ~1, NA = SCH == 1 ? 2 : 1;
   auto bytes = [&](int k) {
-    return ((size_t)bwd_wide_floats(p.L, p.ls, LP, G, k, NA) + ((p.L + 3) & ~3) + 4) * sizeof(float);
+    return ((size_t)bwd_wide_floats(p.L, p.ls, LP, G, k, NA) + 256 + 4) * sizeof(float);
   };
   // every chain of the launch resident at once where possible: the stage depth shrinks first
   const int per_sm = (total + 147) / 148;
