@@ -1006,7 +1006,7 @@ __global__ void __launch_bounds__(256, 3) fwd_live_kernel(const __grid_constant_
     int bi = 0;
     const bool up = e >= 0.f;
     if (R1 && window.R && up) {
-      minplus_narrow<2, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
+      minplus_narrow<TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
       bi <<= 7;
     } else {
       const float hmin = warp_min(h);

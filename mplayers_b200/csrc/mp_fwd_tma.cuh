@@ -2,7 +2,6 @@
 // whose width is a multiple of four (see mp_forward.cu for the sweeps of everything else).
 #pragma once
 #include <cstdlib>
-#include <type_traits>
 
 #include "mp_common.cuh"
 #include "mp_minplus.cuh"
@@ -309,13 +308,12 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
   NarrowWindow window{};
   if constexpr (R1) window = narrow_window(p.ctx, 1, L, lane);
   bool pend = false;  // R1: the argmin of the last pixel is still to be resolved
-  auto narrow_step = [&](auto rw, const float* t, float e) {
-    constexpr int RW = decltype(rw)::value;
+  auto narrow_step = [&](const float* t, float e) {
     const float h = fmaf(rho, r, uu);
     const float uu_next = uu_at(t);
     float best, m;
     int bi = 0;
-    minplus_narrow<RW, TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
+    minplus_narrow<TRAIN>(window, h, e, L, lc, lmask, best, bi, m);
     r = best - m;
     *mw = r;
     if constexpr (TRAIN) {
@@ -328,11 +326,11 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     uu = uu_next;
   };
   // the stage's pixels (s, npix) from tile row t0 and weights e0 on
-  auto narrow_stage = [&](auto rw, int s, int npix, const float* t0, const float* e0) {
+  auto narrow_stage = [&](int s, int npix, const float* t0, const float* e0) {
     if (s > 0 && npix == kTK) {
 #pragma unroll
       for (int k = 0; k < kTK; ++k) {
-        narrow_step(rw, t0 + k * sk, e0[k * ek]);
+        narrow_step(t0 + k * sk, e0[k * ek]);
         advance();
       }
     } else {
@@ -340,7 +338,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
         if (s + k == 0) {
           uu = uu_at(t0);
         } else {
-          narrow_step(rw, t0 + k * sk, e0[k * ek]);
+          narrow_step(t0 + k * sk, e0[k * ek]);
         }
         advance();
       }
@@ -368,7 +366,7 @@ __global__ void __launch_bounds__(160, 1) fwd_tma_kernel(const __grid_constant__
     if (R1 && window.R && __all_sync(0xffffffffu, lane >= npix || e0[lane * ek] >= 0.f)) {
       if (TRAIN && pend) resolve();
       pend = false;
-      narrow_stage(std::integral_constant<int, 2>{}, s, npix, t0, e0);
+      narrow_stage(s, npix, t0, e0);
     } else if (s > 0 && npix == kTK) {
       // full stage: fully unrolled, every tile offset is an immediate
 #pragma unroll

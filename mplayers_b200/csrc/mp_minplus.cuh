@@ -281,33 +281,26 @@ __device__ __forceinline__ NarrowWindow narrow_window(const float* ctx, int rank
   return w;
 }
 
-// The step through such a window of up to RW offsets (those from R to RW - 1 hold the last value: exact as well).  Neighbours
-// come by shuffle; the candidate of a label outside 0 .. L - 1 is NaN, which no minimum takes and nothing equals.  The highest
-// index among equal candidates: inside the window the highest offset; outside it candidates are equal to the saturated
-// minimum gv, and the highest label whose saturated candidate is gv stands for all of them (its window candidate is no
-// larger).  Where all candidates are NaN the index is 0.
-template <int RW, bool TRAIN>
+// The step through such a window.  Neighbours come by shuffle; the candidate of a label outside 0 .. L - 1 is NaN, which no
+// minimum takes and nothing equals.  (With R == 1 the candidates of the neighbours are at the last value: exact as well.)  The
+// highest index among equal candidates: inside the window the highest offset; outside it candidates are equal to the
+// saturated minimum gv, and the highest label whose saturated candidate is gv stands for all of them (its window
+// candidate is no larger).  Where all candidates are NaN the index is 0.
+template <bool TRAIN>
 __device__ __forceinline__ void minplus_narrow(const NarrowWindow& w, float h, float e, int L, int lc,
                                                unsigned lmask, float& best, int& bi, float& m) {
   const float hmin = warp_min(h);
   m = warp_min(fmaf(e, w.least, h));  // fma is monotone (a uniform branch around this reduction: 28 -> 36 us a sweep)
   const float gv = fmaf(e, w.last, hmin);
-  float cand[2 * RW];
-  cand[0] = gv;
-  cand[RW] = fmaf(e, w.c[0], h);
-#pragma unroll
-  for (int k = 1; k < RW; ++k) {
-    const float dn = __shfl_sync(0xffffffffu, h, lc - k), up = __shfl_sync(0xffffffffu, h, lc + k);
-    cand[RW - k] = lc >= k ? fmaf(e, w.c[k], dn) : kNaN;
-    cand[RW + k] = lc + k < L ? fmaf(e, w.c[k], up) : kNaN;
-  }
-  best = min_tree<2 * RW>(cand);
+  const float dn = __shfl_sync(0xffffffffu, h, lc - 1), up = __shfl_sync(0xffffffffu, h, lc + 1);
+  const float cand[4] = {gv, lc >= 1 ? fmaf(e, w.c[1], dn) : kNaN, fmaf(e, w.c[0], h), lc + 1 < L ? fmaf(e, w.c[1], up) : kNaN};
+  best = min_tree<4>(cand);
   if (TRAIN) {
     const unsigned sat = __ballot_sync(0xffffffffu, fmaf(e, w.last, h) == gv) & lmask;
     const int fstar = 31 - __clz(sat);
     int fw = 0;
 #pragma unroll
-    for (int k = 1 - RW; k < RW; ++k) fw = cand[RW + k] == best ? lc + k : fw;
+    for (int k = -1; k <= 1; ++k) fw = cand[2 + k] == best ? lc + k : fw;
     bi = gv == best ? max(fstar, fw) : fw;
   }
 }
