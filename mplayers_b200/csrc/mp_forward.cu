@@ -7,6 +7,8 @@
 // pixels ahead, labels live in registers, and min / argmin use warp-wide redux + ballot.
 //
 //   fwd_warp_kernel : L <= 32, one warp per chain, lane = label, context row in registers.
+//   fwd_live_kernel : L <= 32, launches over several directions (live_use), only the candidates that can be a minimum.
+//   fwd_pair_kernel : 32 < L <= 64, the same with two labels per lane (others: mp_pair_rows.cu, forward_rows_wins).
 //   fwd_cta_kernel  : L  > 32, one CTA per chain, thread = label;
 //                     MODE 1 rank-1 context: windowed O(L*R) evaluation when the context is
 //                            non-decreasing and saturates at offset R, else dense;

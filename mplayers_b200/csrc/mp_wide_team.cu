@@ -58,8 +58,8 @@ __global__ void __launch_bounds__((TW + 1) * 32, TW == 2 ? 7 : 1) fwd_wide_team_
   const int nstages = (len + K - 1) / K;
   const long long ibase = (long long)ch.img * p.H * p.W;
   const int pix0 = ch.h0 * p.W + ch.w0;
+  const bool contiguous = (ch.pstep == 1 || ch.pstep == -1);
   const bool boxed = p.tma_box != 0 && (ch.dir == 2 || ch.dir == 3);
-  const bool contiguous = !boxed && (ch.pstep == 1 || ch.pstep == -1);  // (see fwd_wide_kernel)
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
       mbar_init(&full[i], 1);
@@ -311,8 +311,8 @@ cudaError_t launch_team_d(FwdParams p, cudaStream_t st) {
   p.tma_k = K;
   p.tma_stages = NS;
   TmaMaps maps{};
-  p.tma_box = 0;
-  if (p.dir0 <= 3 && p.dir0 + p.ndirs > 2 && ((size_t)K * p.ls * sizeof(float)) % 128 == 0) {
+  p.tma_box = 0;  // (the columns of an image one pixel wide are contiguous and copied as such)
+  if (p.W > 1 && p.dir0 <= 3 && p.dir0 + p.ndirs > 2 && ((size_t)K * p.ls * sizeof(float)) % 128 == 0) {
     const unsigned long long inner = (unsigned long long)p.W * p.ls, rows = (unsigned long long)p.nimg * p.H;
     if (encode_tmap_2d(&maps.a, p.unary, inner, rows, p.ls, K) &&
         (A == 1 || encode_tmap_2d(&maps.b, p.msg_read, inner, rows * p.D, p.ls, K)))
