@@ -221,7 +221,7 @@ def dominant_kernel(cfg, kind):
     if L <= 64:
         if kind == "bwd":
             return "bwd_quad_kernel" if many else "bwd_pair_kernel"
-        return "fwd_pair_kernel"
+        return "fwd_pair_kernel" if many else "fwd_rows_kernel"
     return "bwd_cta_kernel" if kind == "bwd" else "fwd_cta_tma_kernel"
 
 
