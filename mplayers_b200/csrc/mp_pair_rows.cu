@@ -263,7 +263,7 @@ bool forward_rows_wins(const FwdParams& p, bool train) {
   bool list;
   if (p.dir0 + p.ndirs > 4) {
     if (!first) {
-      list = need >= 1600 || (p.L <= 52 && need >= 1000 && hi <= 3 * lo) || (weights && need >= 500 && 2 * hi <= 5 * lo) ||
+      list = need >= 1600 || (need >= (weights || p.L <= 40 || p.H >= p.W ? 500 : 1000) && (weights || p.L <= 52) && hi <= 3 * lo) ||
              (need >= (p.L <= 52 ? 500 : 1000) && hi <= 2 * lo) || (need >= 500 && 4 * hi <= 5 * lo);
     } else if (weights && p.L <= 40) {
       list = need >= 1600 || (need >= 500 && 2 * hi <= 5 * lo);
